@@ -57,10 +57,19 @@ struct Units {
     __device__ void next() { unit += step; }
 };
 
+// What C holds at W row `n_row` for tokens tok0 .. tok0 + 15 (zeros unless the mode adds to it).  All of it is
+// requested before the first sum is stored: written one after the other, every read would wait behind the store
+// before it (the compiler cannot tell that the addresses differ), a round trip to L2 per row.
+__device__ __forceinline__ void old16(float (&old)[16], int tok0, int n_row, const float* c, int m, int n, int ldc, int mode) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+        old[i] = mode == MODE_ACCUMULATE && tok0 + i < m && n_row < n ? __ldcg(c + (size_t)(tok0 + i) * ldc + n_row) : 0.0f;
+}
+
 // 16 tokens' values of W row `n_row` (this thread's), tokens tok0 .. tok0 + 15.
 __device__ __forceinline__ void finish16(const float (&v)[16], int tok0, int n_row, int lane, float* c,
                                          bf16* out_act, int m, int n, int ldc, int ld_act, int mode,
-                                         const AddGate& add) {
+                                         const AddGate& add, const float (&old)[16]) {
     if (mode == MODE_SWIGLU) {
         // rows of W: 8 gate, their 8 up, ...; lane l (l % 16 < 8) holds a gate row, lane l + 8 its up row
 #pragma unroll
@@ -73,18 +82,11 @@ __device__ __forceinline__ void finish16(const float (&v)[16], int tok0, int n_r
             }
         }
     } else if (n_row < n) {
-        // When adding to C, all old values are requested before the first sum is stored: written
-        // one after the other, every read would wait behind the store before it (the compiler
-        // cannot tell that the addresses differ), a round trip to L2 per row (the down projection
-        // of the 8B shape at 64 rows: 55 -> 34 microseconds).
-        float old[16], gate[16];
+        float gate[16];
         const float bias = add.gate ? add.bias[n_row] : 0.0f;
 #pragma unroll
         for (int i = 0; i < 16; ++i)
             gate[i] = add.gate && tok0 + i < m ? __ldcg(add.gate + (size_t)(tok0 + i) * add.ld + n_row) : 0.0f;
-#pragma unroll
-        for (int i = 0; i < 16; ++i)
-            old[i] = mode == MODE_ACCUMULATE && tok0 + i < m ? __ldcg(c + (size_t)(tok0 + i) * ldc + n_row) : 0.0f;
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
             const int tok = tok0 + i;
@@ -206,10 +208,11 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             float* part = ws + (size_t)u.unit * NTOK * BW;     // [NTOK][128]
 #pragma unroll 1
             for (int t0 = 0; t0 < NTOK; t0 += 16) {
-                float v[16];
+                float v[16], old[16];
+                if (splits == 1) old16(old, t0, n_row, c, m, n, ldc, mode);
                 tmem_load16(tmem_base + ((unsigned)(quarter * 32) << 16) + (unsigned)(buf * NTOK + t0), v);
                 if (splits == 1) {
-                    finish16(v, t0, n_row, lane, c, out_act, m, n, ldc, ld_act, mode, add);
+                    finish16(v, t0, n_row, lane, c, out_act, m, n, ldc, ld_act, mode, add, old);
                 } else if (t0 < m) {
 #pragma unroll
                     for (int i = 0; i < 16; ++i) part[(size_t)(t0 + i) * BW + row_in_tile] = v[i];
@@ -226,37 +229,51 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             epilogue_sync();
             if (*ticket_slot != splits - 1) continue;
             __threadfence();
-            // Other blocks wrote the partial sums, so every load is a round trip to L2 of most of
-            // a microsecond, and this merge is the exposed tail of the tile: the loads of several
-            // splits (as many as the registers hold) are all requested before any is added, and
-            // the additions then follow in ascending order of the split.
-            const float* first = ws + (size_t)tile * splits * NTOK * BW + row_in_tile;
-            constexpr int AT_ONCE = NTOK == 16 ? 8 : NTOK == 32 ? 3 : 1;
-            float acc[NTOK];
+            // Other blocks wrote the partial sums, so every load is a round trip to L2 of most of a microsecond,
+            // and this merge is the exposed tail of the tile.  When the block has no unit left, its ring is free
+            // (all of its MMAs are through) and takes as many splits' sums as fit, all requested at once without a
+            // register: three of 64 tokens, six of 32, eleven of 16, added in ascending order of the split.  What C
+            // holds is requested before them.
+            const float* first = ws + (size_t)tile * splits * NTOK * BW;
+            const int used = min(NTOK, (m + 15) / 16 * 16);      // tokens whose sums were stored
+            float acc[NTOK], old[NTOK / 16][16];
+#pragma unroll
+            for (int i = 0; i < NTOK / 16; ++i) old16(old[i], i * 16, n_row, c, m, n, ldc, mode);
 #pragma unroll
             for (int i = 0; i < NTOK; ++i) acc[i] = 0.0f;
-            for (int s0 = 0; s0 < splits; s0 += AT_ONCE) {
-                float got[AT_ONCE][NTOK];
+            if (u.unit + u.step >= u.num_units) {
+                constexpr int AT_ONCE = STAGES * (T::STAGE_W + T::STAGE_X) / (NTOK * BW * 4);
+                float* ring = reinterpret_cast<float*>(smem);
+                const int piece = (int)threadIdx.x - 64;         // 0 .. 127: the four epilogue warps
+                for (int s0 = 0; s0 < splits; s0 += AT_ONCE) {
+                    const int here = min(AT_ONCE, splits - s0);
+                    if (s0 > 0) epilogue_sync();
+                    for (int j = 0; j < here; ++j)
+                        for (int at = piece * 4; at < used * BW; at += 512)
+                            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(ring + j * NTOK * BW + at)),
+                                         "l"(first + (size_t)(s0 + j) * NTOK * BW + at) : "memory");
+                    asm volatile("cp.async.wait_all;" ::: "memory");
+                    epilogue_sync();
+                    for (int j = 0; j < here; ++j)
 #pragma unroll
-                for (int j = 0; j < AT_ONCE; ++j) {
-                    // a split past the last one is read from the last one and counts as zero
-                    const int sj = s0 + j < splits ? s0 + j : splits - 1;
-                    const float* p = first + (size_t)sj * NTOK * BW;
-#pragma unroll
-                    for (int i = 0; i < NTOK; ++i) got[j][i] = __ldcg(p + (size_t)i * BW);
+                        for (int i = 0; i < NTOK; ++i)
+                            if (i < used) acc[i] += ring[(j * NTOK + i) * BW + row_in_tile];
                 }
+            } else {
+                for (int sj = 0; sj < splits; ++sj) {
+                    const float* p = first + (size_t)sj * NTOK * BW + row_in_tile;
+                    float got[NTOK];
 #pragma unroll
-                for (int j = 0; j < AT_ONCE; ++j) {
-                    const bool live = s0 + j < splits;
+                    for (int i = 0; i < NTOK; ++i) got[i] = i < used ? __ldcg(p + (size_t)i * BW) : 0.0f;
 #pragma unroll
-                    for (int i = 0; i < NTOK; ++i) acc[i] += live ? got[j][i] : 0.0f;
+                    for (int i = 0; i < NTOK; ++i) acc[i] += got[i];
                 }
             }
 #pragma unroll
             for (int t0 = 0; t0 < NTOK; t0 += 16) {
                 if (t0 < m)
                     finish16(*reinterpret_cast<const float(*)[16]>(&acc[t0]), t0, n_row, lane, c, out_act, m, n,
-                             ldc, ld_act, mode, add);
+                             ldc, ld_act, mode, add, old[t0 / 16]);
             }
             if (warp == 2 && lane == 0) tickets[tile] = 0;
         }
@@ -272,19 +289,29 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
 
 int padded_rows(int m) { return m <= 16 ? 16 : m <= 32 ? 32 : 64; }
 
-// The number of splits of K: the one that lets the busiest block stream the fewest blocks of K
-// (each unit costs one more for its epilogue, a split tile two for the merge); smallest on a tie.
+// The number of splits of K.  The grid has `slots` = two blocks per SM.  A lone block takes a k block (16 KB of W) in
+// about 0.29 us, all slots together one per 2.46 ns (the copy bandwidth), so from about 118 tiles on whole tiles keep
+// the memory busy by themselves and every split only adds partial sums to store and merge: one split, or two where
+// the last round of whole tiles would leave most slots idle.  Fewer tiles are cut into as many splits as the slots
+// hold at once, a unit per block.  Times in us at 8 / 32 / 64 rows, against the rule before, which counted one block
+// per SM: 10,240 x 5,120 (80 tiles, 11 -> 3 splits) 30.5 / 36.5 / 57.5 -> 21.3 / 22.9 / 28.3; 5,120 x 8,192 (40 tiles,
+// 11 -> 7) 23.6 / 29.8 / 46.7 -> 18.8 / 22.3 / 28.9 with 6; 51,200 x 5,120 (400 tiles, 4 -> 1) 100 / 144 / 202 -> 85 /
+// 92 / 104; 151,936 x 5,120 (1,187 tiles, 4 -> 1) 266 / 305 -> 237 / 241 at 8 / 32.
 int choose_splits(int n, int k, int sms) {
-    const int tiles = (n + BW - 1) / BW, num_kb = (k + BK - 1) / BK;
-    int best = 1;
-    long long best_cost = -1;
-    for (int s = 1; s <= MAX_SPLITS && s * 2 <= num_kb || s == 1; ++s) {
-        const long long units = (long long)tiles * s;
-        const long long grid = units < sms ? units : sms;
-        const long long cost = ((units + grid - 1) / grid) * ((num_kb + s - 1) / s + 1) + (s > 1 ? 2 : 0);
-        if (best_cost < 0 || cost < best_cost) { best = s; best_cost = cost; }
+    const int tiles = (n + BW - 1) / BW, num_kb = (k + BK - 1) / BK, slots = BLOCKS_PER_SM * sms;
+    if (tiles * 5 < slots * 2) {
+        int s = slots / tiles;
+        if (s > MAX_SPLITS) s = MAX_SPLITS;
+        if (s > num_kb / 2) s = num_kb / 2;
+        return s > 1 ? s : 1;
     }
-    return best;
+    // picoseconds: full rounds at the bandwidth, the rest at the bandwidth or a block's own pace; a split unit's sums
+    auto cost = [&](int s) {
+        const long long units = (long long)tiles * s, kb = (num_kb + s - 1) / s, left = units % slots;
+        const long long tail = left * kb * 2460 > kb * 290000 ? left * kb * 2460 : left ? kb * 290000 : 0;
+        return units / slots * slots * kb * 2460 + tail + (s > 1 ? 3000000 + units * 60000 : 0);
+    };
+    return num_kb >= 4 && cost(2) < cost(1) ? 2 : 1;
 }
 
 int device_sms() {
