@@ -1,0 +1,486 @@
+// Paged flash attention with optional parts for prompt portions on the 5th-generation tensor cores: the same options,
+// cache layouts and precision as attn_options_tc.cu (a window and/or chunks, a score factor per head, a cap, a sink, an
+// output gate, one shared row per token as key and value), whose mma.sync kernel keeps single tokens and every size
+// that this one does not take.
+//
+// Arrangement.  A block has 128 rows, the MMA's M side: the heads of one kv group of 128 / group consecutive tokens of
+// one request, fetched by one 3-D TMA box per 64 elements of the head.  It walks its keys in tiles of 64.  A tile
+// comes as chunks of 64 keys x 64 elements (TMA, 128-byte swizzle, a barrier each).  Score products take every key
+// chunk as K-major B operand; the value products take the chunks of the block's value columns as MN-major B operand:
+// chunks of their own, or with shared rows the very chunks that the scores have used.  Values of more than 256
+// columns are cut into slices, a block each.
+//
+// Softmax weights stay float32 through the second product: a weight is cut into three bfloat16 parts (8 + 8 + 8 bits
+// of its significand) which the softmax threads (one per row) write into tensor memory as the A operand of three
+// products.  So a tile of 64 keys is K / 16 score products of N = 64 and twelve value products, and what bounds it is
+// the tensor core and the shared memory it reads: 1,730 + 1,540 cycles for latent rows of 576 with 256 value columns.
+//
+// Two forms.  Rows of up to 128 elements with values of their own (NS = 1): the weights take the place of the scores,
+// 224 columns of tensor memory, two blocks per SM that fill one another's gaps; a block is the plain chain of
+// scores, softmax, value products.  Wide shared rows (NS = 2): one block per SM, two score buffers, and the next tile's
+// scores issued around the value products of this one.  Where shared memory holds two tiles (rows up to 320) they go in
+// front of them; where it holds one (576: queries 147 KB, a tile 74 KB) the part of the row that is no value of this
+// block goes in front, and the rest, whose chunks the value products still need, behind.
+//
+// Order: warp 0 issues TMA, warp 1 the products, warps 2-5 are the softmax.  Every wait on an mbarrier is bounded: on a
+// timeout the block records status 2, frees its tensor memory and returns.
+#include "sm100.cuh"
+
+namespace {
+
+using namespace sm100;
+
+constexpr int BM = 128, BN = 64;
+constexpr int THREADS = 192;
+constexpr int QCHUNK = BM * 128, CHUNK = BN * 128;    // bytes: 64 elements of every row
+constexpr int MAX_POS = 9;                            // chunks of a tile
+constexpr float LOG2E = 1.4426950408889634f;
+constexpr float RESCALE_STEP = 8.0f;                  // in log2 units
+enum { TI_ERR_BAD_PAGE = 1, TI_ERR_TIMEOUT = 2 };
+
+struct UmmaOptions {
+    int window, chunk;
+    float scale, softcap;
+    const float* head_scale;
+    const float* sink;
+    const float* gate;
+    int gate_stride, gate_per_head;
+};
+
+// How a tile is cut: `chunks` of a key row, `places` chunks of a tile, the last `nv` of them the value chunks of a slice.
+struct Shape {
+    int dk, dv, chunks, places, nv, slices, stages, shared, run;
+};
+
+__device__ __forceinline__ float ex2_approx(float x) {
+    float y;
+    asm("ex2.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float rcp_approx(float x) {
+    float y;
+    asm("rcp.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ int first_visible(int p, const UmmaOptions& o) {
+    int lo = o.window > 0 ? max(0, p - o.window + 1) : 0;
+    if (o.chunk > 0) lo = max(lo, p / o.chunk * o.chunk);
+    return lo;
+}
+// Two floats as three pairs of bfloat16 whose sums are the floats (the upper 16 bits of what is left, three times).
+__device__ __forceinline__ void split3_pair(float x, float y, unsigned& hi, unsigned& mid, unsigned& lo) {
+    const unsigned xb = __float_as_uint(x), yb = __float_as_uint(y);
+    hi = __byte_perm(xb, yb, 0x7632);
+    const float x1 = x - __uint_as_float(xb & 0xffff0000u), y1 = y - __uint_as_float(yb & 0xffff0000u);
+    const unsigned x1b = __float_as_uint(x1), y1b = __float_as_uint(y1);
+    mid = __byte_perm(x1b, y1b, 0x7632);
+    const float x2 = x1 - __uint_as_float(x1b & 0xffff0000u), y2 = y1 - __uint_as_float(y1b & 0xffff0000u);
+    lo = __byte_perm(__float_as_uint(x2), __float_as_uint(y2), 0x7632);
+}
+// D (+)= A B with A from tensor memory (rows in lanes, two bfloat16 of K per 32-bit column).
+__device__ __forceinline__ void umma_bf16_tmem_a(unsigned tmem_d, unsigned tmem_a, unsigned long long db, unsigned idesc,
+                                                 unsigned accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(db), "r"(idesc), "r"(accumulate) : "memory");
+}
+// 16 consecutive 32-bit columns of this thread's lane; completion is awaited by the caller.
+__device__ __forceinline__ void tmem_store16(unsigned taddr, const unsigned (&v)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};\n"
+        ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
+          "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
+        : "memory");
+}
+__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, void* bar, int x, int y, int z) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];\n"
+        ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z) : "memory");
+}
+
+// tiles[i] = {request row, first flat token, tokens (<= BM / group)}
+template <int NS>
+__global__ void __launch_bounds__(THREADS, NS == 1 ? 2 : 1)
+attn_options_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kv,
+                         const int* __restrict__ tiles, const int* __restrict__ positions,
+                         const int* __restrict__ block_table, int bt_stride, int num_pages, int page_size, int num_heads,
+                         int num_kv_heads, Shape sh, UmmaOptions opt, bf16* __restrict__ out, int* __restrict__ status) {
+    constexpr unsigned TMEM_COLS = NS == 1 ? 256 : 512;
+    constexpr unsigned S_AT = NS == 1 ? 128 : 256, P_AT = NS == 1 ? 128 : 384;      // outputs from column 0 on
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    unsigned char* ring = smem + sh.chunks * QCHUNK;
+    unsigned long long* bars = (unsigned long long*)(ring + sh.stages * sh.places * CHUNK);
+    unsigned long long* q_full = bars;
+    unsigned long long* s_full = bars + 1;            // [NS]
+    unsigned long long* s_empty = bars + 3;           // [NS]
+    unsigned long long* p_full = bars + 5;
+    unsigned long long* p_empty = bars + 6;           // value products done: weights may be rewritten, O is up to date
+    unsigned long long* full = bars + 7;              // [stages * places]
+    unsigned long long* empty = full + 2 * MAX_POS;
+    unsigned* tmem_slot = (unsigned*)(empty + 2 * MAX_POS);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int slice = blockIdx.x % sh.slices, kvh = blockIdx.x / sh.slices;
+    const int group = num_heads / num_kv_heads;
+    const int req = tiles[blockIdx.y * 3], tok0 = tiles[blockIdx.y * 3 + 1], ntok = tiles[blockIdx.y * 3 + 2];
+    const int pos_first = positions[tok0], pos_last = pos_first + ntok - 1;
+    const int kv_lo = first_visible(pos_first, opt);
+    const int kt_lo = kv_lo / BN, num_kt = pos_last / BN + 1 - kt_lo;
+    const int early = sh.places - sh.nv;              // places whose chunks only the scores read
+
+    if (threadIdx.x == 0) {
+        mbar_init(q_full, 1);
+        for (int i = 0; i < 2; ++i) { mbar_init(&s_full[i], 1); mbar_init(&s_empty[i], 4); }
+        mbar_init(p_full, 4);
+        mbar_init(p_empty, 1);
+        for (int i = 0; i < sh.stages * sh.places; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
+        mbar_fence_init();
+    }
+    if (warp == 1) tmem_alloc(tmem_slot, TMEM_COLS);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const unsigned tmem_base = *tmem_slot;
+
+    bool ok = true;
+    if (warp == 0) {
+        const int* table = block_table + (size_t)req * bt_stride;
+        const int per_page = num_kv_heads * page_size * (sh.shared ? 1 : 2);      // rows of a page in the pool's 2-D view
+        const int oob_row = num_pages * per_page;                                 // outside the tensor: zeros
+        const int to_v = num_kv_heads * page_size;                                // keys -> values of a page
+        if (lane == 0) {
+            const int tokens = BM / group;
+            mbar_expect_tx(q_full, sh.chunks * tokens * group * 128);
+            for (int c = 0; c < sh.chunks; ++c)
+                tma_load_3d(smem + c * QCHUNK, &map_q, q_full, c * 64, kvh * group, tok0);
+        }
+        for (int j = 0; j < num_kt && ok; ++j) {
+            const int st = j % sh.stages, phase = (j / sh.stages) & 1;
+            int row = oob_row;                        // where this lane's run of keys begins
+            if (lane < BN / sh.run) {
+                const int key0 = (kt_lo + j) * BN + lane * sh.run;
+                if (key0 <= pos_last && key0 + sh.run > kv_lo) {
+                    const int pg = table[key0 / page_size];
+                    if (pg >= 0 && pg < num_pages)
+                        row = pg * per_page + kvh * page_size + key0 % page_size;
+                    else
+                        atomicCAS(status, 0, TI_ERR_BAD_PAGE);
+                }
+            }
+            for (int p = 0; p < sh.places; ++p) {
+                unsigned long long* bar = &full[st * sh.places + p];
+                if (lane == 0) {
+                    ok = mbar_wait(&empty[st * sh.places + p], phase ^ 1);
+                    if (ok) mbar_expect_tx(bar, CHUNK);
+                }
+                ok = __shfl_sync(0xffffffffu, ok, 0);
+                if (!ok) break;
+                int c, y = row;
+                if (sh.shared) {                      // the row's chunks outside the slice, then the slice's
+                    c = p >= early ? slice * sh.nv + p - early : p < slice * sh.nv ? p : p + sh.nv;
+                } else {
+                    c = p < sh.chunks ? p : slice * sh.nv + p - sh.chunks;
+                    if (p >= sh.chunks && row != oob_row) y = row + to_v;
+                }
+                if (lane < BN / sh.run)
+                    tma_load_2d(ring + (st * sh.places + p) * CHUNK + lane * sh.run * 128, &map_kv, bar, c * 64, y);
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            const unsigned idesc_s = umma_idesc(BM, BN);
+            const unsigned idesc_o = umma_idesc(BM, sh.nv * 64, /*b_mn_major=*/true);
+            // scores of tile j from the chunks at places [from, to)
+            auto scores = [&](int j, int from, int to) {
+                const int st = j % sh.stages, phase = (j / sh.stages) & 1;
+                for (int p = from; p < to && ok; ++p) {
+                    ok = mbar_wait(&full[st * sh.places + p], phase);
+                    if (!ok) break;
+                    tc_fence_after();
+                    const int c = !sh.shared ? p : p >= early ? slice * sh.nv + p - early : p < slice * sh.nv ? p : p + sh.nv;
+                    const int steps = min(4, (sh.dk - c * 64) / 16);
+                    const unsigned long long dq = umma_desc(smem + c * QCHUNK);
+                    const unsigned long long dk_ = umma_desc(ring + (st * sh.places + p) * CHUNK);
+                    for (int kk = 0; kk < steps; ++kk)
+                        umma_bf16(tmem_base + S_AT + (NS == 1 ? 0 : (j & 1) * BN), dq + (unsigned long long)(kk * 2),
+                                  dk_ + (unsigned long long)(kk * 2), idesc_s, p > 0 || kk > 0);
+                    if (p < early) umma_commit(&empty[st * sh.places + p]);
+                }
+            };
+            const int all = sh.shared ? sh.places : sh.chunks;
+            ok = mbar_wait(q_full, 0);
+            if (ok) {
+                tc_fence_after();
+                scores(0, 0, all);
+                umma_commit(&s_full[0]);
+            }
+            for (int j = 0; j < num_kt && ok; ++j) {
+                const bool more = j + 1 < num_kt;
+                const int split_at = sh.stages == 2 ? all : early;        // what of the next scores goes in front
+                if (NS == 2 && more) {
+                    const int b = (j + 1) & 1;
+                    ok = mbar_wait(&s_empty[b], (((j + 1) >> 1) & 1) ^ 1);
+                    if (!ok) break;
+                    tc_fence_after();
+                    scores(j + 1, 0, split_at);
+                    if (split_at == all && ok) umma_commit(&s_full[b]);
+                }
+                const int st = j % sh.stages;
+                if (ok) ok = mbar_wait(p_full, j & 1);
+                for (int p = sh.shared ? sh.places : early; p < sh.places && ok; ++p)     // values of their own
+                    ok = mbar_wait(&full[st * sh.places + p], (j / sh.stages) & 1);
+                if (!ok) break;
+                tc_fence_after();
+                const unsigned char* vbuf = ring + (st * sh.places + early) * CHUNK;
+                for (int part = 2; part >= 0; --part)                                     // the smallest parts first
+                    for (int ks = 0; ks < BN / 16; ++ks)
+                        umma_bf16_tmem_a(tmem_base, tmem_base + P_AT + part * 32 + ks * 8,
+                                         umma_desc(vbuf + ks * 2048, CHUNK, 1024), idesc_o, j > 0 || part < 2 || ks > 0);
+                for (int p = early; p < sh.places; ++p) umma_commit(&empty[st * sh.places + p]);
+                umma_commit(p_empty);
+                if (more && NS == 1) {
+                    // the products run in the order of issue: these overwrite the weights when they have been read
+                    scores(j + 1, 0, all);
+                    umma_commit(&s_full[0]);
+                } else if (more && split_at < all) {
+                    scores(j + 1, split_at, all);
+                    umma_commit(&s_full[(j + 1) & 1]);
+                }
+            }
+        }
+    } else {
+        const int quarter = warp & 3;                                             // tensor-memory lanes
+        const int row = quarter * 32 + lane;
+        const int tok = row / group, h = kvh * group + row % group;
+        const bool live = tok < ntok;
+        const int pos_row = live ? pos_first + tok : -1;                          // -1: sees nothing
+        const int lo_row = live ? first_visible(pos_row, opt) : 0;
+        const int lo_last = first_visible(pos_last, opt);
+        const unsigned lane_addr = (unsigned)(quarter * 32) << 16;
+        const float scale = opt.scale * (opt.head_scale && live ? opt.head_scale[h] : 1.0f);
+        const float cap_arg = opt.softcap > 0.0f ? 2.0f * LOG2E / opt.softcap : 0.0f, cap_l2e = opt.softcap * LOG2E;
+        float m_ref = -INFINITY, l_run = 0.0f;
+        for (int j = 0; j < num_kt && ok; ++j) {
+            const int b = NS == 1 ? 0 : j & 1;
+            const int key_lo = (kt_lo + j) * BN;
+            ok = mbar_wait(&s_full[b], (NS == 1 ? j : j >> 1) & 1);
+            if (!ok) break;
+            tc_fence_after();
+            float v[BN];
+#pragma unroll
+            for (int c = 0; c < 2; ++c)
+                tmem_load32(tmem_base + lane_addr + S_AT + b * BN + c * 32, *reinterpret_cast<float(*)[32]>(&v[c * 32]));
+            if (NS == 2) {
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&s_empty[b]);
+            }
+            if (opt.softcap > 0.0f) {                 // cap tanh(v / cap) = cap (1 - 2 / (exp(2 v / cap) + 1))
+#pragma unroll
+                for (int i = 0; i < BN; ++i)
+                    v[i] = cap_l2e * fmaf(-2.0f, rcp_approx(ex2_approx(v[i] * scale * cap_arg) + 1.0f), 1.0f);
+            } else {
+#pragma unroll
+                for (int i = 0; i < BN; ++i) v[i] *= scale * LOG2E;
+            }
+            if (key_lo + BN - 1 > pos_first || key_lo < lo_last) {
+#pragma unroll
+                for (int i = 0; i < BN; ++i)
+                    if (key_lo + i > pos_row || key_lo + i < lo_row) v[i] = -INFINITY;
+            }
+            float m4[4] = {v[0], v[1], v[2], v[3]};
+#pragma unroll
+            for (int i = 4; i < BN; i += 4)
+#pragma unroll
+                for (int u = 0; u < 4; ++u) m4[u] = fmaxf(m4[u], v[i + u]);
+            const float m_new = fmaxf(m_ref, fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])));
+            const bool grow = m_new > m_ref + RESCALE_STEP;                       // also true when m_ref is still -inf
+            if (j > 0) {
+                ok = mbar_wait(p_empty, (j - 1) & 1);
+                if (!ok) break;
+                if (__any_sync(0xffffffffu, grow)) {
+                    // the output so far was built against m_ref: bring it to the new reference
+                    tc_fence_after();
+                    const float factor = grow ? exp2f(m_ref - m_new) : 1.0f;      // 0 if m_ref was -inf
+                    l_run *= factor;
+#pragma unroll 1
+                    for (int c = 0; c < sh.nv * 2; ++c) {
+                        float o[32];
+                        tmem_load32(tmem_base + lane_addr + c * 32, o);
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) o[i] *= factor;
+                        tmem_store32(tmem_base + lane_addr + c * 32, o);
+                    }
+                }
+            }
+            if (grow) m_ref = m_new;
+            const float m_use = m_ref == -INFINITY ? 0.0f : m_ref;
+            float sum[2] = {0.0f, 0.0f};
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                unsigned hi[16], mid[16], lo[16];
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    const float p0 = exp2f(v[c * 32 + 2 * i] - m_use), p1 = exp2f(v[c * 32 + 2 * i + 1] - m_use);
+                    sum[0] += p0;
+                    sum[1] += p1;
+                    split3_pair(p0, p1, hi[i], mid[i], lo[i]);
+                }
+                tmem_store16(tmem_base + lane_addr + P_AT + c * 16, hi);
+                tmem_store16(tmem_base + lane_addr + P_AT + 32 + c * 16, mid);
+                tmem_store16(tmem_base + lane_addr + P_AT + 64 + c * 16, lo);
+            }
+            l_run += sum[0] + sum[1];
+            asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(p_full);
+        }
+        if (ok) ok = mbar_wait(p_empty, (num_kt - 1) & 1);
+        if (ok) {
+            tc_fence_after();
+            const size_t t = (size_t)tok0 + tok;
+            float l = l_run;
+            if (opt.sink && live) l += exp2f(opt.sink[h] * LOG2E - m_ref);
+            float inv = 1.0f / l;
+            const float* gt = opt.gate && live ? opt.gate + t * opt.gate_stride : nullptr;
+            if (gt && opt.gate_per_head) inv *= 1.0f / (1.0f + expf(-gt[h]));
+            const float* ge = gt && !opt.gate_per_head ? gt + (size_t)h * sh.dv + slice * sh.nv * 64 : nullptr;
+            bf16* orow = out + (t * num_heads + h) * sh.dv + slice * sh.nv * 64;
+#pragma unroll 1
+            for (int c = 0; c < sh.nv * 2; ++c) {
+                float v[32];
+                tmem_load32(tmem_base + lane_addr + c * 32, v);
+                if (!live) continue;
+                unsigned packed[16];
+#pragma unroll
+                for (int i = 0; i < 32; i += 2) {
+                    float a = v[i] * inv, d = v[i + 1] * inv;
+                    if (ge) {
+                        a *= 1.0f / (1.0f + expf(-ge[c * 32 + i]));
+                        d *= 1.0f / (1.0f + expf(-ge[c * 32 + i + 1]));
+                    }
+                    __nv_bfloat162 pk = __floats2bfloat162_rn(a, d);
+                    packed[i >> 1] = *reinterpret_cast<unsigned*>(&pk);
+                }
+#pragma unroll
+                for (int q8 = 0; q8 < 2; ++q8)            // whole 32-byte sectors (a row of outputs is 128-byte aligned)
+                    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(orow + c * 32 + q8 * 16),
+                                 "r"(packed[q8 * 8]), "r"(packed[q8 * 8 + 1]), "r"(packed[q8 * 8 + 2]),
+                                 "r"(packed[q8 * 8 + 3]), "r"(packed[q8 * 8 + 4]), "r"(packed[q8 * 8 + 5]),
+                                 "r"(packed[q8 * 8 + 6]), "r"(packed[q8 * 8 + 7]) : "memory");
+            }
+        }
+    }
+    if (!ok) atomicCAS(status, 0, TI_ERR_TIMEOUT);
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_dealloc(tmem_base, TMEM_COLS);
+    }
+}
+
+size_t smem_bytes(const Shape& sh) {
+    return 1024 + (size_t)sh.chunks * QCHUNK + (size_t)sh.stages * sh.places * CHUNK + (7 + 4 * MAX_POS) * 8 + 16;
+}
+
+// The cut of the rows, or `places` = 0 where the kernel does not take them.
+Shape shape_of(int dk, int dv, int page_size, int shared, int group) {
+    Shape sh = {};
+    if (group < 1 || group > BM || dk < 16 || dk % 16 || dv < 64 || dv % 64 || page_size < 16 || page_size % 16) return sh;
+    sh.dk = dk;
+    sh.dv = dv;
+    sh.shared = shared;
+    sh.chunks = (dk + 63) / 64;
+    if (shared) {
+        if (dv > dk || (dv > 256 && dv % 256)) return sh;
+        sh.nv = dv > 256 ? 4 : dv / 64;
+    } else {
+        if (dk != dv || dv > 128) return sh;
+        sh.nv = dv / 64;
+    }
+    sh.slices = dv / (sh.nv * 64);
+    sh.run = BN;
+    while (page_size % sh.run) sh.run /= 2;
+    const int places = shared ? sh.chunks : sh.chunks + sh.nv;
+    if (places > MAX_POS) return sh;
+    sh.places = places;
+    sh.stages = 2;
+    if (smem_bytes(sh) > 227 * 1024) sh.stages = 1;
+    if (smem_bytes(sh) > 227 * 1024 || (!shared && sh.stages == 1)) sh.places = 0;
+    return sh;
+}
+
+int make_map(CUtensorMap* map, const void* base, int rank, const cuuint64_t* dims, const cuuint64_t* strides,
+             const cuuint32_t* box) {
+    EncodeTiled fn = encode_fn();
+    if (!fn) return ti_fail("attn_options_umma: the driver lacks cuTensorMapEncodeTiled");
+    const cuuint32_t elem[3] = {1, 1, 1};
+    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, rank, const_cast<void*>(base), dims, strides, box, elem,
+                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return ti_fail("attn_options_umma: cuTensorMapEncodeTiled failed with %d", (int)r);
+    return 0;
+}
+
+}  // namespace
+
+// Query tokens of a block, or 0 where the kernel does not take these sizes.
+extern "C" int ti_attn_options_umma_tokens(int dk, int dv, int page_size, int shared_rows, int num_heads, int num_kv_heads) {
+    if (num_kv_heads < 1 || num_heads % num_kv_heads) return 0;
+    return shape_of(dk, dv, page_size, shared_rows, num_heads / num_kv_heads).places ? BM / (num_heads / num_kv_heads) : 0;
+}
+
+// q: bfloat16 [num_tokens, num_heads, dk], out: bfloat16 [num_tokens, num_heads, dv], contiguous.  tiles: int32
+// [num_tiles, 3] = {request row, first flat token, tokens}, at most ti_attn_options_umma_tokens consecutive tokens of
+// one request each.  The rest as in ti_attn_options_tc.
+extern "C" int ti_attn_options_umma(const void* q, const int* tiles, int num_tiles, int num_tokens, const int* positions,
+                                    const int* block_table, int bt_stride, const void* pages, int num_pages,
+                                    int page_size, int num_heads, int num_kv_heads, int dk, int dv, int shared_rows,
+                                    int window, int chunk, float scale, float softcap, const float* head_scale,
+                                    const float* sink, const float* gate, int gate_stride, int gate_per_head, void* out,
+                                    int* status, void* stream) {
+    if (num_tiles == 0) return 0;
+    TI_REQUIRE(ti_attn_options_umma_tokens(dk, dv, page_size, shared_rows, num_heads, num_kv_heads) > 0,
+               "attn_options_umma: head sizes %d and %d, page size %d or %d heads over %d kv heads are not supported", dk,
+               dv, page_size, num_heads, num_kv_heads);
+    TI_REQUIRE((uintptr_t)q % 16 == 0 && (uintptr_t)pages % 16 == 0 && (uintptr_t)out % 32 == 0,
+               "attn_options_umma: queries and pages must be 16-byte aligned, the output 32-byte");
+    TI_REQUIRE(num_tiles <= 65535, "attn_options_umma: %d tiles exceed the grid limit", num_tiles);
+    const int group = num_heads / num_kv_heads;
+    const Shape sh = shape_of(dk, dv, page_size, shared_rows, group);
+    const long long pool_rows = (long long)num_pages * num_kv_heads * page_size * (shared_rows ? 1 : 2);
+    TI_REQUIRE(pool_rows < (1LL << 31) - 1, "attn_options_umma: the page pool has too many token slots");
+    CUtensorMap map_q, map_kv;
+    const cuuint64_t qdims[3] = {(cuuint64_t)dk, (cuuint64_t)num_heads, (cuuint64_t)num_tokens};
+    const cuuint64_t qstrides[2] = {(cuuint64_t)dk * 2, (cuuint64_t)num_heads * dk * 2};
+    const cuuint32_t qbox[3] = {64, (cuuint32_t)group, (cuuint32_t)(BM / group)};
+    if (int rc = make_map(&map_q, q, 3, qdims, qstrides, qbox)) return rc;
+    const cuuint64_t kdims[2] = {(cuuint64_t)dk, (cuuint64_t)pool_rows};
+    const cuuint64_t kstrides[1] = {(cuuint64_t)dk * 2};
+    const cuuint32_t kbox[2] = {64, (cuuint32_t)sh.run};
+    if (int rc = make_map(&map_kv, pages, 2, kdims, kstrides, kbox)) return rc;
+    UmmaOptions opt = {window, chunk, scale, softcap, head_scale, sink, gate, gate_stride, gate_per_head};
+    const size_t smem = smem_bytes(sh);
+    const dim3 grid(num_kv_heads * sh.slices, num_tiles);
+    cudaStream_t s = (cudaStream_t)stream;
+#define LAUNCH(NS)                                                                                                \
+    {                                                                                                             \
+        static TiPerDevice configured;                                                                            \
+        if (configured.first_use()) {                                                                             \
+            cudaError_t e = cudaFuncSetAttribute(attn_options_umma_kernel<NS>,                                     \
+                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);         \
+            if (e != cudaSuccess) return ti_fail("attn_options_umma: %s", cudaGetErrorString(e));                  \
+            configured.mark();                                                                                    \
+        }                                                                                                         \
+        attn_options_umma_kernel<NS><<<grid, THREADS, smem, s>>>(map_q, map_kv, tiles, positions, block_table,     \
+            bt_stride, num_pages, page_size, num_heads, num_kv_heads, sh, opt, (bf16*)out, status);               \
+    }
+    if (shared_rows) LAUNCH(2) else LAUNCH(1)
+#undef LAUNCH
+    return ti_check_launch("attn_options_umma");
+}

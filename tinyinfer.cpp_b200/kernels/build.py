@@ -31,7 +31,7 @@ LIBRARIES = {
     "bf16_gated": ["common.cu", "attn_gated_bias_tc.cu", "attn_bias_prefill_tc.cu", "moe_grouped.cu"],
     # attention with optional parts (chunks, caps, sinks, gates, shared rows) and the recurrent mixer
     "mixers": ["common.cu", "attn_options.cu", "head_rows.cu", "wkv.cu"],
-    "bf16_mixers": ["common.cu", "attn_options_tc.cu"],
+    "bf16_mixers": ["common.cu", "attn_options_tc.cu", "attn_options_umma.cu"],
     # recurrent mixers with a matrix state
     "state": ["common.cu", "matrix_state.cu", "matrix_state_decayed.cu"],
     # recurrences per channel and the gates and decays in front of them

@@ -323,11 +323,12 @@ class CudaOps(MixerOps, StateOps):
         prompt-attention kernel's own height.  The 32-bit kernels need none."""
         if act_dtype != torch.bfloat16:
             return []
-        from .step_lists import attention_lists, row_tile_lists
+        from .step_lists import attention_lists, option_tile_lists, row_tile_lists
         self.bf16
         # ... and, where a mixer has announced attention with options, every entry cut into tiles
         # of as many tokens as that kernel's blocks take
-        return attention_lists(self._tile_rows) + row_tile_lists(self._row_tile_tokens)
+        return (attention_lists(self._tile_rows) + row_tile_lists(self._row_tile_tokens)
+                + option_tile_lists(self._option_tile_tokens))
 
     def stream(self) -> int:
         """The CUDA stream (as an integer handle) on which the engine's kernels are launched; a

@@ -42,7 +42,8 @@ def _ptr(t):
 class MixerOps:
     _mixers = None
     _mixers_tc = None
-    use_tc_attention_options = True        # tensor-core kernel of the attention with options (bfloat16)
+    use_tc_attention_options = True        # tensor-core kernels of the attention with options (bfloat16)
+    use_umma_attention_options = True      # ... prompt portions on tcgen05 where the sizes allow
 
     @property
     def _row_tile_tokens(self) -> set:
@@ -51,11 +52,17 @@ class MixerOps:
             found = self.__dict__["_row_tile_set"] = set()
         return found
 
+    @property
+    def _option_tile_tokens(self) -> set:
+        return self.__dict__.setdefault("_option_tile_set", set())
+
     def want_row_tiles(self, num_heads: int, num_kv_heads: int) -> None:
         """A mixer says, when it gets its weights, that it will call ``attention_options`` with these
-        head counts: every step then brings the tile list that the tensor-core kernel walks
-        (``step_lists``); without it the calls run on the CUDA-core kernel."""
+        head counts: every step then brings the tile lists that the tensor-core kernels walk
+        (``step_lists``); without them the calls run on the CUDA-core kernel."""
         self._row_tile_tokens.add(64 // self._group_rows(num_heads, num_kv_heads))
+        if num_heads // num_kv_heads <= 128:
+            self._option_tile_tokens.add(128 // (num_heads // num_kv_heads))
 
     @staticmethod
     def _group_rows(num_heads: int, num_kv_heads: int) -> int:
@@ -85,6 +92,9 @@ class MixerOps:
             b.ti_head_project_tc.argtypes = [_vp, _i, _i, _vp, _i, _i, _vp, _i, _i, _i, _i, _vp]
             b.ti_attn_options_tc.argtypes = [_vp, _vp, _i, _i, _vp, _vp, _i, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _i,
                                              _f, _f, _vp, _vp, _vp, _i, _i, _i, _vp, _vp, _i, _vp, _vp, _vp]
+            b.ti_attn_options_umma_tokens.argtypes = [_i] * 6
+            b.ti_attn_options_umma.argtypes = [_vp, _vp, _i, _i, _vp, _vp, _i, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _i,
+                                               _f, _f, _vp, _vp, _vp, _i, _i, _vp, _vp, _vp]
             self._mixers_tc = b
         return self._mixers_tc
 
@@ -363,6 +373,21 @@ class MixerOps:
         self._must(gate is None or (gate.dtype == torch.float32 and gate.stride(1) == 1 and gate.shape[0] == t
                                     and gate.shape[1] == (num_heads if gate_per_head else num_heads * dv)),
                    "attention_options: the gate must be float32 [T, heads] or [T, heads * dv]")
+        # a step that brings prompt portions: tcgen05, where the head sizes fill its chunks of 64 elements; its single
+        # tokens ride along as tiles of one token
+        tiles = getattr(step, "lists", {}).get(f"option_tiles_{128 // max(1, min(128, num_heads // num_kv_heads))}")
+        if (self.use_tc_attention_options and self.use_umma_attention_options and getattr(step, "max_q_len", 0) > 1
+                and tiles is not None and 0 < tiles.shape[0] <= 65535 and q.dtype == pages.dtype == torch.bfloat16
+                and q.data_ptr() % 16 == 0 and out.data_ptr() % 32 == 0 and pages.data_ptr() % 16 == 0
+                and self.mixers_tc.ti_attn_options_umma_tokens(dk, dv, cache.page_size, int(bool(shared_rows)), num_heads,
+                                                               num_kv_heads)):
+            self._ok(self.mixers_tc.ti_attn_options_umma(
+                q.data_ptr(), tiles.data_ptr(), tiles.shape[0], t, step.positions.data_ptr(), bt.data_ptr(),
+                bt.stride(0), pages.data_ptr(), pages.shape[0], cache.page_size, num_heads, num_kv_heads, dk, dv,
+                int(bool(shared_rows)), int(window or 0), int(chunk or 0), float(scale), float(softcap or 0.0),
+                _ptr(head_scale), _ptr(sink), _ptr(gate), gate.stride(0) if gate is not None else 0,
+                int(bool(gate_per_head)), out.data_ptr(), self.status.data_ptr(), self._stream()), self.mixers_tc)
+            return
         gp = self._group_rows(num_heads, num_kv_heads)
         tiles = getattr(step, "lists", {}).get(f"row_tiles_{64 // gp}")
         if (self.use_tc_attention_options and tiles is not None and 0 < tiles.shape[0] <= 65535 and q.dtype == torch.bfloat16

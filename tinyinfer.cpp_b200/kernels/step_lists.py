@@ -51,9 +51,26 @@ def row_tiles(q_lens: Sequence[int], starts: Sequence[int], tokens: int) -> np.n
     return np.stack([req, cu[req] + lo, np.minimum(tokens, q[req] - lo)], axis=1).astype(np.int64).reshape(-1, 3)
 
 
+def option_tiles(q_lens: Sequence[int], starts: Sequence[int], tokens: int) -> np.ndarray:
+    """The tiles of ``row_tiles`` with the longest contexts first (they take longest); none for a step of single
+    tokens, which another kernel takes."""
+    if max(q_lens, default=0) <= 1:
+        return np.zeros((0, 3), dtype=np.int64)
+    tiles = row_tiles(q_lens, starts, tokens)
+    cu = np.concatenate([[0], np.cumsum(q_lens)])
+    ends = np.asarray(starts, dtype=np.int64)[tiles[:, 0]] + tiles[:, 1] - cu[tiles[:, 0]] + tiles[:, 2]
+    return tiles[np.argsort(-ends, kind="stable")]
+
+
 def row_tile_lists(token_counts: Sequence[int]):
     from ..engine.batch import StepList
     return [StepList(f"row_tiles_{n}", partial(row_tiles, tokens=n)) for n in sorted(set(token_counts))]
+
+
+def option_tile_lists(token_counts: Sequence[int]):
+    from ..engine.batch import StepList
+    return [StepList(f"option_tiles_{n}", partial(option_tiles, tokens=n), uses_starts=True)
+            for n in sorted(set(token_counts))]
 
 
 def attention_lists(tile_heights: Sequence[int]):
