@@ -5,7 +5,7 @@
 //
 // Arrangement.  A block has 128 rows, the MMA's M side: the heads of one kv group of 128 / group consecutive tokens of
 // one request, fetched by one 3-D TMA box per 64 elements of the head.  It walks its keys in tiles of 64.  A tile
-// comes as chunks of 64 keys x 64 elements (TMA, 128-byte swizzle, a barrier each).  Score products take every key
+// comes as chunks of 64 keys x 64 elements (TMA, 128-byte swizzle).  Score products take every key
 // chunk as K-major B operand; the value products take the chunks of the block's value columns as MN-major B operand:
 // chunks of their own, or with shared rows the very chunks that the scores have used.  Values of more than 256
 // columns are cut into slices, a block each.
@@ -18,12 +18,13 @@
 // Two forms.  Rows of up to 128 elements with values of their own (NS = 1): the weights take the place of the scores,
 // 224 columns of tensor memory, two blocks per SM that fill one another's gaps; a block is the plain chain of
 // scores, softmax, value products.  Wide shared rows (NS = 2): one block per SM, two score buffers, and the next tile's
-// scores issued around the value products of this one.  Where shared memory holds two tiles (rows up to 320) they go in
-// front of them; where it holds one (576: queries 147 KB, a tile 74 KB) the part of the row that is no value of this
-// block goes in front, and the rest, whose chunks the value products still need, behind.
+// scores issued beside the value products of this one.  Where shared memory holds two tiles (rows up to 320) they wait
+// for nothing; where it holds one (576: queries 147 KB, a tile 74 KB) the part of the row that is no value of this
+// block comes first, and the rest follows as the value products release its chunks.
 //
-// Order: warp 0 issues TMA, warp 1 the products, warps 2-5 are the softmax.  Every wait on an mbarrier is bounded: on a
-// timeout the block records status 2, frees its tensor memory and returns.
+// Order: warp 0 issues TMA, warp 1 the products (NS = 2: the scores, warp 6 the value products), warps 2-5 are the
+// softmax.  Every wait on an mbarrier is bounded: on a timeout the block records status 2, frees its tensor memory and
+// returns.
 #include "sm100.cuh"
 
 namespace {
@@ -31,7 +32,7 @@ namespace {
 using namespace sm100;
 
 constexpr int BM = 128, BN = 64;
-constexpr int THREADS = 192;
+template <int NS> constexpr int threads_of() { return NS == 1 ? 192 : 224; }
 constexpr int QCHUNK = BM * 128, CHUNK = BN * 128;    // bytes: 64 elements of every row
 constexpr int MAX_POS = 9;                            // chunks of a tile
 constexpr float LOG2E = 1.4426950408889634f;
@@ -102,7 +103,7 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, v
 
 // tiles[i] = {request row, first flat token, tokens (<= BM / group)}
 template <int NS>
-__global__ void __launch_bounds__(THREADS, NS == 1 ? 2 : 1)
+__global__ void __launch_bounds__(threads_of<NS>(), NS == 1 ? 2 : 1)
 attn_options_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kv,
                          const int* __restrict__ tiles, const int* __restrict__ positions,
                          const int* __restrict__ block_table, int bt_stride, int num_pages, int page_size, int num_heads,
@@ -118,9 +119,9 @@ attn_options_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     unsigned long long* s_empty = bars + 3;           // [NS]
     unsigned long long* p_full = bars + 5;
     unsigned long long* p_empty = bars + 6;           // value products done: weights may be rewritten, O is up to date
-    unsigned long long* full = bars + 7;              // [stages * places]
-    unsigned long long* empty = full + 2 * MAX_POS;
-    unsigned* tmem_slot = (unsigned*)(empty + 2 * MAX_POS);
+    unsigned long long* full = bars + 7;              // [stages][2]: the chunks only the scores read, the value chunks
+    unsigned long long* empty = bars + 11;
+    unsigned* tmem_slot = (unsigned*)(bars + 15);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int slice = blockIdx.x % sh.slices, kvh = blockIdx.x / sh.slices;
@@ -130,13 +131,15 @@ attn_options_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     const int kv_lo = first_visible(pos_first, opt);
     const int kt_lo = kv_lo / BN, num_kt = pos_last / BN + 1 - kt_lo;
     const int early = sh.places - sh.nv;              // places whose chunks only the scores read
+    // shared rows: the chunk of the row at place p
+    auto chunk_at = [&](int p) { return p >= early ? slice * sh.nv + p - early : p < slice * sh.nv ? p : p + sh.nv; };
 
     if (threadIdx.x == 0) {
         mbar_init(q_full, 1);
         for (int i = 0; i < 2; ++i) { mbar_init(&s_full[i], 1); mbar_init(&s_empty[i], 4); }
         mbar_init(p_full, 4);
         mbar_init(p_empty, 1);
-        for (int i = 0; i < sh.stages * sh.places; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
+        for (int i = 0; i < 2 * sh.stages; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
         mbar_fence_init();
     }
     if (warp == 1) tmem_alloc(tmem_slot, TMEM_COLS);
@@ -170,85 +173,92 @@ attn_options_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                         atomicCAS(status, 0, TI_ERR_BAD_PAGE);
                 }
             }
-            for (int p = 0; p < sh.places; ++p) {
-                unsigned long long* bar = &full[st * sh.places + p];
+            for (int part = early > 0 ? 0 : 1; part < 2; ++part) {
+                unsigned long long* bar = &full[st * 2 + part];
+                const int from = part == 0 ? 0 : early, to = part == 0 ? early : sh.places;
                 if (lane == 0) {
-                    ok = mbar_wait(&empty[st * sh.places + p], phase ^ 1);
-                    if (ok) mbar_expect_tx(bar, CHUNK);
+                    ok = mbar_wait(&empty[st * 2 + part], phase ^ 1);
+                    if (ok) mbar_expect_tx(bar, (to - from) * CHUNK);
                 }
                 ok = __shfl_sync(0xffffffffu, ok, 0);
                 if (!ok) break;
-                int c, y = row;
-                if (sh.shared) {                      // the row's chunks outside the slice, then the slice's
-                    c = p >= early ? slice * sh.nv + p - early : p < slice * sh.nv ? p : p + sh.nv;
-                } else {
-                    c = p < sh.chunks ? p : slice * sh.nv + p - sh.chunks;
-                    if (p >= sh.chunks && row != oob_row) y = row + to_v;
-                }
-                if (lane < BN / sh.run)
+                if (lane >= BN / sh.run) continue;
+                for (int p = from; p < to; ++p) {
+                    int c, y = row;
+                    if (sh.shared) {                  // the row's chunks outside the slice, then the slice's
+                        c = chunk_at(p);
+                    } else {
+                        c = p < sh.chunks ? p : slice * sh.nv + p - sh.chunks;
+                        if (p >= sh.chunks && row != oob_row) y = row + to_v;
+                    }
                     tma_load_2d(ring + (st * sh.places + p) * CHUNK + lane * sh.run * 128, &map_kv, bar, c * 64, y);
+                }
             }
         }
-    } else if (warp == 1) {
+    } else if (warp == 1 || warp == 6) {
+        // Scores and value products, by one thread (NS = 1: the next scores overwrite the weights, and products run in
+        // the order a thread issues them) or by two (NS = 2: the scores' 36 products of a tile of 576 take a thread
+        // longer to issue than to run).
         if (lane == 0) {
             const unsigned idesc_s = umma_idesc(BM, BN);
             const unsigned idesc_o = umma_idesc(BM, sh.nv * 64, /*b_mn_major=*/true);
-            // scores of tile j from the chunks at places [from, to)
-            auto scores = [&](int j, int from, int to) {
+            const unsigned long long dq = umma_desc(smem), dr = umma_desc(ring), dv_ = umma_desc(ring, CHUNK, 1024);
+            // scores of tile j from the chunks of one part; a last chunk of fewer than 64 elements is filled up with zeros
+            auto scores = [&](int j, int part) {
                 const int st = j % sh.stages, phase = (j / sh.stages) & 1;
-                for (int p = from; p < to && ok; ++p) {
-                    ok = mbar_wait(&full[st * sh.places + p], phase);
-                    if (!ok) break;
-                    tc_fence_after();
-                    const int c = !sh.shared ? p : p >= early ? slice * sh.nv + p - early : p < slice * sh.nv ? p : p + sh.nv;
-                    const int steps = min(4, (sh.dk - c * 64) / 16);
-                    const unsigned long long dq = umma_desc(smem + c * QCHUNK);
-                    const unsigned long long dk_ = umma_desc(ring + (st * sh.places + p) * CHUNK);
-                    for (int kk = 0; kk < steps; ++kk)
-                        umma_bf16(tmem_base + S_AT + (NS == 1 ? 0 : (j & 1) * BN), dq + (unsigned long long)(kk * 2),
-                                  dk_ + (unsigned long long)(kk * 2), idesc_s, p > 0 || kk > 0);
-                    if (p < early) umma_commit(&empty[st * sh.places + p]);
-                }
-            };
-            const int all = sh.shared ? sh.places : sh.chunks;
-            ok = mbar_wait(q_full, 0);
-            if (ok) {
+                const int from = part == 0 ? 0 : early, to = part == 0 ? early : sh.places;
+                if (!ok || from == to) return;
+                ok = mbar_wait(&full[st * 2 + part], phase);
+                if (!ok) return;
                 tc_fence_after();
-                scores(0, 0, all);
-                umma_commit(&s_full[0]);
-            }
-            for (int j = 0; j < num_kt && ok; ++j) {
-                const bool more = j + 1 < num_kt;
-                const int split_at = sh.stages == 2 ? all : early;        // what of the next scores goes in front
-                if (NS == 2 && more) {
-                    const int b = (j + 1) & 1;
-                    ok = mbar_wait(&s_empty[b], (((j + 1) >> 1) & 1) ^ 1);
-                    if (!ok) break;
-                    tc_fence_after();
-                    scores(j + 1, 0, split_at);
-                    if (split_at == all && ok) umma_commit(&s_full[b]);
+                const unsigned to_s = tmem_base + S_AT + (NS == 1 ? 0 : (j & 1) * BN);
+                unsigned long long b = dr + (unsigned long long)((st * sh.places + from) * (CHUNK >> 4));
+                for (int p = from; p < to; ++p, b += CHUNK >> 4) {
+                    const unsigned long long a = dq + (unsigned long long)((sh.shared ? chunk_at(p) : p) * (QCHUNK >> 4));
+                    umma_bf16(to_s, a, b, idesc_s, p > 0);
+#pragma unroll
+                    for (int kk = 1; kk < 4; ++kk) umma_bf16(to_s, a + kk * 2, b + kk * 2, idesc_s, 1);
                 }
+                if (part == 0) umma_commit(&empty[st * 2]);
+            };
+            auto all_scores = [&](int j) {
+                scores(j, 0);
+                if (sh.shared) scores(j, 1);
+                if (ok) umma_commit(&s_full[NS == 1 ? 0 : j & 1]);
+            };
+            auto value_products = [&](int j) {
                 const int st = j % sh.stages;
                 if (ok) ok = mbar_wait(p_full, j & 1);
-                for (int p = sh.shared ? sh.places : early; p < sh.places && ok; ++p)     // values of their own
-                    ok = mbar_wait(&full[st * sh.places + p], (j / sh.stages) & 1);
-                if (!ok) break;
+                if (ok) ok = mbar_wait(&full[st * 2 + 1], (j / sh.stages) & 1);
+                if (!ok) return;
                 tc_fence_after();
-                const unsigned char* vbuf = ring + (st * sh.places + early) * CHUNK;
+                const unsigned long long b = dv_ + (unsigned long long)((st * sh.places + early) * (CHUNK >> 4));
+#pragma unroll
                 for (int part = 2; part >= 0; --part)                                     // the smallest parts first
+#pragma unroll
                     for (int ks = 0; ks < BN / 16; ++ks)
-                        umma_bf16_tmem_a(tmem_base, tmem_base + P_AT + part * 32 + ks * 8,
-                                         umma_desc(vbuf + ks * 2048, CHUNK, 1024), idesc_o, j > 0 || part < 2 || ks > 0);
-                for (int p = early; p < sh.places; ++p) umma_commit(&empty[st * sh.places + p]);
+                        umma_bf16_tmem_a(tmem_base, tmem_base + P_AT + part * 32 + ks * 8, b + (unsigned long long)(ks * (2048 >> 4)),
+                                         idesc_o, j > 0 || part < 2 || ks > 0);
+                umma_commit(&empty[st * 2 + 1]);
                 umma_commit(p_empty);
-                if (more && NS == 1) {
-                    // the products run in the order of issue: these overwrite the weights when they have been read
-                    scores(j + 1, 0, all);
-                    umma_commit(&s_full[0]);
-                } else if (more && split_at < all) {
-                    scores(j + 1, split_at, all);
-                    umma_commit(&s_full[(j + 1) & 1]);
+            };
+            if (warp == 1) {
+                ok = mbar_wait(q_full, 0);
+                if (ok) tc_fence_after();
+                for (int j = 0; j < num_kt && ok; ++j) {
+                    if (NS == 2) {
+                        // value chunks are read by the value products too, which may still run: a part of the scores
+                        // waits for nothing but its own copies
+                        ok = mbar_wait(&s_empty[j & 1], ((j >> 1) & 1) ^ 1);
+                        if (ok) all_scores(j);
+                    } else {
+                        if (j == 0) all_scores(0);
+                        value_products(j);
+                        if (ok && j + 1 < num_kt) all_scores(j + 1);
+                    }
                 }
+            } else {
+                for (int j = 0; j < num_kt && ok; ++j) value_products(j);
             }
         }
     } else {
@@ -260,8 +270,10 @@ attn_options_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
         const int lo_row = live ? first_visible(pos_row, opt) : 0;
         const int lo_last = first_visible(pos_last, opt);
         const unsigned lane_addr = (unsigned)(quarter * 32) << 16;
-        const float scale = opt.scale * (opt.head_scale && live ? opt.head_scale[h] : 1.0f);
-        const float cap_arg = opt.softcap > 0.0f ? 2.0f * LOG2E / opt.softcap : 0.0f, cap_l2e = opt.softcap * LOG2E;
+        const float cap_l2e = opt.softcap * LOG2E;
+        // one factor per score: into the cap's exponent, or into log2 units
+        const float scale = opt.scale * (opt.head_scale && live ? opt.head_scale[h] : 1.0f) *
+                            (opt.softcap > 0.0f ? 2.0f * LOG2E / opt.softcap : LOG2E);
         float m_ref = -INFINITY, l_run = 0.0f;
         for (int j = 0; j < num_kt && ok; ++j) {
             const int b = NS == 1 ? 0 : j & 1;
@@ -281,10 +293,10 @@ attn_options_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             if (opt.softcap > 0.0f) {                 // cap tanh(v / cap) = cap (1 - 2 / (exp(2 v / cap) + 1))
 #pragma unroll
                 for (int i = 0; i < BN; ++i)
-                    v[i] = cap_l2e * fmaf(-2.0f, rcp_approx(ex2_approx(v[i] * scale * cap_arg) + 1.0f), 1.0f);
+                    v[i] = cap_l2e * fmaf(-2.0f, rcp_approx(ex2_approx(v[i] * scale) + 1.0f), 1.0f);
             } else {
 #pragma unroll
-                for (int i = 0; i < BN; ++i) v[i] *= scale * LOG2E;
+                for (int i = 0; i < BN; ++i) v[i] *= scale;
             }
             if (key_lo + BN - 1 > pos_first || key_lo < lo_last) {
 #pragma unroll
@@ -324,7 +336,7 @@ attn_options_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                 unsigned hi[16], mid[16], lo[16];
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
-                    const float p0 = exp2f(v[c * 32 + 2 * i] - m_use), p1 = exp2f(v[c * 32 + 2 * i + 1] - m_use);
+                    const float p0 = ex2_approx(v[c * 32 + 2 * i] - m_use), p1 = ex2_approx(v[c * 32 + 2 * i + 1] - m_use);
                     sum[0] += p0;
                     sum[1] += p1;
                     split3_pair(p0, p1, hi[i], mid[i], lo[i]);
@@ -385,7 +397,7 @@ attn_options_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
 }
 
 size_t smem_bytes(const Shape& sh) {
-    return 1024 + (size_t)sh.chunks * QCHUNK + (size_t)sh.stages * sh.places * CHUNK + (7 + 4 * MAX_POS) * 8 + 16;
+    return 1024 + (size_t)sh.chunks * QCHUNK + (size_t)sh.stages * sh.places * CHUNK + 16 * 8;
 }
 
 // The cut of the rows, or `places` = 0 where the kernel does not take them.
@@ -477,7 +489,7 @@ extern "C" int ti_attn_options_umma(const void* q, const int* tiles, int num_til
             if (e != cudaSuccess) return ti_fail("attn_options_umma: %s", cudaGetErrorString(e));                  \
             configured.mark();                                                                                    \
         }                                                                                                         \
-        attn_options_umma_kernel<NS><<<grid, THREADS, smem, s>>>(map_q, map_kv, tiles, positions, block_table,     \
+        attn_options_umma_kernel<NS><<<grid, threads_of<NS>(), smem, s>>>(map_q, map_kv, tiles, positions, block_table,     \
             bt_stride, num_pages, page_size, num_heads, num_kv_heads, sh, opt, (bf16*)out, status);               \
     }
     if (shared_rows) LAUNCH(2) else LAUNCH(1)

@@ -131,15 +131,33 @@ class Scheduler:
         planned: list[Scheduled] = []
         taken = [0] * len(self.cache.groups)
 
+        # what a request's next n tokens need, asked once per plan (``room`` and ``take`` both want it), against the
+        # free pages as they stand after the last preemption
+        needs: dict = {}
+        free = self.cache.free_pages()
+
+        def need_of(req: Request, n: int) -> list[int]:
+            got = needs.get((req.req_id, n))
+            if got is None:
+                got = needs[req.req_id, n] = self.cache.pages_needed(req.req_id, n)
+            return got
+
         def room(req: Request, n: int) -> bool:
-            need = self.cache.pages_needed(req.req_id, n)
-            free = self.cache.free_pages()
-            return all(k <= f - t for k, f, t in zip(need, free, taken))
+            for k, f, t in zip(need_of(req, n), free, taken):
+                if k > f - t:
+                    return False
+            return True
 
         def take(req: Request, n: int) -> None:
-            for g, k in enumerate(self.cache.pages_needed(req.req_id, n)):
+            for g, k in enumerate(need_of(req, n)):
                 taken[g] += k
             planned.append(Scheduled(req, req.computed, n, req.computed + n == req.num_tokens))
+
+        def preempt(req: Request) -> None:
+            nonlocal free
+            self._preempt(req)
+            needs.clear()
+            free = self.cache.free_pages()
 
         # 1. one token for every decoding request
         for req in list(self.running):
@@ -149,13 +167,14 @@ class Scheduler:
                 victim = self.running[-1]
                 if any(s.request is victim for s in planned):
                     break                         # only older, already planned ones are left
-                self._preempt(victim)
+                preempt(victim)
             if req.state == RUNNING and room(req, 1):
                 take(req, 1)
                 budget -= 1
+        taken_ids = {id(p.request) for p in planned}
         # 2. prompt portions of running requests, oldest first
         for req in self.running:
-            if req.remaining <= 1 or budget < 1 or any(s.request is req for s in planned):
+            if req.remaining <= 1 or budget < 1 or id(req) in taken_ids:
                 continue
             n = self._fit(req, min(req.remaining, budget, self.chunk or req.remaining), room)
             if n:

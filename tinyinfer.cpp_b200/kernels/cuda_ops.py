@@ -35,6 +35,7 @@ argmax(logits, out) / sample(...)            next token per row
 from __future__ import annotations
 
 import ctypes
+import functools
 from typing import Optional
 
 import torch
@@ -62,6 +63,13 @@ def _code(t: torch.Tensor, what: str) -> int:
 
 def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
     return None if t is None else t.data_ptr()
+
+
+def _remember(lib, *names: str) -> None:
+    """Answer a library's size queries (functions of whole numbers alone) from a table of earlier answers: a step
+    asks the same few hundreds of times, and a call through ctypes costs more than the launch it decides about."""
+    for name in names:
+        setattr(lib, name, functools.lru_cache(maxsize=4096)(getattr(lib, name)))
 
 
 def _need(cond: bool, msg: str) -> None:
@@ -186,6 +194,7 @@ class CudaOps(MixerOps, StateOps):
         # (``linear(..., may_pair=True)`` and the product after it) as one launch
         self.pair_few_rows = True
         self.fuse_gated_sums = True       # a gate on the way into the residual in the product's epilogue
+        self._cuts: dict = {}             # (m, n, k[, mode]) -> how a product's K is cut on this device
         self._pending_pair = None         # (a, w, out) of a product that waits for the next one
         self._ffn_counters = None
         self._pending = None              # a held-back ``out += a w^T`` (and the norm of ``out`` after it)
@@ -229,7 +238,7 @@ class CudaOps(MixerOps, StateOps):
                                          _i, _vp, _f, _vp]
         c.ti_scale_rows.argtypes = [_vp, _i, _i, _vp, _i, _i, _vp]
 
-    @property
+    @functools.cached_property
     def bf16(self):
         """The tensor-core kernels of the bfloat16 path, built and loaded when first needed."""
         if self._bf16 is None:
@@ -288,6 +297,11 @@ class CudaOps(MixerOps, StateOps):
             b.ti_attn_prefill_tc2_supported.argtypes = [_i, _i, _i, _i]
             b.ti_attn_prefill_tc2.argtypes = b.ti_attn_prefill_tc.argtypes
             self._tile_rows = (int(b.ti_attn_prefill_tile_rows()), int(b.ti_attn_prefill_tc_tile_rows()))
+            if not hasattr(b.ti_gemm_skinny_supported, "cache_info"):        # (the library is loaded once per process)
+                _remember(b, "ti_gemm_skinny_supported", "ti_gemm_tcgen05_few_supported", "ti_gemm_tcgen05_supported",
+                          "ti_ffn_decode_supported", "ti_attn_out_ffn_decode_supported",
+                          "ti_attn_decode_supported", "ti_attn_decode_blocks_per_sm", "ti_attn_decode_qkv_supported",
+                          "ti_attn_prefill_supported", "ti_attn_prefill_tc_supported", "ti_attn_prefill_tc2_supported")
             self._bf16 = b
         return self._bf16
 
@@ -386,7 +400,7 @@ class CudaOps(MixerOps, StateOps):
             self._ok(fn(a.data_ptr(), w.data_ptr(), _ptr(c), _ptr(out_act), m, n, k, a.stride(0), w.stride(0),
                         ldc, ld_act, mode, self.status.data_ptr(), self._stream()), self.bf16)
             return
-        runs = int(self.bf16.ti_gemm_tcgen05_splits(m, n, k, mode)) if self.split_k_portions else 1
+        runs = self._runs_of(m, n, k, mode) if self.split_k_portions else 1
         ws = torch.empty(runs * m * n, dtype=torch.float32, device=a.device) if runs > 1 else None
         leave = bool(runs > 1 and may_defer and self.norm_adds_runs and c is not None and c.is_contiguous())
         self._ok(fn(a.data_ptr(), w.data_ptr(), _ptr(c), _ptr(out_act), m, n, k, a.stride(0), w.stride(0),
@@ -395,6 +409,28 @@ class CudaOps(MixerOps, StateOps):
             self._pending_runs = (ws, runs, c, mode == 1)
         elif runs > 1:
             self.launches += 1            # the launch that adds the runs
+
+    def _runs_of(self, m: int, n: int, k: int, mode: int) -> int:
+        """In how many runs the tcgen05 product of many rows cuts K."""
+        runs = self._cuts.get((m, n, k, mode))
+        if runs is None:
+            if len(self._cuts) >= 4096:
+                self._cuts.clear()
+            runs = self._cuts[m, n, k, mode] = int(self.bf16.ti_gemm_tcgen05_splits(m, n, k, mode))
+        return runs
+
+    @staticmethod
+    def _kept(step, tag: str, shape: tuple, dtype, device):
+        """A buffer that every layer of a forward pass uses in turn, on the pass's one stream (``step.scratch`` is
+        emptied at a pass's ends); a fresh one where the step keeps nothing."""
+        scratch = getattr(step, "scratch", None)
+        if scratch is None:
+            return torch.empty(shape, dtype=dtype, device=device)
+        key = (tag, shape, dtype)
+        t = scratch.get(key)
+        if t is None:
+            t = scratch[key] = torch.empty(shape, dtype=dtype, device=device)
+        return t
 
     def _few_tc_scratch(self, a, w, mode):
         """Workspace (or None) and tickets of the split-K tcgen05 product for few rows, or None if it does
@@ -405,11 +441,17 @@ class CudaOps(MixerOps, StateOps):
                 or a.data_ptr() % 16 or w.data_ptr() % 16
                 or not self.bf16.ti_gemm_tcgen05_few_supported(m, n, k, a.stride(0), w.stride(0), mode)):
             return None
-        ws_floats, tickets = ctypes.c_longlong(0), ctypes.c_int(0)
-        self.bf16.ti_gemm_tcgen05_few_scratch(m, n, k, ctypes.byref(ws_floats), ctypes.byref(tickets))
-        if self._few_tickets is None or self._few_tickets.numel() < tickets.value:
-            self._few_tickets = self._grown(self._few_tickets, tickets.value, a.device)
-        ws = torch.empty(ws_floats.value, dtype=torch.float32, device=a.device) if ws_floats.value else None
+        cut = self._cuts.get((m, n, k))
+        if cut is None:
+            if len(self._cuts) >= 4096:
+                self._cuts.clear()
+            ws_floats, tickets = ctypes.c_longlong(0), ctypes.c_int(0)
+            self.bf16.ti_gemm_tcgen05_few_scratch(m, n, k, ctypes.byref(ws_floats), ctypes.byref(tickets))
+            cut = self._cuts[m, n, k] = (ws_floats.value, tickets.value)
+        floats, tickets = cut
+        if self._few_tickets is None or self._few_tickets.numel() < tickets:
+            self._few_tickets = self._grown(self._few_tickets, tickets, a.device)
+        ws = torch.empty(floats, dtype=torch.float32, device=a.device) if floats else None
         return ws, self._few_tickets
 
     def _few_tc(self, a, w, c, out_act, mode) -> bool:
@@ -622,7 +664,7 @@ class CudaOps(MixerOps, StateOps):
                 if self._tc_gemm(m, n) is self.bf16.ti_gemm_tcgen05_2sm:
                     self._ok(self.bf16.ti_gemm_tcgen05_2sm_gated(*sizes, *args, status, stream), self.bf16)
                     return
-                runs = int(self.bf16.ti_gemm_tcgen05_splits(m, n, k, 1)) if self.split_k_portions else 1
+                runs = self._runs_of(m, n, k, 1) if self.split_k_portions else 1
                 ws = torch.empty(runs * m * n, dtype=torch.float32, device=a.device) if runs > 1 else None
                 self._ok(self.bf16.ti_gemm_tcgen05_gated(*sizes, _ptr(ws), *args, status, stream), self.bf16)
                 if runs > 1:
@@ -914,7 +956,7 @@ class CudaOps(MixerOps, StateOps):
                  and bt.dtype == torch.int32 and bt.stride(1) == 1
                  and self.bf16.ti_attn_decode_qkv_supported(head_dim, group, cache.page_size))
         if not fused:
-            q = torch.empty((t, num_heads * head_dim), dtype=h.dtype, device=h.device)
+            q = self._kept(step, "queries", (t, num_heads * head_dim), h.dtype, h.device)
             self.qkv_rope_store(h, w_qkv, q_weight, k_weight, eps, rotation, step, cache, q,
                                 num_heads, num_kv_heads, head_dim)
             self.paged_attention(q, step, cache, out, num_heads, num_kv_heads, head_dim, window, scale)
@@ -976,13 +1018,12 @@ class CudaOps(MixerOps, StateOps):
         # dependents only when its own wait has returned; flash-decoding (bound by HBM) then runs
         # beside it on what that wait covered and waits for the prompt kernel at its end.
         beside = decode and prompt_tc and self.attention_side_by_side
+        splits = (self.decode_splits(n_dec, num_kv_heads, step.max_position or step.max_ctx_len, head_dim)
+                  if decode else 0)
 
         def run_decode():
-            splits = self.decode_splits(n_dec, num_kv_heads, step.max_position or step.max_ctx_len, head_dim)
-            part_o = torch.empty((n_dec, num_heads, splits, head_dim), dtype=torch.float32,
-                                 device=q.device)
-            part_ml = torch.empty((n_dec, num_heads, splits, 2), dtype=torch.float32,
-                                  device=q.device)
+            part_o = self._kept(step, "decode_o", (n_dec, num_heads, splits, head_dim), torch.float32, q.device)
+            part_ml = self._kept(step, "decode_ml", (n_dec, num_heads, splits, 2), torch.float32, q.device)
             if self._counters is None or self._counters.numel() < n_dec * num_kv_heads:
                 # zero once; every launch leaves its counters at zero again
                 self._counters = self._grown(self._counters, n_dec * num_kv_heads, q.device)
@@ -1008,8 +1049,7 @@ class CudaOps(MixerOps, StateOps):
                                                                         num_kv_heads))
                 decode_blocks = 0
                 if beside:
-                    decode_blocks = n_dec * num_kv_heads * self.decode_splits(
-                        n_dec, num_kv_heads, step.max_position or step.max_ctx_len, head_dim)
+                    decode_blocks = n_dec * num_kv_heads * splits
                 two, runs = choose_prompt_attention(
                     n_tiles, num_heads, self.num_sms, reach=getattr(step, "portion_reach", 1), window=win,
                     two_heads_ok=pairs_ok, pairs_from=self.tc_attention_pairs_from,
@@ -1017,10 +1057,8 @@ class CudaOps(MixerOps, StateOps):
                     decode_blocks_per_sm=int(self.bf16.ti_attn_decode_blocks_per_sm(head_dim)))
                 part_o = part_ml = None
                 if runs > 1:
-                    part_o = torch.empty((n_tiles, num_heads, runs, big, head_dim), dtype=torch.float32,
-                                         device=q.device)
-                    part_ml = torch.empty((n_tiles, num_heads, runs, big, 2), dtype=torch.float32,
-                                          device=q.device)
+                    part_o = self._kept(step, "prompt_o", (n_tiles, num_heads, runs, big, head_dim), torch.float32, q.device)
+                    part_ml = self._kept(step, "prompt_ml", (n_tiles, num_heads, runs, big, 2), torch.float32, q.device)
                 kernel = self.bf16.ti_attn_prefill_tc2 if two else self.bf16.ti_attn_prefill_tc
                 self._ok(kernel(
                     q.data_ptr(), q.shape[0], tiles.data_ptr(), n_tiles,

@@ -69,7 +69,10 @@ class Attention(Part):
 
     def forward(self, ops, h, residual, step, cache):
         t, dev, act = h.shape[0], h.device, h.dtype
-        out = torch.empty((t, self.nq), dtype=act, device=dev)
+        # one output buffer for all layers of a pass: the product behind has read it before the next layer writes
+        out = step.scratch.get(("attention_out", t, self.nq, act))
+        if out is None:
+            out = step.scratch["attention_out", t, self.nq, act] = torch.empty((t, self.nq), dtype=act, device=dev)
         ops.qkv_attention(h, self.w_qkv, self.q_norm, self.k_norm, self.eps, self.position.rotation(dev),
                           step, cache, out, self.num_heads, self.num_kv_heads, self.head_dim,
                           self.window, self.scale)

@@ -134,6 +134,7 @@ class CausalLM:
             cache = cache_views[(entry.cache_slot, entry.writes_cache)]
             self.blocks[entry.layer].forward(ops, x, step, cache)
         ops.flush()                        # nothing a part asked for may still be held back
+        step.scratch.clear()               # ... and nothing of the pass is kept behind it
         if step.num_logit_rows == 0:
             return torch.empty((0, self.plan.vocab_size), dtype=torch.float32, device=x.device)
         h = self.final_norm.forward_rows(ops, x, step.logit_rows, step.act_dtype)
