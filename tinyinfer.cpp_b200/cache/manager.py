@@ -117,6 +117,7 @@ class CacheManager:
         self._slot_group: dict[int, tuple[int, int]] = {}      # cache slot -> (group, index in group)
         self._state_specs: dict[int, FixedStateSpec] = {}
         self._state_storage: dict[int, torch.Tensor] = {}
+        self._slot_views: dict[int, list] = {}       # state slot -> its states, a list per type
         by_spec: dict[PagedKVSpec, int] = {}
         # a cache slot that keeps several things: every leaf becomes a slot of its own behind the
         # model's, and the slot's view gathers them under their names
@@ -174,8 +175,15 @@ class CacheManager:
         self._touch(req)
         for g in self.groups:
             g.tables[req] = []
-        for t in self._state_storage.values():
-            t[slot].zero_()
+        # the slot's states of one type in one call (a model of six such layers has eleven: a launch each before)
+        views = self._slot_views.get(slot)
+        if views is None:
+            by_type: dict = {}
+            for t in self._state_storage.values():
+                by_type.setdefault(t.dtype, []).append(t[slot])
+            views = self._slot_views[slot] = list(by_type.values())
+        for same in views:
+            torch._foreach_zero_(same)
 
     def _touch(self, req: Hashable) -> None:
         self._versions += 1

@@ -82,12 +82,14 @@ __device__ __forceinline__ float mixed(const float* row, const float* first, int
 template <typename TQ, typename TC>
 __global__ void __launch_bounds__(256)
 qkv_turn_store_kernel(const float* proj, int stride, const RowNorm norm, const ValueMix mix,
-                      const float* __restrict__ inv_freq, int rot, int halves, float mag,
-                      const float* __restrict__ v_inv_freq, int v_rot, int v_halves,
-                      const int* __restrict__ positions, const int* __restrict__ req_of_tok,
-                      const int* __restrict__ block_table, int bt_stride, TC* __restrict__ pages, int num_pages,
+                      const float* inv_freq, int rot, int halves, float mag,
+                      const float* v_inv_freq, int v_rot, int v_halves,
+                      const int* positions, const int* req_of_tok,
+                      const int* block_table, int bt_stride, TC* __restrict__ pages, int num_pages,
                       int page_size, int write_kv, int num_heads, int num_kv_heads, int dk, int dv,
                       TQ* __restrict__ q_out, int* __restrict__ status) {
+    pdl_launch();
+    pdl_wait();
     __shared__ float scratch[32];
     extern __shared__ float2 turn_table[];             // rot/2 entries for queries and keys, then v_rot/2 for values
     const int t = blockIdx.x;
@@ -158,8 +160,10 @@ qkv_turn_store_kernel(const float* proj, int stride, const RowNorm norm, const V
 // block per token, a thread reads and writes both elements of a pair, so the rows may be turned in place
 template <typename T>
 __global__ void __launch_bounds__(256)
-turn_rows_kernel(const T* x, const int* __restrict__ positions, const float* __restrict__ inv_freq, int rot,
+turn_rows_kernel(const T* x, const int* positions, const float* inv_freq, int rot,
                  int halves, float sign, const float* gate, int gate_stride, int num_heads, int n, T* out) {
+    pdl_launch();
+    pdl_wait();
     extern __shared__ float2 turn_table[];
     const int t = blockIdx.x;
     fill_turn_table(turn_table, rot >> 1, sign * (float)positions[t], inv_freq, 1.0f);
@@ -189,13 +193,15 @@ turn_rows_kernel(const T* x, const int* __restrict__ positions, const float* __r
 
 template <typename TQ, typename TC>
 __global__ void __launch_bounds__(256)
-qk_rownorm_rope_store_kernel(const float* proj, int stride, const float* __restrict__ q_weight,
-                             const float* __restrict__ k_weight, float eps,
-                             const float* __restrict__ inv_freq, int rot,
-                             const int* __restrict__ positions, const int* __restrict__ req_of_tok,
-                             const int* __restrict__ block_table, int bt_stride, TC* __restrict__ pages,
+qk_rownorm_rope_store_kernel(const float* proj, int stride, const float* q_weight,
+                             const float* k_weight, float eps,
+                             const float* inv_freq, int rot,
+                             const int* positions, const int* req_of_tok,
+                             const int* block_table, int bt_stride, TC* __restrict__ pages,
                              int num_pages, int page_size, int write_kv, int num_heads, int num_kv_heads,
                              int dk, int dv, TQ* __restrict__ q_out, int* __restrict__ status) {
+    pdl_launch();
+    pdl_wait();
     __shared__ float scratch[32];
     const int t = blockIdx.x;
     const int nq = num_heads * dk, nk = num_kv_heads * dk, nv = num_kv_heads * dv;
@@ -262,7 +268,9 @@ qk_rownorm_rope_store_kernel(const float* proj, int stride, const float* __restr
 // product (a latent that shares its product with other columns)
 template <typename TO>
 __global__ void __launch_bounds__(256)
-slice_rmsnorm_kernel(const float* x, int stride, int n, const float* __restrict__ w, float eps, TO* __restrict__ out) {
+slice_rmsnorm_kernel(const float* x, int stride, int n, const float* w, float eps, TO* __restrict__ out) {
+    pdl_launch();
+    pdl_wait();
     __shared__ float scratch[32];
     const float* row = x + (size_t)blockIdx.x * stride;
     float ss = 0.0f;
@@ -275,11 +283,13 @@ slice_rmsnorm_kernel(const float* x, int stride, int n, const float* __restrict_
 template <typename TQ, typename TC>
 __global__ void __launch_bounds__(256)
 latent_prepare_kernel(const float* qproj, int q_stride, const float* proj, int stride,
-                      const float* __restrict__ latent_weight, float eps,
-                      const float* __restrict__ inv_freq, float mag, const int* __restrict__ positions,
-                      const int* __restrict__ req_of_tok, const int* __restrict__ block_table, int bt_stride,
+                      const float* latent_weight, float eps,
+                      const float* inv_freq, float mag, const int* positions,
+                      const int* req_of_tok, const int* block_table, int bt_stride,
                       TC* __restrict__ pages, int num_pages, int page_size, int num_heads, int dk, int dr,
                       int rank, TQ* __restrict__ q_plain, TQ* __restrict__ q_full, int* __restrict__ status) {
+    pdl_launch();
+    pdl_wait();
     __shared__ float scratch[32];
     const int t = blockIdx.x;
     const int qh = dk + dr, nq = num_heads * qh, row_len = rank + dr;
@@ -342,8 +352,10 @@ template <> __device__ __forceinline__ void load4<float>(const float* p, bool wh
 
 template <typename TI, typename TW, typename TO>
 __global__ void __launch_bounds__(HP_WARPS * 32)
-head_project_kernel(const TI* in, int in_stride_t, int in_stride_h, const TW* __restrict__ w, int n_in,
+head_project_kernel(const TI* in, int in_stride_t, int in_stride_h, const TW* w, int n_in,
                     int n_out, TO* out, int out_stride_t, int out_stride_h, int num_tokens, int vec_ok) {
+    pdl_launch();
+    pdl_wait();
     extern __shared__ __align__(16) float xs[];      // [n_in][HP_TOKENS]; afterwards the warps' partial sums
     const int t0 = blockIdx.x * HP_TOKENS, h = blockIdx.y;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -416,8 +428,10 @@ head_project_kernel(const TI* in, int in_stride_t, int in_stride_h, const TW* __
 // all of k in one thread (no meeting of partial sums).
 template <typename TI, typename TW, typename TO>
 __global__ void __launch_bounds__(128)
-head_project_rows_kernel(const TI* in, int in_stride_t, int in_stride_h, const TW* __restrict__ w, int n_in,
+head_project_rows_kernel(const TI* in, int in_stride_t, int in_stride_h, const TW* w, int n_in,
                          int n_out, TO* out, int out_stride_t, int out_stride_h, int num_tokens) {
+    pdl_launch();
+    pdl_wait();
     extern __shared__ __align__(16) float xs[];      // [n_in][HP_TOKENS]
     const int t0 = blockIdx.x * HP_TOKENS, h = blockIdx.y;
     const int n = blockIdx.z * 128 + threadIdx.x;
@@ -553,13 +567,15 @@ attention_options_kernel(const TQ* q, const int* __restrict__ rows, const int* _
 // A warp takes a head; the values are copied by all.
 template <typename TQ, typename TC>
 __global__ void __launch_bounds__(256)
-qk_headnorm_rope_store_kernel(const float* proj, int stride, const float* __restrict__ q_weight,
-                              const float* __restrict__ k_weight, float eps,
-                              const float* __restrict__ inv_freq, int rot,
-                              const int* __restrict__ positions, const int* __restrict__ req_of_tok,
-                              const int* __restrict__ block_table, int bt_stride, TC* __restrict__ pages,
+qk_headnorm_rope_store_kernel(const float* proj, int stride, const float* q_weight,
+                              const float* k_weight, float eps,
+                              const float* inv_freq, int rot,
+                              const int* positions, const int* req_of_tok,
+                              const int* block_table, int bt_stride, TC* __restrict__ pages,
                               int num_pages, int page_size, int write_kv, int num_heads, int num_kv_heads,
                               int dk, int dv, TQ* __restrict__ q_out, int* __restrict__ status) {
+    pdl_launch();
+    pdl_wait();
     const int t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nq = num_heads * dk, nk = num_kv_heads * dk, nv = num_kv_heads * dv;
     const float* row = proj + (size_t)t * stride;
@@ -630,8 +646,8 @@ extern "C" int ti_qk_rownorm_rope_store(const float* proj, int stride, const flo
     TI_REQUIRE(rot == 0 || inv_freq != nullptr, "qk_rownorm_rope_store: a rotation needs its frequencies");
     cudaStream_t s = (cudaStream_t)stream;
 #define CALL(TQ, TC)                                                                              \
-    (per_head ? qk_headnorm_rope_store_kernel<TQ, TC> : qk_rownorm_rope_store_kernel<TQ, TC>)<<<num_tokens, 256, 0, s>>>( \
-        proj, stride, q_weight, k_weight, eps, inv_freq, rot, positions, req_of_tok, block_table,   \
+    ti_launch_pdl((per_head ? qk_headnorm_rope_store_kernel<TQ, TC> : qk_rownorm_rope_store_kernel<TQ, TC>),          \
+        dim3(num_tokens), dim3(256), 0, s, proj, stride, q_weight, k_weight, eps, inv_freq, rot, positions, req_of_tok, block_table,   \
         bt_stride, (TC*)pages, num_pages, page_size, write_kv, num_heads, num_kv_heads, dk, dv,      \
         (TQ*)q_out, status)
     TI_DISPATCH_QC(q_dtype, cache_dtype, CALL)
@@ -643,8 +659,8 @@ extern "C" int ti_slice_rmsnorm(const float* x, int stride, int num_rows, int n,
                                 void* out, int out_dtype, void* stream) {
     if (num_rows == 0 || n == 0) return 0;
     cudaStream_t s = (cudaStream_t)stream;
-    if (out_dtype == TI_BF16) slice_rmsnorm_kernel<bf16><<<num_rows, 256, 0, s>>>(x, stride, n, weight, eps, (bf16*)out);
-    else if (out_dtype == TI_F32) slice_rmsnorm_kernel<float><<<num_rows, 256, 0, s>>>(x, stride, n, weight, eps, (float*)out);
+    if (out_dtype == TI_BF16) ti_launch_pdl((slice_rmsnorm_kernel<bf16>), dim3(num_rows), dim3(256), 0, s, x, stride, n, weight, eps, (bf16*)out);
+    else if (out_dtype == TI_F32) ti_launch_pdl((slice_rmsnorm_kernel<float>), dim3(num_rows), dim3(256), 0, s, x, stride, n, weight, eps, (float*)out);
     else return ti_fail("slice_rmsnorm: output dtype code %d", out_dtype);
     return ti_check_launch("slice_rmsnorm");
 }
@@ -662,7 +678,7 @@ extern "C" int ti_latent_prepare(const float* qproj, int q_stride, const float* 
     TI_REQUIRE(dr == 0 || inv_freq != nullptr, "latent_prepare: a rotation needs its frequencies");
     cudaStream_t s = (cudaStream_t)stream;
 #define CALL(TQ, TC)                                                                              \
-    latent_prepare_kernel<TQ, TC><<<num_tokens, 256, 0, s>>>(                                      \
+    ti_launch_pdl((latent_prepare_kernel<TQ, TC>), dim3(num_tokens), dim3(256), 0, s, \
         qproj, q_stride, proj, stride, latent_weight, eps, inv_freq, mag, positions, req_of_tok, block_table, bt_stride,  \
         (TC*)pages, num_pages, page_size, num_heads, dk, dr, rank, (TQ*)q_plain, (TQ*)q_full, status)
     TI_DISPATCH_QC(q_dtype, cache_dtype, CALL)
@@ -691,7 +707,7 @@ extern "C" int ti_qkv_turn_store(const float* proj, int stride, int row_norm, fl
     const ValueMix mix{mix_first, mix_stride, mix_share};
     TI_REQUIRE(turn_smem <= 47 * 1024, "qkv_turn_store: rotated widths %d and %d", rot, v_rot);
 #define CALL(TQ, TC)                                                                              \
-    qkv_turn_store_kernel<TQ, TC><<<num_tokens, 256, turn_smem, s>>>(                              \
+    ti_launch_pdl((qkv_turn_store_kernel<TQ, TC>), dim3(num_tokens), dim3(256), turn_smem, s, \
         proj, stride, norm, mix, inv_freq, rot, halves, mag, v_inv_freq, v_rot, v_halves, positions, req_of_tok, \
         block_table, bt_stride, (TC*)pages, num_pages, page_size, write_kv, num_heads, num_kv_heads, dk, dv, \
         (TQ*)q_out, status)
@@ -710,10 +726,10 @@ extern "C" int ti_turn_rows(const void* x, int dtype, const int* positions, cons
     TI_REQUIRE(smem <= 48 * 1024, "turn_rows: a rotated width of %d", rot);
     cudaStream_t s = (cudaStream_t)stream;
     if (dtype == TI_BF16)
-        turn_rows_kernel<bf16><<<num_tokens, 256, smem, s>>>((const bf16*)x, positions, inv_freq, rot, halves, sign, gate,
+        ti_launch_pdl((turn_rows_kernel<bf16>), dim3(num_tokens), dim3(256), smem, s, (const bf16*)x, positions, inv_freq, rot, halves, sign, gate,
                                                             gate_stride, num_heads, n, (bf16*)out);
     else if (dtype == TI_F32)
-        turn_rows_kernel<float><<<num_tokens, 256, smem, s>>>((const float*)x, positions, inv_freq, rot, halves, sign,
+        ti_launch_pdl((turn_rows_kernel<float>), dim3(num_tokens), dim3(256), smem, s, (const float*)x, positions, inv_freq, rot, halves, sign,
                                                              gate, gate_stride, num_heads, n, (float*)out);
     else return ti_fail("turn_rows: dtype code %d", dtype);
     return ti_check_launch("turn_rows");
@@ -739,11 +755,11 @@ extern "C" int ti_head_project(const void* in, int in_dtype, int in_stride_t, in
     const bool few = in_dtype != TI_F32 && (long long)grid.x * grid.y * grid.z <= 512;
 #define CALL(TI_, TW_)                                                                            \
     if (few)                                                                                      \
-        head_project_kernel<TI_, TW_, TI_><<<grid, HP_WARPS * 32, smem, s>>>(                      \
+        ti_launch_pdl((head_project_kernel<TI_, TW_, TI_>), dim3(grid), dim3(HP_WARPS * 32), smem, s, \
             (const TI_*)in, in_stride_t, in_stride_h, (const TW_*)w, n_in, n_out, (TI_*)out,        \
             out_stride_t, out_stride_h, num_tokens, vec_ok);                                       \
     else                                                                                          \
-        head_project_rows_kernel<TI_, TW_, TI_><<<grid, 128, smem, s>>>(                           \
+        ti_launch_pdl((head_project_rows_kernel<TI_, TW_, TI_>), dim3(grid), dim3(128), smem, s, \
             (const TI_*)in, in_stride_t, in_stride_h, (const TW_*)w, n_in, n_out, (TI_*)out,        \
             out_stride_t, out_stride_h, num_tokens)
     if (in_dtype == TI_F32 && w_dtype == TI_F32) { CALL(float, float); }

@@ -115,6 +115,7 @@ attn_options_tc_kernel(const bf16* q, const int* __restrict__ tiles, const int* 
     // KS (at most 16 live rows, decoding): every warp has the same 16 rows and a quarter of a tile's keys
     constexpr int NJ = KS ? BN / 32 : BN / 8;            // 8-key columns of a tile that a warp multiplies
     extern __shared__ __align__(16) unsigned char smem[];
+    pdl_launch();
     const int k_row = dk * 2 + 16;                       // bytes of a staged query or key row
     const int stage_bytes = BN * k_row + (opt.shared_rows ? 0 : BN * V_ROW);
     unsigned char* q_s = smem;
@@ -164,6 +165,7 @@ attn_options_tc_kernel(const bf16* q, const int* __restrict__ tiles, const int* 
     const int warp_pos_lo = pos_first + warp_tok_lo, warp_pos_hi = pos_first + warp_tok_hi;
     const int warp_lo_first = first_visible(warp_pos_lo, opt), warp_lo_last = first_visible(warp_pos_hi, opt);
 
+    pdl_wait();                                          // queries, keys, values and gates come from the kernels before
     // queries into shared memory (part of the first commit group)
     const int chunks = dk / 8;
     for (int c = threadIdx.x; c < BM * chunks; c += WARPS * 32) {
@@ -412,8 +414,10 @@ attn_options_tc_kernel(const bf16* q, const int* __restrict__ tiles, const int* 
 // and a thread has several loads in flight
 __global__ void __launch_bounds__(128)
 attn_options_merge_kernel(const float* part_o, const float* part_ml, int nsplit, int num_heads, int dv,
-                          const float* __restrict__ sink, const float* gate, int gate_stride, int gate_per_head,
+                          const float* sink, const float* gate, int gate_stride, int gate_per_head,
                           bf16* __restrict__ out) {
+    pdl_launch();
+    pdl_wait();
     __shared__ float f_s[64];
     __shared__ float inv_s;
     const int item = blockIdx.x, t = item / num_heads, h = item % num_heads;
@@ -453,8 +457,10 @@ constexpr int HPK = 64;          // rows of W[h] a stage holds
 constexpr int HP_WROW = 128 * 2 + 16;
 
 __global__ void __launch_bounds__(WARPS * 32)
-head_project_tc_kernel(const bf16* x, int x_stride_t, int x_stride_h, const bf16* __restrict__ w, int n_in, int n_out,
+head_project_tc_kernel(const bf16* x, int x_stride_t, int x_stride_h, const bf16* w, int n_in, int n_out,
                        bf16* out, int out_stride_t, int out_stride_h, int num_tokens) {
+    pdl_launch();
+    pdl_wait();
     extern __shared__ __align__(16) unsigned char smem[];
     const int x_row = n_in * 2 + 16;
     unsigned char* xs = smem;
@@ -559,8 +565,7 @@ extern "C" int ti_head_project_tc(const void* x, int x_stride_t, int x_stride_h,
         configured.mark();
     }
     dim3 grid((num_tokens + BM - 1) / BM, num_heads, (n_out + 127) / 128);
-    head_project_tc_kernel<<<grid, WARPS * 32, smem, (cudaStream_t)stream>>>(
-        (const bf16*)x, x_stride_t, x_stride_h, (const bf16*)w, n_in, n_out, (bf16*)out, out_stride_t, out_stride_h,
+    ti_launch_pdl((head_project_tc_kernel), dim3(grid), dim3(WARPS * 32), smem, (cudaStream_t)stream, (const bf16*)x, x_stride_t, x_stride_h, (const bf16*)w, n_in, n_out, (bf16*)out, out_stride_t, out_stride_h,
         num_tokens);
     return ti_check_launch("head_project_tc");
 }
@@ -618,7 +623,7 @@ extern "C" int ti_attn_options_tc(const void* q, const int* tiles, int num_tiles
             configured.mark();                                                                            \
             allowed = 227 * 1024;                                                                         \
         }                                                                                                 \
-        attn_options_tc_kernel<DVS, MODE><<<grid, WARPS * 32, smem, s>>>(                                        \
+        ti_launch_pdl((attn_options_tc_kernel<DVS, MODE>), grid, dim3(WARPS * 32), smem, s,                       \
             (const bf16*)q, tiles, positions, block_table, bt_stride, (const bf16*)pages, num_pages,       \
             page_size, num_heads, num_kv_heads, dk, dv, gp, head_blocks, nsplit, opt, (bf16*)out, part_o,   \
             part_ml, status);                                                                             \
@@ -634,7 +639,7 @@ extern "C" int ti_attn_options_tc(const void* q, const int* tiles, int num_tiles
     if (int rc = ti_check_launch("attn_options_tc")) return rc;
     if (nsplit > 1) {
         const int items = num_tokens * num_heads;
-        attn_options_merge_kernel<<<dim3(items, (dv + 127) / 128), 128, 0, s>>>(part_o, part_ml, nsplit, num_heads, dv, sink, gate, gate_stride,
+        ti_launch_pdl((attn_options_merge_kernel), dim3(dim3(items, (dv + 127) / 128)), dim3(128), 0, s, part_o, part_ml, nsplit, num_heads, dv, sink, gate, gate_stride,
                                                        gate_per_head, (bf16*)out);
         return ti_check_launch("attn_options_merge");
     }

@@ -147,6 +147,7 @@ attn_options_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     __syncthreads();
     tc_fence_after();
     const unsigned tmem_base = *tmem_slot;
+    pdl_wait();        // queries, keys, values and gates come from the kernels before (the next is not released early)
 
     bool ok = true;
     if (warp == 0) {
@@ -489,7 +490,7 @@ extern "C" int ti_attn_options_umma(const void* q, const int* tiles, int num_til
             if (e != cudaSuccess) return ti_fail("attn_options_umma: %s", cudaGetErrorString(e));                  \
             configured.mark();                                                                                    \
         }                                                                                                         \
-        attn_options_umma_kernel<NS><<<grid, threads_of<NS>(), smem, s>>>(map_q, map_kv, tiles, positions, block_table,     \
+        ti_launch_pdl(attn_options_umma_kernel<NS>, grid, dim3(threads_of<NS>()), smem, s, map_q, map_kv, tiles, positions, block_table,     \
             bt_stride, num_pages, page_size, num_heads, num_kv_heads, sh, opt, (bf16*)out, status);               \
     }
     if (shared_rows) LAUNCH(2) else LAUNCH(1)

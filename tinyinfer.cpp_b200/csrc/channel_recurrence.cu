@@ -23,8 +23,10 @@ constexpr int LD_TOKENS = 16, LD_RANK = 32;
 
 template <typename TW>
 __global__ void __launch_bounds__(128)
-low_rank_decay_kernel(const float* low, int low_stride, int rank, const TW* __restrict__ a2,
-                      const float* __restrict__ bias, float inv_tau, int rows, int n, float* __restrict__ out) {
+low_rank_decay_kernel(const float* low, int low_stride, int rank, const TW* a2,
+                      const float* bias, float inv_tau, int rows, int n, float* __restrict__ out) {
+    pdl_launch();
+    pdl_wait();
     __shared__ float ls[LD_RANK][LD_TOKENS];
     const int t0 = blockIdx.y * LD_TOKENS, nt = min(LD_TOKENS, rows - t0);
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -230,7 +232,9 @@ template <> __device__ __forceinline__ void load_weights<float, 4>(const float* 
 // w: [parts][2 per][per], the rows of zr first.  A part's width must be a multiple of 4.
 template <typename TW, typename TO, int NR>
 __global__ void __launch_bounds__(256)
-gated_recurrence_single_kernel(const RecurrenceArgs p, const TW* __restrict__ w, int requests, TO* __restrict__ out) {
+gated_recurrence_single_kernel(const RecurrenceArgs p, const TW* w, int requests, TO* __restrict__ out) {
+    pdl_launch();
+    pdl_wait();
     extern __shared__ __align__(16) float us[];            // [NR][per]
     __shared__ float z[2 * GS_CHANNELS][NR + 1];
     const int slices = (p.per + GS_CHANNELS - 1) / GS_CHANNELS;
@@ -307,6 +311,8 @@ gated_recurrence_single_kernel(const RecurrenceArgs p, const TW* __restrict__ w,
 // x [rows][width] as three bfloat16 rows that add up to it: out[part][row][3][per] (`rows_padded` rows a part)
 __global__ void __launch_bounds__(256)
 split_rows_kernel(const float* x, int stride, int rows, int width, int per, int rows_padded, bf16* __restrict__ out) {
+    pdl_launch();
+    pdl_wait();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;      // four neighbouring columns
     const int quads = width / 4;
     if (i >= (size_t)rows * quads) return;
@@ -351,9 +357,9 @@ extern "C" int ti_low_rank_decay(const float* low, int low_stride, int rank, con
     TI_REQUIRE(grid.y <= 65535, "low_rank_decay: %d rows exceed the grid limit", rows);
     cudaStream_t s = (cudaStream_t)stream;
     if (a2_dtype == TI_BF16)
-        low_rank_decay_kernel<bf16><<<grid, 128, 0, s>>>(low, low_stride, rank, (const bf16*)a2, bias, inv_tau, rows, n, out);
+        ti_launch_pdl((low_rank_decay_kernel<bf16>), dim3(grid), dim3(128), 0, s, low, low_stride, rank, (const bf16*)a2, bias, inv_tau, rows, n, out);
     else if (a2_dtype == TI_F32)
-        low_rank_decay_kernel<float><<<grid, 128, 0, s>>>(low, low_stride, rank, (const float*)a2, bias, inv_tau, rows, n, out);
+        ti_launch_pdl((low_rank_decay_kernel<float>), dim3(grid), dim3(128), 0, s, low, low_stride, rank, (const float*)a2, bias, inv_tau, rows, n, out);
     else return ti_fail("low_rank_decay: matrix dtype code %d", a2_dtype);
     return ti_check_launch("low_rank_decay");
 }
@@ -380,8 +386,8 @@ extern "C" int ti_gated_recurrence(const float* u, int u_stride, const float* ga
     cudaStream_t s = (cudaStream_t)stream;
 #define CALL(CH)                                                                                                     \
     do {                                                                                                             \
-        if (out_dtype == TI_BF16) gated_recurrence_kernel<bf16, CH><<<grid, GR_WARPS * 32, 0, s>>>(a, (bf16*)out);     \
-        else gated_recurrence_kernel<float, CH><<<grid, GR_WARPS * 32, 0, s>>>(a, (float*)out);                        \
+        if (out_dtype == TI_BF16) ti_launch_if_early(false, (gated_recurrence_kernel<bf16, CH>), dim3(grid), dim3(GR_WARPS * 32), 0, s, a, (bf16*)out);     \
+        else ti_launch_if_early(false, (gated_recurrence_kernel<float, CH>), dim3(grid), dim3(GR_WARPS * 32), 0, s, a, (float*)out);                        \
     } while (0)
     if (ch == 32) CALL(32);
     else if (ch == 16) CALL(16);
@@ -413,8 +419,8 @@ extern "C" int ti_gated_recurrence_single(const float* u, int u_stride, const vo
     cudaStream_t s = (cudaStream_t)stream;
 #define CALL(TW, TO)                                                                                                 \
     do {                                                                                                             \
-        if (wide) gated_recurrence_single_kernel<TW, TO, 16><<<grid, 256, smem, s>>>(a, (const TW*)w, requests, (TO*)out); \
-        else gated_recurrence_single_kernel<TW, TO, 8><<<grid, 256, smem, s>>>(a, (const TW*)w, requests, (TO*)out); \
+        if (wide) ti_launch_pdl((gated_recurrence_single_kernel<TW, TO, 16>), dim3(grid), dim3(256), smem, s, a, (const TW*)w, requests, (TO*)out); \
+        else ti_launch_pdl((gated_recurrence_single_kernel<TW, TO, 8>), dim3(grid), dim3(256), smem, s, a, (const TW*)w, requests, (TO*)out); \
     } while (0)
     if (w_dtype == TI_BF16 && out_dtype == TI_BF16) CALL(bf16, bf16);
     else if (w_dtype == TI_BF16 && out_dtype == TI_F32) CALL(bf16, float);
@@ -431,7 +437,7 @@ extern "C" int ti_split_rows(const float* x, int stride, int rows, int width, in
     TI_REQUIRE(per % 4 == 0 && width % per == 0 && rows <= rows_padded && (uintptr_t)out % 8 == 0,
                "split_rows: parts of %d columns (a multiple of 4) of %d", per, width);
     const long long quads = (long long)rows * (width / 4);
-    split_rows_kernel<<<(unsigned)((quads + 255) / 256), 256, 0, (cudaStream_t)stream>>>(x, stride, rows, width, per,
+    ti_launch_pdl((split_rows_kernel), dim3((unsigned)((quads + 255) / 256)), dim3(256), 0, (cudaStream_t)stream, x, stride, rows, width, per,
                                                                                          rows_padded, (bf16*)out);
     return ti_check_launch("split_rows");
 }

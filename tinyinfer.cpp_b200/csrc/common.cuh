@@ -46,9 +46,12 @@ struct TiPerDevice {
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::); }
 
+// `early` false: an ordinary launch, whose blocks start when the kernel before has ended.  A kernel that walks a prompt
+// token by token out of L1 wants that: started under a product that has set the SM's shared memory aside, it keeps that
+// product's small L1 (the wkv walk over 2,048 tokens 283 -> 606 us, the decayed sum 361 -> 474).
 template <typename... KArgs, typename... Args>
-cudaError_t ti_launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
-                          cudaStream_t stream, Args... args) {
+cudaError_t ti_launch_if_early(bool early, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                               cudaStream_t stream, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -58,8 +61,12 @@ cudaError_t ti_launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = early ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
+}
+template <typename... KArgs, typename... Args>
+cudaError_t ti_launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+    return ti_launch_if_early(true, kernel, grid, block, smem, stream, args...);
 }
 
 __device__ __forceinline__ float to_f32(float x) { return x; }

@@ -9,9 +9,11 @@ namespace {
 // The gated sum's normaliser column and running maximum from `carry` into the slots, after every
 // block of the cut launch has read the old ones: one block per (request, head).
 __global__ void __launch_bounds__(64)
-matrix_state_commit_kernel(const float* __restrict__ carry, const int* __restrict__ cu_q,
-                           const int* __restrict__ slots, float* state, long long state_stride, int heads, int dk,
+matrix_state_commit_kernel(const float* carry, const int* cu_q,
+                           const int* slots, float* state, long long state_stride, int heads, int dk,
                            int dv) {
+    pdl_launch();
+    pdl_wait();
     const int req = blockIdx.x, head = blockIdx.y;
     if (cu_q[req] >= cu_q[req + 1]) return;
     const int cols = dv + 1;
@@ -25,9 +27,11 @@ matrix_state_commit_kernel(const float* __restrict__ carry, const int* __restric
 // one warp per (token, head).
 template <typename TO>
 __global__ void __launch_bounds__(256)
-matrix_state_finish_kernel(const float* o_raw, const float* __restrict__ norm_weight, int norm_per_row, float eps,
+matrix_state_finish_kernel(const float* o_raw, const float* norm_weight, int norm_per_row, float eps,
                            const float* gate, int gate_stride, int gate_act, int rows, int heads, int dv,
                            TO* __restrict__ out) {
+    pdl_launch();
+    pdl_wait();
     const int unit = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (unit >= rows * heads) return;
     const int t = unit / heads, head = unit % heads;
@@ -84,6 +88,7 @@ extern "C" int ti_matrix_state(int mode, const float* q, const float* k, const f
     a.heads = heads; a.kv_heads = kv_heads; a.dk = dk; a.dv = dv;
     a.out = out; a.out_bf16 = out_dtype == TI_BF16; a.o_raw = o_raw; a.carry = carry;
     a.cut = col_block != 0;
+    a.single = rows == requests;
     a.vec4 = ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v)) % 16 == 0 &&
               reinterpret_cast<uintptr_t>(decay) % 16 == 0 && decay_stride % 4 == 0 && q_stride % 4 == 0 && k_stride % 4 == 0 && v_stride % 4 == 0 && dk % 4 == 0 && dv % 4 == 0) ? 1 : 0;
     cudaStream_t s = (cudaStream_t)stream;
@@ -96,16 +101,16 @@ extern "C" int ti_matrix_state(int mode, const float* q, const float* k, const f
     if (int rc = ti_check_launch("matrix_state")) return rc;
     if (col_block != 0) {
         if (mode == MODE_GATED_SUM) {
-            matrix_state_commit_kernel<<<dim3(requests, heads), 64, 0, s>>>(carry, cu_q, slots, state, state_stride,
+            ti_launch_pdl((matrix_state_commit_kernel), dim3(dim3(requests, heads)), dim3(64), 0, s, carry, cu_q, slots, state, state_stride,
                                                                             heads, dk, dv);
             if (int rc = ti_check_launch("matrix_state_commit")) return rc;
         }
         const int blocks = (rows * heads + 7) / 8;
         if (out_dtype == TI_BF16)
-            matrix_state_finish_kernel<bf16><<<blocks, 256, 0, s>>>(o_raw, norm_weight, norm_per_row, eps, gate,
+            ti_launch_pdl((matrix_state_finish_kernel<bf16>), dim3(blocks), dim3(256), 0, s, o_raw, norm_weight, norm_per_row, eps, gate,
                                                                      gate_stride, gate_act, rows, heads, dv, (bf16*)out);
         else
-            matrix_state_finish_kernel<float><<<blocks, 256, 0, s>>>(o_raw, norm_weight, norm_per_row, eps, gate,
+            ti_launch_pdl((matrix_state_finish_kernel<float>), dim3(blocks), dim3(256), 0, s, o_raw, norm_weight, norm_per_row, eps, gate,
                                                                       gate_stride, gate_act, rows, heads, dv, (float*)out);
         return ti_check_launch("matrix_state_finish");
     }

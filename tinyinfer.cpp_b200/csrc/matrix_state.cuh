@@ -65,6 +65,7 @@ struct MatrixStateArgs {
     float* carry;                                         // [requests, heads, dk + 1] float32 (columns cut, gated sum)
     int vec4;                                             // q, k, v rows and the heads in them start on 16 bytes
     int cut;                                              // a head's columns lie over several blocks
+    int single;                                           // a token per request
 };
 
 __device__ __forceinline__ float softplusf_(float z) { return z > 20.0f ? z : log1pf(expf(z)); }
@@ -120,6 +121,7 @@ template <int MODE, int DMAX, int CB, int LANES> struct StateBlock {
 template <int MODE, int DMAX, int CB, int LANES>
 __global__ void __launch_bounds__(StateBlock<MODE, DMAX, CB, LANES>::threads, StateBlock<MODE, DMAX, CB, LANES>::resident)
 matrix_state_kernel(const MatrixStateArgs p) {
+    pdl_wait();
     constexpr int TT = TileTokens<MODE, DMAX, CB>::value;
     constexpr bool DECAYED = MODE == MODE_DECAYED_SUM;
     constexpr int VPT = VLANES / LANES;                   // virtual lanes a thread plays: 4 or 1
@@ -441,7 +443,7 @@ template <int MODE, int DMAX>
 int launch_cb(const MatrixStateArgs& a, int requests, int cb, int col_blocks, cudaStream_t s) {
     dim3 grid(requests, a.heads, col_blocks);
 #define TI_MS_GO(CB_, LANES_) \
-    matrix_state_kernel<MODE, DMAX, CB_, LANES_><<<grid, StateBlock<MODE, DMAX, CB_, LANES_>::threads, 0, s>>>(a)
+    ti_launch_if_early(a.single, (matrix_state_kernel<MODE, DMAX, CB_, LANES_>), dim3(grid), dim3(StateBlock<MODE, DMAX, CB_, LANES_>::threads), 0, s, a)
     if (a.cut && cb == 8) TI_MS_GO(8, 16);
     else if (a.cut && cb == 16) TI_MS_GO(16, 16);
     else if (a.cut && cb == 32) TI_MS_GO(32, 16);

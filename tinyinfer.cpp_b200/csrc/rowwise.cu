@@ -197,8 +197,10 @@ rmsnorm_vec_kernel(float* __restrict__ x, const float* __restrict__ w, const int
 // up_j = gu[t, inter + j].  Interleaved layout (groups of 8 gate columns followed by their 8 up
 // columns): gate_j = gu[t, 16 (j / 8) + j % 8], up_j eight columns further.
 template <typename TO>
-__global__ void swiglu_kernel(const float* __restrict__ gu, int inter, size_t total,
+__global__ void swiglu_kernel(const float* gu, int inter, size_t total,
                               int interleaved, TO* __restrict__ y) {
+    pdl_launch();
+    pdl_wait();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total) return;
     const size_t t = i / inter, j = i % inter;
@@ -406,9 +408,9 @@ extern "C" int ti_swiglu(const float* gu, int num_tokens, int inter, int interle
     cudaStream_t s = (cudaStream_t)stream;
     const unsigned blocks = (unsigned)((total + 255) / 256);
     if (out_dtype == TI_BF16)
-        swiglu_kernel<bf16><<<blocks, 256, 0, s>>>(gu, inter, total, interleaved, (bf16*)out);
+        ti_launch_pdl((swiglu_kernel<bf16>), dim3(blocks), dim3(256), 0, s, gu, inter, total, interleaved, (bf16*)out);
     else if (out_dtype == TI_F32)
-        swiglu_kernel<float><<<blocks, 256, 0, s>>>(gu, inter, total, interleaved, (float*)out);
+        ti_launch_pdl((swiglu_kernel<float>), dim3(blocks), dim3(256), 0, s, gu, inter, total, interleaved, (float*)out);
     else
         return ti_fail("swiglu: output dtype code %d is not float32 or bfloat16", out_dtype);
     return ti_check_launch("swiglu");

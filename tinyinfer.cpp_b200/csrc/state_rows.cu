@@ -43,11 +43,13 @@ constexpr int MAX_TAPS = 16;
 
 template <typename TO>
 __global__ void __launch_bounds__(256)
-causal_conv_rows_kernel(const float* x, int x_stride, const float* __restrict__ w, int taps, int channels,
-                        const int* __restrict__ req_of_tok, const int* __restrict__ cu_q,
-                        const int* __restrict__ slots, const float* state, size_t state_stride,
-                        size_t state_offset, int add_input, int silu, int renew, const float* __restrict__ in_bias,
-                        const float* __restrict__ bias, TO* __restrict__ out, int out_stride) {
+causal_conv_rows_kernel(const float* x, int x_stride, const float* w, int taps, int channels,
+                        const int* req_of_tok, const int* cu_q,
+                        const int* slots, const float* state, size_t state_stride,
+                        size_t state_offset, int add_input, int silu, int renew, const float* in_bias,
+                        const float* bias, TO* __restrict__ out, int out_stride) {
+    pdl_launch();
+    pdl_wait();
     const int t = blockIdx.x;
     const int c = blockIdx.y * blockDim.x + threadIdx.x;
     if (c >= channels) return;
@@ -82,9 +84,11 @@ causal_conv_rows_kernel(const float* x, int x_stride, const float* __restrict__ 
 // state[slot] <- the last taps - 1 inputs of the request after this step: rows of this step, or,
 // where the portion is shorter than that, the rows the state held moved up.
 __global__ void __launch_bounds__(256)
-conv_tail_store_kernel(const float* x, int x_stride, int taps, int channels, const int* __restrict__ cu_q,
-                       const int* __restrict__ slots, float* state, size_t state_stride, size_t state_offset,
-                       const float* __restrict__ in_bias) {
+conv_tail_store_kernel(const float* x, int x_stride, int taps, int channels, const int* cu_q,
+                       const int* slots, float* state, size_t state_stride, size_t state_offset,
+                       const float* in_bias) {
+    pdl_launch();
+    pdl_wait();
     const int r = blockIdx.y;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= channels) return;
@@ -104,8 +108,10 @@ conv_tail_store_kernel(const float* x, int x_stride, int taps, int channels, con
 // shared memory in a fixed order); the block's warps take the groups `blockDim / 32 / wpg` at a time.
 template <typename TO, bool ADD>
 __global__ void __launch_bounds__(256)
-group_norm_rows_kernel(const float* x, const float* __restrict__ w, const int* __restrict__ rows, int groups,
+group_norm_rows_kernel(const float* x, const float* w, const int* rows, int groups,
                        int n, float eps, TO* __restrict__ out, float* residual, int res_stride, int wpg) {
+    pdl_launch();
+    pdl_wait();
     __shared__ float part[8];
     const int r = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     const float* xr = x + (size_t)(rows ? rows[r] : r) * n;
@@ -136,7 +142,9 @@ group_norm_rows_kernel(const float* x, const float* __restrict__ w, const int* _
 }
 
 __global__ void __launch_bounds__(256)
-depth_mix_kernel(float* x, float* hist, size_t layer_elems, int index, const float* __restrict__ w, size_t n) {
+depth_mix_kernel(float* x, float* hist, size_t layer_elems, int index, const float* w, size_t n) {
+    pdl_launch();
+    pdl_wait();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float cur = x[i];
@@ -150,6 +158,8 @@ depth_mix_kernel(float* x, float* hist, size_t layer_elems, int index, const flo
 __global__ void __launch_bounds__(256)
 add_scaled_kernel(float* dst, int dst_stride, const float* a, float sa, const float* b, float sb, int rows,
                   int cols) {
+    pdl_launch();
+    pdl_wait();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (size_t)rows * cols) return;
     const int r = (int)(i / cols), c = (int)(i % cols);
@@ -162,6 +172,8 @@ template <typename TO>
 __global__ void __launch_bounds__(256)
 glu_rows_kernel(const float* gu, int inter, size_t total, int interleaved, int kind, float limit, float alpha,
                 TO* __restrict__ out) {
+    pdl_launch();
+    pdl_wait();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total) return;
     const size_t t = i / inter;
@@ -190,9 +202,11 @@ __device__ __forceinline__ float tanh_norm_one(float x, float alpha, float w, fl
 
 template <typename TO, bool ADD, int VEC>
 __global__ void __launch_bounds__(256)
-tanh_norm_rows_kernel(const float* __restrict__ x, const int* __restrict__ rows, int n, float alpha,
-                      const float* __restrict__ w, const float* __restrict__ b, TO* __restrict__ out,
+tanh_norm_rows_kernel(const float* x, const int* rows, int n, float alpha,
+                      const float* w, const float* b, TO* __restrict__ out,
                       float* residual, int res_stride) {
+    pdl_launch();
+    pdl_wait();
     const size_t r = blockIdx.x;
     const int c = (blockIdx.y * blockDim.x + threadIdx.x) * VEC;
     if (c >= n) return;
@@ -220,9 +234,11 @@ tanh_norm_rows_kernel(const float* __restrict__ x, const int* __restrict__ rows,
 // residual += tanh(a1 y) w1 + b1, then out = tanh(a2 residual) w2 + b2
 template <typename TO, int VEC>
 __global__ void __launch_bounds__(256)
-tanh_norm_pair_kernel(const float* __restrict__ y, int n, float a1, const float* __restrict__ w1,
-                      const float* __restrict__ b1, float* residual, int res_stride, float a2,
-                      const float* __restrict__ w2, const float* __restrict__ b2, TO* __restrict__ out) {
+tanh_norm_pair_kernel(const float* y, int n, float a1, const float* w1,
+                      const float* b1, float* residual, int res_stride, float a2,
+                      const float* w2, const float* b2, TO* __restrict__ out) {
+    pdl_launch();
+    pdl_wait();
     const size_t r = blockIdx.x;
     const int c = (blockIdx.y * blockDim.x + threadIdx.x) * VEC;
     if (c >= n) return;
@@ -250,10 +266,12 @@ tanh_norm_pair_kernel(const float* __restrict__ y, int n, float a1, const float*
 // out[t] = table[token] + bigram[row]; a block per token
 template <typename TW>
 __global__ void __launch_bounds__(256)
-embed_bigram_kernel(const TW* __restrict__ table, const TW* __restrict__ bigram, const int* __restrict__ tokens, int n,
+embed_bigram_kernel(const TW* table, const TW* bigram, const int* tokens, int n,
                     int vocab, long long buckets, long long mul_prev, long long mul_cur,
-                    const int* __restrict__ positions, const int* __restrict__ req_of_tok, const int* __restrict__ cu_q,
-                    const int* __restrict__ slots, int* kept, size_t kept_stride, float* __restrict__ out) {
+                    const int* positions, const int* req_of_tok, const int* cu_q,
+                    const int* slots, int* kept, size_t kept_stride, float* __restrict__ out) {
+    pdl_launch();
+    pdl_wait();
     __shared__ long long row_s;
     const int t = blockIdx.x;
     const int token = min(max(tokens[t], 0), vocab - 1);
@@ -305,9 +323,11 @@ template <int VEC> __device__ __forceinline__ float row_scale(const float* row, 
 
 template <typename TO, int VEC>
 __global__ void __launch_bounds__(256)
-rmsnorm_shift_kernel(const float* x, int n, const float* __restrict__ w, float eps, const float* __restrict__ mu,
-                     const int* __restrict__ req_of_tok, const int* __restrict__ cu_q, const int* __restrict__ slots,
+rmsnorm_shift_kernel(const float* x, int n, const float* w, float eps, const float* mu,
+                     const int* req_of_tok, const int* cu_q, const int* slots,
                      float* kept, size_t kept_stride, TO* __restrict__ out, TO* __restrict__ shifted) {
+    pdl_launch();
+    pdl_wait();
     __shared__ float scratch[32];
     const int t = blockIdx.x, r = req_of_tok[t];
     const int first = cu_q[r], last = cu_q[r + 1] - 1;
@@ -342,7 +362,9 @@ rmsnorm_shift_kernel(const float* x, int n, const float* __restrict__ w, float e
 template <int VEC>
 __global__ void __launch_bounds__(256)
 gated_add_kernel(float* x, int x_stride, const float* y, int y_stride, const float* gate, int gate_stride,
-                 const float* __restrict__ bias, float scale, int n) {
+                 const float* bias, float scale, int n) {
+    pdl_launch();
+    pdl_wait();
     const size_t r = blockIdx.x;
     const int c = (blockIdx.y * blockDim.x + threadIdx.x) * VEC;
     if (c >= n) return;
@@ -356,17 +378,23 @@ gated_add_kernel(float* x, int x_stride, const float* y, int y_stride, const flo
 }
 
 __global__ void cap_rows_kernel(float* __restrict__ x, size_t total, float cap) {
+    pdl_launch();
+    pdl_wait();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < total) x[i] = cap * tanhf(x[i] / cap);
 }
 
 template <typename TO>
 __global__ void unary_rows_kernel(const float* x, size_t total, int kind, TO* __restrict__ out) {
+    pdl_launch();
+    pdl_wait();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < total) out[i] = from_f32<TO>(unary_activation(kind, x[i]));
 }
 
-__global__ void add_row_kernel(float* __restrict__ x, int stride, const float* __restrict__ row, int cols, size_t total) {
+__global__ void add_row_kernel(float* __restrict__ x, int stride, const float* row, int cols, size_t total) {
+    pdl_launch();
+    pdl_wait();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total) return;
     const int c = (int)(i % cols);
@@ -386,11 +414,11 @@ extern "C" int ti_causal_conv_rows(const float* x, int x_stride, const float* w,
     dim3 grid(rows, (channels + 255) / 256);
     cudaStream_t s = (cudaStream_t)stream;
     if (out_dtype == TI_BF16)
-        causal_conv_rows_kernel<bf16><<<grid, 256, 0, s>>>(x, x_stride, w, taps, channels, req_of_tok, cu_q, slots, state,
+        ti_launch_pdl((causal_conv_rows_kernel<bf16>), dim3(grid), dim3(256), 0, s, x, x_stride, w, taps, channels, req_of_tok, cu_q, slots, state,
                                                            (size_t)state_stride, (size_t)state_offset, add_input, silu,
                                                            renew, in_bias, bias, (bf16*)out, out_stride);
     else if (out_dtype == TI_F32)
-        causal_conv_rows_kernel<float><<<grid, 256, 0, s>>>(x, x_stride, w, taps, channels, req_of_tok, cu_q, slots, state,
+        ti_launch_pdl((causal_conv_rows_kernel<float>), dim3(grid), dim3(256), 0, s, x, x_stride, w, taps, channels, req_of_tok, cu_q, slots, state,
                                                             (size_t)state_stride, (size_t)state_offset, add_input, silu,
                                                             renew, in_bias, bias, (float*)out, out_stride);
     else return ti_fail("causal_conv_rows: output dtype code %d", out_dtype);
@@ -403,7 +431,7 @@ extern "C" int ti_conv_tail_store(const float* x, int x_stride, int taps, int ch
     if (requests == 0 || channels == 0 || taps <= 1) return 0;
     TI_REQUIRE(taps <= MAX_TAPS, "conv_tail_store: %d taps (at most %d)", taps, MAX_TAPS);
     dim3 grid((channels + 255) / 256, requests);
-    conv_tail_store_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(x, x_stride, taps, channels, cu_q, slots, state,
+    ti_launch_pdl((conv_tail_store_kernel), dim3(grid), dim3(256), 0, (cudaStream_t)stream, x, x_stride, taps, channels, cu_q, slots, state,
                                                                     (size_t)state_stride, (size_t)state_offset, in_bias);
     return ti_check_launch("conv_tail_store");
 }
@@ -417,12 +445,12 @@ extern "C" int ti_group_norm_rows(const float* x, const float* w, const int* row
     const int threads = (groups >= 8 ? 8 : groups) * wpg * 32;
     if (residual != nullptr) {
         TI_REQUIRE(rows == nullptr, "group_norm_rows: rows are not gathered when adding to a residual");
-        group_norm_rows_kernel<float, true><<<num_rows, threads, 0, s>>>(x, w, rows, groups, n, eps, nullptr, residual,
+        ti_launch_pdl((group_norm_rows_kernel<float, true>), dim3(num_rows), dim3(threads), 0, s, x, w, rows, groups, n, eps, nullptr, residual,
                                                                         res_stride, wpg);
     } else if (out_dtype == TI_BF16) {
-        group_norm_rows_kernel<bf16, false><<<num_rows, threads, 0, s>>>(x, w, rows, groups, n, eps, (bf16*)out, nullptr, 0, wpg);
+        ti_launch_pdl((group_norm_rows_kernel<bf16, false>), dim3(num_rows), dim3(threads), 0, s, x, w, rows, groups, n, eps, (bf16*)out, nullptr, 0, wpg);
     } else if (out_dtype == TI_F32) {
-        group_norm_rows_kernel<float, false><<<num_rows, threads, 0, s>>>(x, w, rows, groups, n, eps, (float*)out, nullptr, 0, wpg);
+        ti_launch_pdl((group_norm_rows_kernel<float, false>), dim3(num_rows), dim3(threads), 0, s, x, w, rows, groups, n, eps, (float*)out, nullptr, 0, wpg);
     } else {
         return ti_fail("group_norm_rows: output dtype code %d", out_dtype);
     }
@@ -432,7 +460,7 @@ extern "C" int ti_group_norm_rows(const float* x, const float* w, const int* row
 extern "C" int ti_depth_mix(float* x, float* hist, long long layer_elems, int index, const float* w, void* stream) {
     if (layer_elems == 0) return 0;
     const int blocks = (int)((layer_elems + 255) / 256);
-    depth_mix_kernel<<<blocks, 256, 0, (cudaStream_t)stream>>>(x, hist, (size_t)layer_elems, index, w, (size_t)layer_elems);
+    ti_launch_pdl((depth_mix_kernel), dim3(blocks), dim3(256), 0, (cudaStream_t)stream, x, hist, (size_t)layer_elems, index, w, (size_t)layer_elems);
     return ti_check_launch("depth_mix");
 }
 
@@ -440,7 +468,7 @@ extern "C" int ti_add_scaled(float* dst, int dst_stride, const float* a, float s
                              int cols, void* stream) {
     if (rows == 0 || cols == 0) return 0;
     const size_t n = (size_t)rows * cols;
-    add_scaled_kernel<<<(int)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(dst, dst_stride, a, sa, b, sb, rows, cols);
+    ti_launch_pdl((add_scaled_kernel), dim3((int)((n + 255) / 256)), dim3(256), 0, (cudaStream_t)stream, dst, dst_stride, a, sa, b, sb, rows, cols);
     return ti_check_launch("add_scaled");
 }
 
@@ -453,9 +481,9 @@ extern "C" int ti_glu_rows(const float* gu, int num_tokens, int inter, int inter
     const int blocks = (int)((total + 255) / 256);
     cudaStream_t s = (cudaStream_t)stream;
     if (out_dtype == TI_BF16)
-        glu_rows_kernel<bf16><<<blocks, 256, 0, s>>>(gu, inter, total, interleaved, kind, limit, alpha, (bf16*)out);
+        ti_launch_pdl((glu_rows_kernel<bf16>), dim3(blocks), dim3(256), 0, s, gu, inter, total, interleaved, kind, limit, alpha, (bf16*)out);
     else if (out_dtype == TI_F32)
-        glu_rows_kernel<float><<<blocks, 256, 0, s>>>(gu, inter, total, interleaved, kind, limit, alpha, (float*)out);
+        ti_launch_pdl((glu_rows_kernel<float>), dim3(blocks), dim3(256), 0, s, gu, inter, total, interleaved, kind, limit, alpha, (float*)out);
     else return ti_fail("glu_rows: output dtype code %d", out_dtype);
     return ti_check_launch("glu_rows");
 }
@@ -475,7 +503,7 @@ extern "C" int ti_tanh_norm_rows(const float* x, const int* rows, int num_rows, 
     const dim3 grid(num_rows, (n + (four ? 1023 : 255)) / (four ? 1024 : 256));
     TI_REQUIRE(grid.y <= 65535, "tanh_norm_rows: rows of %d elements", n);
 #define CALL(TO, ADD, VEC)                                                                            \
-    tanh_norm_rows_kernel<TO, ADD, VEC><<<grid, 256, 0, s>>>(x, rows, n, alpha, w, b, (TO*)(ADD ? nullptr : out), \
+    ti_launch_pdl((tanh_norm_rows_kernel<TO, ADD, VEC>), dim3(grid), dim3(256), 0, s, x, rows, n, alpha, w, b, (TO*)(ADD ? nullptr : out), \
                                                              residual, res_stride)
     if (residual != nullptr) {
         TI_REQUIRE(rows == nullptr, "tanh_norm_rows: rows are not gathered when adding to a residual");
@@ -500,7 +528,7 @@ extern "C" int ti_embed_bigram(const void* table, const void* bigram, int dtype,
                "embed_bigram: factors must lie in [0, buckets), and buckets below 2^31");
     cudaStream_t s = (cudaStream_t)stream;
 #define CALL(TW)                                                                                                   \
-    embed_bigram_kernel<TW><<<num_tokens, 256, 0, s>>>((const TW*)table, (const TW*)bigram, tokens, n, vocab, buckets,  \
+    ti_launch_pdl((embed_bigram_kernel<TW>), dim3(num_tokens), dim3(256), 0, s, (const TW*)table, (const TW*)bigram, tokens, n, vocab, buckets,  \
                                                        mul_prev, mul_cur, positions, req_of_tok, cu_q, slots, kept, \
                                                        (size_t)kept_stride, out)
     if (dtype == TI_BF16) CALL(bf16);
@@ -517,7 +545,7 @@ extern "C" int ti_rmsnorm_shift(const float* x, int num_rows, int n, const float
     cudaStream_t s = (cudaStream_t)stream;
     const bool four = kept_stride % 4 == 0 && rows_of_four(n, 0, {x, w, mu, kept, out, shifted});
 #define CALL(TO, VEC)                                                                                              \
-    rmsnorm_shift_kernel<TO, VEC><<<num_rows, 256, 0, s>>>(x, n, w, eps, mu, req_of_tok, cu_q, slots, kept,         \
+    ti_launch_pdl((rmsnorm_shift_kernel<TO, VEC>), dim3(num_rows), dim3(256), 0, s, x, n, w, eps, mu, req_of_tok, cu_q, slots, kept,         \
                                                            (size_t)kept_stride, (TO*)out, (TO*)shifted)
     if (out_dtype == TI_BF16) { if (four) CALL(bf16, 4); else CALL(bf16, 1); }
     else if (out_dtype == TI_F32) { if (four) CALL(float, 4); else CALL(float, 1); }
@@ -533,15 +561,15 @@ extern "C" int ti_gated_add(float* x, int x_stride, const float* y, int y_stride
     const bool four = y_stride % 4 == 0 && gate_stride % 4 == 0 && rows_of_four(n, x_stride, {x, y, gate, bias});
     const dim3 grid(rows, (n + (four ? 1023 : 255)) / (four ? 1024 : 256));
     TI_REQUIRE(grid.y <= 65535, "gated_add: rows of %d elements", n);
-    if (four) gated_add_kernel<4><<<grid, 256, 0, s>>>(x, x_stride, y, y_stride, gate, gate_stride, bias, scale, n);
-    else gated_add_kernel<1><<<grid, 256, 0, s>>>(x, x_stride, y, y_stride, gate, gate_stride, bias, scale, n);
+    if (four) ti_launch_pdl((gated_add_kernel<4>), dim3(grid), dim3(256), 0, s, x, x_stride, y, y_stride, gate, gate_stride, bias, scale, n);
+    else ti_launch_pdl((gated_add_kernel<1>), dim3(grid), dim3(256), 0, s, x, x_stride, y, y_stride, gate, gate_stride, bias, scale, n);
     return ti_check_launch("gated_add");
 }
 
 extern "C" int ti_cap_rows(float* x, long long total, float cap, void* stream) {
     if (total == 0) return 0;
     TI_REQUIRE(cap > 0.0f, "cap_rows: the cap must be positive");
-    cap_rows_kernel<<<(unsigned)((total + 255) / 256), 256, 0, (cudaStream_t)stream>>>(x, (size_t)total, cap);
+    ti_launch_pdl((cap_rows_kernel), dim3((unsigned)((total + 255) / 256)), dim3(256), 0, (cudaStream_t)stream, x, (size_t)total, cap);
     return ti_check_launch("cap_rows");
 }
 
@@ -550,8 +578,8 @@ extern "C" int ti_unary_rows(const float* x, long long total, int kind, void* ou
     TI_REQUIRE(kind == ACT_RELU2, "unary_rows: activation kind %d", kind);
     const unsigned blocks = (unsigned)((total + 255) / 256);
     cudaStream_t s = (cudaStream_t)stream;
-    if (out_dtype == TI_BF16) unary_rows_kernel<bf16><<<blocks, 256, 0, s>>>(x, (size_t)total, kind, (bf16*)out);
-    else if (out_dtype == TI_F32) unary_rows_kernel<float><<<blocks, 256, 0, s>>>(x, (size_t)total, kind, (float*)out);
+    if (out_dtype == TI_BF16) ti_launch_pdl((unary_rows_kernel<bf16>), dim3(blocks), dim3(256), 0, s, x, (size_t)total, kind, (bf16*)out);
+    else if (out_dtype == TI_F32) ti_launch_pdl((unary_rows_kernel<float>), dim3(blocks), dim3(256), 0, s, x, (size_t)total, kind, (float*)out);
     else return ti_fail("unary_rows: output dtype code %d", out_dtype);
     return ti_check_launch("unary_rows");
 }
@@ -559,7 +587,7 @@ extern "C" int ti_unary_rows(const float* x, long long total, int kind, void* ou
 extern "C" int ti_add_row(float* x, int stride, const float* row, int rows, int cols, void* stream) {
     const size_t total = (size_t)rows * cols;
     if (total == 0) return 0;
-    add_row_kernel<<<(unsigned)((total + 255) / 256), 256, 0, (cudaStream_t)stream>>>(x, stride, row, cols, total);
+    ti_launch_pdl((add_row_kernel), dim3((unsigned)((total + 255) / 256)), dim3(256), 0, (cudaStream_t)stream, x, stride, row, cols, total);
     return ti_check_launch("add_row");
 }
 
@@ -572,7 +600,7 @@ extern "C" int ti_tanh_norm_pair(const float* y, int num_rows, int n, float a1, 
     const dim3 grid(num_rows, (n + (four ? 1023 : 255)) / (four ? 1024 : 256));
     TI_REQUIRE(grid.y <= 65535, "tanh_norm_pair: rows of %d elements", n);
 #define CALL(TO, VEC) \
-    tanh_norm_pair_kernel<TO, VEC><<<grid, 256, 0, s>>>(y, n, a1, w1, b1, residual, res_stride, a2, w2, b2, (TO*)out)
+    ti_launch_pdl((tanh_norm_pair_kernel<TO, VEC>), dim3(grid), dim3(256), 0, s, y, n, a1, w1, b1, residual, res_stride, a2, w2, b2, (TO*)out)
     if (out_dtype == TI_BF16) { if (four) CALL(bf16, 4); else CALL(bf16, 1); }
     else if (out_dtype == TI_F32) { if (four) CALL(float, 4); else CALL(float, 1); }
     else return ti_fail("tanh_norm_pair: output dtype code %d", out_dtype);

@@ -23,10 +23,12 @@ namespace {
 
 template <typename TH>
 __global__ void __launch_bounds__(256)
-token_shift_mix_kernel(const TH* h, const float* __restrict__ mu, int n_mix, int width, int num_tokens,
-                       const int* __restrict__ req_of_tok, const int* __restrict__ cu_q,
-                       const int* __restrict__ slots, const float* state, size_t state_stride,
+token_shift_mix_kernel(const TH* h, const float* mu, int n_mix, int width, int num_tokens,
+                       const int* req_of_tok, const int* cu_q,
+                       const int* slots, const float* state, size_t state_stride,
                        size_t prev_offset, TH* __restrict__ out) {
+    pdl_launch();
+    pdl_wait();
     const int t = blockIdx.x;
     const int r = req_of_tok[t];
     const bool first = t == cu_q[r];
@@ -67,6 +69,7 @@ wkv_recurrence_kernel(const float* r, const float* k, const float* v, const floa
                       const int* __restrict__ cu_q, const int* __restrict__ slots, float* state,
                       size_t state_stride, size_t prev_offset, int num_heads, int d,
                       TO* __restrict__ out, float* __restrict__ o_raw) {
+    pdl_wait();
     constexpr int WKV_TT = (DMAX > 64 ? 8 : 16) / (JS == 1 ? 2 : 1);   // tokens per staged tile (48 KB of shared memory at most)
     constexpr int WKV_IS = wkv_lanes(DMAX, JS);
     constexpr int NI = DMAX / WKV_IS;                    // state rows per thread
@@ -214,8 +217,10 @@ wkv_recurrence_kernel(const float* r, const float* k, const float* v, const floa
 // a warp per (token, head)
 template <typename TO>
 __global__ void __launch_bounds__(256)
-wkv_finish_kernel(const float* o_raw, const float* g, int g_stride, const float* __restrict__ norm_weight, float eps,
+wkv_finish_kernel(const float* o_raw, const float* g, int g_stride, const float* norm_weight, float eps,
                   int num_items, int num_heads, int d, TO* __restrict__ out) {
+    pdl_launch();
+    pdl_wait();
     const int item = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (item >= num_items) return;
     const int t = item / num_heads, head = item % num_heads;
@@ -231,12 +236,16 @@ wkv_finish_kernel(const float* o_raw, const float* g, int g_stride, const float*
 
 template <typename TO>
 __global__ void tanh_rows_kernel(const float* x, size_t n, TO* __restrict__ out) {
+    pdl_launch();
+    pdl_wait();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) out[i] = from_f32<TO>(tanhf(x[i]));
 }
 
 template <typename TO>
 __global__ void xielu_rows_kernel(const float* x, size_t n, float ap, float aq, TO* __restrict__ out) {
+    pdl_launch();
+    pdl_wait();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float z = x[i];
@@ -253,10 +262,10 @@ extern "C" int ti_token_shift_mix(const void* h, int h_dtype, const float* mu, i
     if (num_tokens == 0) return 0;
     cudaStream_t s = (cudaStream_t)stream;
     if (h_dtype == TI_F32)
-        token_shift_mix_kernel<float><<<num_tokens, 256, 0, s>>>((const float*)h, mu, n_mix, width, num_tokens,
+        ti_launch_pdl((token_shift_mix_kernel<float>), dim3(num_tokens), dim3(256), 0, s, (const float*)h, mu, n_mix, width, num_tokens,
             req_of_tok, cu_q, slots, state, (size_t)state_stride, (size_t)prev_offset, (float*)out);
     else if (h_dtype == TI_BF16)
-        token_shift_mix_kernel<bf16><<<num_tokens, 256, 0, s>>>((const bf16*)h, mu, n_mix, width, num_tokens,
+        ti_launch_pdl((token_shift_mix_kernel<bf16>), dim3(num_tokens), dim3(256), 0, s, (const bf16*)h, mu, n_mix, width, num_tokens,
             req_of_tok, cu_q, slots, state, (size_t)state_stride, (size_t)prev_offset, (bf16*)out);
     else
         return ti_fail("token_shift_mix: dtype code %d is not supported", h_dtype);
@@ -279,7 +288,7 @@ extern "C" int ti_wkv_recurrence(const float* r, const float* k, const float* v,
     dim3 grid(num_requests, num_heads, col_split);
     cudaStream_t s = (cudaStream_t)stream;
 #define LAUNCH(TH, DMAX, JS)                                                                       \
-    wkv_recurrence_kernel<TH, TH, DMAX, JS><<<grid, DMAX / JS * wkv_lanes(DMAX, JS), 0, s>>>(                      \
+    ti_launch_if_early(num_tokens == num_requests, (wkv_recurrence_kernel<TH, TH, DMAX, JS>), grid, dim3(DMAX / JS * wkv_lanes(DMAX, JS)), 0, s,                      \
         r, k, v, g, a, in_stride, w0, u, norm_weight, eps, (const TH*)h, width, cu_q, slots, state,    \
         (size_t)state_stride, (size_t)prev_offset, num_heads, d, (TH*)out, o_raw)
 #define CALL(TH)                                                                                   \
@@ -287,7 +296,7 @@ extern "C" int ti_wkv_recurrence(const float* r, const float* k, const float* v,
         if (d <= 32) LAUNCH(TH, 32, 4); else if (d <= 64) LAUNCH(TH, 64, 4); else LAUNCH(TH, 128, 4); \
         if (int rc = ti_check_launch("wkv_recurrence")) return rc;                                 \
         const int items = num_tokens * num_heads;                                                  \
-        wkv_finish_kernel<TH><<<(items + 7) / 8, 256, 0, s>>>(o_raw, g, in_stride, norm_weight, eps, items, \
+        ti_launch_pdl((wkv_finish_kernel<TH>), dim3((items + 7) / 8), dim3(256), 0, s, o_raw, g, in_stride, norm_weight, eps, items, \
                                                             num_heads, d, (TH*)out);               \
         return ti_check_launch("wkv_finish");                                                      \
     }                                                                                              \
@@ -304,8 +313,8 @@ extern "C" int ti_tanh_rows(const float* x, long long n, void* out, int out_dtyp
     if (n == 0) return 0;
     cudaStream_t s = (cudaStream_t)stream;
     const unsigned blocks = (unsigned)((n + 255) / 256);
-    if (out_dtype == TI_F32) tanh_rows_kernel<float><<<blocks, 256, 0, s>>>(x, (size_t)n, (float*)out);
-    else if (out_dtype == TI_BF16) tanh_rows_kernel<bf16><<<blocks, 256, 0, s>>>(x, (size_t)n, (bf16*)out);
+    if (out_dtype == TI_F32) ti_launch_pdl((tanh_rows_kernel<float>), dim3(blocks), dim3(256), 0, s, x, (size_t)n, (float*)out);
+    else if (out_dtype == TI_BF16) ti_launch_pdl((tanh_rows_kernel<bf16>), dim3(blocks), dim3(256), 0, s, x, (size_t)n, (bf16*)out);
     else return ti_fail("tanh_rows: dtype code %d is not supported", out_dtype);
     return ti_check_launch("tanh_rows");
 }
@@ -315,8 +324,8 @@ extern "C" int ti_xielu_rows(const float* x, long long n, float ap, float aq, vo
     if (n == 0) return 0;
     cudaStream_t s = (cudaStream_t)stream;
     const unsigned blocks = (unsigned)((n + 255) / 256);
-    if (out_dtype == TI_F32) xielu_rows_kernel<float><<<blocks, 256, 0, s>>>(x, (size_t)n, ap, aq, (float*)out);
-    else if (out_dtype == TI_BF16) xielu_rows_kernel<bf16><<<blocks, 256, 0, s>>>(x, (size_t)n, ap, aq, (bf16*)out);
+    if (out_dtype == TI_F32) ti_launch_pdl((xielu_rows_kernel<float>), dim3(blocks), dim3(256), 0, s, x, (size_t)n, ap, aq, (float*)out);
+    else if (out_dtype == TI_BF16) ti_launch_pdl((xielu_rows_kernel<bf16>), dim3(blocks), dim3(256), 0, s, x, (size_t)n, ap, aq, (bf16*)out);
     else return ti_fail("xielu_rows: dtype code %d is not supported", out_dtype);
     return ti_check_launch("xielu_rows");
 }
