@@ -12,8 +12,15 @@
 //
 // Softmax weights stay float32 through the second product: a weight is cut into three bfloat16 parts (8 + 8 + 8 bits
 // of its significand) which the softmax threads (one per row) write into tensor memory as the A operand of three
-// products.  So a tile of 64 keys is K / 16 score products of N = 64 and twelve value products, and what bounds it is
-// the tensor core and the shared memory it reads: 1,730 + 1,540 cycles for latent rows of 576 with 256 value columns.
+// products.  So a tile of 64 keys is K / 16 score products of N = 64 and twelve value products.
+//
+// What bounds it (clock stamps in the roles).  Latent rows of 576 with 256 value columns: 7,000 cycles a tile, a chain of
+// 12 value products (137 each), the reload of the value chunks, the last 16 of 36 score products (98 each, issue as much
+// as operand reads) and the softmax; rows of 288: 4,300.  Heads of 128 with a cap: 6,800 a tile and block, of which the
+// softmax takes 4,300, two blocks at a time.  16 heads over 2,048 tokens at positions 0 / 2,048: latent 576 259 / 743 us
+// (416 / 1,232 with one issuing thread and a barrier per chunk), latent 288 93 / 244 (143 / 387), heads of 128 over 4 kv
+// heads with a cap 145 / 281 (177 / 343).  The mma.sync kernel took 2,114 us for the first and 322 for the last as the
+// mean of such two launches.  Steps without a portion stay with that kernel: it cuts a row's keys over blocks.
 //
 // Two forms.  Rows of up to 128 elements with values of their own (NS = 1): the weights take the place of the scores,
 // 224 columns of tensor memory, two blocks per SM that fill one another's gaps; a block is the plain chain of
