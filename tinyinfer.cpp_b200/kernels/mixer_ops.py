@@ -374,7 +374,10 @@ class MixerOps:
                                     and gate.shape[1] == (num_heads if gate_per_head else num_heads * dv)),
                    "attention_options: the gate must be float32 [T, heads] or [T, heads * dv]")
         # a step that brings prompt portions: tcgen05, where the head sizes fill its chunks of 64 elements; its single
-        # tokens ride along as tiles of one token
+        # tokens ride along as tiles of one token.  us against the mma.sync kernel, 16 heads, portions of 2 / 64 / 256
+        # tokens and 64 behind 2,000: shared rows of 576 11.3 / 12.2 / 24.3 / 129 against 21.0 / 23.3 / 47.7 / 292, of 288
+        # 10.8 / 11.6 / 17.8 / 82 against 17.3 / 18.5 / 39.7 / 230, heads of 128 (4 kv heads, a cap) 9.5 / 9.9 / 19.9 / 116
+        # against 9.1 / 11.4 / 29.4 / 203, of 64 7.4 / 7.7 / 13.8 / 73 against 6.5 / 8.5 / 20.4 / 137
         tiles = getattr(step, "lists", {}).get(f"option_tiles_{128 // max(1, min(128, num_heads // num_kv_heads))}")
         if (self.use_tc_attention_options and self.use_umma_attention_options and getattr(step, "max_q_len", 0) > 1
                 and tiles is not None and 0 < tiles.shape[0] <= 65535 and q.dtype == pages.dtype == torch.bfloat16
