@@ -1,6 +1,5 @@
-"""The split-K tcgen05 product of few rows where its rule changes: tiles cut into as many splits as the grid holds (merged
-through the block's ring in one, two and three rounds), whole tiles, and two splits of more units than the grid (merged
-while other units wait)."""
+"""The split-K tcgen05 product of few rows where its rule changes: few tiles cut into two to six splits, whole tiles, and
+two splits of more units than the grid holds."""
 import pytest
 import torch
 

@@ -57,19 +57,10 @@ struct Units {
     __device__ void next() { unit += step; }
 };
 
-// What C holds at W row `n_row` for tokens tok0 .. tok0 + 15 (zeros unless the mode adds to it).  All of it is
-// requested before the first sum is stored: written one after the other, every read would wait behind the store
-// before it (the compiler cannot tell that the addresses differ), a round trip to L2 per row.
-__device__ __forceinline__ void old16(float (&old)[16], int tok0, int n_row, const float* c, int m, int n, int ldc, int mode) {
-#pragma unroll
-    for (int i = 0; i < 16; ++i)
-        old[i] = mode == MODE_ACCUMULATE && tok0 + i < m && n_row < n ? __ldcg(c + (size_t)(tok0 + i) * ldc + n_row) : 0.0f;
-}
-
 // 16 tokens' values of W row `n_row` (this thread's), tokens tok0 .. tok0 + 15.
 __device__ __forceinline__ void finish16(const float (&v)[16], int tok0, int n_row, int lane, float* c,
                                          bf16* out_act, int m, int n, int ldc, int ld_act, int mode,
-                                         const AddGate& add, const float (&old)[16]) {
+                                         const AddGate& add) {
     if (mode == MODE_SWIGLU) {
         // rows of W: 8 gate, their 8 up, ...; lane l (l % 16 < 8) holds a gate row, lane l + 8 its up row
 #pragma unroll
@@ -82,11 +73,18 @@ __device__ __forceinline__ void finish16(const float (&v)[16], int tok0, int n_r
             }
         }
     } else if (n_row < n) {
-        float gate[16];
+        // When adding to C, all old values are requested before the first sum is stored: written
+        // one after the other, every read would wait behind the store before it (the compiler
+        // cannot tell that the addresses differ), a round trip to L2 per row (the down projection
+        // of the 8B shape at 64 rows: 55 -> 34 microseconds).
+        float old[16], gate[16];
         const float bias = add.gate ? add.bias[n_row] : 0.0f;
 #pragma unroll
         for (int i = 0; i < 16; ++i)
             gate[i] = add.gate && tok0 + i < m ? __ldcg(add.gate + (size_t)(tok0 + i) * add.ld + n_row) : 0.0f;
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+            old[i] = mode == MODE_ACCUMULATE && tok0 + i < m ? __ldcg(c + (size_t)(tok0 + i) * ldc + n_row) : 0.0f;
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
             const int tok = tok0 + i;
@@ -208,11 +206,10 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             float* part = ws + (size_t)u.unit * NTOK * BW;     // [NTOK][128]
 #pragma unroll 1
             for (int t0 = 0; t0 < NTOK; t0 += 16) {
-                float v[16], old[16];
-                if (splits == 1) old16(old, t0, n_row, c, m, n, ldc, mode);
+                float v[16];
                 tmem_load16(tmem_base + ((unsigned)(quarter * 32) << 16) + (unsigned)(buf * NTOK + t0), v);
                 if (splits == 1) {
-                    finish16(v, t0, n_row, lane, c, out_act, m, n, ldc, ld_act, mode, add, old);
+                    finish16(v, t0, n_row, lane, c, out_act, m, n, ldc, ld_act, mode, add);
                 } else if (t0 < m) {
 #pragma unroll
                     for (int i = 0; i < 16; ++i) part[(size_t)(t0 + i) * BW + row_in_tile] = v[i];
@@ -229,51 +226,37 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             epilogue_sync();
             if (*ticket_slot != splits - 1) continue;
             __threadfence();
-            // Other blocks wrote the partial sums, so every load is a round trip to L2 of most of a microsecond,
-            // and this merge is the exposed tail of the tile.  When the block has no unit left, its ring is free
-            // (all of its MMAs are through) and takes as many splits' sums as fit, all requested at once without a
-            // register: three of 64 tokens, six of 32, eleven of 16, added in ascending order of the split.  What C
-            // holds is requested before them.
-            const float* first = ws + (size_t)tile * splits * NTOK * BW;
-            const int used = min(NTOK, (m + 15) / 16 * 16);      // tokens whose sums were stored
-            float acc[NTOK], old[NTOK / 16][16];
-#pragma unroll
-            for (int i = 0; i < NTOK / 16; ++i) old16(old[i], i * 16, n_row, c, m, n, ldc, mode);
+            // Other blocks wrote the partial sums, so every load is a round trip to L2 of most of
+            // a microsecond, and this merge is the exposed tail of the tile: the loads of several
+            // splits (as many as the registers hold) are all requested before any is added, and
+            // the additions then follow in ascending order of the split.
+            const float* first = ws + (size_t)tile * splits * NTOK * BW + row_in_tile;
+            constexpr int AT_ONCE = NTOK == 16 ? 8 : NTOK == 32 ? 3 : 1;
+            float acc[NTOK];
 #pragma unroll
             for (int i = 0; i < NTOK; ++i) acc[i] = 0.0f;
-            if (u.unit + u.step >= u.num_units) {
-                constexpr int AT_ONCE = STAGES * (T::STAGE_W + T::STAGE_X) / (NTOK * BW * 4);
-                float* ring = reinterpret_cast<float*>(smem);
-                const int piece = (int)threadIdx.x - 64;         // 0 .. 127: the four epilogue warps
-                for (int s0 = 0; s0 < splits; s0 += AT_ONCE) {
-                    const int here = min(AT_ONCE, splits - s0);
-                    if (s0 > 0) epilogue_sync();
-                    for (int j = 0; j < here; ++j)
-                        for (int at = piece * 4; at < used * BW; at += 512)
-                            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(ring + j * NTOK * BW + at)),
-                                         "l"(first + (size_t)(s0 + j) * NTOK * BW + at) : "memory");
-                    asm volatile("cp.async.wait_all;" ::: "memory");
-                    epilogue_sync();
-                    for (int j = 0; j < here; ++j)
+            for (int s0 = 0; s0 < splits; s0 += AT_ONCE) {
+                float got[AT_ONCE][NTOK];
 #pragma unroll
-                        for (int i = 0; i < NTOK; ++i)
-                            if (i < used) acc[i] += ring[(j * NTOK + i) * BW + row_in_tile];
+                for (int j = 0; j < AT_ONCE; ++j) {
+                    // a split past the last one is read from the last one and counts as zero
+                    const int sj = s0 + j < splits ? s0 + j : splits - 1;
+                    const float* p = first + (size_t)sj * NTOK * BW;
+#pragma unroll
+                    for (int i = 0; i < NTOK; ++i) got[j][i] = __ldcg(p + (size_t)i * BW);
                 }
-            } else {
-                for (int sj = 0; sj < splits; ++sj) {
-                    const float* p = first + (size_t)sj * NTOK * BW + row_in_tile;
-                    float got[NTOK];
 #pragma unroll
-                    for (int i = 0; i < NTOK; ++i) got[i] = i < used ? __ldcg(p + (size_t)i * BW) : 0.0f;
+                for (int j = 0; j < AT_ONCE; ++j) {
+                    const bool live = s0 + j < splits;
 #pragma unroll
-                    for (int i = 0; i < NTOK; ++i) acc[i] += got[i];
+                    for (int i = 0; i < NTOK; ++i) acc[i] += live ? got[j][i] : 0.0f;
                 }
             }
 #pragma unroll
             for (int t0 = 0; t0 < NTOK; t0 += 16) {
                 if (t0 < m)
                     finish16(*reinterpret_cast<const float(*)[16]>(&acc[t0]), t0, n_row, lane, c, out_act, m, n,
-                             ldc, ld_act, mode, add, old[t0 / 16]);
+                             ldc, ld_act, mode, add);
             }
             if (warp == 2 && lane == 0) tickets[tile] = 0;
         }
@@ -289,18 +272,19 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
 
 int padded_rows(int m) { return m <= 16 ? 16 : m <= 32 ? 32 : 64; }
 
-// The number of splits of K.  The grid has `slots` = two blocks per SM.  A lone block takes a k block (16 KB of W) in
-// about 0.29 us, all slots together one per 2.46 ns (the copy bandwidth), so from about 118 tiles on whole tiles keep
-// the memory busy by themselves and every split only adds partial sums to store and merge: one split, or two where
-// the last round of whole tiles would leave most slots idle.  Fewer tiles are cut into as many splits as the slots
-// hold at once, a unit per block.  Times in us at 8 / 32 / 64 rows, against the rule before, which counted one block
-// per SM: 10,240 x 5,120 (80 tiles, 11 -> 3 splits) 30.5 / 36.5 / 57.5 -> 21.3 / 22.9 / 28.3; 5,120 x 8,192 (40 tiles,
-// 11 -> 7) 23.6 / 29.8 / 46.7 -> 18.8 / 22.3 / 28.9 with 6; 51,200 x 5,120 (400 tiles, 4 -> 1) 100 / 144 / 202 -> 85 /
-// 92 / 104; 151,936 x 5,120 (1,187 tiles, 4 -> 1) 266 / 305 -> 237 / 241 at 8 / 32.
+// The number of splits of K.  The grid has two blocks per SM.  A lone block takes a k block (16 KB of W) in about 0.29
+// us, all of them together one per 2.46 ns (the copy bandwidth), so from about 118 tiles on whole tiles keep the memory
+// busy by themselves and every split only adds partial sums to store and merge: one split, or two where the last round of
+// whole tiles would leave most slots idle.  Fewer tiles are cut until there are five units for every four SMs; more units
+// stream no faster and merge longer.  Times in us at 8 / 32 rows, against the rule before, which counted one block per
+// SM: 10,240 x 5,120 (80 tiles, 9 -> 3 splits) 30.5 / 36.5 -> 21.3 / 22.9, 5,120 x 8,192 (40 tiles, 11 -> 5) 23.5 / 29.9
+// -> 20.0 / 22.0, 51,200 x 5,120 (400 tiles, 4 -> 1) 100 / 144 -> 85 / 92 (at 64 rows 202 -> 104), 24,576 x 4,096 (192
+// tiles, 3 -> 1) 39.6 / 52.7 -> 36.5 / 42.3 (at 64 rows 73 -> 52), 32,768 x 2,048 (256 tiles, 4 -> 1) 36.6 / 46.3 -> 23.5 /
+// 25.0 (at 64 rows 65 -> 29), 4,096 x 12,288 (32 tiles, 9 -> 6) 23.2 / 26.5 -> 23.5 / 25.3.
 int choose_splits(int n, int k, int sms) {
     const int tiles = (n + BW - 1) / BW, num_kb = (k + BK - 1) / BK, slots = BLOCKS_PER_SM * sms;
     if (tiles * 5 < slots * 2) {
-        int s = slots / tiles;
+        int s = (sms * 5 / 4 + tiles - 1) / tiles;
         if (s > MAX_SPLITS) s = MAX_SPLITS;
         if (s > num_kb / 2) s = num_kb / 2;
         return s > 1 ? s : 1;
