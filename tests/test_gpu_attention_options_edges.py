@@ -1,0 +1,81 @@
+"""Prompt portions of the attention with options against float64 where the order of the kernel's roles matters."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from test_gpu_attention_options_umma import _attend
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from tinyinfer_b200.kernels import CudaOps
+    return CudaOps(DEV)
+
+
+def _check(ops, heads, kv, dk, dv, shared, page, ctx, new, opt={}, shape_keys=None):
+    """Attends the last ``new[r]`` of ``ctx[r]`` tokens of every request and compares every row with float64."""
+    from tinyinfer_b200.kernels.step_lists import option_tiles, row_tiles
+    g = torch.Generator(device=DEV).manual_seed(dk + dv + heads)
+    ti = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    rnd = lambda *s: torch.randn(s, generator=g, device=DEV)
+    blocks = [-(-c // page) for c in ctx]
+    count = sum(blocks) + 2
+    order = torch.randperm(count, generator=torch.Generator().manual_seed(3)).tolist()
+    table = torch.full((len(ctx), max(blocks)), -1, dtype=torch.int32)
+    q = rnd(sum(new), heads, dk).bfloat16()
+    keys = [rnd(c, kv, dk).bfloat16() for c in ctx]
+    if shape_keys is not None:
+        q, keys = shape_keys(q, keys)
+    values = [k[:, :, :dv] for k in keys] if shared else [rnd(c, kv, dv).bfloat16() for c in ctx]
+    pages = torch.zeros((count, kv * page * (dk if shared else dk + dv)), dtype=torch.bfloat16, device=DEV)
+    for r, c in enumerate(ctx):
+        for b in range(blocks[r]):
+            table[r, b] = order.pop()
+            n = min(page, c - b * page)
+            at = pages[table[r, b]]
+            at[:kv * page * dk].view(kv, page, dk)[:, :n] = keys[r][b * page:b * page + n].transpose(0, 1)
+            if not shared:
+                at[kv * page * dk:].view(kv, page, dv)[:, :n] = values[r][b * page:b * page + n].transpose(0, 1)
+    starts = [c - n for c, n in zip(ctx, new)]
+    positions = [p for s, c in zip(starts, ctx) for p in range(s, c)]
+    t, group = len(positions), heads // kv
+    gp = ops._group_rows(heads, kv)
+    lists = {f"row_tiles_{64 // gp}": ti(row_tiles(new, starts, 64 // gp).tolist()).view(-1, 3),
+             f"option_tiles_{128 // group}": ti(option_tiles(new, starts, 128 // group).tolist()).view(-1, 3)}
+    step = SimpleNamespace(positions=ti(positions), req_of_tok=ti([r for r, n in enumerate(new) for _ in range(n)]),
+                           scratch={}, lists=lists, max_position=max(ctx), max_ctx_len=max(ctx), max_q_len=max(new))
+    cache = SimpleNamespace(pages=pages, block_table=table.to(DEV), page_size=page, writes=True)
+    scale = 2.0 * dk ** -0.5
+    out = torch.full((t, heads * dv), 9.0, dtype=torch.bfloat16, device=DEV)
+    ops.attention_options(q.reshape(t, -1), step, cache, out, heads, kv, dk, dv, scale, window=opt.get("window"),
+                          chunk=opt.get("chunk"), softcap=opt.get("cap"), shared_rows=shared)
+    ops.check_status()
+    at = 0
+    for r, n in enumerate(new):
+        want = _attend(q[at:at + n].double(), keys[r].double(), values[r].double(), step.positions[at:at + n].long(), scale,
+                       opt, None, None)
+        diff = (out[at:at + n].double().view(n, heads, dv) - want).abs()
+        # half a unit of bfloat16, and float32 scores of size dk that shift a weight by some 1e-5
+        assert bool((diff <= want.abs() * 2.0 ** -8 + 1e-4).all()), (r, float(diff.max()))
+        at += n
+
+
+SIZES = [(16, 1, 576, 512, True, 64), (16, 1, 288, 256, True, 64), (16, 4, 128, 128, False, 64), (16, 4, 64, 64, False, 32)]
+
+
+@pytest.mark.parametrize("heads,kv,dk,dv,shared,page", SIZES)
+def test_weights_replaced_without_a_new_reference(ops, heads, kv, dk, dv, shared, page):
+    """A row's largest score lies in its first tile of keys, so that no later tile brings the outputs to a new reference:
+    every tile's weights replace the ones before directly behind the value products that read them.  Portions of as
+    many blocks as fill every SM, over some thirty tiles of keys."""
+    def first_tile_wins(q, keys):
+        q[:, :, 0] = 4.0                       # a common direction: the first 64 keys stand out in it, the others fall off
+        for k in keys:
+            k[:64, :, 0] = 3.0
+            k[64:, :, 0] = torch.linspace(1.0, -1.0, k.shape[0], device=DEV)[64:, None].bfloat16()
+        return q, keys
+    _check(ops, heads, kv, dk, dv, shared, page, [2000, 1700, 90], [600, 500, 90], shape_keys=first_tile_wins)

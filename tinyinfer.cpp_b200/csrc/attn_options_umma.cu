@@ -321,9 +321,9 @@ attn_options_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             if (j > 0) {
                 ok = mbar_wait(p_empty, (j - 1) & 1);
                 if (!ok) break;
+                tc_fence_after();      // behind the value products, which have read the weights that this tile's replace
                 if (__any_sync(0xffffffffu, grow)) {
                     // the output so far was built against m_ref: bring it to the new reference
-                    tc_fence_after();
                     const float factor = grow ? exp2f(m_ref - m_new) : 1.0f;      // 0 if m_ref was -inf
                     l_run *= factor;
 #pragma unroll 1
