@@ -62,6 +62,7 @@ def _check(ops, heads, kv, dk, dv, shared, page, ctx, new, opt={}, shape_keys=No
         # half a unit of bfloat16, and float32 scores of size dk that shift a weight by some 1e-5
         assert bool((diff <= want.abs() * 2.0 ** -8 + 1e-4).all()), (r, float(diff.max()))
         at += n
+    return out
 
 
 SIZES = [(16, 1, 576, 512, True, 64), (16, 1, 288, 256, True, 64), (16, 4, 128, 128, False, 64), (16, 4, 64, 64, False, 32)]
@@ -79,3 +80,13 @@ def test_weights_replaced_without_a_new_reference(ops, heads, kv, dk, dv, shared
             k[64:, :, 0] = torch.linspace(1.0, -1.0, k.shape[0], device=DEV)[64:, None].bfloat16()
         return q, keys
     _check(ops, heads, kv, dk, dv, shared, page, [2000, 1700, 90], [600, 500, 90], shape_keys=first_tile_wins)
+
+
+@pytest.mark.parametrize("heads,kv,size,page", [(16, 4, 128, 64), (16, 4, 64, 16), (6, 6, 128, 16)])
+@pytest.mark.parametrize("cap", [None, 5.0])
+def test_scores_behind_the_weights_they_replace(ops, heads, kv, size, page, cap):
+    """Heads with values of their own: a tile's scores come into the columns of tensor memory that hold the last part of
+    the weights of the tile before.  Two blocks on every SM over an odd and an even number of tiles; repeated launches
+    give the same bits."""
+    outs = [_check(ops, heads, kv, size, size, False, page, [4100, 2048, 65], [1300, 1024, 65], {"cap": cap}) for _ in range(3)]
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])

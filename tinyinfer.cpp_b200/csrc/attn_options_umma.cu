@@ -22,9 +22,11 @@
 // heads with a cap 145 / 281 (177 / 343).  The mma.sync kernel took 2,114 us for the first and 322 for the last as the
 // mean of such two launches.  Steps without a portion stay with that kernel: it cuts a row's keys over blocks.
 //
-// Two forms.  Rows of up to 128 elements with values of their own (NS = 1): the weights take the place of the scores,
-// 224 columns of tensor memory, two blocks per SM that fill one another's gaps; a block is the plain chain of
-// scores, softmax, value products.  Wide shared rows (NS = 2): one block per SM, two score buffers, and the next tile's
+// Two forms.  Rows of up to 128 elements with values of their own (NS = 1): two blocks per SM that fill one another's
+// gaps, with 256 columns of tensor memory each: outputs up to 128, scores 64, weights 96, of which the last 32 lie where
+// the scores were if the outputs take 128.  There the next scores wait for the products with that part (heads of 128
+// without a cap, 256 tokens behind 2,000: 91 -> 96 us); a block is the plain chain of scores, softmax, value products.
+// Wide shared rows (NS = 2): one block per SM, two score buffers, and the next tile's
 // scores issued beside the value products of this one.  Where shared memory holds two tiles (rows up to 320) they wait
 // for nothing; where it holds one (576: queries 147 KB, a tile 74 KB) the part of the row that is no value of this
 // block comes first, and the rest follows as the value products release its chunks.
@@ -108,15 +110,19 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, v
         ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z) : "memory");
 }
 
-// tiles[i] = {request row, first flat token, tokens (<= BM / group)}
-template <int NS>
+// tiles[i] = {request row, first flat token, tokens (<= BM / group)}; NV: chunks of value columns (NS = 1)
+template <int NS, int NV>
 __global__ void __launch_bounds__(threads_of<NS>(), NS == 1 ? 2 : 1)
 attn_options_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kv,
                          const int* __restrict__ tiles, const int* __restrict__ positions,
                          const int* __restrict__ block_table, int bt_stride, int num_pages, int page_size, int num_heads,
                          int num_kv_heads, Shape sh, UmmaOptions opt, bf16* __restrict__ out, int* __restrict__ status) {
     constexpr unsigned TMEM_COLS = NS == 1 ? 256 : 512;
-    constexpr unsigned S_AT = NS == 1 ? 128 : 256, P_AT = NS == 1 ? 128 : 384;      // outputs from column 0 on
+    // Columns of tensor memory: outputs from 0 on, scores, the three parts of the weights (32 columns each).  128 columns
+    // of outputs (NS = 1) leave no room for the last part, which lies where the scores were.
+    constexpr bool LO_IN_SCORES = NS == 1 && NV == 2;
+    constexpr unsigned S_AT = NS == 2 ? 256 : NV * 64, HI_AT = S_AT + NS * BN, MID_AT = HI_AT + 32;
+    constexpr unsigned LO_AT = LO_IN_SCORES ? S_AT : MID_AT + 32;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     unsigned char* ring = smem + sh.chunks * QCHUNK;
@@ -128,7 +134,8 @@ attn_options_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     unsigned long long* p_empty = bars + 6;           // value products done: weights may be rewritten, O is up to date
     unsigned long long* full = bars + 7;              // [stages][2]: the chunks only the scores read, the value chunks
     unsigned long long* empty = bars + 11;
-    unsigned* tmem_slot = (unsigned*)(bars + 15);
+    unsigned long long* lo_read = bars + 15;          // LO_IN_SCORES: the products with the last part of the weights are done
+    unsigned* tmem_slot = (unsigned*)(bars + 16);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int slice = blockIdx.x % sh.slices, kvh = blockIdx.x / sh.slices;
@@ -146,6 +153,7 @@ attn_options_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
         for (int i = 0; i < 2; ++i) { mbar_init(&s_full[i], 1); mbar_init(&s_empty[i], 4); }
         mbar_init(p_full, 4);
         mbar_init(p_empty, 1);
+        mbar_init(lo_read, 1);
         for (int i = 0; i < 2 * sh.stages; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
         mbar_fence_init();
     }
@@ -204,9 +212,10 @@ attn_options_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             }
         }
     } else if (warp == 1 || warp == 6) {
-        // Scores and value products, by one thread (NS = 1: the next scores overwrite the weights, and products run in
-        // the order a thread issues them) or by two (NS = 2: the scores' 36 products of a tile of 576 take a thread
-        // longer to issue than to run).
+        // Scores and value products, by one thread (NS = 1) or by two (NS = 2: the scores' 36 products of a tile of 576
+        // take a thread longer to issue than to run).  Products into different accumulators may run in another order
+        // than they are issued in, so the next scores, where they replace the last part of the weights, wait for the
+        // products that read it; the products with the other two parts keep the tensor cores busy meanwhile.
         if (lane == 0) {
             const unsigned idesc_s = umma_idesc(BM, BN);
             const unsigned idesc_o = umma_idesc(BM, sh.nv * 64, /*b_mn_major=*/true);
@@ -242,11 +251,14 @@ attn_options_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                 tc_fence_after();
                 const unsigned long long b = dv_ + (unsigned long long)((st * sh.places + early) * (CHUNK >> 4));
 #pragma unroll
-                for (int part = 2; part >= 0; --part)                                     // the smallest parts first
+                for (int part = 2; part >= 0; --part) {                                   // the smallest parts first
+                    const unsigned a = tmem_base + (part == 2 ? LO_AT : part == 1 ? MID_AT : HI_AT);
 #pragma unroll
                     for (int ks = 0; ks < BN / 16; ++ks)
-                        umma_bf16_tmem_a(tmem_base, tmem_base + P_AT + part * 32 + ks * 8, b + (unsigned long long)(ks * (2048 >> 4)),
-                                         idesc_o, j > 0 || part < 2 || ks > 0);
+                        umma_bf16_tmem_a(tmem_base, a + ks * 8, b + (unsigned long long)(ks * (2048 >> 4)), idesc_o,
+                                         j > 0 || part < 2 || ks > 0);
+                    if (LO_IN_SCORES && part == 2) umma_commit(lo_read);
+                }
                 umma_commit(&empty[st * 2 + 1]);
                 umma_commit(p_empty);
             };
@@ -262,7 +274,10 @@ attn_options_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                     } else {
                         if (j == 0) all_scores(0);
                         value_products(j);
-                        if (ok && j + 1 < num_kt) all_scores(j + 1);
+                        if (ok && j + 1 < num_kt) {
+                            if (LO_IN_SCORES) ok = mbar_wait(lo_read, j & 1);
+                            if (ok) all_scores(j + 1);
+                        }
                     }
                 }
             } else {
@@ -349,9 +364,9 @@ attn_options_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                     sum[1] += p1;
                     split3_pair(p0, p1, hi[i], mid[i], lo[i]);
                 }
-                tmem_store16(tmem_base + lane_addr + P_AT + c * 16, hi);
-                tmem_store16(tmem_base + lane_addr + P_AT + 32 + c * 16, mid);
-                tmem_store16(tmem_base + lane_addr + P_AT + 64 + c * 16, lo);
+                tmem_store16(tmem_base + lane_addr + HI_AT + c * 16, hi);
+                tmem_store16(tmem_base + lane_addr + MID_AT + c * 16, mid);
+                tmem_store16(tmem_base + lane_addr + LO_AT + c * 16, lo);
             }
             l_run += sum[0] + sum[1];
             asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
@@ -405,7 +420,7 @@ attn_options_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
 }
 
 size_t smem_bytes(const Shape& sh) {
-    return 1024 + (size_t)sh.chunks * QCHUNK + (size_t)sh.stages * sh.places * CHUNK + 16 * 8;
+    return 1024 + (size_t)sh.chunks * QCHUNK + (size_t)sh.stages * sh.places * CHUNK + 17 * 8;
 }
 
 // The cut of the rows, or `places` = 0 where the kernel does not take them.
@@ -488,19 +503,20 @@ extern "C" int ti_attn_options_umma(const void* q, const int* tiles, int num_til
     const size_t smem = smem_bytes(sh);
     const dim3 grid(num_kv_heads * sh.slices, num_tiles);
     cudaStream_t s = (cudaStream_t)stream;
-#define LAUNCH(NS)                                                                                                \
+#define LAUNCH(NS, NV)                                                                                            \
     {                                                                                                             \
         static TiPerDevice configured;                                                                            \
         if (configured.first_use()) {                                                                             \
-            cudaError_t e = cudaFuncSetAttribute(attn_options_umma_kernel<NS>,                                     \
+            cudaError_t e = cudaFuncSetAttribute(attn_options_umma_kernel<NS, NV>,                                 \
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);         \
             if (e != cudaSuccess) return ti_fail("attn_options_umma: %s", cudaGetErrorString(e));                  \
             configured.mark();                                                                                    \
         }                                                                                                         \
-        ti_launch_pdl(attn_options_umma_kernel<NS>, grid, dim3(threads_of<NS>()), smem, s, map_q, map_kv, tiles, positions, block_table,     \
-            bt_stride, num_pages, page_size, num_heads, num_kv_heads, sh, opt, (bf16*)out, status);               \
+        ti_launch_pdl(attn_options_umma_kernel<NS, NV>, grid, dim3(threads_of<NS>()), smem, s, map_q, map_kv,      \
+                      tiles, positions, block_table, bt_stride, num_pages, page_size, num_heads, num_kv_heads, sh, \
+                      opt, (bf16*)out, status);                                                                   \
     }
-    if (shared_rows) LAUNCH(2) else LAUNCH(1)
+    if (shared_rows) LAUNCH(2, 0) else if (sh.nv == 1) LAUNCH(1, 1) else LAUNCH(1, 2)
 #undef LAUNCH
     return ti_check_launch("attn_options_umma");
 }
