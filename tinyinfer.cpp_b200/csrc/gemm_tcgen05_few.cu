@@ -272,30 +272,32 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
 
 int padded_rows(int m) { return m <= 16 ? 16 : m <= 32 ? 32 : 64; }
 
-// The number of splits of K.  The grid has two blocks per SM.  A lone block takes a k block (16 KB of W) in about 0.29
-// us, all of them together one per 2.46 ns (the copy bandwidth), so from about 118 tiles on whole tiles keep the memory
-// busy by themselves and every split only adds partial sums to store and merge: one split, or two where the last round of
-// whole tiles would leave most slots idle.  Fewer tiles are cut until there are five units for every four SMs; more units
-// stream no faster and merge longer.  Times in us at 8 / 32 rows, against the rule before, which counted one block per
-// SM: 10,240 x 5,120 (80 tiles, 9 -> 3 splits) 30.5 / 36.5 -> 21.3 / 22.9, 5,120 x 8,192 (40 tiles, 11 -> 5) 23.5 / 29.9
-// -> 20.0 / 22.0, 51,200 x 5,120 (400 tiles, 4 -> 1) 100 / 144 -> 85 / 92 (at 64 rows 202 -> 104), 24,576 x 4,096 (192
-// tiles, 3 -> 1) 39.6 / 52.7 -> 36.5 / 42.3 (at 64 rows 73 -> 52), 32,768 x 2,048 (256 tiles, 4 -> 1) 36.6 / 46.3 -> 23.5 /
-// 25.0 (at 64 rows 65 -> 29), 4,096 x 12,288 (32 tiles, 9 -> 6) 23.2 / 26.5 -> 23.5 / 25.3.
+// The number of splits of K: the one of least cost, smallest on a tie.  The cost is a model of the time in picoseconds,
+// its constants fitted on a B200 to the splits of 268 matrices (8 to 1,187 tiles, K of 1,024 to 28,672, more than 32 MB) at
+// 8, 32 and 64 rows.  Two blocks per SM take the units in rounds.  All of them together stream a k block (16 KB of W) in
+// 2 ns; the last round takes as long as its whole stream, a lone block's pace (330 ns a k block) or that of the SMs with
+// two of its blocks (2 x 230 ns), whichever is longest, so 96 tiles want three splits (288 units) and not two (192: some
+// SMs have two, others one).  A round starts and ends in 4.4 us; splits cost partial sums to store and to merge.
+// The chosen split is 0.4 % slower than the fastest of its matrix on average, at most 11 % (4,096 x 5,120 at 8 rows).
+// Against five units for every four SMs and whole tiles from 118 on, us at 8 / 32 / 64 rows: 38,016 x 14,336 (297 tiles, 1
+// -> 4 splits) 217 / 219 / 230 -> 173 / 180 / 198, 12,288 x 2,048 (96 tiles, 2 -> 3) 14.6 / 15.9 / 20.3 -> 13.4 / 14.8 /
+// 19.9, 2,048 x 12,288 (16 tiles, 12 -> 9) 16.4 / 19.7 / 27.6 -> 16.4 / 18.2 / 25.1; against the rule before that, which
+// counted one block per SM: 51,200 x 5,120 (400 tiles, 4 -> 1) 100 / 144 / 202 -> 85 / 92 / 104, 10,240 x 5,120 (80 tiles,
+// 9 -> 3) 30.5 / 36.5 / 57.5 -> 21.3 / 22.9 / 28.3.
 int choose_splits(int n, int k, int sms) {
-    const int tiles = (n + BW - 1) / BW, num_kb = (k + BK - 1) / BK, slots = BLOCKS_PER_SM * sms;
-    if (tiles * 5 < slots * 2) {
-        int s = (sms * 5 / 4 + tiles - 1) / tiles;
-        if (s > MAX_SPLITS) s = MAX_SPLITS;
-        if (s > num_kb / 2) s = num_kb / 2;
-        return s > 1 ? s : 1;
-    }
-    // picoseconds: full rounds at the bandwidth, the rest at the bandwidth or a block's own pace; a split unit's sums
-    auto cost = [&](int s) {
-        const long long units = (long long)tiles * s, kb = (num_kb + s - 1) / s, left = units % slots;
-        const long long tail = left * kb * 2460 > kb * 290000 ? left * kb * 2460 : left ? kb * 290000 : 0;
-        return units / slots * slots * kb * 2460 + tail + (s > 1 ? 3000000 + units * 60000 : 0);
+    const long long tiles = (n + BW - 1) / BW, num_kb = (k + BK - 1) / BK, slots = BLOCKS_PER_SM * sms;
+    auto cost = [&](long long s) {
+        const long long units = tiles * s, kb = (num_kb + s - 1) / s, left = units % slots;
+        long long pace = left * 2000, busiest = (left + sms - 1) / sms * 230000;
+        if (pace < busiest) pace = busiest;
+        if (pace < 330000) pace = 330000;
+        return units / slots * (slots * kb * 2000 + 4400000) + (left ? kb * pace + 4400000 : 0) +
+               (s > 1 ? 660000 + s * 400000 + units * 5000 : 0);
     };
-    return num_kb >= 4 && cost(2) < cost(1) ? 2 : 1;
+    int best = 1;
+    for (int s = 2; s <= MAX_SPLITS && s * 2 <= num_kb; ++s)
+        if (cost(s) < cost(best)) best = s;
+    return best;
 }
 
 int device_sms() {
