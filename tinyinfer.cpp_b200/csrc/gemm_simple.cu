@@ -306,13 +306,7 @@ gemm_rows_kernel(const float* a, const TW* __restrict__ w, float* c, int m, int 
 
 template <typename TW, int MT>
 int launch_rows(const float* a, const TW* w, float* c, int m, int n, int k, int lda, int ldw, int ldc, int accumulate,
-                cudaStream_t s) {
-    const int spans = (k + SPAN - 1) / SPAN;
-    const int most = sizeof(TW) == 2 ? 4 : 2;                    // shared memory: 33 KB of float32 weights a warp
-    const int ws = spans < most ? spans : most;
-    // one span: four column groups share the rows of A where there are columns enough for all SMs
-    const int wc = ws == 1 && n > 2048 ? 4 : 1;
-    const size_t smem = rows_smem<TW>(ws, wc, MT);
+                int ws, int wc, size_t smem, cudaStream_t s) {
     static TiPerDevice seen;
     if (seen.first_use()) {
         if (cudaFuncSetAttribute(gemm_rows_kernel<TW, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) !=
@@ -346,31 +340,65 @@ int launch_tiles(const TA* a, const TW* w, float* c, int m, int n, int k, int ld
     return ti_check_launch("gemm_simple");
 }
 
-template <typename TW>
-int launch_few(const float* a, const TW* w, float* c, int m, int n, int k, int lda, int ldw, int ldc, int accumulate,
-               cudaStream_t s) {
-    if (m == 1) return launch_rows<TW, 1>(a, w, c, m, n, k, lda, ldw, ldc, accumulate, s);
-    if (m == 2) return launch_rows<TW, 2>(a, w, c, m, n, k, lda, ldw, ldc, accumulate, s);
-    if (m <= 4) return launch_rows<TW, 4>(a, w, c, m, n, k, lda, ldw, ldc, accumulate, s);
-    return launch_rows<TW, 8>(a, w, c, m, n, k, lda, ldw, ldc, accumulate, s);
+int device_sms() {
+    int device = 0, sms = 0;
+    cudaGetDevice(&device);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    return sms;
 }
-template <typename TW>
-int launch_few(const bf16*, const TW*, float*, int, int, int, int, int, int, int, cudaStream_t) { return -1; }
+
+// Whether the streaming kernel takes a product of up to 32 rows (both kernels give the same bits): by a model of the two
+// times in ns, fitted to 2,926 products (8 to 32,768 columns, K of 8 to 12,288, 1 to 32 rows, both types of weights).  The
+// streaming kernel passes a round's weights once for every MT rows and holds few blocks on an SM; a tile of 64 rows costs
+// the same whatever it holds, and groups of warps beside one another slow each other down.  The choice lies 0.5 % above
+// the faster one on average.  us, streaming / tiles: float32 weights, 32 rows of 8 x 8 23 / 2.3, 17 of 128 x 64 21.5 / 4.3,
+// 32 of 4,096 x 12,288 1,410 / 342, 8 of 1,024 x 1,024 16 / 29; bfloat16 weights, 17 rows of 12,288 x 1,024 60 / 63, 4 of
+// 1,024 x 3,072 9.5 / 91.
+bool rows_pay(int m, int n, int k, int w_size, int mt, int ws, int wc, size_t smem) {
+    const int sms = device_sms();
+    const double kk = k < SEG ? k : SEG, segs = (k + SEG - 1) / SEG;
+    const int blocks = (n + wc * COLS - 1) / (wc * COLS), rounds = ((int)segs + 4 * ws - 1) / (4 * ws);
+    const int per_sm = (int)(227 * 1024 / (smem + 1024)) < 16 ? (int)(227 * 1024 / (smem + 1024)) : 16;
+    const int waves = (blocks + sms * per_sm - 1) / (sms * per_sm), passes = (m + mt - 1) / mt;
+    const double rows = 480 + (double)waves * rounds * (640 + passes * (730 + 370 * mt + kk * (6.8 + 3.2 * mt)));
+    const double beside = segs < 4 ? segs : 4, alone = (int)(segs + 3) / 4;
+    const double shared = segs * ((n + BN - 1) / BN) * 0.43 / sms;
+    const double tiles = 1500 + (int)(kk + BK - 1) / BK * 880 * (1 + 0.32 * (beside - 1)) * (alone > shared ? alone : shared);
+    return rows < tiles;
+}
 
 template <typename TA, typename TW>
 int launch(const TA* a, const TW* w, float* c, int m, int n, int k, int lda, int ldw, int ldc, int accumulate,
            cudaStream_t s) {
-    // Up to 32 rows by the streaming kernel: a tile of 64 rows pays for 64 whatever it holds (17 rows of 1,024 x
-    // 2,048: 38 against 65 us, of 151,936 x 1,024: 454 against 528 us, of 4,096 x 1,024: 28 against 35 us).
     // Operands that cannot be read 16 bytes at a time take the tiles, whose loader falls back to single elements.
-    constexpr bool f32_rows = sizeof(TA) == 4;
-    if (f32_rows && m <= MAX_ROWS && aligned16<TA>(a, lda) && aligned16<TW>(w, ldw) && k % (16 / (int)sizeof(TW)) == 0 &&
-        k % 4 == 0)
-        return launch_few(a, w, c, m, n, k, lda, ldw, ldc, accumulate, s);
-    if (!(aligned16<TA>(a, lda) && aligned16<TW>(w, ldw)))
-        return launch_tiles<TA, TW, 2, false>(a, w, c, m, n, k, lda, ldw, ldc, accumulate, s);
-    if (k <= 2 * SEG) return launch_tiles<TA, TW, 2, true>(a, w, c, m, n, k, lda, ldw, ldc, accumulate, s);
-    return launch_tiles<TA, TW, 4, true>(a, w, c, m, n, k, lda, ldw, ldc, accumulate, s);
+    const bool aligned = aligned16<TA>(a, lda) && aligned16<TW>(w, ldw);
+    if constexpr (sizeof(TA) == 4) {
+        if (m <= MAX_ROWS && aligned && k % (16 / (int)sizeof(TW)) == 0 && k % 4 == 0) {
+            const int mt = m <= 2 ? m : m <= 4 ? 4 : 8, spans = (k + SPAN - 1) / SPAN;
+            const int most = sizeof(TW) == 2 ? 4 : 2;            // shared memory: 33 KB of float32 weights a warp
+            const int ws = spans < most ? spans : most;
+            // one span: four column groups share the rows of A where there are columns enough for all SMs
+            const int wc = ws == 1 && n > 2048 ? 4 : 1;
+            const size_t smem = rows_smem<TW>(ws, wc, mt);
+            if (rows_pay(m, n, k, sizeof(TW), mt, ws, wc, smem)) {
+                if (mt == 1) return launch_rows<TW, 1>(a, w, c, m, n, k, lda, ldw, ldc, accumulate, ws, wc, smem, s);
+                if (mt == 2) return launch_rows<TW, 2>(a, w, c, m, n, k, lda, ldw, ldc, accumulate, ws, wc, smem, s);
+                if (mt == 4) return launch_rows<TW, 4>(a, w, c, m, n, k, lda, ldw, ldc, accumulate, ws, wc, smem, s);
+                return launch_rows<TW, 8>(a, w, c, m, n, k, lda, ldw, ldc, accumulate, ws, wc, smem, s);
+            }
+        }
+    }
+    // Groups of warps by segments and tiles; a group without a segment still helps to store a tile, and leaves room for
+    // fewer tiles on an SM.  us at one, two and four groups (float32): 2,048 x 32,768 x 256 759 / 896 / 1,323, 100 x 4,096 x
+    // 64 5.6 / 5.9 / 5.0, 466 x 1,000 x 1,001 (rows not aligned) 66 / 65 / 37.
+    const long long tiles = (long long)((n + BN - 1) / BN) * ((m + BM - 1) / BM);
+    const int sms = device_sms();
+    const int groups = tiles <= sms || k > 2 * SEG ? 4 : tiles <= 2 * sms || k > SEG ? 2 : 1;
+#define TILES(G)                                                                                          \
+    (aligned ? launch_tiles<TA, TW, G, true>(a, w, c, m, n, k, lda, ldw, ldc, accumulate, s)               \
+             : launch_tiles<TA, TW, G, false>(a, w, c, m, n, k, lda, ldw, ldc, accumulate, s))
+    return groups == 4 ? TILES(4) : groups == 2 ? TILES(2) : TILES(1);
+#undef TILES
 }
 
 }  // namespace
