@@ -17,6 +17,7 @@ constexpr int MAX_HEAD_DIM = 256;
 constexpr int WARPS = 4;
 
 enum { TI_ERR_BAD_PAGE = 1 };
+template <int N> struct Int { static constexpr int value = N; };
 
 template <typename TQ, typename TC>
 __global__ void __launch_bounds__(WARPS * 32)
@@ -301,18 +302,17 @@ qk_norm_rope_store_one_kernel(const float* qkv, int qkv_stride,
 // ATT_WARPS, ...), each with an online softmax of its own, merged at the end: an order that depends on the row
 // alone.  A warp's time is the latency of its loads and of the sum over its lanes, so it asks for the keys and
 // values of AHEAD keys at once and adds their dot products side by side; the online softmax then takes them one
-// after the other.  PER_LANE elements of a head per lane.  (One key at a time and four warps: the 72 calls of a pass
-// over three prompts of up to 197 tokens and eight more steps, 16 heads of 128, took 9.6 of its 60 ms; with the keys
-// asked for ahead the calls of a pass that overlap their neighbours' ends show 3.7 ms.)
+// after the other (so AHEAD changes no bit), and fewer keys than that are taken in halves.  PER_LANE elements of a head
+// per lane.  Keys asked for ahead cost registers and so blocks on an SM: many blocks cover one another's latency and take
+// one key at a time (see the launch).
 constexpr int ATT_WARPS = 8;
 
-template <typename TQ, typename TC, int PER_LANE>
-__global__ void __launch_bounds__(ATT_WARPS * 32)
+template <typename TQ, typename TC, int PER_LANE, int AHEAD>
+__global__ void __launch_bounds__(ATT_WARPS * 32, AHEAD > 1 ? 1 : PER_LANE <= 4 ? 8 : 4)
 paged_attention_simple_kernel(const TQ* q, const int* __restrict__ rows, const int* __restrict__ positions,
                               const int* __restrict__ req_of_tok, const int* __restrict__ block_table, int bt_stride,
                               const TC* pages, int num_pages, int page_size, int num_heads, int num_kv_heads,
                               int head_dim, int window, float scale, TQ* out, int* __restrict__ status) {
-    constexpr int AHEAD = PER_LANE > 4 ? 4 : 8;
     __shared__ float so[ATT_WARPS][32 * PER_LANE];
     __shared__ float sm[ATT_WARPS], sl[ATT_WARPS];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -336,16 +336,17 @@ paged_attention_simple_kernel(const TQ* q, const int* __restrict__ rows, const i
     float m = -INFINITY, l = 0.0f;
     bool bad = false;
     const size_t to_values = (size_t)num_kv_heads * page_size * head_dim;
-    for (int p0 = lo + warp; p0 <= pos; p0 += AHEAD * ATT_WARPS) {
-        TC kv[AHEAD][PER_LANE], vv[AHEAD][PER_LANE];
-        bool there[AHEAD];
+    // N keys, ATT_WARPS apart, of which the last is no later than pos
+    auto take = [&](int p0, auto n) {
+        constexpr int N = decltype(n)::value;
+        TC kv[N][PER_LANE], vv[N][PER_LANE];
+        bool there[N];
 #pragma unroll
-        for (int j = 0; j < AHEAD; ++j) {
+        for (int j = 0; j < N; ++j) {
             const int p = p0 + j * ATT_WARPS;
-            const int page = p <= pos ? table[p / page_size] : 0;
-            const bool known = page >= 0 && page < num_pages;
-            bad |= !known;
-            there[j] = p <= pos && known;
+            const int page = table[p / page_size];
+            there[j] = page >= 0 && page < num_pages;
+            bad |= !there[j];
             const TC* kp = pages + (((size_t)page * 2 * num_kv_heads + kvh) * page_size + p % page_size) * head_dim;
 #pragma unroll
             for (int i = 0; i < PER_LANE; ++i) {
@@ -355,9 +356,9 @@ paged_attention_simple_kernel(const TQ* q, const int* __restrict__ rows, const i
                 vv[j][i] = on ? kp[to_values + d] : from_f32<TC>(0.0f);
             }
         }
-        float s[AHEAD];
+        float s[N];
 #pragma unroll
-        for (int j = 0; j < AHEAD; ++j) {
+        for (int j = 0; j < N; ++j) {
             s[j] = 0.0f;
 #pragma unroll
             for (int i = 0; i < PER_LANE; ++i) s[j] = fmaf(qv[i], to_f32(kv[j][i]), s[j]);
@@ -365,9 +366,9 @@ paged_attention_simple_kernel(const TQ* q, const int* __restrict__ rows, const i
 #pragma unroll
         for (int x = 16; x > 0; x >>= 1)
 #pragma unroll
-            for (int j = 0; j < AHEAD; ++j) s[j] += __shfl_xor_sync(0xffffffffu, s[j], x);
+            for (int j = 0; j < N; ++j) s[j] += __shfl_xor_sync(0xffffffffu, s[j], x);
 #pragma unroll
-        for (int j = 0; j < AHEAD; ++j) {
+        for (int j = 0; j < N; ++j) {
             if (!there[j]) continue;
             const float sc = s[j] * scale;
             const float m_new = fmaxf(m, sc);
@@ -378,12 +379,18 @@ paged_attention_simple_kernel(const TQ* q, const int* __restrict__ rows, const i
             for (int i = 0; i < PER_LANE; ++i) o[i] = fmaf(pr, to_f32(vv[j][i]), o[i] * alpha);
             m = m_new;
         }
-    }
+    };
+    int p = lo + warp;
+    for (; p + (AHEAD - 1) * ATT_WARPS <= pos; p += AHEAD * ATT_WARPS) take(p, Int<AHEAD>{});
+    if (AHEAD > 4 && p + 3 * ATT_WARPS <= pos) { take(p, Int<4>{}); p += 4 * ATT_WARPS; }
+    if (AHEAD > 2 && p + ATT_WARPS <= pos) { take(p, Int<2>{}); p += 2 * ATT_WARPS; }
+    if (p <= pos) take(p, Int<1>{});
     if (bad && lane == 0) atomicCAS(status, 0, TI_ERR_BAD_PAGE);
 #pragma unroll
     for (int i = 0; i < PER_LANE; ++i) so[warp][lane + 32 * i] = o[i];
     if (lane == 0) { sm[warp] = m; sl[warp] = l; }
     __syncthreads();
+    if (threadIdx.x >= 32 * PER_LANE) return;
     float mm = -INFINITY;
 #pragma unroll
     for (int w = 0; w < ATT_WARPS; ++w) mm = fmaxf(mm, sm[w]);
@@ -395,7 +402,8 @@ paged_attention_simple_kernel(const TQ* q, const int* __restrict__ rows, const i
     }
     const float inv = 1.0f / ltot;
     TQ* oh = out + ((size_t)t * num_heads + h) * head_dim;
-    for (int d = threadIdx.x; d < head_dim; d += ATT_WARPS * 32) {
+    if (threadIdx.x < head_dim) {
+        const int d = threadIdx.x;
         float acc = 0.0f;
 #pragma unroll
         for (int w = 0; w < ATT_WARPS; ++w) acc = fmaf(so[w][d], wt[w], acc);
@@ -482,18 +490,33 @@ extern "C" int ti_paged_attention_simple(const void* q, int q_dtype, const int* 
                num_heads, num_kv_heads);
     dim3 grid(num_rows, num_heads);
     cudaStream_t s = (cudaStream_t)stream;
+    // Few blocks wait for their loads, many cover one another's.  us at 8 / 4 / 1 keys ahead, 16 heads of 128: 3 requests
+    // with one token at 200 keys (48 blocks) 8.2 / 8.7 / 13, 16 tokens of one at up to 30 keys (256) 4.1 / 4.4 / 4.6, of 8
+    // requests 64 tokens each (8,192) 92 / 67 / 59, of 64 requests 16 tokens each (16,384) 111 / 77 / 54 (one key at a time
+    // by four warps: 54, 11, 82 and 57)
+    int device = 0, sms = 0;
+    cudaGetDevice(&device);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    const long long blocks = (long long)num_rows * num_heads;
     const int per_lane = head_dim <= 32 ? 1 : head_dim <= 64 ? 2 : head_dim <= 128 ? 4 : 8;
-#define LAUNCH(TQ, TC, N)                                                                       \
-    ti_launch_pdl(paged_attention_simple_kernel<TQ, TC, N>, grid, dim3(ATT_WARPS * 32), 0, s,   \
+#define LAUNCH(TQ, TC, N, A)                                                                    \
+    ti_launch_pdl(paged_attention_simple_kernel<TQ, TC, N, A>, grid, dim3(ATT_WARPS * 32), 0, s, \
         (const TQ*)q, rows, positions, req_of_tok, block_table, bt_stride, (const TC*)pages,     \
         num_pages, page_size, num_heads, num_kv_heads, head_dim, window, scale, (TQ*)out, status)
-#define CALL(TQ, TC)                                                                           \
-    if (per_lane == 1) LAUNCH(TQ, TC, 1);                                                       \
-    else if (per_lane == 2) LAUNCH(TQ, TC, 2);                                                  \
-    else if (per_lane == 4) LAUNCH(TQ, TC, 4);                                                  \
-    else LAUNCH(TQ, TC, 8)
+#define PICK(TQ, TC, N)                                                                         \
+    {                                                                                           \
+        if (blocks <= sms) LAUNCH(TQ, TC, N, 8);                                                 \
+        else if (blocks <= 2 * sms) LAUNCH(TQ, TC, N, 4);                                        \
+        else LAUNCH(TQ, TC, N, 1);                                                               \
+    }
+#define CALL(TQ, TC)                                                                            \
+    if (per_lane == 1) PICK(TQ, TC, 1)                                                           \
+    else if (per_lane == 2) PICK(TQ, TC, 2)                                                      \
+    else if (per_lane == 4) PICK(TQ, TC, 4)                                                      \
+    else PICK(TQ, TC, 8)
     TI_DISPATCH_QC(q_dtype, cache_dtype, CALL)
 #undef CALL
+#undef PICK
 #undef LAUNCH
     return ti_check_launch("paged_attention_simple");
 }
