@@ -16,8 +16,10 @@ def ops():
     return CudaOps(DEV)
 
 
-def _check(ops, heads, kv, dk, dv, shared, page, ctx, new, opt={}, shape_keys=None):
-    """Attends the last ``new[r]`` of ``ctx[r]`` tokens of every request and compares every row with float64."""
+def _check(ops, heads, kv, dk, dv, shared, page, ctx, new, opt={}, shape_keys=None, left=0.0, released=False):
+    """Attends the last ``new[r]`` of ``ctx[r]`` tokens of every request and compares every row with float64.  ``left`` fills
+    what earlier requests have left in the pool (a number, or "large" for rows of random large numbers); ``released``:
+    pages wholly in front of the first visible key of a request's first new token are gone from its table."""
     from tinyinfer_b200.kernels.step_lists import option_tiles, row_tiles
     g = torch.Generator(device=DEV).manual_seed(dk + dv + heads)
     ti = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
@@ -31,7 +33,8 @@ def _check(ops, heads, kv, dk, dv, shared, page, ctx, new, opt={}, shape_keys=No
     if shape_keys is not None:
         q, keys = shape_keys(q, keys)
     values = [k[:, :, :dv] for k in keys] if shared else [rnd(c, kv, dv).bfloat16() for c in ctx]
-    pages = torch.zeros((count, kv * page * (dk if shared else dk + dv)), dtype=torch.bfloat16, device=DEV)
+    pages = torch.empty((count, kv * page * (dk if shared else dk + dv)), dtype=torch.bfloat16, device=DEV)
+    pages.copy_(1000.0 * rnd(*pages.shape)) if left == "large" else pages.fill_(left)
     for r, c in enumerate(ctx):
         for b in range(blocks[r]):
             table[r, b] = order.pop()
@@ -41,6 +44,11 @@ def _check(ops, heads, kv, dk, dv, shared, page, ctx, new, opt={}, shape_keys=No
             if not shared:
                 at[kv * page * dk:].view(kv, page, dv)[:, :n] = values[r][b * page:b * page + n].transpose(0, 1)
     starts = [c - n for c, n in zip(ctx, new)]
+    if released:
+        for r, start in enumerate(starts):
+            first = max(0, start - opt["window"] + 1) if opt.get("window") else start // opt["chunk"] * opt["chunk"]
+            pages[table[r, :first // page].long()] = float("nan")
+            table[r, :first // page] = -1
     positions = [p for s, c in zip(starts, ctx) for p in range(s, c)]
     t, group = len(positions), heads // kv
     gp = ops._group_rows(heads, kv)
@@ -90,3 +98,16 @@ def test_scores_behind_the_weights_they_replace(ops, heads, kv, size, page, cap)
     give the same bits."""
     outs = [_check(ops, heads, kv, size, size, False, page, [4100, 2048, 65], [1300, 1024, 65], {"cap": cap}) for _ in range(3)]
     assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+
+
+@pytest.mark.parametrize("heads,kv,dk,dv,shared,page", SIZES + [(24, 1, 96, 64, True, 16), (6, 2, 128, 128, False, 16)])
+@pytest.mark.parametrize("left", [float("nan"), float("inf"), "large"])
+@pytest.mark.parametrize("opt", [{}, {"window": 70}, {"chunk": 150, "cap": 4.0}])
+def test_what_earlier_requests_left(ops, monkeypatch, heads, kv, dk, dv, shared, page, left, opt):
+    """A reused page holds infinities and NaN behind a context's end, and pages that a window or a chunk has passed are
+    gone: no query may see either, on tcgen05, on mma.sync, and in a step of single tokens."""
+    ctx, new = [64, 1, 65, 400, 63, 200, 130, 77], [64, 1, 65, 140, 3, 1, 2, 77]
+    for umma in (True, False):
+        monkeypatch.setattr(ops, "use_umma_attention_options", umma)
+        _check(ops, heads, kv, dk, dv, shared, page, ctx, new, opt, left=left, released=bool(opt))
+    _check(ops, heads, kv, dk, dv, shared, page, ctx, [1] * len(ctx), opt, left=left, released=bool(opt))

@@ -195,18 +195,23 @@ attn_options_tc_kernel(const bf16* q, const int* __restrict__ tiles, const int* 
                 }
             }
             const bool valid = pg >= 0;
+            // rows outside the keys of this block's queries come as zeros: behind the request's last token a page may hold
+            // what an earlier request left, and a weight of zero times an infinity is not zero
+            const int own_lo = max(0, kv_lo - key0);
+            const unsigned own_rows = valid ? min(16, pos_last + 1 - key0) - own_lo : 0;
+            auto own = [&](int row) { return (unsigned)(row - own_lo) < own_rows; };
             const bf16* base = pages + (valid ? (size_t)pg * page_elems : 0);
             const bf16* ksrc = base + (valid ? ((size_t)kvh * page_size + key0 % page_size) * dk : 0);
             for (int c = threadIdx.x; c < 16 * chunks; c += WARPS * 32)
                 cp_async16(kdst + (size_t)(r * 16 + c / chunks) * k_row + (c % chunks) * 16,
-                           ksrc + (valid ? c * 8 : 0), valid);
+                           ksrc + (valid ? c * 8 : 0), own(c / chunks));
             if (!opt.shared_rows) {
                 const bf16* vsrc = base + (valid ? v_base + ((size_t)kvh * page_size + key0 % page_size) * dv
                                                        + slice * DVS : 0);
                 constexpr int VCH = DVS / 8;
                 for (int c = threadIdx.x; c < 16 * VCH; c += WARPS * 32)
                     cp_async16(vdst + (size_t)(r * 16 + c / VCH) * V_ROW + (c % VCH) * 16,
-                               vsrc + (valid ? (size_t)(c / VCH) * dv + (c % VCH) * 8 : 0), valid);
+                               vsrc + (valid ? (size_t)(c / VCH) * dv + (c % VCH) * 8 : 0), own(c / VCH));
             }
         }
     };

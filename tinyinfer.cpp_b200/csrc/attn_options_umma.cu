@@ -34,6 +34,8 @@
 // Order: warp 0 issues TMA, warp 1 the products (NS = 2: the scores, warp 6 the value products), warps 2-5 are the
 // softmax.  Every wait on an mbarrier is bounded: on a timeout the block records status 2, frees its tensor memory and
 // returns.
+#include <utility>
+
 #include "sm100.cuh"
 
 namespace {
@@ -114,6 +116,7 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, v
 template <int NS, int NV>
 __global__ void __launch_bounds__(threads_of<NS>(), NS == 1 ? 2 : 1)
 attn_options_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kv,
+                         const __grid_constant__ CUtensorMap map_8, const __grid_constant__ CUtensorMap map_1,
                          const int* __restrict__ tiles, const int* __restrict__ positions,
                          const int* __restrict__ block_table, int bt_stride, int num_pages, int page_size, int num_heads,
                          int num_kv_heads, Shape sh, UmmaOptions opt, bf16* __restrict__ out, int* __restrict__ status) {
@@ -178,18 +181,33 @@ attn_options_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
         }
         for (int j = 0; j < num_kt && ok; ++j) {
             const int st = j % sh.stages, phase = (j / sh.stages) & 1;
-            int row = oob_row;                        // where this lane's run of keys begins
-            if (lane < BN / sh.run) {
-                const int key0 = (kt_lo + j) * BN + lane * sh.run;
-                if (key0 <= pos_last && key0 + sh.run > kv_lo) {
-                    const int pg = table[key0 / page_size];
-                    if (pg >= 0 && pg < num_pages)
-                        row = pg * per_page + kvh * page_size + key0 % page_size;
-                    else
-                        atomicCAS(status, 0, TI_ERR_BAD_PAGE);
-                }
-            }
+            const int base = (kt_lo + j) * BN, from_row = kv_lo - base, to_row = pos_last + 1 - base;
+            // where `height` rows of the tile from row `at` on begin in the pool
+            auto place = [&](int at, int height) {
+                const int key0 = base + at;
+                if (at >= to_row || at + height <= from_row) return oob_row;
+                const int pg = table[key0 / page_size];
+                if (pg >= 0 && pg < num_pages) return pg * per_page + kvh * page_size + key0 % page_size;
+                atomicCAS(status, 0, TI_ERR_BAD_PAGE);
+                return oob_row;
+            };
+            // this lane's rows of the tile: a run of keys
+            const CUtensorMap* map = &map_kv;
+            bool mine = lane < BN / sh.run;
+            int at = lane * sh.run, row = mine ? place(at, sh.run) : oob_row;
             for (int part = early > 0 ? 0 : 1; part < 2; ++part) {
+                if (part == 1 && (from_row > 0 || to_row < BN)) {
+                    // Values outside the keys that this block's queries see must be zeros: behind the request's last token
+                    // a page may hold what an earlier request left, and a weight of zero times an infinity is not zero.
+                    // They come in groups of eight rows, a group at either end row by row (lanes 8 to 15, 16 to 23).
+                    const int cut = to_row < BN && to_row % 8 ? to_row / 8 : -1;
+                    const int cut_lo = from_row > 0 && from_row % 8 && from_row / 8 != cut ? from_row / 8 : -1;
+                    const int eight = lane < 8 ? lane : lane < 16 ? cut : cut_lo;
+                    map = lane < 8 ? &map_8 : &map_1;
+                    mine = lane < 8 ? lane != cut && lane != cut_lo : lane < 24 && eight >= 0;
+                    at = eight * 8 + (lane < 8 ? 0 : lane % 8);
+                    row = mine ? place(at, lane < 8 ? 8 : 1) : oob_row;
+                }
                 unsigned long long* bar = &full[st * 2 + part];
                 const int from = part == 0 ? 0 : early, to = part == 0 ? early : sh.places;
                 if (lane == 0) {
@@ -198,7 +216,7 @@ attn_options_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                 }
                 ok = __shfl_sync(0xffffffffu, ok, 0);
                 if (!ok) break;
-                if (lane >= BN / sh.run) continue;
+                if (!mine) continue;
                 for (int p = from; p < to; ++p) {
                     int c, y = row;
                     if (sh.shared) {                  // the row's chunks outside the slice, then the slice's
@@ -207,7 +225,7 @@ attn_options_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                         c = p < sh.chunks ? p : slice * sh.nv + p - sh.chunks;
                         if (p >= sh.chunks && row != oob_row) y = row + to_v;
                     }
-                    tma_load_2d(ring + (st * sh.places + p) * CHUNK + lane * sh.run * 128, &map_kv, bar, c * 64, y);
+                    tma_load_2d(ring + (st * sh.places + p) * CHUNK + at * 128, map, bar, c * 64, y);
                 }
             }
         }
@@ -490,15 +508,17 @@ extern "C" int ti_attn_options_umma(const void* q, const int* tiles, int num_til
     const Shape sh = shape_of(dk, dv, page_size, shared_rows, group);
     const long long pool_rows = (long long)num_pages * num_kv_heads * page_size * (shared_rows ? 1 : 2);
     TI_REQUIRE(pool_rows < (1LL << 31) - 1, "attn_options_umma: the page pool has too many token slots");
-    CUtensorMap map_q, map_kv;
+    CUtensorMap map_q, map_kv, map_8, map_1;
     const cuuint64_t qdims[3] = {(cuuint64_t)dk, (cuuint64_t)num_heads, (cuuint64_t)num_tokens};
     const cuuint64_t qstrides[2] = {(cuuint64_t)dk * 2, (cuuint64_t)num_heads * dk * 2};
     const cuuint32_t qbox[3] = {64, (cuuint32_t)group, (cuuint32_t)(BM / group)};
     if (int rc = make_map(&map_q, q, 3, qdims, qstrides, qbox)) return rc;
     const cuuint64_t kdims[2] = {(cuuint64_t)dk, (cuuint64_t)pool_rows};
     const cuuint64_t kstrides[1] = {(cuuint64_t)dk * 2};
-    const cuuint32_t kbox[2] = {64, (cuuint32_t)sh.run};
-    if (int rc = make_map(&map_kv, pages, 2, kdims, kstrides, kbox)) return rc;
+    for (auto [map, rows] : {std::pair<CUtensorMap*, int>{&map_kv, sh.run}, {&map_8, 8}, {&map_1, 1}}) {
+        const cuuint32_t kbox[2] = {64, (cuuint32_t)rows};
+        if (int rc = make_map(map, pages, 2, kdims, kstrides, kbox)) return rc;
+    }
     UmmaOptions opt = {window, chunk, scale, softcap, head_scale, sink, gate, gate_stride, gate_per_head};
     const size_t smem = smem_bytes(sh);
     const dim3 grid(num_kv_heads * sh.slices, num_tiles);
@@ -513,7 +533,7 @@ extern "C" int ti_attn_options_umma(const void* q, const int* tiles, int num_til
             configured.mark();                                                                                    \
         }                                                                                                         \
         ti_launch_pdl(attn_options_umma_kernel<NS, NV>, grid, dim3(threads_of<NS>()), smem, s, map_q, map_kv,      \
-                      tiles, positions, block_table, bt_stride, num_pages, page_size, num_heads, num_kv_heads, sh, \
+                      map_8, map_1, tiles, positions, block_table, bt_stride, num_pages, page_size, num_heads, num_kv_heads, sh, \
                       opt, (bf16*)out, status);                                                                   \
     }
     if (shared_rows) LAUNCH(2, 0) else if (sh.nv == 1) LAUNCH(1, 1) else LAUNCH(1, 2)
