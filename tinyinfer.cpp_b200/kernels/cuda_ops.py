@@ -65,11 +65,20 @@ def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
     return None if t is None else t.data_ptr()
 
 
-def _remember(lib, *names: str) -> None:
-    """Answer a library's size queries (functions of whole numbers alone) from a table of earlier answers: a step
-    asks the same few hundreds of times, and a call through ctypes costs more than the launch it decides about."""
-    for name in names:
-        setattr(lib, name, functools.lru_cache(maxsize=4096)(getattr(lib, name)))
+class _Remembering:
+    """A library whose size queries (``names``: functions of whole numbers and of the device) are answered from tables
+    of earlier answers: a step asks the same few hundreds of times, and a call through ctypes costs more than the
+    launch it decides about.  A kernel set has one of its own, since another may run on a device with other answers."""
+
+    def __init__(self, lib, *names: str):
+        self._lib = lib
+        for name in names:
+            setattr(self, name, functools.lru_cache(maxsize=4096)(getattr(lib, name)))
+
+    def __getattr__(self, name):                     # everything else is the library's, looked up once
+        found = getattr(self._lib, name)
+        setattr(self, name, found)
+        return found
 
 
 def _need(cond: bool, msg: str) -> None:
@@ -297,12 +306,11 @@ class CudaOps(MixerOps, StateOps):
             b.ti_attn_prefill_tc2_supported.argtypes = [_i, _i, _i, _i]
             b.ti_attn_prefill_tc2.argtypes = b.ti_attn_prefill_tc.argtypes
             self._tile_rows = (int(b.ti_attn_prefill_tile_rows()), int(b.ti_attn_prefill_tc_tile_rows()))
-            if not hasattr(b.ti_gemm_skinny_supported, "cache_info"):        # (the library is loaded once per process)
-                _remember(b, "ti_gemm_skinny_supported", "ti_gemm_tcgen05_few_supported", "ti_gemm_tcgen05_supported",
-                          "ti_ffn_decode_supported", "ti_attn_out_ffn_decode_supported",
-                          "ti_attn_decode_supported", "ti_attn_decode_blocks_per_sm", "ti_attn_decode_qkv_supported",
-                          "ti_attn_prefill_supported", "ti_attn_prefill_tc_supported", "ti_attn_prefill_tc2_supported")
-            self._bf16 = b
+            self._bf16 = _Remembering(
+                b, "ti_gemm_skinny_supported", "ti_gemm_tcgen05_few_supported", "ti_gemm_tcgen05_supported",
+                "ti_ffn_decode_supported", "ti_attn_out_ffn_decode_supported",
+                "ti_attn_decode_supported", "ti_attn_decode_blocks_per_sm", "ti_attn_decode_qkv_supported",
+                "ti_attn_prefill_supported", "ti_attn_prefill_tc_supported", "ti_attn_prefill_tc2_supported")
         return self._bf16
 
     @property
