@@ -170,6 +170,14 @@ def test_a_step_is_classed_by_how_far_its_portions_reach_back():
         assert batch.portion_reach == want
 
 
+def test_a_step_knows_whether_its_contexts_are_one_tile_of_keys():
+    from tinyinfer_b200.engine.batch import ONE_TILE, build_step_batch
+    entries = [StepEntry("a", [1] * 4, []), StepEntry("b", [2], [0])]
+    for starts, want in (([0, 0], True), ([ONE_TILE - 4, ONE_TILE - 1], True), ([ONE_TILE - 3, 0], False), ([0, ONE_TILE], False)):
+        batch = build_step_batch(entries, starts, [[list(range(8)), list(range(8))]], [0, 1], torch.float32, "cpu")
+        assert batch.one_tile == want
+
+
 def test_which_prompt_attention_kernel_takes_a_step():
     """The choice between the one-head and the two-heads tcgen05 prompt kernels and the number of
     runs a tile's keys are cut into follow from the step's shape (B200: 148 SMs)."""

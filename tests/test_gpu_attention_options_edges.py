@@ -16,7 +16,7 @@ def ops():
     return CudaOps(DEV)
 
 
-def _check(ops, heads, kv, dk, dv, shared, page, ctx, new, opt={}, shape_keys=None, left=0.0, released=False):
+def _check(ops, heads, kv, dk, dv, shared, page, ctx, new, opt={}, shape_keys=None, left=0.0, released=False, one_tile=False):
     """Attends the last ``new[r]`` of ``ctx[r]`` tokens of every request and compares every row with float64.  ``left`` fills
     what earlier requests have left in the pool (a number, or "large" for rows of random large numbers); ``released``:
     pages wholly in front of the first visible key of a request's first new token are gone from its table."""
@@ -55,7 +55,8 @@ def _check(ops, heads, kv, dk, dv, shared, page, ctx, new, opt={}, shape_keys=No
     lists = {f"row_tiles_{64 // gp}": ti(row_tiles(new, starts, 64 // gp).tolist()).view(-1, 3),
              f"option_tiles_{128 // group}": ti(option_tiles(new, starts, 128 // group).tolist()).view(-1, 3)}
     step = SimpleNamespace(positions=ti(positions), req_of_tok=ti([r for r, n in enumerate(new) for _ in range(n)]),
-                           scratch={}, lists=lists, max_position=max(ctx), max_ctx_len=max(ctx), max_q_len=max(new))
+                           scratch={}, lists=lists, max_position=max(ctx), max_ctx_len=max(ctx), max_q_len=max(new),
+                           one_tile=one_tile)
     cache = SimpleNamespace(pages=pages, block_table=table.to(DEV), page_size=page, writes=True)
     scale = 2.0 * dk ** -0.5
     out = torch.full((t, heads * dv), 9.0, dtype=torch.bfloat16, device=DEV)
@@ -111,3 +112,17 @@ def test_what_earlier_requests_left(ops, monkeypatch, heads, kv, dk, dv, shared,
         monkeypatch.setattr(ops, "use_umma_attention_options", umma)
         _check(ops, heads, kv, dk, dv, shared, page, ctx, new, opt, left=left, released=bool(opt))
     _check(ops, heads, kv, dk, dv, shared, page, ctx, [1] * len(ctx), opt, left=left, released=bool(opt))
+
+
+@pytest.mark.parametrize("heads,kv,size,most", [(16, 4, 64, 8), (16, 4, 128, 2), (6, 6, 128, 8), (8, 1, 64, 4), (16, 1, 128, 0)])
+def test_short_portions_in_one_tile_of_keys(ops, monkeypatch, heads, kv, size, most):
+    """A step whose contexts all end in their first tile of keys takes the tcgen05 kernel for portions of more than
+    ``most`` tokens; any step with a longer context takes it."""
+    taken = []
+    real = ops.mixers_tc.ti_attn_options_umma
+    monkeypatch.setattr(ops.mixers_tc, "ti_attn_options_umma", lambda *a: taken.append(1) or real(*a))
+    for tokens in (2, 4, 8, 9):
+        for ctx, one_tile in (([64, 20], True), ([64, 65], False)):
+            taken.clear()
+            _check(ops, heads, kv, size, size, False, 64, ctx, [tokens, 1], one_tile=one_tile)
+            assert bool(taken) == (not one_tile or tokens > most)

@@ -70,6 +70,7 @@ class StepBatch:
     logit_rows: torch.Tensor         # [K] flat token indices whose logits are wanted
     state_slots: torch.Tensor        # [R] state slot of each request
     max_position: int = 0            # the model's longest context (bounds that do not vary by step)
+    one_tile: bool = False           # every context ends within ONE_TILE keys (a class of steps like portion_reach)
     packed_size: int = 0             # int32 values in the packed device buffer
     block_tables: list[torch.Tensor] = field(default_factory=list)   # per group [R, blocks]
     lists: dict = field(default_factory=dict)     # name -> int32 device tensor of a registered StepList
@@ -93,6 +94,7 @@ def build_lists(lists: Sequence[StepList], q_lens: Sequence[int], starts: Sequen
 
 SHORT_CONTEXT = 1536    # keys: up to here a prompt portion's attention walks few tiles of keys
 LONG_CONTEXT = 6144     # keys: from here on it is a long walk
+ONE_TILE = 64           # keys: no longer contexts and every row's attention walks a single tile of keys
 
 
 def portion_reach(q_lens, ctx_lens) -> int:
@@ -174,7 +176,7 @@ def build_step_batch(entries: Sequence[StepEntry], starts: Sequence[int],
         num_tokens=t, num_requests=r, num_logit_rows=k, act_dtype=act_dtype,
         q_lens=q_lens, q_starts=list(starts), ctx_lens=ctx,
         max_q_len=max(q_lens, default=0), max_ctx_len=max(ctx, default=0),
-        portion_reach=portion_reach(q_lens, ctx),
+        portion_reach=portion_reach(q_lens, ctx), one_tile=max(ctx, default=0) <= ONE_TILE,
         token_ids=view("tok"), positions=view("pos"), req_of_tok=view("roft"), cu_q=view("cu"),
         q_start_dev=view("qs"), ctx_len_dev=view("ctx"), logit_rows=view("rows"),
         state_slots=view("slots"),

@@ -270,10 +270,10 @@ class StepGraphs(_OfEngine):
     def run(self, entries, starts, tables, slots):
         """Logits of the step, or None if the step should run eagerly (a shape seen for the first time)."""
         eng = self.engine
-        from .batch import portion_reach
+        from .batch import ONE_TILE, portion_reach
         lens = [len(e.tokens) for e in entries]
-        key = (tuple(lens), tuple(tuple(e.want) for e in entries),
-               portion_reach(lens, [s + n for s, n in zip(starts, lens)]))
+        ends = [s + n for s, n in zip(starts, lens)]
+        key = (tuple(lens), tuple(tuple(e.want) for e in entries), portion_reach(lens, ends), max(ends) <= ONE_TILE)
         ent = self.graphs.get(key)
         build = dict(act_dtype=eng.dtype, device=eng.device, min_blocks=self.width,
                      max_position=eng.plan.max_position, lists=eng.step_lists)

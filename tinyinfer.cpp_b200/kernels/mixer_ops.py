@@ -374,12 +374,20 @@ class MixerOps:
                                     and gate.shape[1] == (num_heads if gate_per_head else num_heads * dv)),
                    "attention_options: the gate must be float32 [T, heads] or [T, heads * dv]")
         # a step that brings prompt portions: tcgen05, where the head sizes fill its chunks of 64 elements; its single
-        # tokens ride along as tiles of one token.  us against the mma.sync kernel, 16 heads, portions of 2 / 64 / 256
-        # tokens and 64 behind 2,000: shared rows of 576 11.3 / 12.2 / 24.3 / 129 against 21.0 / 23.3 / 47.7 / 292, of 288
-        # 10.8 / 11.6 / 17.8 / 82 against 17.3 / 18.5 / 39.7 / 230, heads of 128 (4 kv heads, a cap) 9.5 / 9.9 / 19.9 / 116
-        # against 9.1 / 11.4 / 29.4 / 203, of 64 7.4 / 7.7 / 13.8 / 73 against 6.5 / 8.5 / 20.4 / 137
+        # tokens ride along as tiles of one token.  us against the mma.sync kernel, 16 heads (one kv head over shared rows,
+        # else 4), portions of 2 / 64 / 256 tokens, 64 behind 2,000, and 2 / 64 tokens beside 32 single ones at 2,000:
+        #   shared rows of 576     14.3 / 13.8 / 25.8, 135, 134 / 136   against  22.1 / 23.2 / 48.0, 297, 284 / 286
+        #   shared rows of 288     14.2 / 13.1 / 19.4, 89, 86 / 86      against  18.7 / 19.4 / 41.6, 233, 223 / 222
+        #   heads of 128, a cap    10.5 / 10.8 / 21.8, 128, 141 / 144   against  9.3 / 12.3 / 29.8, 203, 204 / 205
+        #   heads of 64            8.4 / 8.4 / 15.1, 80, 84 / 84        against  6.9 / 8.9 / 20.7, 137, 134 / 135
+        # Not where every context is one tile of keys and every portion a few rows of a tile (2, 4, 8 tokens of heads of
+        # 64 over 4 kv heads, one request: 8.2 / 8.2 / 7.9 against 6.9 / 7.9 / 8.2, 64 requests: 9.6 / 9.5 / 9.7 against
+        # 8.2 / 9.0 / 9.0; of heads of 128 10.2 / 10.0 / 10.0 against 9.2 / 11.5 / 11.4).
         tiles = getattr(step, "lists", {}).get(f"option_tiles_{128 // max(1, min(128, num_heads // num_kv_heads))}")
-        if (self.use_tc_attention_options and self.use_umma_attention_options and getattr(step, "max_q_len", 0) > 1
+        group = num_heads // max(1, num_kv_heads)
+        brief = (not shared_rows and getattr(step, "one_tile", False)
+                 and getattr(step, "max_q_len", 0) * group <= (32 if dv <= 64 else 8))
+        if (self.use_tc_attention_options and self.use_umma_attention_options and getattr(step, "max_q_len", 0) > 1 and not brief
                 and tiles is not None and 0 < tiles.shape[0] <= 65535 and q.dtype == pages.dtype == torch.bfloat16
                 and q.data_ptr() % 16 == 0 and out.data_ptr() % 32 == 0 and pages.data_ptr() % 16 == 0
                 and self.mixers_tc.ti_attn_options_umma_tokens(dk, dv, cache.page_size, int(bool(shared_rows)), num_heads,
