@@ -659,8 +659,10 @@ extern "C" int ti_slice_rmsnorm(const float* x, int stride, int num_rows, int n,
                                 void* out, int out_dtype, void* stream) {
     if (num_rows == 0 || n == 0) return 0;
     cudaStream_t s = (cudaStream_t)stream;
-    if (out_dtype == TI_BF16) ti_launch_pdl((slice_rmsnorm_kernel<bf16>), dim3(num_rows), dim3(256), 0, s, x, stride, n, weight, eps, (bf16*)out);
-    else if (out_dtype == TI_F32) ti_launch_pdl((slice_rmsnorm_kernel<float>), dim3(num_rows), dim3(256), 0, s, x, stride, n, weight, eps, (float*)out);
+    if (out_dtype == TI_BF16) ti_launch_pdl(slice_rmsnorm_kernel<bf16>, dim3(num_rows), dim3(256), 0, s, x, stride, n,
+                                            weight, eps, (bf16*)out);
+    else if (out_dtype == TI_F32) ti_launch_pdl(slice_rmsnorm_kernel<float>, dim3(num_rows), dim3(256), 0, s, x,
+                                                stride, n, weight, eps, (float*)out);
     else return ti_fail("slice_rmsnorm: output dtype code %d", out_dtype);
     return ti_check_launch("slice_rmsnorm");
 }
@@ -726,11 +728,11 @@ extern "C" int ti_turn_rows(const void* x, int dtype, const int* positions, cons
     TI_REQUIRE(smem <= 48 * 1024, "turn_rows: a rotated width of %d", rot);
     cudaStream_t s = (cudaStream_t)stream;
     if (dtype == TI_BF16)
-        ti_launch_pdl((turn_rows_kernel<bf16>), dim3(num_tokens), dim3(256), smem, s, (const bf16*)x, positions, inv_freq, rot, halves, sign, gate,
-                                                            gate_stride, num_heads, n, (bf16*)out);
+        ti_launch_pdl(turn_rows_kernel<bf16>, dim3(num_tokens), dim3(256), smem, s, (const bf16*)x, positions,
+                      inv_freq, rot, halves, sign, gate, gate_stride, num_heads, n, (bf16*)out);
     else if (dtype == TI_F32)
-        ti_launch_pdl((turn_rows_kernel<float>), dim3(num_tokens), dim3(256), smem, s, (const float*)x, positions, inv_freq, rot, halves, sign,
-                                                             gate, gate_stride, num_heads, n, (float*)out);
+        ti_launch_pdl(turn_rows_kernel<float>, dim3(num_tokens), dim3(256), smem, s, (const float*)x, positions,
+                      inv_freq, rot, halves, sign, gate, gate_stride, num_heads, n, (float*)out);
     else return ti_fail("turn_rows: dtype code %d", dtype);
     return ti_check_launch("turn_rows");
 }

@@ -1,5 +1,7 @@
 // Paged flash attention with optional parts on the tensor cores (bfloat16 operands, mma.sync
-// m16n8k16), for prompt portions and single decoded tokens alike.
+// m16n8k16), for prompt portions and single decoded tokens alike.  Steps with portions run here only
+// where attn_options_umma.cu (tcgen05) does not take them: rows of more than 576 elements, values of a
+// size of their own, few rows within one tile of keys.
 //
 // The options are those of attention_options (attn_options.cu): a window and/or chunks of
 // positions, a score factor per head, a cap on the score, a sink in the softmax, an output gate
@@ -24,7 +26,7 @@
 // also takes the weights in full float32: a weight is split into three bfloat16 parts (8 + 8 + 8
 // bits of its significand), each multiplies the bfloat16 values on the tensor cores, and the
 // three products are added in the float32 accumulator.
-#include "common.cuh"
+#include "attn_options.cuh"
 
 namespace {
 
@@ -59,28 +61,6 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], const unsigned (&a)[4], 
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-// Two floats as three pairs of bfloat16 whose sums are the floats: the upper 16 bits of a float
-// are a bfloat16 (truncated), what is left is exact in float32 and is cut the same way again;
-// after three cuts nothing of the 24-bit significand is left.
-__device__ __forceinline__ void split3_pair(float x, float y, unsigned& hi, unsigned& mid, unsigned& lo) {
-    const unsigned xb = __float_as_uint(x), yb = __float_as_uint(y);
-    hi = __byte_perm(xb, yb, 0x7632);
-    const float x1 = x - __uint_as_float(xb & 0xffff0000u), y1 = y - __uint_as_float(yb & 0xffff0000u);
-    const unsigned x1b = __float_as_uint(x1), y1b = __float_as_uint(y1);
-    mid = __byte_perm(x1b, y1b, 0x7632);
-    const float x2 = x1 - __uint_as_float(x1b & 0xffff0000u), y2 = y1 - __uint_as_float(y1b & 0xffff0000u);
-    lo = __byte_perm(__float_as_uint(x2), __float_as_uint(y2), 0x7632);
-}
-__device__ __forceinline__ float ex2_approx(float x) {
-    float y;
-    asm("ex2.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-__device__ __forceinline__ float rcp_approx(float x) {
-    float y;
-    asm("rcp.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
 
 struct TcOptions {
     int window, chunk;
@@ -91,11 +71,7 @@ struct TcOptions {
     int gate_stride, gate_per_head, shared_rows;
 };
 
-__device__ __forceinline__ int first_visible(int p, const TcOptions& o) {
-    int lo = o.window > 0 ? max(0, p - o.window + 1) : 0;
-    if (o.chunk > 0) lo = max(lo, p / o.chunk * o.chunk);
-    return lo;
-}
+__device__ __forceinline__ int first_visible(int p, const TcOptions& o) { return first_key_seen(p, o.window, o.chunk); }
 
 // tiles[i] = {request row, first flat token, tokens (<= 64 / gp)}
 // MODE 0: the warps of a block have 16 rows each.  MODE 1 (KS): all have the same 16 rows and a quarter
@@ -570,8 +546,9 @@ extern "C" int ti_head_project_tc(const void* x, int x_stride_t, int x_stride_h,
         configured.mark();
     }
     dim3 grid((num_tokens + BM - 1) / BM, num_heads, (n_out + 127) / 128);
-    ti_launch_pdl((head_project_tc_kernel), dim3(grid), dim3(WARPS * 32), smem, (cudaStream_t)stream, (const bf16*)x, x_stride_t, x_stride_h, (const bf16*)w, n_in, n_out, (bf16*)out, out_stride_t, out_stride_h,
-        num_tokens);
+    ti_launch_pdl(head_project_tc_kernel, dim3(grid), dim3(WARPS * 32), smem, (cudaStream_t)stream, (const bf16*)x,
+                  x_stride_t, x_stride_h, (const bf16*)w, n_in, n_out, (bf16*)out, out_stride_t, out_stride_h,
+                  num_tokens);
     return ti_check_launch("head_project_tc");
 }
 
@@ -644,8 +621,8 @@ extern "C" int ti_attn_options_tc(const void* q, const int* tiles, int num_tiles
     if (int rc = ti_check_launch("attn_options_tc")) return rc;
     if (nsplit > 1) {
         const int items = num_tokens * num_heads;
-        ti_launch_pdl((attn_options_merge_kernel), dim3(dim3(items, (dv + 127) / 128)), dim3(128), 0, s, part_o, part_ml, nsplit, num_heads, dv, sink, gate, gate_stride,
-                                                       gate_per_head, (bf16*)out);
+        ti_launch_pdl(attn_options_merge_kernel, dim3(items, (dv + 127) / 128), dim3(128), 0, s, part_o, part_ml,
+                      nsplit, num_heads, dv, sink, gate, gate_stride, gate_per_head, (bf16*)out);
         return ti_check_launch("attn_options_merge");
     }
     return 0;

@@ -36,6 +36,7 @@
 // returns.
 #include <utility>
 
+#include "attn_options.cuh"
 #include "sm100.cuh"
 
 namespace {
@@ -64,31 +65,7 @@ struct Shape {
     int dk, dv, chunks, places, nv, slices, stages, shared, run;
 };
 
-__device__ __forceinline__ float ex2_approx(float x) {
-    float y;
-    asm("ex2.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-__device__ __forceinline__ float rcp_approx(float x) {
-    float y;
-    asm("rcp.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-__device__ __forceinline__ int first_visible(int p, const UmmaOptions& o) {
-    int lo = o.window > 0 ? max(0, p - o.window + 1) : 0;
-    if (o.chunk > 0) lo = max(lo, p / o.chunk * o.chunk);
-    return lo;
-}
-// Two floats as three pairs of bfloat16 whose sums are the floats (the upper 16 bits of what is left, three times).
-__device__ __forceinline__ void split3_pair(float x, float y, unsigned& hi, unsigned& mid, unsigned& lo) {
-    const unsigned xb = __float_as_uint(x), yb = __float_as_uint(y);
-    hi = __byte_perm(xb, yb, 0x7632);
-    const float x1 = x - __uint_as_float(xb & 0xffff0000u), y1 = y - __uint_as_float(yb & 0xffff0000u);
-    const unsigned x1b = __float_as_uint(x1), y1b = __float_as_uint(y1);
-    mid = __byte_perm(x1b, y1b, 0x7632);
-    const float x2 = x1 - __uint_as_float(x1b & 0xffff0000u), y2 = y1 - __uint_as_float(y1b & 0xffff0000u);
-    lo = __byte_perm(__float_as_uint(x2), __float_as_uint(y2), 0x7632);
-}
+__device__ __forceinline__ int first_visible(int p, const UmmaOptions& o) { return first_key_seen(p, o.window, o.chunk); }
 // D (+)= A B with A from tensor memory (rows in lanes, two bfloat16 of K per 32-bit column).
 __device__ __forceinline__ void umma_bf16_tmem_a(unsigned tmem_d, unsigned tmem_a, unsigned long long db, unsigned idesc,
                                                  unsigned accumulate) {

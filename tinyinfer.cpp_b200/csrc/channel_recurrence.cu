@@ -357,9 +357,11 @@ extern "C" int ti_low_rank_decay(const float* low, int low_stride, int rank, con
     TI_REQUIRE(grid.y <= 65535, "low_rank_decay: %d rows exceed the grid limit", rows);
     cudaStream_t s = (cudaStream_t)stream;
     if (a2_dtype == TI_BF16)
-        ti_launch_pdl((low_rank_decay_kernel<bf16>), dim3(grid), dim3(128), 0, s, low, low_stride, rank, (const bf16*)a2, bias, inv_tau, rows, n, out);
+        ti_launch_pdl(low_rank_decay_kernel<bf16>, dim3(grid), dim3(128), 0, s, low, low_stride, rank,
+                      (const bf16*)a2, bias, inv_tau, rows, n, out);
     else if (a2_dtype == TI_F32)
-        ti_launch_pdl((low_rank_decay_kernel<float>), dim3(grid), dim3(128), 0, s, low, low_stride, rank, (const float*)a2, bias, inv_tau, rows, n, out);
+        ti_launch_pdl(low_rank_decay_kernel<float>, dim3(grid), dim3(128), 0, s, low, low_stride, rank,
+                      (const float*)a2, bias, inv_tau, rows, n, out);
     else return ti_fail("low_rank_decay: matrix dtype code %d", a2_dtype);
     return ti_check_launch("low_rank_decay");
 }
@@ -386,8 +388,10 @@ extern "C" int ti_gated_recurrence(const float* u, int u_stride, const float* ga
     cudaStream_t s = (cudaStream_t)stream;
 #define CALL(CH)                                                                                                     \
     do {                                                                                                             \
-        if (out_dtype == TI_BF16) ti_launch_if_early(false, (gated_recurrence_kernel<bf16, CH>), dim3(grid), dim3(GR_WARPS * 32), 0, s, a, (bf16*)out);     \
-        else ti_launch_if_early(false, (gated_recurrence_kernel<float, CH>), dim3(grid), dim3(GR_WARPS * 32), 0, s, a, (float*)out);                        \
+        if (out_dtype == TI_BF16) ti_launch_if_early(false, (gated_recurrence_kernel<bf16, CH>), dim3(grid), \
+            dim3(GR_WARPS * 32), 0, s, a, (bf16*)out);                                                       \
+        else ti_launch_if_early(false, (gated_recurrence_kernel<float, CH>), dim3(grid), dim3(GR_WARPS * 32), 0, \
+            s, a, (float*)out);                                                                                  \
     } while (0)
     if (ch == 32) CALL(32);
     else if (ch == 16) CALL(16);
@@ -419,8 +423,10 @@ extern "C" int ti_gated_recurrence_single(const float* u, int u_stride, const vo
     cudaStream_t s = (cudaStream_t)stream;
 #define CALL(TW, TO)                                                                                                 \
     do {                                                                                                             \
-        if (wide) ti_launch_pdl((gated_recurrence_single_kernel<TW, TO, 16>), dim3(grid), dim3(256), smem, s, a, (const TW*)w, requests, (TO*)out); \
-        else ti_launch_pdl((gated_recurrence_single_kernel<TW, TO, 8>), dim3(grid), dim3(256), smem, s, a, (const TW*)w, requests, (TO*)out); \
+        if (wide) ti_launch_pdl((gated_recurrence_single_kernel<TW, TO, 16>), dim3(grid), dim3(256), smem, s, a, \
+            (const TW*)w, requests, (TO*)out);                                                                   \
+        else ti_launch_pdl((gated_recurrence_single_kernel<TW, TO, 8>), dim3(grid), dim3(256), smem, s, a, \
+            (const TW*)w, requests, (TO*)out);                                                             \
     } while (0)
     if (w_dtype == TI_BF16 && out_dtype == TI_BF16) CALL(bf16, bf16);
     else if (w_dtype == TI_BF16 && out_dtype == TI_F32) CALL(bf16, float);
@@ -437,7 +443,7 @@ extern "C" int ti_split_rows(const float* x, int stride, int rows, int width, in
     TI_REQUIRE(per % 4 == 0 && width % per == 0 && rows <= rows_padded && (uintptr_t)out % 8 == 0,
                "split_rows: parts of %d columns (a multiple of 4) of %d", per, width);
     const long long quads = (long long)rows * (width / 4);
-    ti_launch_pdl((split_rows_kernel), dim3((unsigned)((quads + 255) / 256)), dim3(256), 0, (cudaStream_t)stream, x, stride, rows, width, per,
-                                                                                         rows_padded, (bf16*)out);
+    ti_launch_pdl(split_rows_kernel, dim3((unsigned)((quads + 255) / 256)), dim3(256), 0, (cudaStream_t)stream, x,
+                  stride, rows, width, per, rows_padded, (bf16*)out);
     return ti_check_launch("split_rows");
 }

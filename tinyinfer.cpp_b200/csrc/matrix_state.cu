@@ -101,17 +101,17 @@ extern "C" int ti_matrix_state(int mode, const float* q, const float* k, const f
     if (int rc = ti_check_launch("matrix_state")) return rc;
     if (col_block != 0) {
         if (mode == MODE_GATED_SUM) {
-            ti_launch_pdl((matrix_state_commit_kernel), dim3(dim3(requests, heads)), dim3(64), 0, s, carry, cu_q, slots, state, state_stride,
-                                                                            heads, dk, dv);
+            ti_launch_pdl(matrix_state_commit_kernel, dim3(requests, heads), dim3(64), 0, s, carry, cu_q, slots,
+                          state, state_stride, heads, dk, dv);
             if (int rc = ti_check_launch("matrix_state_commit")) return rc;
         }
         const int blocks = (rows * heads + 7) / 8;
         if (out_dtype == TI_BF16)
-            ti_launch_pdl((matrix_state_finish_kernel<bf16>), dim3(blocks), dim3(256), 0, s, o_raw, norm_weight, norm_per_row, eps, gate,
-                                                                     gate_stride, gate_act, rows, heads, dv, (bf16*)out);
+            ti_launch_pdl(matrix_state_finish_kernel<bf16>, dim3(blocks), dim3(256), 0, s, o_raw, norm_weight,
+                          norm_per_row, eps, gate, gate_stride, gate_act, rows, heads, dv, (bf16*)out);
         else
-            ti_launch_pdl((matrix_state_finish_kernel<float>), dim3(blocks), dim3(256), 0, s, o_raw, norm_weight, norm_per_row, eps, gate,
-                                                                      gate_stride, gate_act, rows, heads, dv, (float*)out);
+            ti_launch_pdl(matrix_state_finish_kernel<float>, dim3(blocks), dim3(256), 0, s, o_raw, norm_weight,
+                          norm_per_row, eps, gate, gate_stride, gate_act, rows, heads, dv, (float*)out);
         return ti_check_launch("matrix_state_finish");
     }
     return 0;

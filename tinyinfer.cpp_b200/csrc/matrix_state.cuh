@@ -443,7 +443,8 @@ template <int MODE, int DMAX>
 int launch_cb(const MatrixStateArgs& a, int requests, int cb, int col_blocks, cudaStream_t s) {
     dim3 grid(requests, a.heads, col_blocks);
 #define TI_MS_GO(CB_, LANES_) \
-    ti_launch_if_early(a.single, (matrix_state_kernel<MODE, DMAX, CB_, LANES_>), dim3(grid), dim3(StateBlock<MODE, DMAX, CB_, LANES_>::threads), 0, s, a)
+    ti_launch_if_early(a.single, (matrix_state_kernel<MODE, DMAX, CB_, LANES_>), dim3(grid), \
+                       dim3(StateBlock<MODE, DMAX, CB_, LANES_>::threads), 0, s, a)
     if (a.cut && cb == 8) TI_MS_GO(8, 16);
     else if (a.cut && cb == 16) TI_MS_GO(16, 16);
     else if (a.cut && cb == 32) TI_MS_GO(32, 16);

@@ -414,13 +414,13 @@ extern "C" int ti_causal_conv_rows(const float* x, int x_stride, const float* w,
     dim3 grid(rows, (channels + 255) / 256);
     cudaStream_t s = (cudaStream_t)stream;
     if (out_dtype == TI_BF16)
-        ti_launch_pdl((causal_conv_rows_kernel<bf16>), dim3(grid), dim3(256), 0, s, x, x_stride, w, taps, channels, req_of_tok, cu_q, slots, state,
-                                                           (size_t)state_stride, (size_t)state_offset, add_input, silu,
-                                                           renew, in_bias, bias, (bf16*)out, out_stride);
+        ti_launch_pdl(causal_conv_rows_kernel<bf16>, dim3(grid), dim3(256), 0, s, x, x_stride, w, taps, channels,
+                      req_of_tok, cu_q, slots, state, (size_t)state_stride, (size_t)state_offset, add_input, silu,
+                      renew, in_bias, bias, (bf16*)out, out_stride);
     else if (out_dtype == TI_F32)
-        ti_launch_pdl((causal_conv_rows_kernel<float>), dim3(grid), dim3(256), 0, s, x, x_stride, w, taps, channels, req_of_tok, cu_q, slots, state,
-                                                            (size_t)state_stride, (size_t)state_offset, add_input, silu,
-                                                            renew, in_bias, bias, (float*)out, out_stride);
+        ti_launch_pdl(causal_conv_rows_kernel<float>, dim3(grid), dim3(256), 0, s, x, x_stride, w, taps, channels,
+                      req_of_tok, cu_q, slots, state, (size_t)state_stride, (size_t)state_offset, add_input, silu,
+                      renew, in_bias, bias, (float*)out, out_stride);
     else return ti_fail("causal_conv_rows: output dtype code %d", out_dtype);
     return ti_check_launch("causal_conv_rows");
 }
@@ -431,8 +431,8 @@ extern "C" int ti_conv_tail_store(const float* x, int x_stride, int taps, int ch
     if (requests == 0 || channels == 0 || taps <= 1) return 0;
     TI_REQUIRE(taps <= MAX_TAPS, "conv_tail_store: %d taps (at most %d)", taps, MAX_TAPS);
     dim3 grid((channels + 255) / 256, requests);
-    ti_launch_pdl((conv_tail_store_kernel), dim3(grid), dim3(256), 0, (cudaStream_t)stream, x, x_stride, taps, channels, cu_q, slots, state,
-                                                                    (size_t)state_stride, (size_t)state_offset, in_bias);
+    ti_launch_pdl(conv_tail_store_kernel, dim3(grid), dim3(256), 0, (cudaStream_t)stream, x, x_stride, taps, channels,
+                  cu_q, slots, state, (size_t)state_stride, (size_t)state_offset, in_bias);
     return ti_check_launch("conv_tail_store");
 }
 
@@ -445,12 +445,14 @@ extern "C" int ti_group_norm_rows(const float* x, const float* w, const int* row
     const int threads = (groups >= 8 ? 8 : groups) * wpg * 32;
     if (residual != nullptr) {
         TI_REQUIRE(rows == nullptr, "group_norm_rows: rows are not gathered when adding to a residual");
-        ti_launch_pdl((group_norm_rows_kernel<float, true>), dim3(num_rows), dim3(threads), 0, s, x, w, rows, groups, n, eps, nullptr, residual,
-                                                                        res_stride, wpg);
+        ti_launch_pdl(group_norm_rows_kernel<float, true>, dim3(num_rows), dim3(threads), 0, s, x, w, rows, groups, n,
+                      eps, nullptr, residual, res_stride, wpg);
     } else if (out_dtype == TI_BF16) {
-        ti_launch_pdl((group_norm_rows_kernel<bf16, false>), dim3(num_rows), dim3(threads), 0, s, x, w, rows, groups, n, eps, (bf16*)out, nullptr, 0, wpg);
+        ti_launch_pdl(group_norm_rows_kernel<bf16, false>, dim3(num_rows), dim3(threads), 0, s, x, w, rows, groups, n,
+                      eps, (bf16*)out, nullptr, 0, wpg);
     } else if (out_dtype == TI_F32) {
-        ti_launch_pdl((group_norm_rows_kernel<float, false>), dim3(num_rows), dim3(threads), 0, s, x, w, rows, groups, n, eps, (float*)out, nullptr, 0, wpg);
+        ti_launch_pdl(group_norm_rows_kernel<float, false>, dim3(num_rows), dim3(threads), 0, s, x, w, rows, groups,
+                      n, eps, (float*)out, nullptr, 0, wpg);
     } else {
         return ti_fail("group_norm_rows: output dtype code %d", out_dtype);
     }
@@ -460,7 +462,8 @@ extern "C" int ti_group_norm_rows(const float* x, const float* w, const int* row
 extern "C" int ti_depth_mix(float* x, float* hist, long long layer_elems, int index, const float* w, void* stream) {
     if (layer_elems == 0) return 0;
     const int blocks = (int)((layer_elems + 255) / 256);
-    ti_launch_pdl((depth_mix_kernel), dim3(blocks), dim3(256), 0, (cudaStream_t)stream, x, hist, (size_t)layer_elems, index, w, (size_t)layer_elems);
+    ti_launch_pdl(depth_mix_kernel, dim3(blocks), dim3(256), 0, (cudaStream_t)stream, x, hist, (size_t)layer_elems,
+                  index, w, (size_t)layer_elems);
     return ti_check_launch("depth_mix");
 }
 
@@ -468,7 +471,8 @@ extern "C" int ti_add_scaled(float* dst, int dst_stride, const float* a, float s
                              int cols, void* stream) {
     if (rows == 0 || cols == 0) return 0;
     const size_t n = (size_t)rows * cols;
-    ti_launch_pdl((add_scaled_kernel), dim3((int)((n + 255) / 256)), dim3(256), 0, (cudaStream_t)stream, dst, dst_stride, a, sa, b, sb, rows, cols);
+    ti_launch_pdl(add_scaled_kernel, dim3((int)((n + 255) / 256)), dim3(256), 0, (cudaStream_t)stream, dst,
+                  dst_stride, a, sa, b, sb, rows, cols);
     return ti_check_launch("add_scaled");
 }
 
@@ -481,9 +485,11 @@ extern "C" int ti_glu_rows(const float* gu, int num_tokens, int inter, int inter
     const int blocks = (int)((total + 255) / 256);
     cudaStream_t s = (cudaStream_t)stream;
     if (out_dtype == TI_BF16)
-        ti_launch_pdl((glu_rows_kernel<bf16>), dim3(blocks), dim3(256), 0, s, gu, inter, total, interleaved, kind, limit, alpha, (bf16*)out);
+        ti_launch_pdl(glu_rows_kernel<bf16>, dim3(blocks), dim3(256), 0, s, gu, inter, total, interleaved, kind,
+                      limit, alpha, (bf16*)out);
     else if (out_dtype == TI_F32)
-        ti_launch_pdl((glu_rows_kernel<float>), dim3(blocks), dim3(256), 0, s, gu, inter, total, interleaved, kind, limit, alpha, (float*)out);
+        ti_launch_pdl(glu_rows_kernel<float>, dim3(blocks), dim3(256), 0, s, gu, inter, total, interleaved, kind,
+                      limit, alpha, (float*)out);
     else return ti_fail("glu_rows: output dtype code %d", out_dtype);
     return ti_check_launch("glu_rows");
 }
@@ -503,7 +509,8 @@ extern "C" int ti_tanh_norm_rows(const float* x, const int* rows, int num_rows, 
     const dim3 grid(num_rows, (n + (four ? 1023 : 255)) / (four ? 1024 : 256));
     TI_REQUIRE(grid.y <= 65535, "tanh_norm_rows: rows of %d elements", n);
 #define CALL(TO, ADD, VEC)                                                                            \
-    ti_launch_pdl((tanh_norm_rows_kernel<TO, ADD, VEC>), dim3(grid), dim3(256), 0, s, x, rows, n, alpha, w, b, (TO*)(ADD ? nullptr : out), \
+    ti_launch_pdl((tanh_norm_rows_kernel<TO, ADD, VEC>), dim3(grid), dim3(256), 0, s, x, rows, n, alpha, w, b, \
+        (TO*)(ADD ? nullptr : out),                                                                            \
                                                              residual, res_stride)
     if (residual != nullptr) {
         TI_REQUIRE(rows == nullptr, "tanh_norm_rows: rows are not gathered when adding to a residual");
@@ -528,7 +535,8 @@ extern "C" int ti_embed_bigram(const void* table, const void* bigram, int dtype,
                "embed_bigram: factors must lie in [0, buckets), and buckets below 2^31");
     cudaStream_t s = (cudaStream_t)stream;
 #define CALL(TW)                                                                                                   \
-    ti_launch_pdl((embed_bigram_kernel<TW>), dim3(num_tokens), dim3(256), 0, s, (const TW*)table, (const TW*)bigram, tokens, n, vocab, buckets,  \
+    ti_launch_pdl((embed_bigram_kernel<TW>), dim3(num_tokens), dim3(256), 0, s, (const TW*)table,   \
+        (const TW*)bigram, tokens, n, vocab, buckets,                                               \
                                                        mul_prev, mul_cur, positions, req_of_tok, cu_q, slots, kept, \
                                                        (size_t)kept_stride, out)
     if (dtype == TI_BF16) CALL(bf16);
@@ -545,7 +553,8 @@ extern "C" int ti_rmsnorm_shift(const float* x, int num_rows, int n, const float
     cudaStream_t s = (cudaStream_t)stream;
     const bool four = kept_stride % 4 == 0 && rows_of_four(n, 0, {x, w, mu, kept, out, shifted});
 #define CALL(TO, VEC)                                                                                              \
-    ti_launch_pdl((rmsnorm_shift_kernel<TO, VEC>), dim3(num_rows), dim3(256), 0, s, x, n, w, eps, mu, req_of_tok, cu_q, slots, kept,         \
+    ti_launch_pdl((rmsnorm_shift_kernel<TO, VEC>), dim3(num_rows), dim3(256), 0, s, x, n, w, eps, mu, req_of_tok, \
+        cu_q, slots, kept,                                                                                        \
                                                            (size_t)kept_stride, (TO*)out, (TO*)shifted)
     if (out_dtype == TI_BF16) { if (four) CALL(bf16, 4); else CALL(bf16, 1); }
     else if (out_dtype == TI_F32) { if (four) CALL(float, 4); else CALL(float, 1); }
@@ -561,15 +570,18 @@ extern "C" int ti_gated_add(float* x, int x_stride, const float* y, int y_stride
     const bool four = y_stride % 4 == 0 && gate_stride % 4 == 0 && rows_of_four(n, x_stride, {x, y, gate, bias});
     const dim3 grid(rows, (n + (four ? 1023 : 255)) / (four ? 1024 : 256));
     TI_REQUIRE(grid.y <= 65535, "gated_add: rows of %d elements", n);
-    if (four) ti_launch_pdl((gated_add_kernel<4>), dim3(grid), dim3(256), 0, s, x, x_stride, y, y_stride, gate, gate_stride, bias, scale, n);
-    else ti_launch_pdl((gated_add_kernel<1>), dim3(grid), dim3(256), 0, s, x, x_stride, y, y_stride, gate, gate_stride, bias, scale, n);
+    if (four) ti_launch_pdl(gated_add_kernel<4>, dim3(grid), dim3(256), 0, s, x, x_stride, y, y_stride, gate,
+                            gate_stride, bias, scale, n);
+    else ti_launch_pdl(gated_add_kernel<1>, dim3(grid), dim3(256), 0, s, x, x_stride, y, y_stride, gate, gate_stride,
+                       bias, scale, n);
     return ti_check_launch("gated_add");
 }
 
 extern "C" int ti_cap_rows(float* x, long long total, float cap, void* stream) {
     if (total == 0) return 0;
     TI_REQUIRE(cap > 0.0f, "cap_rows: the cap must be positive");
-    ti_launch_pdl((cap_rows_kernel), dim3((unsigned)((total + 255) / 256)), dim3(256), 0, (cudaStream_t)stream, x, (size_t)total, cap);
+    ti_launch_pdl(cap_rows_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, (cudaStream_t)stream, x,
+                  (size_t)total, cap);
     return ti_check_launch("cap_rows");
 }
 
@@ -578,8 +590,10 @@ extern "C" int ti_unary_rows(const float* x, long long total, int kind, void* ou
     TI_REQUIRE(kind == ACT_RELU2, "unary_rows: activation kind %d", kind);
     const unsigned blocks = (unsigned)((total + 255) / 256);
     cudaStream_t s = (cudaStream_t)stream;
-    if (out_dtype == TI_BF16) ti_launch_pdl((unary_rows_kernel<bf16>), dim3(blocks), dim3(256), 0, s, x, (size_t)total, kind, (bf16*)out);
-    else if (out_dtype == TI_F32) ti_launch_pdl((unary_rows_kernel<float>), dim3(blocks), dim3(256), 0, s, x, (size_t)total, kind, (float*)out);
+    if (out_dtype == TI_BF16) ti_launch_pdl(unary_rows_kernel<bf16>, dim3(blocks), dim3(256), 0, s, x, (size_t)total,
+                                            kind, (bf16*)out);
+    else if (out_dtype == TI_F32) ti_launch_pdl(unary_rows_kernel<float>, dim3(blocks), dim3(256), 0, s, x,
+                                                (size_t)total, kind, (float*)out);
     else return ti_fail("unary_rows: output dtype code %d", out_dtype);
     return ti_check_launch("unary_rows");
 }
@@ -587,7 +601,8 @@ extern "C" int ti_unary_rows(const float* x, long long total, int kind, void* ou
 extern "C" int ti_add_row(float* x, int stride, const float* row, int rows, int cols, void* stream) {
     const size_t total = (size_t)rows * cols;
     if (total == 0) return 0;
-    ti_launch_pdl((add_row_kernel), dim3((unsigned)((total + 255) / 256)), dim3(256), 0, (cudaStream_t)stream, x, stride, row, cols, total);
+    ti_launch_pdl(add_row_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, (cudaStream_t)stream, x,
+                  stride, row, cols, total);
     return ti_check_launch("add_row");
 }
 
@@ -599,8 +614,9 @@ extern "C" int ti_tanh_norm_pair(const float* y, int num_rows, int n, float a1, 
     const bool four = rows_of_four(n, res_stride, {y, w1, b1, w2, b2, out, residual});
     const dim3 grid(num_rows, (n + (four ? 1023 : 255)) / (four ? 1024 : 256));
     TI_REQUIRE(grid.y <= 65535, "tanh_norm_pair: rows of %d elements", n);
-#define CALL(TO, VEC) \
-    ti_launch_pdl((tanh_norm_pair_kernel<TO, VEC>), dim3(grid), dim3(256), 0, s, y, n, a1, w1, b1, residual, res_stride, a2, w2, b2, (TO*)out)
+#define CALL(TO, VEC)                                                                                            \
+    ti_launch_pdl((tanh_norm_pair_kernel<TO, VEC>), dim3(grid), dim3(256), 0, s, y, n, a1, w1, b1, residual,      \
+                  res_stride, a2, w2, b2, (TO*)out)
     if (out_dtype == TI_BF16) { if (four) CALL(bf16, 4); else CALL(bf16, 1); }
     else if (out_dtype == TI_F32) { if (four) CALL(float, 4); else CALL(float, 1); }
     else return ti_fail("tanh_norm_pair: output dtype code %d", out_dtype);

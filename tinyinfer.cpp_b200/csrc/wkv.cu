@@ -262,11 +262,13 @@ extern "C" int ti_token_shift_mix(const void* h, int h_dtype, const float* mu, i
     if (num_tokens == 0) return 0;
     cudaStream_t s = (cudaStream_t)stream;
     if (h_dtype == TI_F32)
-        ti_launch_pdl((token_shift_mix_kernel<float>), dim3(num_tokens), dim3(256), 0, s, (const float*)h, mu, n_mix, width, num_tokens,
-            req_of_tok, cu_q, slots, state, (size_t)state_stride, (size_t)prev_offset, (float*)out);
+        ti_launch_pdl(token_shift_mix_kernel<float>, dim3(num_tokens), dim3(256), 0, s, (const float*)h, mu, n_mix,
+                      width, num_tokens, req_of_tok, cu_q, slots, state, (size_t)state_stride, (size_t)prev_offset,
+                      (float*)out);
     else if (h_dtype == TI_BF16)
-        ti_launch_pdl((token_shift_mix_kernel<bf16>), dim3(num_tokens), dim3(256), 0, s, (const bf16*)h, mu, n_mix, width, num_tokens,
-            req_of_tok, cu_q, slots, state, (size_t)state_stride, (size_t)prev_offset, (bf16*)out);
+        ti_launch_pdl(token_shift_mix_kernel<bf16>, dim3(num_tokens), dim3(256), 0, s, (const bf16*)h, mu, n_mix,
+                      width, num_tokens, req_of_tok, cu_q, slots, state, (size_t)state_stride, (size_t)prev_offset,
+                      (bf16*)out);
     else
         return ti_fail("token_shift_mix: dtype code %d is not supported", h_dtype);
     return ti_check_launch("token_shift_mix");
@@ -288,7 +290,8 @@ extern "C" int ti_wkv_recurrence(const float* r, const float* k, const float* v,
     dim3 grid(num_requests, num_heads, col_split);
     cudaStream_t s = (cudaStream_t)stream;
 #define LAUNCH(TH, DMAX, JS)                                                                       \
-    ti_launch_if_early(num_tokens == num_requests, (wkv_recurrence_kernel<TH, TH, DMAX, JS>), grid, dim3(DMAX / JS * wkv_lanes(DMAX, JS)), 0, s,                      \
+    ti_launch_if_early(num_tokens == num_requests, (wkv_recurrence_kernel<TH, TH, DMAX, JS>), grid, \
+        dim3(DMAX / JS * wkv_lanes(DMAX, JS)), 0, s,                                                \
         r, k, v, g, a, in_stride, w0, u, norm_weight, eps, (const TH*)h, width, cu_q, slots, state,    \
         (size_t)state_stride, (size_t)prev_offset, num_heads, d, (TH*)out, o_raw)
 #define CALL(TH)                                                                                   \
@@ -296,7 +299,8 @@ extern "C" int ti_wkv_recurrence(const float* r, const float* k, const float* v,
         if (d <= 32) LAUNCH(TH, 32, 4); else if (d <= 64) LAUNCH(TH, 64, 4); else LAUNCH(TH, 128, 4); \
         if (int rc = ti_check_launch("wkv_recurrence")) return rc;                                 \
         const int items = num_tokens * num_heads;                                                  \
-        ti_launch_pdl((wkv_finish_kernel<TH>), dim3((items + 7) / 8), dim3(256), 0, s, o_raw, g, in_stride, norm_weight, eps, items, \
+        ti_launch_pdl((wkv_finish_kernel<TH>), dim3((items + 7) / 8), dim3(256), 0, s, o_raw, g, in_stride, \
+            norm_weight, eps, items,                                                                        \
                                                             num_heads, d, (TH*)out);               \
         return ti_check_launch("wkv_finish");                                                      \
     }                                                                                              \
@@ -313,8 +317,10 @@ extern "C" int ti_tanh_rows(const float* x, long long n, void* out, int out_dtyp
     if (n == 0) return 0;
     cudaStream_t s = (cudaStream_t)stream;
     const unsigned blocks = (unsigned)((n + 255) / 256);
-    if (out_dtype == TI_F32) ti_launch_pdl((tanh_rows_kernel<float>), dim3(blocks), dim3(256), 0, s, x, (size_t)n, (float*)out);
-    else if (out_dtype == TI_BF16) ti_launch_pdl((tanh_rows_kernel<bf16>), dim3(blocks), dim3(256), 0, s, x, (size_t)n, (bf16*)out);
+    if (out_dtype == TI_F32) ti_launch_pdl(tanh_rows_kernel<float>, dim3(blocks), dim3(256), 0, s, x, (size_t)n,
+                                           (float*)out);
+    else if (out_dtype == TI_BF16) ti_launch_pdl(tanh_rows_kernel<bf16>, dim3(blocks), dim3(256), 0, s, x, (size_t)n,
+                                                 (bf16*)out);
     else return ti_fail("tanh_rows: dtype code %d is not supported", out_dtype);
     return ti_check_launch("tanh_rows");
 }
@@ -324,8 +330,10 @@ extern "C" int ti_xielu_rows(const float* x, long long n, float ap, float aq, vo
     if (n == 0) return 0;
     cudaStream_t s = (cudaStream_t)stream;
     const unsigned blocks = (unsigned)((n + 255) / 256);
-    if (out_dtype == TI_F32) ti_launch_pdl((xielu_rows_kernel<float>), dim3(blocks), dim3(256), 0, s, x, (size_t)n, ap, aq, (float*)out);
-    else if (out_dtype == TI_BF16) ti_launch_pdl((xielu_rows_kernel<bf16>), dim3(blocks), dim3(256), 0, s, x, (size_t)n, ap, aq, (bf16*)out);
+    if (out_dtype == TI_F32) ti_launch_pdl(xielu_rows_kernel<float>, dim3(blocks), dim3(256), 0, s, x, (size_t)n, ap,
+                                           aq, (float*)out);
+    else if (out_dtype == TI_BF16) ti_launch_pdl(xielu_rows_kernel<bf16>, dim3(blocks), dim3(256), 0, s, x, (size_t)n,
+                                                 ap, aq, (bf16*)out);
     else return ti_fail("xielu_rows: dtype code %d is not supported", out_dtype);
     return ti_check_launch("xielu_rows");
 }

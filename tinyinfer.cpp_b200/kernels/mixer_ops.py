@@ -415,7 +415,9 @@ class MixerOps:
             # over shared rows, the slices of the value columns (2)
             mode = 0 if not single else 2 if (shared_rows and 1 < slices <= 4) else 1 if gp <= 16 else 0
             if mode == 0 and shared_rows and dv % 256 == 0:
-                slices = dv // 256                    # prompt portions over shared rows: 256 columns a block
+                # prompt portions over shared rows that the tcgen05 kernel does not take (rows of more than 576
+                # elements, more than 128 heads): 256 columns a block
+                slices = dv // 256
             head_blocks = -(-(num_heads // num_kv_heads) // (min(gp, 16) if mode == 2 else gp))
             blocks = tiles.shape[0] * num_kv_heads * head_blocks * (1 if mode == 2 else slices)
             per_sm = self._key_run_blocks_per_sm(dk, dv // slices, shared_rows)
