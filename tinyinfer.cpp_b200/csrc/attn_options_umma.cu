@@ -17,10 +17,10 @@
 // What bounds it (clock stamps in the roles).  Latent rows of 576 with 256 value columns: 7,000 cycles a tile, a chain of
 // 12 value products (137 each), the reload of the value chunks, the last 16 of 36 score products (98 each, issue as much
 // as operand reads) and the softmax; rows of 288: 4,300.  Heads of 128 with a cap: 6,800 a tile and block, of which the
-// softmax takes 4,300, two blocks at a time.  16 heads over 2,048 tokens at positions 0 / 2,048: latent 576 259 / 743 us
-// (416 / 1,232 with one issuing thread and a barrier per chunk), latent 288 93 / 244 (143 / 387), heads of 128 over 4 kv
-// heads with a cap 145 / 281 (177 / 343).  The mma.sync kernel took 2,114 us for the first and 322 for the last as the
-// mean of such two launches.  Steps without a portion stay with that kernel: it cuts a row's keys over blocks.
+// softmax takes 4,300, two blocks at a time.  16 heads over 2,048 tokens at positions 0 / 2,048, us, against the mma.sync
+// kernel: latent 576 258 / 744 against 1,217 / 3,152 (416 / 1,232 with one issuing thread and a barrier per chunk), latent
+// 288 91 / 251 against 387 / 916, heads of 128 over 4 kv heads with a cap 132 / 269 against 317 / 766, of 64 with a cap
+// 123 / 249 against 210 / 558.  Steps without a portion stay with that kernel: it cuts a row's keys over blocks.
 //
 // Two forms.  Rows of up to 128 elements with values of their own (NS = 1): two blocks per SM that fill one another's
 // gaps, with 256 columns of tensor memory each: outputs up to 128, scores 64, weights 96, of which the last 32 lie where
