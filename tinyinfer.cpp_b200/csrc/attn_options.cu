@@ -29,19 +29,12 @@
 // depends on the row alone, so a row's bits do not depend on the batch or on how a prompt was cut.
 // Page layout without `shared_rows`: keys [kv head][slot][dk], behind them values [kv head][slot][dv].
 #include "common.cuh"
+#include "head_units.cuh"
 
 namespace {
 
 constexpr int WARPS = 4;
 enum { TI_ERR_BAD_PAGE = 1 };
-
-__device__ __forceinline__ float turned(const float* x, int j, float pos, const float* inv_freq, float unit) {
-    // element j (inside the rotated width) of a head x after the turn; `unit` scales both inputs
-    float s, c;
-    sincosf(pos * inv_freq[j >> 1], &s, &c);
-    const float a = x[j] * unit, b = x[j ^ 1] * unit;
-    return (j & 1) ? a * c + b * s : a * c - b * s;
-}
 
 // The turn of a head by a table of the token's cosines and sines (`cs[pair]`, made once per token: the angle
 // depends on the position and the pair alone, not on the head).  A head of n elements whose first `rot` are
@@ -156,6 +149,123 @@ qkv_turn_store_kernel(const float* proj, int stride, const RowNorm norm, const V
     }
 }
 
+// The same where heads and turned widths fall into units of four elements: a thread keeps NU units of the query
+// and key row in registers, so that the row is read once, four elements a load; cosines, sines and the page are looked
+// up before the wait, values go through while the norms' loads are on their way, and both norms' sums meet at one
+// barrier.  One block per token; what bounds it is the block's chain of latencies, once in a step of single tokens and as
+// often as blocks follow one another on an SM for many.  AHEAD: the weights are asked for before the wait; many tokens
+// rather have more blocks an SM.  16 query and 4 key heads, norms over whole rows, us element by element (a sine per
+// element) -> now at one and 2,048 tokens: heads of 64 5.6 -> 2.9, 19.4 -> 14.2, of 128 8.6 -> 3.3, 33 -> 17.8 (with
+// blocks of 512 threads 26.1).
+struct RowHeads {
+    const float* proj; int stride;
+    RowNorm norm; ValueMix mix;
+    const float* inv_freq; int rot, halves; float mag;
+    const float* v_inv_freq; int v_rot, v_halves;
+    const int* positions; const int* req_of_tok; const int* block_table; int bt_stride;
+    int num_pages, page_size, write_kv, num_heads, num_kv_heads, dk, dv;
+};
+
+template <typename TQ, typename TC, int THREADS, int NU, bool AHEAD>
+__global__ void __launch_bounds__(THREADS, 1024 / THREADS)
+row_heads_units_kernel(const RowHeads p, TC* __restrict__ pages, TQ* __restrict__ q_out, int* __restrict__ status) {
+    extern __shared__ __align__(16) float2 turn_table[];
+    constexpr int WARPS_ = THREADS / 32;
+    __shared__ float sums[2][WARPS_];
+    const int t = blockIdx.x, tid = threadIdx.x, pos = p.positions[t];
+    const int hu = p.dk >> 2, qu = p.num_heads * hu, total = qu + (p.write_kv ? p.num_kv_heads * hu : 0);
+    const int nq = p.num_heads * p.dk, nk = p.num_kv_heads * p.dk;
+    float2* vcs = turn_table + (p.rot >> 1);
+    pdl_launch();
+    fill_turn_table(turn_table, p.rot >> 1, (float)pos, p.inv_freq, p.mag);
+    TC* page = nullptr;                                // the token's page: keys of head 0
+    if (p.write_kv) {
+        fill_turn_table(vcs, p.v_rot >> 1, (float)pos, p.v_inv_freq, 1.0f);
+        const int id = p.block_table[(size_t)p.req_of_tok[t] * p.bt_stride + pos / p.page_size];
+        if (id >= 0 && id < p.num_pages) page = pages + (size_t)id * p.num_kv_heads * p.page_size * (p.dk + p.dv);
+        else if (tid == 0) atomicCAS(status, 0, TI_ERR_BAD_PAGE);
+    }
+    const int slot = pos % p.page_size;
+    // unit i: its head (query heads, behind them key heads) and its place there
+    auto head_of = [&](int i) { return i / hu; };
+    auto place_of = [&](int i) { return i - i / hu * hu; };
+    auto weight_of = [&](int i) {
+        const float* weight = i < qu ? p.norm.q_weight : p.norm.k_weight;
+        if (i >= total || !p.norm.on || !weight) return make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+        const int u = place_of(i);
+        return load_unit(weight + (head_of(i) - (i < qu ? 0 : p.num_heads)) * p.dk, u, u < p.rot >> 2, p.halves, p.rot >> 1);
+    };
+    float4 w[NU], x[NU];
+    if (AHEAD) {
+#pragma unroll
+        for (int j = 0; j < NU; ++j) w[j] = weight_of(tid + THREADS * j);
+    }
+    __syncthreads();                                   // the turn tables
+    pdl_wait();
+    const float* row = p.proj + (size_t)t * p.stride;
+    float2 ss = make_float2(0.0f, 0.0f);               // of the query row, of the key row
+#pragma unroll
+    for (int j = 0; j < NU; ++j) {
+        const int i = tid + THREADS * j;
+        x[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (i < total) {
+            const int u = place_of(i);
+            x[j] = load_unit(row + head_of(i) * p.dk, u, u < p.rot >> 2, p.halves, p.rot >> 1);
+        }
+    }
+    if (page) {
+        const int vu = p.dv >> 2;
+        const float* first = p.mix.first ? p.mix.first + (size_t)t * p.mix.stride : nullptr;
+        TC* values = page + (size_t)p.num_kv_heads * p.page_size * p.dk;
+        for (int i = tid; i < p.num_kv_heads * vu; i += THREADS) {
+            const int g = i / vu, u = i - g * vu;
+            const bool turned = u < p.v_rot >> 2;
+            float4 v = load_unit(row + nq + nk + g * p.dv, u, turned, p.v_halves, p.v_rot >> 1);
+            if (first) {
+                const float4 f = load_unit(first + g * p.dv, u, turned, p.v_halves, p.v_rot >> 1);
+                const float own = 1.0f - p.mix.share;
+                v = make_float4(own * v.x + p.mix.share * f.x, own * v.y + p.mix.share * f.y, own * v.z + p.mix.share * f.z,
+                                own * v.w + p.mix.share * f.w);
+            }
+            if (turned) v = turn_unit(v, vcs, u);
+            store_unit<TC>(values + ((size_t)g * p.page_size + slot) * p.dv, u, turned, p.v_halves, p.v_rot >> 1, v);
+        }
+    }
+    float inv_q = 1.0f, inv_k = 1.0f;
+    if (p.norm.on) {
+#pragma unroll
+        for (int j = 0; j < NU; ++j) {
+            const float s = fmaf(x[j].w, x[j].w, fmaf(x[j].z, x[j].z, fmaf(x[j].y, x[j].y, x[j].x * x[j].x)));
+            if (tid + THREADS * j < qu) ss.x += s; else ss.y += s;
+        }
+        ss = make_float2(warp_sum(ss.x), warp_sum(ss.y));
+        if ((tid & 31) == 0) { sums[0][tid >> 5] = ss.x; sums[1][tid >> 5] = ss.y; }
+        __syncthreads();
+        ss = make_float2(0.0f, 0.0f);
+#pragma unroll
+        for (int i = 0; i < WARPS_; ++i) { ss.x += sums[0][i]; ss.y += sums[1][i]; }
+        inv_q = 1.0f / sqrtf(ss.x / (float)nq + p.norm.eps);
+        inv_k = 1.0f / sqrtf(ss.y / (float)nk + p.norm.eps);
+    }
+#pragma unroll
+    for (int j = 0; j < NU; ++j) {
+        const int i = tid + THREADS * j;
+        if (i >= total) break;
+        const int h = head_of(i), u = place_of(i);
+        const bool turned = u < p.rot >> 2;
+        const float inv = i < qu ? inv_q : inv_k;
+        float4 v = x[j];
+        if (p.norm.on) {
+            if (!AHEAD) w[j] = weight_of(i);
+            v = make_float4(v.x * inv * w[j].x, v.y * inv * w[j].y, v.z * inv * w[j].z, v.w * inv * w[j].w);
+        }
+        if (turned) v = turn_unit(v, turn_table, u);
+        if (i < qu) store_unit<TQ>(q_out + (size_t)t * nq + h * p.dk, u, turned, p.halves, p.rot >> 1, v);
+        else if (page) store_unit<TC>(page + ((size_t)(h - p.num_heads) * p.page_size + slot) * p.dk, u, turned, p.halves,
+                                      p.rot >> 1, v);
+    }
+}
+
 // x[t, h, :] turned by sign * position over its first `rot` elements, then times sigmoid(gate[t, h * n + j]); a
 // block per token, a thread reads and writes both elements of a pair, so the rows may be turned in place
 template <typename T>
@@ -191,79 +301,6 @@ turn_rows_kernel(const T* x, const int* positions, const float* inv_freq, int ro
     }
 }
 
-template <typename TQ, typename TC>
-__global__ void __launch_bounds__(256)
-qk_rownorm_rope_store_kernel(const float* proj, int stride, const float* q_weight,
-                             const float* k_weight, float eps,
-                             const float* inv_freq, int rot,
-                             const int* positions, const int* req_of_tok,
-                             const int* block_table, int bt_stride, TC* __restrict__ pages,
-                             int num_pages, int page_size, int write_kv, int num_heads, int num_kv_heads,
-                             int dk, int dv, TQ* __restrict__ q_out, int* __restrict__ status) {
-    pdl_launch();
-    pdl_wait();
-    __shared__ float scratch[32];
-    const int t = blockIdx.x;
-    const int nq = num_heads * dk, nk = num_kv_heads * dk, nv = num_kv_heads * dv;
-    const float* row = proj + (size_t)t * stride;
-    const int pos_i = positions[t];
-    const float pos = (float)pos_i;
-    float ss = 0.0f;
-    for (int e = threadIdx.x; e < nq; e += blockDim.x) ss = fmaf(row[e], row[e], ss);
-    const float inv_q = 1.0f / sqrtf(block_sum(ss, scratch) / (float)nq + eps);
-    for (int e = threadIdx.x; e < nq; e += blockDim.x) {
-        const int j = e % dk;
-        const float* head = row + (e - j);
-        const float* w = q_weight ? q_weight + (e - j) : nullptr;
-        float y;
-        if (j < rot) {
-            // the weight belongs to the element, so it is applied before the turn
-            float s, c;
-            sincosf(pos * inv_freq[j >> 1], &s, &c);
-            const float a = head[j] * inv_q * (w ? w[j] : 1.0f);
-            const float b = head[j ^ 1] * inv_q * (w ? w[j ^ 1] : 1.0f);
-            y = (j & 1) ? a * c + b * s : a * c - b * s;
-        } else {
-            y = head[j] * inv_q * (w ? w[j] : 1.0f);
-        }
-        q_out[(size_t)t * nq + e] = from_f32<TQ>(y);
-    }
-    if (!write_kv) return;
-    const int page = block_table[(size_t)req_of_tok[t] * bt_stride + pos_i / page_size];
-    if (page < 0 || page >= num_pages) {
-        if (threadIdx.x == 0) atomicCAS(status, 0, TI_ERR_BAD_PAGE);
-        return;
-    }
-    const int slot = pos_i % page_size;
-    TC* base = pages + (size_t)page * num_kv_heads * page_size * (dk + dv);
-    const float* krow = row + nq;
-    ss = 0.0f;
-    for (int e = threadIdx.x; e < nk; e += blockDim.x) ss = fmaf(krow[e], krow[e], ss);
-    const float inv_k = 1.0f / sqrtf(block_sum(ss, scratch) / (float)nk + eps);
-    for (int e = threadIdx.x; e < nk; e += blockDim.x) {
-        const int j = e % dk, g = e / dk;
-        const float* head = krow + (e - j);
-        const float* w = k_weight ? k_weight + (e - j) : nullptr;
-        float y;
-        if (j < rot) {
-            float s, c;
-            sincosf(pos * inv_freq[j >> 1], &s, &c);
-            const float a = head[j] * inv_k * (w ? w[j] : 1.0f);
-            const float b = head[j ^ 1] * inv_k * (w ? w[j ^ 1] : 1.0f);
-            y = (j & 1) ? a * c + b * s : a * c - b * s;
-        } else {
-            y = head[j] * inv_k * (w ? w[j] : 1.0f);
-        }
-        base[((size_t)g * page_size + slot) * dk + j] = from_f32<TC>(y);
-    }
-    TC* vbase = base + (size_t)num_kv_heads * page_size * dk;
-    const float* vrow = krow + nk;
-    for (int e = threadIdx.x; e < nv; e += blockDim.x) {
-        const int j = e % dv, g = e / dv;
-        vbase[((size_t)g * page_size + slot) * dv + j] = from_f32<TC>(vrow[e]);
-    }
-}
-
 // out[t, :] = x[t, :n] / sqrt(mean(x[t, :n]^2) + eps) * w over rows with a stride: the norm of a column slice of a
 // product (a latent that shares its product with other columns)
 template <typename TO>
@@ -280,7 +317,11 @@ slice_rmsnorm_kernel(const float* x, int stride, int n, const float* w, float ep
         out[(size_t)blockIdx.x * n + e] = from_f32<TO>(row[e] * inv * (w ? w[e] : 1.0f));
 }
 
-template <typename TQ, typename TC>
+// Grid: tokens x 2; the first block of a token has its query heads, the second its latent and key part.  UNITS: all parts
+// are multiples of four elements on aligned rows, which then travel four at a time, a thread's loads together.  Cosines
+// and sines are made before the wait, once per token instead of once per head.  16 heads, latent of 512: one token 6.6 ->
+// 1.9 us, 2,048 tokens 23.4 -> 9.7.
+template <typename TQ, typename TC, bool UNITS>
 __global__ void __launch_bounds__(256)
 latent_prepare_kernel(const float* qproj, int q_stride, const float* proj, int stride,
                       const float* latent_weight, float eps,
@@ -288,139 +329,176 @@ latent_prepare_kernel(const float* qproj, int q_stride, const float* proj, int s
                       const int* req_of_tok, const int* block_table, int bt_stride,
                       TC* __restrict__ pages, int num_pages, int page_size, int num_heads, int dk, int dr,
                       int rank, TQ* __restrict__ q_plain, TQ* __restrict__ q_full, int* __restrict__ status) {
-    pdl_launch();
-    pdl_wait();
+    extern __shared__ __align__(16) float2 cs[];
     __shared__ float scratch[32];
-    const int t = blockIdx.x;
-    const int qh = dk + dr, nq = num_heads * qh, row_len = rank + dr;
-    const float* row = qproj + (size_t)t * q_stride;
-    const int pos_i = positions[t];
-    const float pos = (float)pos_i;
-    for (int e = threadIdx.x; e < nq; e += blockDim.x) {
-        const int j = e % qh, h = e / qh;
-        if (j < dk) q_plain[((size_t)t * num_heads + h) * dk + j] = from_f32<TQ>(row[e]);
-        else q_full[((size_t)t * num_heads + h) * row_len + rank + (j - dk)] =
-                 from_f32<TQ>(mag * turned(row + h * qh + dk, j - dk, pos, inv_freq, 1.0f));
-    }
-    const int page = block_table[(size_t)req_of_tok[t] * bt_stride + pos_i / page_size];
-    if (page < 0 || page >= num_pages) {
-        if (threadIdx.x == 0) atomicCAS(status, 0, TI_ERR_BAD_PAGE);
+    const int t = blockIdx.x, tid = threadIdx.x, pos = positions[t];
+    const int qh = dk + dr, row_len = rank + dr;
+    pdl_launch();
+    fill_turn_table(cs, dr >> 1, (float)pos, inv_freq, mag);
+    __syncthreads();
+    auto pair = [&](const float* x, int j) {             // element j of the turned part x
+        const float2 f = cs[j >> 1];
+        return (j & 1) ? x[j] * f.x + x[j ^ 1] * f.y : x[j] * f.x - x[j ^ 1] * f.y;
+    };
+    if (blockIdx.y == 0) {
+        pdl_wait();
+        const float* row = qproj + (size_t)t * q_stride;
+        TQ* plain = q_plain + (size_t)t * num_heads * dk;
+        TQ* full = q_full + (size_t)t * num_heads * row_len + rank;
+        if (UNITS) {
+            const int hu = qh >> 2, total = num_heads * hu;
+            for (int i0 = tid; i0 < total; i0 += 4 * 256) {
+                float4 v[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if (i0 + 256 * j < total) v[j] = *reinterpret_cast<const float4*>(row + 4 * (i0 + 256 * j));
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int i = i0 + 256 * j;
+                    if (i >= total) break;
+                    const int h = i / hu, u = i - h * hu, r = u - (dk >> 2);
+                    if (r < 0) {
+                        store_unit<TQ>(plain + (size_t)h * dk, u, false, 0, 0, v[j]);
+                    } else {
+                        const float4 pairs = make_float4(v[j].x, v[j].z, v[j].y, v[j].w);
+                        store_unit<TQ>(full + (size_t)h * row_len, r, true, 0, 0, turn_unit(pairs, cs, r));
+                    }
+                }
+            }
+        } else {
+            for (int e = tid; e < num_heads * qh; e += 256) {
+                const int j = e % qh, h = e / qh;
+                if (j < dk) plain[(size_t)h * dk + j] = from_f32<TQ>(row[e]);
+                else full[(size_t)h * row_len + (j - dk)] = from_f32<TQ>(pair(row + h * qh + dk, j - dk));
+            }
+        }
         return;
     }
-    TC* dst = pages + ((size_t)page * page_size + pos_i % page_size) * row_len;
-    const float* lat = proj + (size_t)t * stride;
-    float ss = 0.0f;
-    for (int e = threadIdx.x; e < rank; e += blockDim.x) ss = fmaf(lat[e], lat[e], ss);
-    const float inv = 1.0f / sqrtf(block_sum(ss, scratch) / (float)rank + eps);
-    for (int e = threadIdx.x; e < rank; e += blockDim.x)
-        dst[e] = from_f32<TC>(lat[e] * inv * (latent_weight ? latent_weight[e] : 1.0f));
-    for (int e = threadIdx.x; e < dr; e += blockDim.x)
-        dst[rank + e] = from_f32<TC>(mag * turned(lat + rank, e, pos, inv_freq, 1.0f));
-}
-
-// out[t, h, n] = sum_k in[t, h, k] * w[h, k, n]; a block has 16 tokens of one head and 128 columns.
-// Its eight warps take an eighth of k each, a lane four neighbouring columns (8 bytes of a weight row
-// a load, eight loads in flight), so that a step of few tokens, whose grid is a block or a few per
-// head, still has the weights of a head on their way at once; the tokens' inputs lie in shared
-// memory with the tokens of one k side by side (read four at a time, the same address for the whole
-// warp), and the warps' partial sums meet in shared memory in a fixed order.
-constexpr int HP_TOKENS = 16;
-constexpr int HP_WARPS = 8;
-
-template <typename TW> __device__ __forceinline__ void load4(const TW* p, bool whole, int left, float (&w)[4]);
-template <> __device__ __forceinline__ void load4<bf16>(const bf16* p, bool whole, int left, float (&w)[4]) {
-    if (whole) {
-        const uint2 raw = *reinterpret_cast<const uint2*>(p);
-        const __nv_bfloat162 lo = *reinterpret_cast<const __nv_bfloat162*>(&raw.x);
-        const __nv_bfloat162 hi = *reinterpret_cast<const __nv_bfloat162*>(&raw.y);
-        w[0] = __bfloat162float(lo.x); w[1] = __bfloat162float(lo.y);
-        w[2] = __bfloat162float(hi.x); w[3] = __bfloat162float(hi.y);
-    } else {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) w[i] = i < left ? __bfloat162float(p[i]) : 0.0f;
-    }
-}
-template <> __device__ __forceinline__ void load4<float>(const float* p, bool whole, int left, float (&w)[4]) {
-    if (whole) {
-        const float4 raw = *reinterpret_cast<const float4*>(p);
-        w[0] = raw.x; w[1] = raw.y; w[2] = raw.z; w[3] = raw.w;
-    } else {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) w[i] = i < left ? p[i] : 0.0f;
-    }
-}
-
-template <typename TI, typename TW, typename TO>
-__global__ void __launch_bounds__(HP_WARPS * 32)
-head_project_kernel(const TI* in, int in_stride_t, int in_stride_h, const TW* w, int n_in,
-                    int n_out, TO* out, int out_stride_t, int out_stride_h, int num_tokens, int vec_ok) {
-    pdl_launch();
+    const int page = block_table[(size_t)req_of_tok[t] * bt_stride + pos / page_size];
     pdl_wait();
-    extern __shared__ __align__(16) float xs[];      // [n_in][HP_TOKENS]; afterwards the warps' partial sums
-    const int t0 = blockIdx.x * HP_TOKENS, h = blockIdx.y;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int n0 = blockIdx.z * 128 + lane * 4;      // this lane's first column
-    const int nt = min(HP_TOKENS, num_tokens - t0);
-    for (int e = threadIdx.x; e < HP_TOKENS * n_in; e += HP_WARPS * 32) {
-        const int tt = e / n_in, k = e % n_in;
-        xs[k * HP_TOKENS + tt] =
-            tt < nt ? to_f32(in[(size_t)(t0 + tt) * in_stride_t + (size_t)h * in_stride_h + k]) : 0.0f;
+    if (page < 0 || page >= num_pages) {
+        if (tid == 0) atomicCAS(status, 0, TI_ERR_BAD_PAGE);
+        return;
+    }
+    TC* dst = pages + ((size_t)page * page_size + pos % page_size) * row_len;
+    const float* lat = proj + (size_t)t * stride;
+    if (UNITS && rank <= 4 * 256) {                      // the latent in registers: read once
+        const bool mine = 4 * tid < rank;
+        float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (mine) v = *reinterpret_cast<const float4*>(lat + 4 * tid);
+        for (int r = tid; r < dr >> 2; r += 256)
+            store_unit<TC>(dst + rank, r, true, 0, 0, turn_unit(load_unit(lat + rank, r, true, 0, 0), cs, r));
+        const float ss = fmaf(v.w, v.w, fmaf(v.z, v.z, fmaf(v.y, v.y, v.x * v.x)));
+        const float inv = 1.0f / sqrtf(block_sum(ss, scratch) / (float)rank + eps);
+        if (!mine) return;
+        float4 w = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+        if (latent_weight) w = *reinterpret_cast<const float4*>(latent_weight + 4 * tid);
+        store_unit<TC>(dst, tid, false, 0, 0, make_float4(v.x * inv * w.x, v.y * inv * w.y, v.z * inv * w.z, v.w * inv * w.w));
+        return;
+    }
+    float ss = 0.0f;
+    for (int e = tid; e < rank; e += 256) ss = fmaf(lat[e], lat[e], ss);
+    const float inv = 1.0f / sqrtf(block_sum(ss, scratch) / (float)rank + eps);
+    for (int e = tid; e < rank; e += 256)
+        dst[e] = from_f32<TC>(lat[e] * inv * (latent_weight ? latent_weight[e] : 1.0f));
+    for (int e = tid; e < dr; e += 256) dst[rank + e] = from_f32<TC>(pair(lat + rank, e));
+}
+
+// out[t, h, n] = sum_k in[t, h, k] * w[h, k, n], bfloat16, for few tokens: a block has up to TT tokens of one head and 32
+// columns, a thread four neighbouring columns (8 bytes of a weight row a load) and every 32nd k.  What bounds it is the
+// weights' way from memory, so all blocks of a head together ask for all of them at once, and up to KP rows a thread
+// before the wait for the kernel before; the tokens' inputs lie in shared memory with the tokens of one k side by side,
+// and the threads' sums meet by shuffles and in shared memory in a fixed order.  16 heads, us at one token: 128 -> 512
+// 5.7 -> 2.7, 512 -> 128 15.5 -> 2.9 (blocks of 128 columns: 16 of them, an eighth of k a warp).
+constexpr int HP_TOKENS = 16;      // most tokens of a block
+constexpr int HP_COLS = 32, HP_GROUPS = 32, HP_THREADS = HP_COLS / 4 * HP_GROUPS;
+
+__device__ __forceinline__ uint2 load4(const bf16* p, bool whole, int left) {
+    if (whole) return *reinterpret_cast<const uint2*>(p);
+    bf16 v[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = i < left ? p[i] : __float2bfloat16_rn(0.0f);
+    const __nv_bfloat162 lo = __halves2bfloat162(v[0], v[1]), hi = __halves2bfloat162(v[2], v[3]);
+    return make_uint2(*reinterpret_cast<const unsigned*>(&lo), *reinterpret_cast<const unsigned*>(&hi));
+}
+
+template <int TT, int KP>
+__global__ void __launch_bounds__(HP_THREADS)
+head_project_few_kernel(const bf16* in, int in_stride_t, int in_stride_h, const bf16* __restrict__ w, int n_in,
+                        int n_out, bf16* out, int out_stride_t, int out_stride_h, int num_tokens, int vec_ok) {
+    extern __shared__ __align__(16) float xs[];      // [n_in][TT]; afterwards the warps' partial sums [8][TT][HP_COLS]
+    const int t0 = blockIdx.x * TT, h = blockIdx.y, tid = threadIdx.x, kg = tid >> 3;
+    const int n0 = blockIdx.z * HP_COLS + (tid & 7) * 4;
+    const int nt = min(TT, num_tokens - t0), left = n_out - n0;
+    const bool whole = vec_ok && left >= 4;
+    const bf16* wh = w + (size_t)h * n_in * n_out + n0;
+    pdl_launch();
+    uint2 wv[KP];
+    auto fetch = [&](int k0) {
+#pragma unroll
+        for (int i = 0; i < KP; ++i) {
+            const int k = k0 + kg + HP_GROUPS * i;
+            wv[i] = make_uint2(0u, 0u);
+            if (k < n_in && left > 0) wv[i] = load4(wh + (size_t)k * n_out, whole, left);
+        }
+    };
+    fetch(0);
+    pdl_wait();
+    for (int k = tid; k < n_in; k += HP_THREADS) {
+        const bf16* src = in + (size_t)t0 * in_stride_t + (size_t)h * in_stride_h + k;
+        float x[TT];                                 // all tokens' loads together
+#pragma unroll
+        for (int tt = 0; tt < TT; ++tt) x[tt] = tt < nt ? to_f32(src[(size_t)tt * in_stride_t]) : 0.0f;
+#pragma unroll
+        for (int tt = 0; tt < TT; tt += 4) store4(xs + k * TT + tt, make_float4(x[tt], x[tt + 1], x[tt + 2], x[tt + 3]));
     }
     __syncthreads();
-    float acc[HP_TOKENS][4];
+    float acc[TT][4];
 #pragma unroll
-    for (int i = 0; i < HP_TOKENS; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.0f;
-    const int left = n_out - n0;                     // columns of this lane that exist
-    if (left > 0) {
-        const bool whole = vec_ok && left >= 4;
-        const TW* wh = w + (size_t)h * n_in * n_out + n0;
-        const int per = (n_in + HP_WARPS - 1) / HP_WARPS;
-        const int k_end = min(n_in, (warp + 1) * per);
-#pragma unroll 8
-        for (int k = warp * per; k < k_end; ++k) {
-            float wv[4];
-            load4<TW>(wh + (size_t)k * n_out, whole, left, wv);
-            const float4* x4 = reinterpret_cast<const float4*>(xs + k * HP_TOKENS);
+    for (int i = 0; i < TT; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.0f;
+    for (int k0 = 0; k0 < n_in; k0 += HP_GROUPS * KP) {
+        if (k0) fetch(k0);
 #pragma unroll
-            for (int i = 0; i < HP_TOKENS / 4; ++i) {
-                const float4 x = x4[i];
+        for (int i = 0; i < KP; ++i) {
+            const int k = k0 + kg + HP_GROUPS * i;
+            if (k >= n_in) break;
+            const __nv_bfloat162 lo = *reinterpret_cast<const __nv_bfloat162*>(&wv[i].x);
+            const __nv_bfloat162 hi = *reinterpret_cast<const __nv_bfloat162*>(&wv[i].y);
+            const float wf[4] = {__bfloat162float(lo.x), __bfloat162float(lo.y), __bfloat162float(hi.x), __bfloat162float(hi.y)};
+            const float4* x4 = reinterpret_cast<const float4*>(xs + k * TT);
+#pragma unroll
+            for (int q = 0; q < TT / 4; ++q) {
+                const float4 x = x4[q];
                 const float xv[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
                 for (int a = 0; a < 4; ++a)
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) acc[4 * i + a][c] = fmaf(xv[a], wv[c], acc[4 * i + a][c]);
+                    for (int c = 0; c < 4; ++c) acc[4 * q + a][c] = fmaf(xv[a], wf[c], acc[4 * q + a][c]);
             }
         }
     }
-    // the warps' sums meet in a fixed order (the upper half of the warps hands its sums to the lower
-    // half, three times), so a row's bits are the same in every run
-    float4* meet = reinterpret_cast<float4*>(xs);    // [warp][HP_TOKENS][32 lanes] of four columns
 #pragma unroll
-    for (int half = HP_WARPS / 2; half >= 1; half /= 2) {
-        __syncthreads();                             // the inputs, or the round before, have been read
-        if (warp >= half && warp < 2 * half) {
+    for (int i = 0; i < TT; ++i)
 #pragma unroll
-            for (int i = 0; i < HP_TOKENS; ++i)
-                meet[((warp - half) * HP_TOKENS + i) * 32 + lane] = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+        for (int c = 0; c < 4; ++c) {
+            acc[i][c] += __shfl_xor_sync(0xffffffffu, acc[i][c], 8);
+            acc[i][c] += __shfl_xor_sync(0xffffffffu, acc[i][c], 16);
         }
-        __syncthreads();
-        if (warp < half) {
+    __syncthreads();                                 // the inputs have been read
+    if ((tid & 31) < 8) {
 #pragma unroll
-            for (int i = 0; i < HP_TOKENS; ++i) {
-                const float4 o = meet[(warp * HP_TOKENS + i) * 32 + lane];
-                acc[i][0] += o.x; acc[i][1] += o.y; acc[i][2] += o.z; acc[i][3] += o.w;
-            }
-        }
+        for (int i = 0; i < TT; ++i)
+            *reinterpret_cast<float4*>(xs + ((tid >> 5) * TT + i) * HP_COLS + (tid & 7) * 4) =
+                make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
     }
-    if (warp == 0 && left > 0) {
+    __syncthreads();
+    for (int e = tid; e < nt * HP_COLS; e += HP_THREADS) {
+        const int tt = e / HP_COLS, c = e % HP_COLS, n = blockIdx.z * HP_COLS + c;
+        if (n >= n_out) continue;
+        float sum = 0.0f;
 #pragma unroll
-        for (int i = 0; i < HP_TOKENS; ++i) {
-            if (i >= nt) break;
-            TO* dst = out + (size_t)(t0 + i) * out_stride_t + (size_t)h * out_stride_h + n0;
-#pragma unroll
-            for (int c = 0; c < 4; ++c)
-                if (c < left) dst[c] = from_f32<TO>(acc[i][c]);
-        }
+        for (int i = 0; i < HP_THREADS / 32; ++i) sum += xs[(i * TT + tt) * HP_COLS + c];
+        out[(size_t)(t0 + tt) * out_stride_t + (size_t)h * out_stride_h + n] = __float2bfloat16_rn(sum);
     }
 }
 
@@ -562,69 +640,6 @@ attention_options_kernel(const TQ* q, const int* __restrict__ rows, const int* _
     }
 }
 
-// The same with a norm per head: every query head and every key head is divided by its own
-// sqrt(mean(head^2) + eps) and multiplied by a weight of dk elements that all heads share.
-// A warp takes a head; the values are copied by all.
-template <typename TQ, typename TC>
-__global__ void __launch_bounds__(256)
-qk_headnorm_rope_store_kernel(const float* proj, int stride, const float* q_weight,
-                              const float* k_weight, float eps,
-                              const float* inv_freq, int rot,
-                              const int* positions, const int* req_of_tok,
-                              const int* block_table, int bt_stride, TC* __restrict__ pages,
-                              int num_pages, int page_size, int write_kv, int num_heads, int num_kv_heads,
-                              int dk, int dv, TQ* __restrict__ q_out, int* __restrict__ status) {
-    pdl_launch();
-    pdl_wait();
-    const int t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int nq = num_heads * dk, nk = num_kv_heads * dk, nv = num_kv_heads * dv;
-    const float* row = proj + (size_t)t * stride;
-    const int pos_i = positions[t];
-    const float pos = (float)pos_i;
-    TC* base = nullptr;
-    int slot = 0;
-    if (write_kv) {
-        const int page = block_table[(size_t)req_of_tok[t] * bt_stride + pos_i / page_size];
-        if (page < 0 || page >= num_pages) {
-            if (threadIdx.x == 0) atomicCAS(status, 0, TI_ERR_BAD_PAGE);
-            return;
-        }
-        slot = pos_i % page_size;
-        base = pages + (size_t)page * num_kv_heads * page_size * (dk + dv);
-    }
-    const int units = num_heads + (write_kv ? num_kv_heads : 0);
-    for (int u = warp; u < units; u += 8) {
-        const bool is_q = u < num_heads;
-        const int h = is_q ? u : u - num_heads;
-        const float* head = row + (is_q ? 0 : nq) + (size_t)h * dk;
-        const float* w = is_q ? q_weight : k_weight;
-        float ss = 0.0f;
-        for (int j = lane; j < dk; j += 32) ss = fmaf(head[j], head[j], ss);
-        const float inv = 1.0f / sqrtf(warp_sum(ss) / (float)dk + eps);
-        for (int j = lane; j < dk; j += 32) {
-            float y;
-            if (j < rot) {
-                float s, c;
-                sincosf(pos * inv_freq[j >> 1], &s, &c);
-                const float a = head[j] * inv * (w ? w[j] : 1.0f);
-                const float b = head[j ^ 1] * inv * (w ? w[j ^ 1] : 1.0f);
-                y = (j & 1) ? a * c + b * s : a * c - b * s;
-            } else {
-                y = head[j] * inv * (w ? w[j] : 1.0f);
-            }
-            if (is_q) q_out[(size_t)t * nq + (size_t)h * dk + j] = from_f32<TQ>(y);
-            else base[((size_t)h * page_size + slot) * dk + j] = from_f32<TC>(y);
-        }
-    }
-    if (!write_kv) return;
-    TC* vbase = base + (size_t)num_kv_heads * page_size * dk;
-    const float* vrow = row + nq + nk;
-    for (int e = threadIdx.x; e < nv; e += blockDim.x) {
-        const int j = e % dv, g = e / dv;
-        vbase[((size_t)g * page_size + slot) * dv + j] = from_f32<TC>(vrow[e]);
-    }
-}
-
 }  // namespace
 
 #define TI_DISPATCH_QC(qd, cd, CALL)                                               \
@@ -632,6 +647,45 @@ qk_headnorm_rope_store_kernel(const float* proj, int stride, const float* q_weig
     else if (qd == TI_BF16 && cd == TI_BF16) { CALL(bf16, bf16); }                 \
     else if (qd == TI_F32 && cd == TI_BF16) { CALL(float, bf16); }                 \
     else return ti_fail("attention: dtype codes q=%d cache=%d are not supported", qd, cd);
+
+// Rows of whole heads (RowHeads) to pages and queries: in units of four elements where the sizes and addresses allow it
+// and the query and key rows together fit into two units a thread of a block, else element by element.
+static int launch_row_heads(const char* what, const RowHeads& p, int num_tokens, void* pages, int cache_dtype, void* q_out,
+                            int q_dtype, int* status, cudaStream_t s) {
+    auto aligned = [](const void* x) { return (uintptr_t)x % 16 == 0; };
+    const size_t smem = (size_t)(p.rot / 2 + p.v_rot / 2) * sizeof(float2);      // the token's cosines and sines
+    TI_REQUIRE(smem <= 47 * 1024, "%s: rotated widths %d and %d", what, p.rot, p.v_rot);
+    const int units = (p.num_heads + p.num_kv_heads) * p.dk / 4;
+    const bool fits = p.dk % 4 == 0 && p.dv % 4 == 0 && p.rot % 4 == 0 && p.v_rot % 4 == 0 && p.stride % 4 == 0 &&
+                      (p.mix.first == nullptr || p.mix.stride % 4 == 0) && units <= 2048 && aligned(p.proj) &&
+                      aligned(p.norm.q_weight) && aligned(p.norm.k_weight) && aligned(p.mix.first) && aligned(pages) &&
+                      aligned(q_out);
+#define UNITS(TQ, TC, N, NU, AHEAD)                                                                                             \
+    ti_launch_pdl((row_heads_units_kernel<TQ, TC, N, NU, AHEAD>), dim3(num_tokens), dim3(N), smem, s, p, (TC*)pages, (TQ*)q_out, status)
+#define CALL(TQ, TC)                                                                                                 \
+    if (!fits)                                                                                                       \
+        ti_launch_pdl((qkv_turn_store_kernel<TQ, TC>), dim3(num_tokens), dim3(256), smem, s, p.proj, p.stride, p.norm, \
+                      p.mix, p.inv_freq, p.rot, p.halves, p.mag, p.v_inv_freq, p.v_rot, p.v_halves, p.positions,       \
+                      p.req_of_tok, p.block_table, p.bt_stride, (TC*)pages, p.num_pages, p.page_size, p.write_kv,      \
+                      p.num_heads, p.num_kv_heads, p.dk, p.dv, (TQ*)q_out, status);                                    \
+    else if (units <= 512) UNITS(TQ, TC, 256, 2, true);                                                              \
+    else if (units <= 1024 && num_tokens < 256) UNITS(TQ, TC, 512, 2, true);                                         \
+    else if (units <= 1024) UNITS(TQ, TC, 256, 4, false);                                                            \
+    else UNITS(TQ, TC, 1024, 2, true)
+    TI_DISPATCH_QC(q_dtype, cache_dtype, CALL)
+#undef CALL
+#undef UNITS
+    return ti_check_launch(what);
+}
+
+extern "C" int ti_heads_prepare_store(const float* proj, int stride, const float* bias, const float* q_weight,
+                                      const float* k_weight, int pre_norm, int post_norm, float eps,
+                                      const float* inv_freq, int rot, int halves, float mag, float temp_coef,
+                                      int temp_every, int values_from_keys, const int* positions,
+                                      const int* req_of_tok, const int* block_table, int bt_stride, void* pages,
+                                      int cache_dtype, int num_pages, int page_size, int write_kv, int num_tokens,
+                                      int num_heads, int num_kv_heads, int dk, int dv, void* q_out, int q_dtype,
+                                      int* status, void* stream);
 
 extern "C" int ti_qk_rownorm_rope_store(const float* proj, int stride, const float* q_weight,
                                         const float* k_weight, float eps, const float* inv_freq, int rot,
@@ -644,15 +698,17 @@ extern "C" int ti_qk_rownorm_rope_store(const float* proj, int stride, const flo
     TI_REQUIRE(rot >= 0 && rot <= dk && rot % 2 == 0, "qk_rownorm_rope_store: rotated width %d must be even "
                "and at most the head size %d", rot, dk);
     TI_REQUIRE(rot == 0 || inv_freq != nullptr, "qk_rownorm_rope_store: a rotation needs its frequencies");
-    cudaStream_t s = (cudaStream_t)stream;
-#define CALL(TQ, TC)                                                                              \
-    ti_launch_pdl((per_head ? qk_headnorm_rope_store_kernel<TQ, TC> : qk_rownorm_rope_store_kernel<TQ, TC>),          \
-        dim3(num_tokens), dim3(256), 0, s, proj, stride, q_weight, k_weight, eps, inv_freq, rot, positions, req_of_tok, block_table,   \
-        bt_stride, (TC*)pages, num_pages, page_size, write_kv, num_heads, num_kv_heads, dk, dv,      \
-        (TQ*)q_out, status)
-    TI_DISPATCH_QC(q_dtype, cache_dtype, CALL)
-#undef CALL
-    return ti_check_launch("qk_rownorm_rope_store");
+    TI_REQUIRE(q_dtype == cache_dtype || q_dtype == TI_F32, "qk_rownorm_rope_store: dtype codes q=%d cache=%d are not "
+               "supported", q_dtype, cache_dtype);
+    if (per_head)                                       // heads normed one by one: head_rows.cu
+        return ti_heads_prepare_store(proj, stride, nullptr, q_weight, k_weight, 1, 0, eps, inv_freq, rot, 0, 1.0f, 0.0f, 0, 0,
+                                      positions, req_of_tok, block_table, bt_stride, pages, cache_dtype, num_pages, page_size,
+                                      write_kv, num_tokens, num_heads, num_kv_heads, dk, dv, q_out, q_dtype, status, stream);
+    const RowHeads p{proj, stride, {1, eps, q_weight, k_weight}, {nullptr, 0, 0.0f}, inv_freq, rot, 0, 1.0f, nullptr, 0, 0,
+                     positions, req_of_tok, block_table, bt_stride, num_pages, page_size, write_kv, num_heads, num_kv_heads,
+                     dk, dv};
+    return launch_row_heads("qk_rownorm_rope_store", p, num_tokens, pages, cache_dtype, q_out, q_dtype, status,
+                            (cudaStream_t)stream);
 }
 
 extern "C" int ti_slice_rmsnorm(const float* x, int stride, int num_rows, int n, const float* weight, float eps,
@@ -679,10 +735,15 @@ extern "C" int ti_latent_prepare(const float* qproj, int q_stride, const float* 
     TI_REQUIRE(dr >= 0 && dr % 2 == 0, "latent_prepare: the rotated width %d must be even", dr);
     TI_REQUIRE(dr == 0 || inv_freq != nullptr, "latent_prepare: a rotation needs its frequencies");
     cudaStream_t s = (cudaStream_t)stream;
+    auto aligned = [](const void* x) { return (uintptr_t)x % 16 == 0; };
+    const size_t smem = (size_t)(dr / 2) * sizeof(float2);
+    TI_REQUIRE(smem <= 47 * 1024, "latent_prepare: a rotated width of %d", dr);
+    const bool units = dk % 4 == 0 && dr % 4 == 0 && rank % 4 == 0 && q_stride % 4 == 0 && stride % 4 == 0 && aligned(qproj) &&
+                       aligned(proj) && aligned(latent_weight) && aligned(pages) && aligned(q_plain) && aligned(q_full);
 #define CALL(TQ, TC)                                                                              \
-    ti_launch_pdl((latent_prepare_kernel<TQ, TC>), dim3(num_tokens), dim3(256), 0, s, \
-        qproj, q_stride, proj, stride, latent_weight, eps, inv_freq, mag, positions, req_of_tok, block_table, bt_stride,  \
-        (TC*)pages, num_pages, page_size, num_heads, dk, dr, rank, (TQ*)q_plain, (TQ*)q_full, status)
+    ti_launch_pdl((units ? latent_prepare_kernel<TQ, TC, true> : latent_prepare_kernel<TQ, TC, false>), dim3(num_tokens, 2), \
+        dim3(256), smem, s, qproj, q_stride, proj, stride, latent_weight, eps, inv_freq, mag, positions, req_of_tok,  \
+        block_table, bt_stride, (TC*)pages, num_pages, page_size, num_heads, dk, dr, rank, (TQ*)q_plain, (TQ*)q_full, status)
     TI_DISPATCH_QC(q_dtype, cache_dtype, CALL)
 #undef CALL
     return ti_check_launch("latent_prepare");
@@ -703,19 +764,10 @@ extern "C" int ti_qkv_turn_store(const float* proj, int stride, int row_norm, fl
                "even and at most their head size %d", v_rot, dv);
     TI_REQUIRE((rot == 0 || inv_freq != nullptr) && (v_rot == 0 || v_inv_freq != nullptr),
                "qkv_turn_store: a rotation needs its frequencies");
-    cudaStream_t s = (cudaStream_t)stream;
-    const size_t turn_smem = (size_t)(rot / 2 + v_rot / 2) * sizeof(float2);      // the token's cosines and sines
-    const RowNorm norm{row_norm, eps, q_weight, k_weight};
-    const ValueMix mix{mix_first, mix_stride, mix_share};
-    TI_REQUIRE(turn_smem <= 47 * 1024, "qkv_turn_store: rotated widths %d and %d", rot, v_rot);
-#define CALL(TQ, TC)                                                                              \
-    ti_launch_pdl((qkv_turn_store_kernel<TQ, TC>), dim3(num_tokens), dim3(256), turn_smem, s, \
-        proj, stride, norm, mix, inv_freq, rot, halves, mag, v_inv_freq, v_rot, v_halves, positions, req_of_tok, \
-        block_table, bt_stride, (TC*)pages, num_pages, page_size, write_kv, num_heads, num_kv_heads, dk, dv, \
-        (TQ*)q_out, status)
-    TI_DISPATCH_QC(q_dtype, cache_dtype, CALL)
-#undef CALL
-    return ti_check_launch("qkv_turn_store");
+    const RowHeads p{proj, stride, {row_norm, eps, q_weight, k_weight}, {mix_first, mix_stride, mix_share}, inv_freq, rot,
+                     halves, mag, v_inv_freq, v_rot, v_halves, positions, req_of_tok, block_table, bt_stride, num_pages,
+                     page_size, write_kv, num_heads, num_kv_heads, dk, dv};
+    return launch_row_heads("qkv_turn_store", p, num_tokens, pages, cache_dtype, q_out, q_dtype, status, (cudaStream_t)stream);
 }
 
 extern "C" int ti_turn_rows(const void* x, int dtype, const int* positions, const float* inv_freq, int rot, int halves,
@@ -742,28 +794,35 @@ extern "C" int ti_head_project(const void* in, int in_dtype, int in_stride_t, in
                                int out_stride_h, int num_tokens, int num_heads, void* stream) {
     if (num_tokens == 0 || num_heads == 0) return 0;
     TI_REQUIRE(in_dtype == out_dtype, "head_project: input and output must have one dtype");
-    size_t smem = (size_t)HP_TOKENS * n_in * sizeof(float);
-    const size_t meet = (size_t)(HP_WARPS / 2) * HP_TOKENS * 128 * sizeof(float);     // where the warps' sums meet
-    if (smem < meet) smem = meet;
+    const size_t smem = (size_t)HP_TOKENS * n_in * sizeof(float);
     TI_REQUIRE(smem <= 48 * 1024, "head_project: %d inputs per head are more than the kernel stages", n_in);
-    dim3 grid((num_tokens + HP_TOKENS - 1) / HP_TOKENS, num_heads, (n_out + 127) / 128);
-    // four columns a load where every group of four starts on a multiple of the load's size
-    const int vec_ok = n_out % 4 == 0 && (uintptr_t)w % 16 == 0;
     cudaStream_t s = (cudaStream_t)stream;
-    // few blocks (a step of single tokens): the form whose warps split k, so that a head's weights are
-    // on their way at once; many blocks: a thread per column with all of k.  (A row's bits can differ
-    // between the two forms; within a form they depend on the row alone.)
-    // Float32 rows always take the second form: their bits must not depend on the step around them.
-    const bool few = in_dtype != TI_F32 && (long long)grid.x * grid.y * grid.z <= 512;
+    // Up to 64 tokens in bfloat16 (a step of single tokens): the form whose threads split k, so that a head's weights are
+    // on their way at once; else a thread per column with all of k.  (A row's bits can differ between the two forms;
+    // within a form they depend on the row alone.)  Float32 rows always take the second form: their bits must not depend
+    // on the step around them.
+    if (in_dtype == TI_BF16 && w_dtype == TI_BF16 && num_tokens <= 64) {
+        const int vec_ok = n_out % 4 == 0 && (uintptr_t)w % 8 == 0;      // four columns a load
+        const int tt = num_tokens <= 4 ? 4 : num_tokens <= 8 ? 8 : 16;
+        const dim3 grid((num_tokens + tt - 1) / tt, num_heads, (n_out + HP_COLS - 1) / HP_COLS);
+        const size_t inputs = (size_t)tt * n_in * sizeof(float), meet = (size_t)(HP_THREADS / 32) * tt * HP_COLS * sizeof(float);
+#define LAUNCH(TT, KP)                                                                                              \
+    ti_launch_pdl((head_project_few_kernel<TT, KP>), grid, dim3(HP_THREADS), inputs > meet ? inputs : meet, s,        \
+        (const bf16*)in, in_stride_t, in_stride_h, (const bf16*)w, n_in, n_out, (bf16*)out, out_stride_t, out_stride_h, \
+        num_tokens, vec_ok)
+        if (n_in <= HP_GROUPS * 4) {
+            if (tt == 4) LAUNCH(4, 4); else if (tt == 8) LAUNCH(8, 4); else LAUNCH(16, 4);
+        } else {
+            if (tt == 4) LAUNCH(4, 16); else if (tt == 8) LAUNCH(8, 16); else LAUNCH(16, 16);
+        }
+#undef LAUNCH
+        return ti_check_launch("head_project");
+    }
+    dim3 grid((num_tokens + HP_TOKENS - 1) / HP_TOKENS, num_heads, (n_out + 127) / 128);
 #define CALL(TI_, TW_)                                                                            \
-    if (few)                                                                                      \
-        ti_launch_pdl((head_project_kernel<TI_, TW_, TI_>), dim3(grid), dim3(HP_WARPS * 32), smem, s, \
-            (const TI_*)in, in_stride_t, in_stride_h, (const TW_*)w, n_in, n_out, (TI_*)out,        \
-            out_stride_t, out_stride_h, num_tokens, vec_ok);                                       \
-    else                                                                                          \
-        ti_launch_pdl((head_project_rows_kernel<TI_, TW_, TI_>), dim3(grid), dim3(128), smem, s, \
-            (const TI_*)in, in_stride_t, in_stride_h, (const TW_*)w, n_in, n_out, (TI_*)out,        \
-            out_stride_t, out_stride_h, num_tokens)
+    ti_launch_pdl((head_project_rows_kernel<TI_, TW_, TI_>), dim3(grid), dim3(128), smem, s,        \
+        (const TI_*)in, in_stride_t, in_stride_h, (const TW_*)w, n_in, n_out, (TI_*)out,            \
+        out_stride_t, out_stride_h, num_tokens)
     if (in_dtype == TI_F32 && w_dtype == TI_F32) { CALL(float, float); }
     else if (in_dtype == TI_F32 && w_dtype == TI_BF16) { CALL(float, bf16); }
     else if (in_dtype == TI_BF16 && w_dtype == TI_BF16) { CALL(bf16, bf16); }

@@ -15,6 +15,7 @@
 // that do not fall into such units take a kernel with a warp per head and a pass per norm.  All arithmetic is
 // float32; a head's bits depend on its row alone.
 #include "common.cuh"
+#include "head_units.cuh"
 
 namespace {
 
@@ -75,34 +76,6 @@ template <int LANES> __device__ __forceinline__ float group_sum(float v) {
     return v;
 }
 
-// Unit u of a head: elements (x0, y0) and (x1, y1) are the pairs of the turn, or four neighbours outside of it.
-__device__ __forceinline__ float4 load_unit(const float* p, int u, bool turned, int halves, int half) {
-    if (turned && halves) {
-        const float2 x = *reinterpret_cast<const float2*>(p + 2 * u), y = *reinterpret_cast<const float2*>(p + 2 * u + half);
-        return make_float4(x.x, x.y, y.x, y.y);
-    }
-    const float4 v = *reinterpret_cast<const float4*>(p + 4 * u);
-    return turned ? make_float4(v.x, v.z, v.y, v.w) : v;
-}
-template <typename T> __device__ __forceinline__ void store2(T* p, float a, float b) {
-    if constexpr (sizeof(T) == 2) *reinterpret_cast<__nv_bfloat162*>(p) = __floats2bfloat162_rn(a, b);
-    else *reinterpret_cast<float2*>(p) = make_float2(a, b);
-}
-template <typename T>
-__device__ __forceinline__ void store_unit(T* p, int u, bool turned, int halves, int half, float4 v) {
-    if (turned && halves) {
-        store2<T>(p + 2 * u, v.x, v.y);
-        store2<T>(p + 2 * u + half, v.z, v.w);
-        return;
-    }
-    if (turned) v = make_float4(v.x, v.z, v.y, v.w);
-    if constexpr (sizeof(T) == 2) {
-        __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
-        *reinterpret_cast<uint2*>(p + 4 * u) = make_uint2(*reinterpret_cast<unsigned*>(&a), *reinterpret_cast<unsigned*>(&b));
-    } else {
-        *reinterpret_cast<float4*>(p + 4 * u) = v;
-    }
-}
 __device__ __forceinline__ float squares(float4 v) { return fmaf(v.w, v.w, fmaf(v.z, v.z, fmaf(v.y, v.y, v.x * v.x))); }
 __device__ __forceinline__ void times(float4& v, float f) { v.x *= f; v.y *= f; v.z *= f; v.w *= f; }
 
@@ -132,7 +105,7 @@ __device__ __forceinline__ void prepare_head(const Heads& p, const float* row, i
         const float mean_of = 1.0f / (float)n;
         float last = KIND == ITEM_QUERY ? factor : 1.0f;
         if (p.pre_norm) {
-            const float inv = rsqrtf(fmaf(group_sum<LANES>(ss), mean_of, p.eps));
+            const float inv = 1.0f / sqrtf(fmaf(group_sum<LANES>(ss), mean_of, p.eps));
             const float* w = KIND == ITEM_QUERY ? p.q_weight : p.k_weight;
             if (w) {
 #pragma unroll
@@ -151,15 +124,13 @@ __device__ __forceinline__ void prepare_head(const Heads& p, const float* row, i
         for (int j = 0; j < NU; ++j) {
             const int u = lane + LANES * j;
             if (u >= turned_units) continue;
-            const float4 f = *reinterpret_cast<const float4*>(cs + 2 * u);     // two pairs' (cosine, sine)
-            v[j] = make_float4(v[j].x * f.x - v[j].z * f.y, v[j].y * f.z - v[j].w * f.w,
-                               v[j].z * f.x + v[j].x * f.y, v[j].w * f.z + v[j].y * f.w);
+            v[j] = turn_unit(v[j], cs, u);
         }
         if (p.post_norm) {
             float sq = 0.0f;
 #pragma unroll
             for (int j = 0; j < NU; ++j) sq += squares(v[j]);
-            last *= rsqrtf(fmaf(group_sum<LANES>(sq), mean_of, p.eps));
+            last *= 1.0f / sqrtf(fmaf(group_sum<LANES>(sq), mean_of, p.eps));
         }
 #pragma unroll
         for (int j = 0; j < NU; ++j) times(v[j], last);

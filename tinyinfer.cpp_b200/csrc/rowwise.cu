@@ -16,6 +16,17 @@ __global__ void embed_kernel(const TW* __restrict__ table, const int* __restrict
     for (int i = threadIdx.x; i < hidden; i += blockDim.x) o[i] = to_f32(row[i]);
 }
 
+// The same four elements a thread, one piece of a row a thread: a row waits for memory once instead of once per piece (the
+// first launch of a step, its rows always cold: 64 rows of 5,120 13.2 us in passes of one element a thread).
+template <typename TW>
+__global__ void __launch_bounds__(256)
+embed4_kernel(const TW* __restrict__ table, const int* __restrict__ tokens, int hidden, float* __restrict__ out) {
+    pdl_launch();
+    pdl_wait();
+    const int t = blockIdx.x, c = (blockIdx.y * 256 + threadIdx.x) * 4;
+    if (c < hidden) store4(out + (size_t)t * hidden + c, load4_f32(table + (size_t)tokens[t] * hidden + c));
+}
+
 // out[r, :] = x[src(r), :] * (1 / sqrt(mean(x^2) + eps)) * w, src(r) = rows ? rows[r] : r
 template <typename TO>
 __global__ void rmsnorm_kernel(const float* x, const float* __restrict__ w,
@@ -317,12 +328,16 @@ extern "C" int ti_embed(const void* table, int table_dtype, const int* tokens, i
                         int hidden, float* out, void* stream) {
     if (num_tokens == 0) return 0;
     cudaStream_t s = (cudaStream_t)stream;
-    if (table_dtype == TI_BF16)
-        ti_launch_pdl(embed_kernel<bf16>, num_tokens, 256, 0, s, (const bf16*)table, tokens, hidden, out);
-    else if (table_dtype == TI_F32)
-        ti_launch_pdl(embed_kernel<float>, num_tokens, 256, 0, s, (const float*)table, tokens, hidden, out);
+    const bool four = hidden % 4 == 0 && (uintptr_t)table % 16 == 0 && (uintptr_t)out % 16 == 0;
+    const dim3 grid4(num_tokens, (hidden / 4 + 255) / 256);
+#define CALL(TW)                                                                                              \
+    if (four) ti_launch_pdl(embed4_kernel<TW>, grid4, 256, 0, s, (const TW*)table, tokens, hidden, out);        \
+    else ti_launch_pdl(embed_kernel<TW>, num_tokens, 256, 0, s, (const TW*)table, tokens, hidden, out)
+    if (table_dtype == TI_BF16) { CALL(bf16); }
+    else if (table_dtype == TI_F32) { CALL(float); }
     else
         return ti_fail("embed: table dtype code %d is not float32 or bfloat16", table_dtype);
+#undef CALL
     return ti_check_launch("embed");
 }
 

@@ -266,7 +266,7 @@ tanh_norm_pair_kernel(const float* y, int n, float a1, const float* w1,
 // out[t] = table[token] + bigram[row]; a block per token
 template <typename TW>
 __global__ void __launch_bounds__(256)
-embed_bigram_kernel(const TW* table, const TW* bigram, const int* tokens, int n,
+embed_bigram_kernel(const TW* __restrict__ table, const TW* __restrict__ bigram, const int* tokens, int n, int four,
                     int vocab, long long buckets, long long mul_prev, long long mul_cur,
                     const int* positions, const int* req_of_tok, const int* cu_q,
                     const int* slots, int* kept, size_t kept_stride, float* __restrict__ out) {
@@ -289,6 +289,14 @@ embed_bigram_kernel(const TW* table, const TW* bigram, const int* tokens, int n,
     __syncthreads();
     const TW* a = table + (size_t)token * n;
     const TW* b = bigram + (size_t)row_s * n;
+    if (four) {                                            // four elements a load
+#pragma unroll 4
+        for (int c = threadIdx.x * 4; c < n; c += blockDim.x * 4) {
+            const float4 x = load4_f32(a + c), y = load4_f32(b + c);
+            store4(out + (size_t)t * n + c, make_float4(x.x + y.x, x.y + y.y, x.z + y.z, x.w + y.w));
+        }
+        return;
+    }
     for (int c = threadIdx.x; c < n; c += blockDim.x) out[(size_t)t * n + c] = to_f32(a[c]) + to_f32(b[c]);
 }
 
@@ -534,9 +542,10 @@ extern "C" int ti_embed_bigram(const void* table, const void* bigram, int dtype,
     TI_REQUIRE(buckets >= 1 && buckets < (1LL << 31) && mul_prev >= 0 && mul_prev < buckets && mul_cur >= 0 && mul_cur < buckets,
                "embed_bigram: factors must lie in [0, buckets), and buckets below 2^31");
     cudaStream_t s = (cudaStream_t)stream;
+    const int four = rows_of_four(n, 0, {table, bigram, out});
 #define CALL(TW)                                                                                                   \
     ti_launch_pdl((embed_bigram_kernel<TW>), dim3(num_tokens), dim3(256), 0, s, (const TW*)table,   \
-        (const TW*)bigram, tokens, n, vocab, buckets,                                               \
+        (const TW*)bigram, tokens, n, four, vocab, buckets,                                            \
                                                        mul_prev, mul_cur, positions, req_of_tok, cu_q, slots, kept, \
                                                        (size_t)kept_stride, out)
     if (dtype == TI_BF16) CALL(bf16);
