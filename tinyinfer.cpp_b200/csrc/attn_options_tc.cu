@@ -19,7 +19,11 @@
 // Few rows (decoding) cut the keys of a row into runs of tiles, a block each, whose unnormalised
 // results a second launch adds (attn_options_merge); and when a tile has at most 16 rows (single
 // tokens, up to 16 heads per kv head) the four warps of a block share those rows and take a
-// quarter of every tile's keys each, meeting in shared memory at the end.
+// quarter of every tile's keys each, meeting in shared memory at the end.  What bounds such a step is a block's chain of
+// latencies: pages are looked up a tile ahead, the first tile's keys (older than the step, but for the token's own row) are
+// on their way before the wait, a run without keys leaves its maximum and nothing else.  us a layer, before -> now, 16 heads:
+// of 64 over 4 kv heads, 8 requests of 200 to 530 keys 10.6 -> 9.9, 4 of 400 to 1,030 14.7 -> 9.9, 64 of 600 31 -> 28; of
+// 128, 16 requests of 1,500 37 -> 33; over shared rows of 288, 8 requests 18.1 -> 14.0, of 576, 16 of 1,500 50 -> 46.
 //
 // Precision.  Scores, cap (with the hardware's float32 exponential and reciprocal, relative error
 // about 2^-22), softmax weights and sums are float32.  The weighted sum of the values
@@ -88,6 +92,7 @@ attn_options_tc_kernel(const bf16* q, const int* __restrict__ tiles, const int* 
     constexpr int NT_O = DVS / 8;
     constexpr bool KS = MODE == 1;
     constexpr int V_ROW = DVS * 2 + 16;
+    constexpr int QROWS = MODE == 0 ? BM : 16;           // rows of queries that are staged
     // KS (at most 16 live rows, decoding): every warp has the same 16 rows and a quarter of a tile's keys
     constexpr int NJ = KS ? BN / 32 : BN / 8;            // 8-key columns of a tile that a warp multiplies
     extern __shared__ __align__(16) unsigned char smem[];
@@ -95,7 +100,7 @@ attn_options_tc_kernel(const bf16* q, const int* __restrict__ tiles, const int* 
     const int k_row = dk * 2 + 16;                       // bytes of a staged query or key row
     const int stage_bytes = BN * k_row + (opt.shared_rows ? 0 : BN * V_ROW);
     unsigned char* q_s = smem;
-    unsigned char* ring = smem + BM * k_row;
+    unsigned char* ring = smem + QROWS * k_row;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, tq = lane & 3;
     const int rbase = MODE == 0 ? warp * 16 : 0, kbase = KS ? warp * 16 : 0;
@@ -141,63 +146,117 @@ attn_options_tc_kernel(const bf16* q, const int* __restrict__ tiles, const int* 
     const int warp_pos_lo = pos_first + warp_tok_lo, warp_pos_hi = pos_first + warp_tok_hi;
     const int warp_lo_first = first_visible(warp_pos_lo, opt), warp_lo_last = first_visible(warp_pos_hi, opt);
 
-    pdl_wait();                                          // queries, keys, values and gates come from the kernels before
-    // queries into shared memory (part of the first commit group)
+    // queries into shared memory
     const int chunks = dk / 8;
-    for (int c = threadIdx.x; c < BM * chunks; c += WARPS * 32) {
-        const int i = c / chunks, part = c % chunks;
-        const int h = row_head(i);
-        const bf16* src = h >= 0 ? q + ((size_t)(tok0 + row_token(i)) * num_heads + h) * dk + part * 8 : q;
-        cp_async16(q_s + (size_t)i * k_row + part * 16, src, h >= 0);
-    }
+    // a row of queries or keys is copied by a run of lanes (a power of two, at most a warp), so that no copy divides
+    const int lanes_log2 = chunks <= 8 ? 3 : chunks <= 16 ? 4 : 5, row_step = WARPS * 32 >> lanes_log2;
+    const int row_first = threadIdx.x >> lanes_log2, chunk_first = threadIdx.x & ((1 << lanes_log2) - 1);
+    auto issue_queries = [&]() {
+        for (int i = row_first; i < QROWS; i += row_step) {
+            const int h = row_head(i);
+            const bf16* src = h >= 0 ? q + ((size_t)(tok0 + row_token(i)) * num_heads + h) * dk : q;
+            for (int c = chunk_first; c < chunks; c += 1 << lanes_log2)
+                cp_async16(q_s + (size_t)i * k_row + c * 16, src + c * 8, h >= 0);
+        }
+    };
 
     float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.0f, 0.0f};
     float o[NT_O][4];
 #pragma unroll
     for (int i = 0; i < NT_O; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.0f;
 
-    auto issue = [&](int kt, int stage) {
+    // the pages of a tile's four runs of 16 keys (-2: nothing of this block's), few rows: looked up a tile ahead
+    int page_of[BN / 16];
+    auto lookup = [&](int kt) {
+#pragma unroll
+        for (int r = 0; r < BN / 16; ++r) {
+            const int key0 = kt * BN + r * 16;
+            page_of[r] = key0 <= pos_last && key0 + 16 > kv_lo ? table[key0 / page_size] : -2;
+        }
+    };
+    // `held`: a key that is left out for now (its row is being written), or -1
+    auto issue = [&](int kt, int stage, int held) {
+        if (MODE == 0) lookup(kt);                       // (registers are short there)
         unsigned char* kdst = ring + (size_t)stage * stage_bytes;
         unsigned char* vdst = kdst + BN * k_row;
 #pragma unroll
         for (int r = 0; r < BN / 16; ++r) {              // four runs of 16 keys, each inside one page
             const int key0 = kt * BN + r * 16;
-            int pg = -1;
-            if (key0 <= pos_last && key0 + 16 > kv_lo) {
-                pg = table[key0 / page_size];
-                if (pg < 0 || pg >= num_pages) {
-                    if (threadIdx.x == 0) atomicCAS(status, 0, 1);
-                    pg = -1;
-                }
-            }
-            const bool valid = pg >= 0;
+            const int pg = page_of[r];
+            const bool valid = pg >= 0 && pg < num_pages;
+            if (!valid && pg != -2 && threadIdx.x == 0) atomicCAS(status, 0, 1);
             // rows outside the keys of this block's queries come as zeros: behind the request's last token a page may hold
             // what an earlier request left, and a weight of zero times an infinity is not zero
             const int own_lo = max(0, kv_lo - key0);
             const unsigned own_rows = valid ? min(16, pos_last + 1 - key0) - own_lo : 0;
             auto own = [&](int row) { return (unsigned)(row - own_lo) < own_rows; };
+            auto skip = [&](int row) { return MODE != 0 && key0 + row == held; };
             const bf16* base = pages + (valid ? (size_t)pg * page_elems : 0);
             const bf16* ksrc = base + (valid ? ((size_t)kvh * page_size + key0 % page_size) * dk : 0);
-            for (int c = threadIdx.x; c < 16 * chunks; c += WARPS * 32)
-                cp_async16(kdst + (size_t)(r * 16 + c / chunks) * k_row + (c % chunks) * 16,
-                           ksrc + (valid ? c * 8 : 0), own(c / chunks));
+            for (int i = row_first; i < 16; i += row_step) {
+                if (skip(i)) continue;
+                const bool live = own(i);
+                const bf16* src = ksrc + (live ? (size_t)i * dk : 0);
+                unsigned char* dst = kdst + (size_t)(r * 16 + i) * k_row;
+                for (int c = chunk_first; c < chunks; c += 1 << lanes_log2) cp_async16(dst + c * 16, src + c * 8, live);
+            }
             if (!opt.shared_rows) {
                 const bf16* vsrc = base + (valid ? v_base + ((size_t)kvh * page_size + key0 % page_size) * dv
                                                        + slice * DVS : 0);
                 constexpr int VCH = DVS / 8;
                 for (int c = threadIdx.x; c < 16 * VCH; c += WARPS * 32)
-                    cp_async16(vdst + (size_t)(r * 16 + c / VCH) * V_ROW + (c % VCH) * 16,
-                               vsrc + (valid ? (size_t)(c / VCH) * dv + (c % VCH) * 8 : 0), own(c / VCH));
+                    if (!skip(c / VCH))
+                        cp_async16(vdst + (size_t)(r * 16 + c / VCH) * V_ROW + (c % VCH) * 16,
+                                   vsrc + (valid ? (size_t)(c / VCH) * dv + (c % VCH) * 8 : 0), own(c / VCH));
             }
         }
     };
+    // the held key's row
+    auto issue_held = [&](int kt, int stage) {
+        const int row = pos_last - kt * BN, pg = table[pos_last / page_size], in_page = pos_last % page_size;
+        const bool valid = pg >= 0 && pg < num_pages;     // (reported by `issue` where it is not)
+        unsigned char* kdst = ring + (size_t)stage * stage_bytes;
+        const bf16* base = pages + (valid ? (size_t)pg * page_elems : 0);
+        const bf16* ksrc = base + (valid ? ((size_t)kvh * page_size + in_page) * dk : 0);
+        for (int c = threadIdx.x; c < chunks; c += WARPS * 32)
+            cp_async16(kdst + (size_t)row * k_row + c * 16, ksrc + (valid ? c * 8 : 0), valid);
+        if (!opt.shared_rows) {
+            const bf16* vsrc = base + (valid ? v_base + ((size_t)kvh * page_size + in_page) * dv + slice * DVS : 0);
+            for (int c = threadIdx.x; c < DVS / 8; c += WARPS * 32)
+                cp_async16(kdst + BN * k_row + (size_t)row * V_ROW + c * 16, vsrc + (valid ? c * 8 : 0), valid);
+        }
+    };
 
-    if (kt_lo < kt_hi) issue(kt_lo, 0);
+    if (MODE != 0 && kt_lo < kt_hi) lookup(kt_lo);
+    if (MODE != 0 && ntok == 1) {
+        // a single token: all keys but its own are older than this step, so the first tile is on its way while the
+        // kernels before still run; the own key's row follows behind the wait
+        const bool last = kt_lo < kt_hi && kt_lo == pos_last / BN;
+        if (kt_lo < kt_hi) issue(kt_lo, 0, pos_last);
+        pdl_wait();
+        if (nsplit > 1 && kt_lo >= kt_hi) {
+            // a run without keys: the merging launch leaves it out by its maximum and reads nothing else of it
+            if (threadIdx.x < QROWS && (MODE == 2 || slice == 0)) {
+                const int h = row_head(threadIdx.x);
+                const size_t at = ((size_t)tok0 * num_heads + h) * nsplit + split;
+                if (h >= 0) { part_ml[at * 2] = -INFINITY; part_ml[at * 2 + 1] = 0.0f; }
+            }
+            return;
+        }
+        issue_queries();
+        if (last) issue_held(kt_lo, 0);
+    } else {
+        pdl_wait();                                       // queries, keys, values and gates come from the kernels before
+        issue_queries();
+        if (kt_lo < kt_hi) issue(kt_lo, 0, -1);
+    }
     cp_async_commit();
+    if (MODE != 0 && kt_lo + 1 < kt_hi) lookup(kt_lo + 1);
     const int ksteps = dk / 16;
     for (int kt = kt_lo; kt < kt_hi; ++kt) {
         const int stage = (kt - kt_lo) % STAGES;
-        if (kt + 1 < kt_hi) issue(kt + 1, (kt + 1 - kt_lo) % STAGES);
+        if (kt + 1 < kt_hi) issue(kt + 1, (kt + 1 - kt_lo) % STAGES, -1);
+        if (MODE != 0 && kt + 2 < kt_hi) lookup(kt + 2);
         cp_async_commit();
         cp_async_wait<1>();
         __syncthreads();
@@ -401,6 +460,7 @@ attn_options_merge_kernel(const float* part_o, const float* part_ml, int nsplit,
     pdl_wait();
     __shared__ float f_s[64];
     __shared__ float inv_s;
+    __shared__ int live_s;                           // runs up to the last one that has seen a key
     const int item = blockIdx.x, t = item / num_heads, h = item % num_heads;
     const float* ml = part_ml + (size_t)item * nsplit * 2;
     if (threadIdx.x < 32) {
@@ -412,18 +472,24 @@ attn_options_merge_kernel(const float* part_o, const float* part_ml, int nsplit,
         l = warp_sum(l);
         if (sink) l += exp2f(sink[h] * LOG2E - m);
         f_s[lane] = f0; f_s[lane + 32] = f1;
+        const unsigned lo = __ballot_sync(0xffffffffu, f0 != 0.0f), hi = __ballot_sync(0xffffffffu, f1 != 0.0f);
         if (lane == 0) {
             float inv = 1.0f / l;
             if (gate && gate_per_head) inv *= 1.0f / (1.0f + expf(-gate[(size_t)t * gate_stride + h]));
             inv_s = inv;
+            live_s = hi ? 64 - __clz(hi) : 32 - __clz(lo);
         }
     }
     __syncthreads();
     const float* po = part_o + (size_t)item * nsplit * dv;
+    const int live = live_s;
     for (int d = blockIdx.y * 128 + threadIdx.x; d < dv; d += 128 * gridDim.y) {
         float acc = 0.0f;
 #pragma unroll 8
-        for (int z = 0; z < nsplit; ++z) acc = fmaf(po[(size_t)z * dv + d], f_s[z], acc);
+        for (int z = 0; z < live; ++z) {             // what a run without keys has left is not read
+            const float f = f_s[z], x = f != 0.0f ? po[(size_t)z * dv + d] : 0.0f;
+            acc = fmaf(x, f, acc);
+        }
         acc *= inv_s;
         if (gate && !gate_per_head) acc *= 1.0f / (1.0f + expf(-gate[(size_t)t * gate_stride + (size_t)h * dv + d]));
         out[(size_t)item * dv + d] = __float2bfloat16_rn(acc);
@@ -509,18 +575,18 @@ head_project_tc_kernel(const bf16* x, int x_stride_t, int x_stride_h, const bf16
 
 int value_slice(int dv) { return dv % 128 == 0 ? 128 : dv % 64 == 0 ? 64 : dv % 32 == 0 ? 32 : 16; }
 
-size_t smem_bytes(int dk, int dv, int shared_rows) {
+size_t smem_bytes(int dk, int dv, int shared_rows, int query_rows) {
     const size_t k_row = (size_t)dk * 2 + 16, v_row = (size_t)value_slice(dv) * 2 + 16;
     const size_t ring = STAGES * (BN * k_row + (shared_rows ? 0 : BN * v_row));
     const size_t meet = (size_t)WARPS * 16 * (value_slice(dv) + 2) * sizeof(float);     // where split warps meet
-    return BM * k_row + (ring > meet ? ring : meet);
+    return query_rows * k_row + (ring > meet ? ring : meet);
 }
 
 }  // namespace
 
 extern "C" int ti_attn_options_tc_supported(int dk, int dv, int page_size, int shared_rows) {
     return dk >= 16 && dk % 16 == 0 && dv >= 16 && dv % 16 == 0 && page_size >= 16 && page_size % 16 == 0 &&
-           (!shared_rows || dv <= dk) && smem_bytes(dk, dv, shared_rows) <= 227 * 1024;
+           (!shared_rows || dv <= dk) && smem_bytes(dk, dv, shared_rows, BM) <= 227 * 1024;
 }
 
 extern "C" int ti_head_project_tc_supported(int n_in, int n_out, int x_stride_t, int x_stride_h) {
@@ -588,12 +654,16 @@ extern "C" int ti_attn_options_tc(const void* q, const int* tiles, int num_tiles
     // prompt portions over shared rows: 256 value columns a block where they divide, so that the score
     // product of a wide row is repeated half as often (such a block fills an SM's shared memory anyway)
     const int dvs = (shared_rows && key_split == 0 && dv % 256 == 0) ? 256 : value_slice(dv);
-    const size_t smem = smem_bytes(dk, dv, shared_rows);
+    const size_t smem = smem_bytes(dk, dv, shared_rows, key_split ? 16 : BM);
     TcOptions opt = {window, chunk, scale, softcap, head_scale, sink, gate, gate_stride, gate_per_head, shared_rows};
     TI_REQUIRE(key_split != 2 || (shared_rows && dv / dvs <= WARPS), "attn_options_tc: a warp per slice needs shared rows "
                "and at most %d slices", WARPS);
     dim3 grid(num_kv_heads * head_blocks * (key_split == 2 ? 1 : dv / dvs), num_tiles, nsplit);
     cudaStream_t s = (cudaStream_t)stream;
+    // Single tokens: 164 KB of shared memory an SM are room for the blocks that the caller counts on, and the products
+    // behind this kernel, which start under it and keep the split it leaves, read their rows from the L1 that remains
+    // (three rows of 2,048, the two feed-forward products behind it: 16 + 15 us with three blocks' worth set aside, 12 + 10
+    // with this).
 #define LAUNCH(DVS, MODE)                                                                                       \
     {                                                                                                     \
         static TiPerDevice configured;                                                                    \
@@ -602,6 +672,8 @@ extern "C" int ti_attn_options_tc(const void* q, const int* tiles, int num_tiles
             cudaError_t e = cudaFuncSetAttribute(attn_options_tc_kernel<DVS, MODE>,                             \
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024); \
             if (e != cudaSuccess) return ti_fail("attn_options_tc: %s", cudaGetErrorString(e));           \
+            if (MODE != 0)                                                                                \
+                cudaFuncSetAttribute(attn_options_tc_kernel<DVS, MODE>, cudaFuncAttributePreferredSharedMemoryCarveout, 72); \
             configured.mark();                                                                            \
             allowed = 227 * 1024;                                                                         \
         }                                                                                                 \
