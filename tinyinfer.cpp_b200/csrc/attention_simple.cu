@@ -10,6 +10,7 @@
 // [slot][head_dim]; a token at position p of request r lies in page block_table[r][p / page_size],
 // slot p % page_size.
 #include "common.cuh"
+#include "tape.cuh"
 
 namespace {
 
@@ -520,3 +521,6 @@ extern "C" int ti_paged_attention_simple(const void* q, int q_dtype, const int* 
 #undef LAUNCH
     return ti_check_launch("paged_attention_simple");
 }
+
+TI_TAPED(ti_qk_norm_rope_store)
+TI_TAPED(ti_paged_attention_simple)

@@ -383,6 +383,7 @@ extern "C" int ti_attn_decode_qkv(const float* qkv, int width, const float* q_we
 
 // ---- the variant that allocates nothing (declared and described in attn_decode_noalloc.h) ----
 #include "attn_decode_noalloc.h"
+#include "tape.cuh"
 
 #include <mutex>
 
@@ -439,3 +440,5 @@ extern "C" int ti_attn_decode_noalloc(const void* q, const int* rows, int num_ro
                           num_pages, page_size, num_heads, num_kv_heads, head_dim, window, scale,
                           num_splits, part_o, part_ml, out, status, stream);
 }
+
+TI_TAPED(ti_attn_decode_fused)

@@ -8,6 +8,7 @@
 // values run on the tensor cores (mma.sync m16n8k16), the softmax is online and float32.
 // The causal and window masks are applied only in tiles that touch an edge.
 #include "common.cuh"
+#include "tape.cuh"
 
 namespace {
 
@@ -303,3 +304,5 @@ extern "C" int ti_attn_prefill(const void* q, const int* tiles, int num_tiles, c
 #undef CASE
     return ti_fail("attn_prefill: head_dim %d", head_dim);
 }
+
+TI_TAPED(ti_attn_prefill)

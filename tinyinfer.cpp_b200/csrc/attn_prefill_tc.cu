@@ -23,6 +23,7 @@
 // Every wait on an mbarrier is bounded; on a timeout the block records status 2, frees its tensor
 // memory and returns.
 #include "sm100.cuh"
+#include "tape.cuh"
 
 namespace {
 
@@ -466,3 +467,6 @@ extern "C" int ti_attn_prefill_tc_merge(const int* tiles, int num_tiles, int num
                   part_ml, num_heads, splits, (bf16*)out);
     return ti_check_launch("attn_prefill_tc_merge");
 }
+
+TI_TAPED(ti_attn_prefill_tc)
+TI_TAPED(ti_attn_prefill_tc_merge)

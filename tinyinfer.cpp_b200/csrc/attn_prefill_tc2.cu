@@ -30,6 +30,7 @@
 // Every wait on an mbarrier is bounded; on a timeout the block records status 2, frees its tensor
 // memory and returns.
 #include "sm100.cuh"
+#include "tape.cuh"
 
 namespace {
 
@@ -438,3 +439,5 @@ extern "C" int ti_attn_prefill_tc2(const void* q, int num_tokens, const int* til
                   window, run, scale * LOG2E, (bf16*)out, part_o, part_ml, status, hold_dependents);
     return ti_check_launch("attn_prefill_tc2");
 }
+
+TI_TAPED(ti_attn_prefill_tc2)

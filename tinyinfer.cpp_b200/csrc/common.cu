@@ -37,3 +37,18 @@ void TiPerDevice::mark() {
     const int dev = current_device_slot();
     if (dev >= 0) done[dev] = true;
 }
+
+// Repeats a tape of launches for `layers` layers.  Call c is `calls[c]` (an entry point's `_taped` form) with the slots from
+// first_slot[c] on; before a layer's calls, slot patch_slot[p] of every patch p gets that layer's value.  Returns 0, or one
+// more than the number of the call that failed (its library keeps the message).
+extern "C" int ti_tape_run(const void* const* calls, const int* first_slot, int num_calls, unsigned long long* slots,
+                           const int* patch_slot, int num_patches, const unsigned long long* patch_values, int layers) {
+    typedef int (*Taped)(const unsigned long long*);
+    for (int layer = 0; layer < layers; ++layer) {
+        const unsigned long long* values = patch_values + (size_t)layer * num_patches;
+        for (int p = 0; p < num_patches; ++p) slots[patch_slot[p]] = values[p];
+        for (int c = 0; c < num_calls; ++c)
+            if (((Taped)calls[c])(slots + first_slot[c])) return c + 1;
+    }
+    return 0;
+}

@@ -25,6 +25,7 @@
 // wait for the rest; their waits then run out and both report status 2.  An engine launches on
 // one stream; who steps several engines concurrently on one GPU turns this kernel off.)
 #include "sm100.cuh"
+#include "tape.cuh"
 
 namespace {
 
@@ -554,3 +555,6 @@ extern "C" int ti_attn_out_ffn_decode(const void* attn, const void* w_o, const f
     a.ld_act = ld_act; a.ldc = ldc; a.counters = counters; a.status = status;
     return m <= 8 ? launch<1, 12, true>(a, (cudaStream_t)stream) : launch<2, 6, true>(a, (cudaStream_t)stream);
 }
+
+TI_TAPED(ti_ffn_decode)
+TI_TAPED(ti_attn_out_ffn_decode)

@@ -10,6 +10,7 @@
 // starts at zero.  So an output element's value does not depend on M, on the tile it falls in or
 // on its neighbours, and a product of few rows can give its segments to different lanes.
 #include "common.cuh"
+#include "tape.cuh"
 
 namespace {
 
@@ -420,3 +421,5 @@ extern "C" int ti_gemm_simple(const void* a, int a_dtype, const void* w, int w_d
         return launch((const bf16*)a, (const bf16*)w, c, m, n, k, lda, ldw, ldc, accumulate, s);
     return ti_fail("gemm: dtype codes %d x %d are not float32/bfloat16", a_dtype, w_dtype);
 }
+
+TI_TAPED(ti_gemm_simple)

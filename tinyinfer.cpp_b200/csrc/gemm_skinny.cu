@@ -16,6 +16,7 @@
 // one value per output.
 #include "common.cuh"
 #include "glu.cuh"
+#include "tape.cuh"
 
 namespace {
 
@@ -303,3 +304,5 @@ extern "C" int ti_gemm_skinny_unary(const void* a, const void* w, void* out_act,
     TI_REQUIRE(act == ACT_RELU2, "gemm_skinny_unary: activation %d", act);
     return skinny(a, w, nullptr, out_act, m, n, k, lda, ldw, 0, ld_act, MODE_UNARY, act, 0.0f, 0.0f, stream);
 }
+
+TI_TAPED(ti_gemm_skinny)

@@ -25,6 +25,7 @@
 // is bounded: on a timeout the block records status 2, frees its tensor memory and returns.
 #include "qkv_epilogue.cuh"
 #include "glu.cuh"
+#include "tape.cuh"
 
 namespace {
 
@@ -618,3 +619,7 @@ extern "C" int ti_rope_table(const int* positions, const float* inv_freq, int nu
                   num_tokens, half, table);
     return ti_check_launch("rope_table");
 }
+
+TI_TAPED(ti_gemm_tcgen05)
+TI_TAPED(ti_gemm_tcgen05_add_runs)
+TI_TAPED(ti_gemm_tcgen05_qkv)

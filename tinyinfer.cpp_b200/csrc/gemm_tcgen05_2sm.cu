@@ -17,6 +17,7 @@
 // through the cluster barrier at the end, freeing their tensor memory.
 #include "qkv_epilogue.cuh"
 #include "glu.cuh"
+#include "tape.cuh"
 
 namespace {
 
@@ -353,3 +354,6 @@ extern "C" int ti_gemm_tcgen05_2sm_qkv(const void* a, const void* w, int m, int 
                           (bf16*)pages, num_pages, page_size, write_kv, num_heads, num_kv_heads, (bf16*)q_out};
     return launch_pairs(a, w, e, nullptr, nullptr, m, n, k, lda, ldw, 0, 0, MODE_QKV, status, stream);
 }
+
+TI_TAPED(ti_gemm_tcgen05_2sm)
+TI_TAPED(ti_gemm_tcgen05_2sm_qkv)

@@ -19,6 +19,7 @@
 // records status 2, frees its tensor memory and returns.
 #include "sm100.cuh"
 #include "glu.cuh"
+#include "tape.cuh"
 
 namespace {
 
@@ -383,3 +384,5 @@ extern "C" int ti_gemm_tcgen05_few_gated(const void* a, const void* w, float* c,
     return few(a, w, c, nullptr, m, n, k, lda, ldw, ldc, 0, MODE_ACCUMULATE, ws, tickets, status, stream,
                AddGate{gate, ld_gate, bias, scale});
 }
+
+TI_TAPED(ti_gemm_tcgen05_few)

@@ -1,6 +1,7 @@
 // Row-wise kernels: token embedding, RMSNorm (optionally of gathered rows), SwiGLU, argmax.
 // All arithmetic is float32; results are rounded once to the output type.
 #include "common.cuh"
+#include "tape.cuh"
 
 namespace {
 
@@ -437,3 +438,7 @@ extern "C" int ti_argmax(const float* logits, int rows, int vocab, int* out, voi
     argmax_kernel<<<rows, 1024, 0, (cudaStream_t)stream>>>(logits, vocab, out);
     return ti_check_launch("argmax");
 }
+
+TI_TAPED(ti_rmsnorm)
+TI_TAPED(ti_rmsnorm_merge)
+TI_TAPED(ti_swiglu)

@@ -1,0 +1,128 @@
+"""Launches of one layer, recorded and repeated for the layers like it.
+
+A step of a new shape runs eagerly, and its layers ask the kernel set for the same launches one after the other: the same
+entry points with the same sizes, only over other weights and other pages.  Choosing and issuing them in Python costs 13 to
+18 us a launch, several times what the launch itself takes.  So the second of a run of alike layers is run in Python with its
+calls recorded, and the layers behind it repeat them natively (``ti_tape_run``) with the pointers to what a layer owns
+replaced.  The first layer is not the one recorded because it has no layer in front of it whose last product waits to be added
+(``_pending_runs``).
+
+What makes a recording valid: every launch went through an entry point that has a taped form (else the number of launches and
+of recorded calls differ), no torch operation but allocations and views took place, nothing is held back at the layer's end
+that was not held back at its start, and the layers' own tensors agree in type, shape, strides and alignment.  A recording
+lives for one pass and holds the tensors allocated under it until the pass has issued its last launch.
+"""
+from __future__ import annotations
+
+import ctypes
+import struct
+
+import torch
+from torch.utils._python_dispatch import TorchDispatchMode
+
+_VIEWS = {"view", "slice", "select", "alias", "unsqueeze", "as_strided", "expand", "permute", "transpose", "detach"}
+
+
+class _Allocations(TorchDispatchMode):
+    """Keeps every tensor that is allocated under it and notices any other operation on data."""
+
+    def __init__(self):
+        super().__init__()
+        self.held: list = []
+        self.pure = True
+
+    def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+        out = func(*args, **(kwargs or {}))
+        name = func.overloadpacket.__name__
+        if name == "empty":
+            self.held.append(out)
+        elif name not in _VIEWS:
+            self.pure = False
+        return out
+
+
+class _Tap:
+    """A kernel library whose launches are recorded on their way."""
+
+    def __init__(self, lib, calls: list):
+        self._lib, self._calls = lib, calls
+
+    def __getattr__(self, name):
+        found = getattr(self._lib, name)
+        taped = getattr(self._lib, name + "_taped", None)
+        if taped is not None:
+            fn, calls, lib = found, self._calls, self._lib
+            address = ctypes.cast(taped, ctypes.c_void_p).value
+
+            def found(*args):
+                calls.append((address, lib, fn.argtypes, args))
+                return fn(*args)
+        setattr(self, name, found)
+        return found
+
+
+def _slot(kind, value) -> int:
+    if kind is ctypes.c_float:
+        return struct.unpack("<I", struct.pack("<f", value))[0]
+    return (0 if value is None else int(value)) & 0xFFFFFFFFFFFFFFFF
+
+
+def signature(tensors) -> tuple:
+    """What two layers' own tensors must agree in for one layer's launches to serve the other."""
+    return tuple((t.dtype, t.shape, t.stride(), t.data_ptr() % 32, getattr(t, "_ti_interleaved", None)) for t in tensors)
+
+
+def record(ops, run, mine):
+    """Runs one layer through ``run()`` and returns its launches as ``replay(layers)``, which takes the own tensors of each
+    layer to repeat them for (in the order of ``mine``, this layer's); None if they cannot be repeated."""
+    calls: list = []
+    start = ops._pending_runs
+    had_more = ops._pending is not None or ops._pending_pair is not None
+    libs = {"core": ops.core, "bf16": ops.__dict__.get("bf16")}
+    issued = ops.issued
+    with _Allocations() as watch:
+        try:
+            for name, lib in libs.items():
+                if lib is not None:
+                    ops.__dict__[name] = _Tap(lib, calls)
+            run()
+        finally:
+            for name, lib in libs.items():
+                if lib is not None:
+                    ops.__dict__[name] = lib
+    end = ops._pending_runs
+    if (not watch.pure or had_more or ops._pending is not None or ops._pending_pair is not None
+            or (start is None) != (end is None) or len(calls) != ops.issued - issued):
+        return None
+    renamed = {}
+    if start is not None:                  # the runs that the layer in front left, and those that this one leaves
+        if start[1:2] != end[1:2] or start[2] is not end[2] or start[3] != end[3]:
+            return None
+        renamed[start[0].data_ptr()] = end[0].data_ptr()
+    place = {t.data_ptr(): i for i, t in enumerate(mine)}
+    if len(place) != len(mine):
+        return None
+    first, slots, patches, sources = [], [], [], []
+    for _, _, kinds, args in calls:
+        if kinds is None or len(kinds) != len(args):
+            return None
+        first.append(len(slots))
+        for kind, value in zip(kinds, args):
+            if kind is ctypes.c_void_p and value:
+                if value in place:
+                    patches.append(len(slots))
+                    sources.append(place[value])
+                value = renamed.get(value, value)
+            slots.append(_slot(kind, value))
+    n = len(calls)
+    packed = ((ctypes.c_void_p * n)(*[c[0] for c in calls]), (ctypes.c_int * n)(*first), n,
+              (ctypes.c_ulonglong * max(1, len(slots)))(*slots), (ctypes.c_int * max(1, len(patches)))(*patches), len(patches))
+
+    def replay(layers):
+        values = [own[s] for own in ([t.data_ptr() for t in layer] for layer in layers) for s in sources]
+        rc = ops.core.ti_tape_run(*packed, (ctypes.c_ulonglong * max(1, len(values)))(*values), len(layers))
+        ops.launches += n * len(layers)
+        ops.issued += n * len(layers)
+        return None if rc == 0 else calls[rc - 1][1]
+    replay.held = (watch.held, start)      # alive until the last launch has been issued
+    return replay

@@ -67,6 +67,9 @@ class Attention(Part):
     def cache_spec(self):
         return PagedKVSpec(self.num_kv_heads, self.head_dim, self.window)
 
+    def own_tensors(self):
+        return [self.w_qkv, self.w_o, self.q_norm, self.k_norm]
+
     def forward(self, ops, h, residual, step, cache):
         t, dev, act = h.shape[0], h.device, h.dtype
         # one output buffer for all layers of a pass: the product behind has read it before the next layer writes

@@ -118,6 +118,11 @@ class Part:
     def load_weights(self, tensors: Mapping[str, torch.Tensor], ops: Any) -> None:
         """Take the tensors named in ``weight_specs`` (already on the device, dtype as stored)."""
 
+    def own_tensors(self):
+        """The device tensors that the part's launches read and that another part of the same specification has in
+        its place, in a fixed order; None: not stated (its layer is then never repeated from a recording)."""
+        return None
+
     def step_lists(self) -> list:
         """Integer lists (``engine.batch.StepList``) that this part wants built on the host for
         every step and handed to it as ``step.lists[name]``."""

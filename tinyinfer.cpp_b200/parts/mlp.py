@@ -40,6 +40,9 @@ class SwiGLU(Part):
         self.w_gate_up = ops.pack_gate_up(g, u)
         self.w_down = ops.pack_linear(tensors["down_proj.weight"])
 
+    def own_tensors(self):
+        return [self.w_gate_up, self.w_down]
+
     def forward(self, ops, h, residual, step):
         ops.swiglu_ffn(h, self.w_gate_up, self.w_down, residual, may_defer=True)
 

@@ -47,6 +47,15 @@ class CausalLM:
             for role, part in parts.items():
                 if part is not None:
                     self._named.append((lp.names[role], part))
+        # how many entries of the schedule, from each on, run layers of the same specification on slots of their own
+        self._alike = [1] * len(plan.schedule)
+        for i in range(len(plan.schedule) - 2, -1, -1):
+            a, b = plan.schedule[i], plan.schedule[i + 1]
+            la, lb = plan.layers[a.layer], plan.layers[b.layer]
+            if (b.enter is None and a.layer != b.layer and a.writes_cache and b.writes_cache
+                    and all(getattr(la, f) == getattr(lb, f) for f in (
+                        "block", "mixer", "ffn", "mixer_norm", "ffn_norm", "mixer_post_norm", "ffn_post_norm"))):
+                self._alike[i] = self._alike[i + 1] + 1
 
     # ---- weights -------------------------------------------------------------------------
     def expected_tensors(self) -> dict[str, WeightSpec]:
@@ -128,11 +137,26 @@ class CausalLM:
         else:
             self.embedding.forward(ops, step.token_ids, x)
         x0 = x.clone() if self.junction is not None else None      # the embedding output, for the junction
-        for entry in self.plan.schedule:
-            if entry.enter is not None:
-                self.junction.forward(ops, x, x0, entry.enter, step)
-            cache = cache_views[(entry.cache_slot, entry.writes_cache)]
-            self.blocks[entry.layer].forward(ops, x, step, cache)
+        at, schedule = 0, self.plan.schedule
+        while at < len(schedule):
+            if schedule[at].enter is not None:
+                self.junction.forward(ops, x, x0, schedule[at].enter, step)
+            count = self._alike[at] if hasattr(ops, "repeat_layers") else 1
+            parts = [(self.blocks[e.layer], cache_views[(e.cache_slot, e.writes_cache)]) for e in schedule[at:at + count]]
+
+            def own(k):
+                mine, view = parts[k][0].own_tensors(), parts[k][1]
+                pages, first = getattr(view, "pages", None), parts[0][1]      # one kind of pages, by one block table
+                same = mine is not None and pages is not None and view.block_table is getattr(first, "block_table", None)
+                return mine + [pages] if same else None
+
+            def run(k):
+                parts[k][0].forward(ops, x, step, parts[k][1])
+            if count > 1:
+                ops.repeat_layers(count, run, own)
+            else:
+                run(0)
+            at += count
         ops.flush()                        # nothing a part asked for may still be held back
         step.scratch.clear()               # ... and nothing of the pass is kept behind it
         if step.num_logit_rows == 0:

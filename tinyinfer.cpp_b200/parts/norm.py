@@ -37,6 +37,9 @@ class RMSNorm(Part):
         if self.factor != 1.0:
             self.weight = self.factor * self.weight
 
+    def own_tensors(self):
+        return [self.weight]
+
     def forward(self, ops, x: torch.Tensor, out_dtype: torch.dtype) -> torch.Tensor:
         out = torch.empty((x.shape[0], self.size), dtype=out_dtype, device=x.device)
         ops.rmsnorm(x, self.weight, self.eps, out)
