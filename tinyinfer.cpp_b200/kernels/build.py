@@ -22,7 +22,7 @@ CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
 
 # library name -> sources (each library is self-contained and links common.cu)
 LIBRARIES = {
-    "core": ["common.cu", "rowwise.cu", "gemm_simple.cu", "attention_simple.cu", "attn_gated_bias.cu",
+    "core": ["common.cu", "rowwise.cu", "gemm_simple.cu", "gemm_split.cu", "attention_simple.cu", "attn_gated_bias.cu",
              "moe_simple.cu", "sampling.cu"],
     "bf16": ["common.cu", "gemm_skinny.cu", "gemm_tcgen05.cu", "gemm_tcgen05_2sm.cu",
              "gemm_tcgen05_few.cu", "ffn_decode.cu", "attn_decode.cu", "attn_prefill.cu", "attn_prefill_tc.cu",

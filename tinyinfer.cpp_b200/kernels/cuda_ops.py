@@ -176,6 +176,11 @@ class CudaOps(MixerOps, StateOps):
         # larger weights gain 15-50 % on tcgen05)
         self.few_tc_min_bytes = 1 << 25
         self._few_tickets = None
+        # float32 rows times bfloat16 weights on the tensor cores, from this many weights on (smaller ones: a launch of
+        # the multiply-add kernel is shorter, 128 x 128 at one row 2.6 against 4.0 us; at 256 x 256 one row pays 4.9 for
+        # 3.4, three save 4.9 for 7.0, 64 7.2 for 14.7)
+        self.split_products = True
+        self.split_from = 1 << 16
         # prompt attention with two heads per block (csrc/attn_prefill_tc2.cu) from this many
         # (head, tile) pairs per SM on (None: never)
         self.tc_attention_pairs_from = 3
@@ -236,6 +241,8 @@ class CudaOps(MixerOps, StateOps):
             _vp, _i, _vp, _vp]
         c.ti_paged_attention_simple.argtypes = [
             _vp, _i, _vp, _vp, _vp, _vp, _i, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _f, _vp, _vp, _vp]
+        c.ti_gemm_split_scratch.argtypes = [_i, _i, _i, ctypes.POINTER(ctypes.c_longlong), ctypes.POINTER(ctypes.c_int)]
+        c.ti_gemm_split.argtypes = [_vp, _vp, _vp] + [_i] * 7 + [_vp, _vp, _vp, _vp]
         c.ti_sample.argtypes = [_vp, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp]
         c.ti_embed_sinusoid.argtypes = [_vp, _i, _vp, _vp, _vp, _f, _i, _i, _vp, _vp]
         c.ti_qkv_bias_norm_store.argtypes = [_vp, _i, _vp, _vp, _vp, _f, _vp, _vp, _vp, _i, _vp, _i, _i, _i,
@@ -663,10 +670,37 @@ class CudaOps(MixerOps, StateOps):
                         m, n, k, a.stride(0), w.stride(0), out.stride(0), mode)):
                 self._run_tc_gemm(a, w, out, None, m, n, k, out.stride(0), 0, mode, may_defer=may_defer)
                 return
+        if self._split_product(a, w, out, accumulate):
+            return
         self._ok(self.core.ti_gemm_simple(
             a.data_ptr(), _code(a, "linear"), w.data_ptr(), _code(w, "linear"), out.data_ptr(),
             m, n, k, a.stride(0), w.stride(0), out.stride(0), int(bool(accumulate)),
             self._stream()))
+
+    def _split_product(self, a, w, out, accumulate) -> bool:
+        """Runs a product of float32 rows with bfloat16 weights on the tensor cores, the rows in three exact parts
+        (csrc/gemm_split.cu), if it applies.  The rule looks at the weights alone: a row's bits must not depend on how
+        many rows run beside it."""
+        m, k = a.shape
+        n = w.shape[0]
+        if not (self.split_products and a.dtype == torch.float32 and w.dtype == torch.bfloat16
+                and w.data_ptr() % 16 == 0 and w.stride(0) % 8 == 0 and n * k >= self.split_from and m > 0):
+            return False
+        cut = self._cuts.get(("split", m, n, k))
+        if cut is None:
+            if len(self._cuts) >= 4096:
+                self._cuts.clear()
+            floats, tickets = ctypes.c_longlong(0), ctypes.c_int(0)
+            self.core.ti_gemm_split_scratch(m, n, k, ctypes.byref(floats), ctypes.byref(tickets))
+            cut = self._cuts["split", m, n, k] = (floats.value, tickets.value)
+        floats, tickets = cut
+        if tickets and (self._few_tickets is None or self._few_tickets.numel() < tickets):
+            self._few_tickets = self._grown(self._few_tickets, tickets, a.device)
+        ws = torch.empty(floats, dtype=torch.float32, device=a.device) if floats else None
+        self._ok(self.core.ti_gemm_split(
+            a.data_ptr(), w.data_ptr(), out.data_ptr(), m, n, k, a.stride(0), w.stride(0), out.stride(0),
+            int(bool(accumulate)), _ptr(ws), _ptr(self._few_tickets), self.status.data_ptr(), self._stream()))
+        return True
 
     def _linear_gated_sum(self, a, w, target):
         """``x += scale * sigmoid(gate + bias) * (a @ w.T)`` for a ``parts.base.GatedSum`` (without a gate ``x +=
