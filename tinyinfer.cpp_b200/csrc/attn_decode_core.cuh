@@ -9,6 +9,7 @@
 namespace attn_decode_core {
 
 
+template <bool V> struct Flag { static constexpr bool value = V; };
 constexpr int TILE = 32;       // keys per tile
 constexpr int STAGES = 3;
 constexpr int MAX_SPLITS = 256;
@@ -215,7 +216,8 @@ __device__ __forceinline__ void decode_item(
 
     if (PDL) pdl_launch();
     if (my_lo < my_hi) {
-        auto issue = [&](int tile, int stage) {
+        // `without_own`: the row's own key is left out for now (it is being written)
+        auto issue = [&](int tile, int stage, auto without_own) {
             unsigned char* kdst = smem + (size_t)stage * 2 * TILE * ROW_BYTES;
             unsigned char* vdst = kdst + TILE * ROW_BYTES;
             // a tile is two runs of 16 keys; a run lies inside one page and is contiguous there
@@ -241,6 +243,7 @@ __device__ __forceinline__ void decode_item(
                 for (int i = 0; i < 16 * CHUNKS / 32; ++i) {
                     const int c = i * 32 + lane;                 // 16-byte chunk of the run
                     const int off = (r * 16 + c / CHUNKS) * ROW_BYTES + (c % CHUNKS) * 16;
+                    if (decltype(without_own)::value && key0 + c / CHUNKS == pos) continue;
                     cp_async16(kdst + off, ksrc + (valid ? i * 256 : 0), valid);
                     cp_async16(vdst + off, vsrc + (valid ? i * 256 : 0), valid);
                 }
@@ -249,19 +252,39 @@ __device__ __forceinline__ void decode_item(
 
         // Keys of earlier steps do not depend on the kernel before this one; the new token's own
         // key and value (in the tile that holds `pos`) and the queries do.  So the first tiles
-        // are requested before waiting for that kernel.
+        // are requested before waiting for that kernel, the tile of the own key without its row,
+        // which follows behind the wait (16 heads, 8 kv heads, us a layer at one request of 20 to 256
+        // keys 5.9 to 6.1 with that tile behind the wait -> 4.6 to 4.9, eight of 50 to 250 6.4 to 7.2 ->
+        // 5.1 to 6.1; letting one block have the two to six tiles of a short row, so that nothing is
+        // merged, takes 5.4 to 10.2).
         const int new_tile = pos / TILE;
-        int early = 0;
+        int early = 0, held_stage = -1;
 #pragma unroll
         for (int s = 0; s < STAGES - 1; ++s) {
-            if (PDL && early == s && my_lo + s < my_hi && my_lo + s < new_tile) {
-                issue(my_lo + s, s);
-                cp_async_commit();
+            if (PDL && !LATE_WAIT && my_lo + s < my_hi) {
+                const bool own = my_lo + s == new_tile;
+                if (own) {
+                    issue(my_lo + s, s, Flag<true>{});
+                    held_stage = s;
+                } else {
+                    issue(my_lo + s, s, Flag<false>{});
+                    cp_async_commit();
+                }
                 ++early;
             }
         }
         if (PDL && !LATE_WAIT) pdl_wait();
         prologue();
+        if (held_stage >= 0) {                       // (always the last of the early tiles)
+            const int pg = table[pos / page_size], in = lane % CHUNKS;
+            const bool valid = pg >= 0 && pg < num_pages;
+            if (lane < 2 * CHUNKS) {
+                const bf16* src = pages + (valid ? (((size_t)pg * 2 * num_kv_heads + kvh) * page_size + pos % page_size) * HD + in * 8 : 0);
+                cp_async16(smem + ((size_t)held_stage * 2 + lane / CHUNKS) * TILE * ROW_BYTES + (pos % TILE) * ROW_BYTES + in * 16,
+                           src + (valid && lane >= CHUNKS ? kv_stride : 0), valid);
+            }
+            cp_async_commit();
+        }
         // queries of the group as the A operand: row r of the tile is head kvh*group + r
         unsigned qa[KSTEPS][4];
 #pragma unroll
@@ -283,12 +306,12 @@ __device__ __forceinline__ void decode_item(
 #pragma unroll
         for (int s = 0; s < STAGES - 1; ++s) {
             if (s < early) continue;
-            if (my_lo + s < my_hi) issue(my_lo + s, s);
+            if (my_lo + s < my_hi) issue(my_lo + s, s, Flag<false>{});
             cp_async_commit();
         }
         for (int tile = my_lo; tile < my_hi; ++tile) {
             const int stage = (tile - my_lo) % STAGES;
-            if (tile + STAGES - 1 < my_hi) issue(tile + STAGES - 1, (tile - my_lo + STAGES - 1) % STAGES);
+            if (tile + STAGES - 1 < my_hi) issue(tile + STAGES - 1, (tile - my_lo + STAGES - 1) % STAGES, Flag<false>{});
             cp_async_commit();
             cp_async_wait<STAGES - 1>();
             __syncwarp();
