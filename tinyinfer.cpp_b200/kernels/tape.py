@@ -18,26 +18,30 @@ import ctypes
 import struct
 
 import torch
-from torch.utils._python_dispatch import TorchDispatchMode
+from torch.overrides import TorchFunctionMode
 
-_VIEWS = {"view", "slice", "select", "alias", "unsqueeze", "as_strided", "expand", "permute", "transpose", "detach"}
+# what a layer may ask of a tensor, and views of it: nothing of these runs on the device
+_QUESTIONS = {"data_ptr", "stride", "is_contiguous", "numel", "size", "dim", "element_size", "__get__", "__len__", "__hash__",
+              "view", "unflatten"}
 
 
-class _Allocations(TorchDispatchMode):
-    """Keeps every tensor that is allocated under it and notices any other operation on data."""
+class _Allocations(TorchFunctionMode):
+    """Keeps every tensor that is allocated under it and notices any other operation on data.  (A function mode: a dispatch
+    mode would bring some 900 modules with its first use, 3 to 5 s.)"""
 
     def __init__(self):
         super().__init__()
         self.held: list = []
         self.pure = True
 
-    def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+    def __torch_function__(self, func, types, args=(), kwargs=None):
         out = func(*args, **(kwargs or {}))
-        name = func.overloadpacket.__name__
-        if name == "empty":
-            self.held.append(out)
-        elif name not in _VIEWS:
-            self.pure = False
+        name = getattr(func, "__name__", "")
+        if name not in _QUESTIONS:
+            if func is torch.empty or func is torch.empty_like:
+                self.held.append(out)
+            else:
+                self.pure = False
         return out
 
 
