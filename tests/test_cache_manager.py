@@ -129,3 +129,30 @@ def test_state_slots_are_zeroed_on_reuse():
     # paged views carry the group's table and this layer's pages (one more page than the pool)
     pv = m.view(1, False, ["table"], None)
     assert pv.pages.shape == (5, 2, 2, 16, 16) and pv.block_table == "table" and not pv.writes
+
+
+def test_new_requests_find_zeros_in_their_slots_and_touch_no_other():
+    """Slots that are neighbours and slots that are not, admitted together and alone, states of two types."""
+    import torch
+    from tinyinfer_b200.cache import CacheManager
+    from tinyinfer_b200.parts.base import FixedStateSpec
+    m = CacheManager([FixedStateSpec((3,)), FixedStateSpec((2, 2), torch.int32), FixedStateSpec((5,))], page_size=4, num_pages=1,
+                     max_requests=6, kv_dtype=torch.float32, device="cpu")
+    states = [m.view(i, True, [], None).state for i in range(3)]
+
+    def check(zero):
+        for s in states:
+            for slot in range(s.shape[0]):
+                assert bool((s[slot] == 0).all()) == (slot in zero), slot
+            s.fill_(7)
+    for s in states:
+        s.fill_(7)
+    m.reserve_step([(r, 1) for r in "abcd"])
+    check({m.state_slot(r) for r in "abcd"})
+    m.free_request("b")
+    m.reserve_step([("e", 1), ("a", 1), ("f", 1)])
+    check({m.state_slot(r) for r in "ef"})
+    m.free_request("a")
+    m.add_request("g")
+    check({m.state_slot("g")})
+    assert sorted(m.state_slot(r) for r in "cdefg") == [0, 1, 2, 3, 4]

@@ -117,7 +117,6 @@ class CacheManager:
         self._slot_group: dict[int, tuple[int, int]] = {}      # cache slot -> (group, index in group)
         self._state_specs: dict[int, FixedStateSpec] = {}
         self._state_storage: dict[int, torch.Tensor] = {}
-        self._slot_views: dict[int, list] = {}       # state slot -> its states, a list per type
         by_spec: dict[PagedKVSpec, int] = {}
         # a cache slot that keeps several things: every leaf becomes a slot of its own behind the
         # model's, and the slot's view gathers them under their names
@@ -169,21 +168,30 @@ class CacheManager:
     def add_request(self, req: Hashable) -> None:
         if req in self._lengths:
             raise KeyError(f"request {req!r} is already live")
-        slot = self.state_slots.take()
-        self._lengths[req] = 0
-        self._state_slot[req] = slot
-        self._touch(req)
-        for g in self.groups:
-            g.tables[req] = []
-        # the slot's states of one type in one call (a model of six such layers has eleven: a launch each before)
-        views = self._slot_views.get(slot)
-        if views is None:
+        self._admit([req])
+
+    def _admit(self, reqs: Sequence[Hashable]) -> None:
+        """Makes the requests live, each with a state slot of zeros.  Neighbouring slots are zeroed together, the states
+        of one type in one call (32 requests with eleven states each: a launch a request and type took 0.6 ms of host)."""
+        slots = []
+        for req in reqs:
+            slots.append(self.state_slots.take())
+            self._lengths[req] = 0
+            self._state_slot[req] = slots[-1]
+            self._touch(req)
+            for g in self.groups:
+                g.tables[req] = []
+        slots.sort()
+        first = 0
+        for i, slot in enumerate(slots):
+            if i + 1 < len(slots) and slots[i + 1] == slot + 1:
+                continue
             by_type: dict = {}
             for t in self._state_storage.values():
-                by_type.setdefault(t.dtype, []).append(t[slot])
-            views = self._slot_views[slot] = list(by_type.values())
-        for same in views:
-            torch._foreach_zero_(same)
+                by_type.setdefault(t.dtype, []).append(t[slots[first]:slot + 1])
+            for same in by_type.values():
+                torch._foreach_zero_(same)
+            first = i + 1
 
     def _touch(self, req: Hashable) -> None:
         self._versions += 1
@@ -265,8 +273,8 @@ class CacheManager:
             if k > self.groups[g].pool.num_free:
                 raise OutOfPages(
                     f"the step needs {k} pages of group {g}, {self.groups[g].pool.num_free} are free")
-        for req in new:
-            self.add_request(req)
+        if new:
+            self._admit(new)
         starts = []
         for (req, n), mine in zip(items, per_item):          # the pages are there: hand them out
             for k, g in zip(mine, self.groups):
