@@ -438,6 +438,52 @@ def test_linear_on_pairs_of_sms(ops, shape):
     ops.check_status()
 
 
+@pytest.mark.parametrize("kind", ["silu", "clamped", "gelu_tanh", "relu2"])
+@pytest.mark.parametrize("shape", [(2048, 2048, 264), (1100, 3344, 136), (2563, 1296, 72), (4099, 2576, 1096)])
+def test_activations_on_pairs_of_sms(ops, shape, kind):
+    """A product with an activation behind it on pairs of SMs: the one-SM kernel's bits (both add k in one order), at
+    sizes with ragged rows, columns and k; against float64 within the sum's error passed through the activation and one
+    bfloat16 rounding (2^-8).  The activations' slopes stay below 4 for these sums (|z| < 1.3)."""
+    m, n, k = shape
+    a, w = _rand((m, k), torch.bfloat16), _rand((n, k), torch.bfloat16, seed=1, scale=0.2 / k ** 0.5)
+    down = _rand((8, n // 2), torch.bfloat16, seed=2)
+    assert ops._tc_glu(m, n, k, kind) is ops.bf16.ti_gemm_tcgen05_2sm_glu
+
+    def run():
+        if kind == "relu2":
+            y = torch.full((m, n), float("nan"), dtype=torch.bfloat16, device=DEV)
+            ops.linear_unary(a, w, kind, y)
+            return y
+        y = torch.zeros((m, 8), device=DEV)
+        ops.glu_ffn(a, ops.pack_gate_up(w[: n // 2], w[n // 2:]), down, y, kind, 0.5, 1.7)
+        return y
+
+    got = run()
+    ops.use_2sm_gemm = False
+    try:
+        one = run()
+    finally:
+        ops.use_2sm_gemm = True
+    ops.check_status()
+    assert torch.equal(got, one), "pair kernel and one-SM kernel differ"
+    z = a.double() @ w.double().T
+    e = 4 * 1.3 * _sum_rtol(k)
+    if kind == "relu2":
+        want = z.clamp(min=0).square()
+        assert ((got.double() - want).abs() <= 2.0 ** -8 * want + e).all()
+        return
+    g, u = z[:, : n // 2], z[:, n // 2:]
+    if kind == "silu":
+        act = torch.nn.functional.silu(g) * u
+    elif kind == "clamped":
+        act = g.clamp(max=0.5) * torch.sigmoid(1.7 * g.clamp(max=0.5)) * (u.clamp(-0.5, 0.5) + 1)
+    else:
+        act = torch.nn.functional.gelu(g, approximate="tanh") * u
+    want = act @ down.double().T
+    bound = (2.0 ** -8 * act.abs() + e) @ down.double().abs().T + _sum_rtol(n // 2) * want.abs().max()
+    assert ((got.double() - want).abs() <= bound).all()
+
+
 @pytest.mark.parametrize("m", [1, 8, 40, 64, 100])
 @pytest.mark.parametrize("hk", [(128, 320), (1024, 3072), (80, 176), (64, 24)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])

@@ -6,8 +6,9 @@
 // crosses from L2 to an SM; the one-SM kernel is bound by that path.  The leader (rank 0) issues
 // tcgen05.mma.cta_group::2 (256 x 256 x 16): the tensor cores of both SMs read both blocks' shared
 // memory at the same offsets, and each SM accumulates its 128 rows x 256 columns in its own tensor
-// memory.  Both blocks run the same epilogue on their own rows (store, accumulate, SwiGLU, or the
-// QKV epilogue of qkv_epilogue.cuh: head norm, rotation and the store into the paged cache).
+// memory.  Both blocks run the same epilogue on their own rows (store, accumulate, SwiGLU, the
+// QKV epilogue of qkv_epilogue.cuh: head norm, rotation and the store into the paged cache, or
+// another activation of glu.cuh).
 //
 // Barriers: a stage's "full" barrier lives in the leader and counts the bytes of both blocks' TMA
 // loads (loads of the peer name the leader's barrier); "empty" and "accumulator full" are signalled
@@ -37,7 +38,7 @@ template <int BN> struct Pair {
     static constexpr unsigned TMEM_COLS = 2 * BN;
 };
 
-enum { MODE_STORE = 0, MODE_ACCUMULATE = 1, MODE_SWIGLU = 2, MODE_QKV = 3 };
+enum { MODE_STORE = 0, MODE_ACCUMULATE = 1, MODE_SWIGLU = 2, MODE_QKV = 3, MODE_UNARY = 4 };
 enum { TI_ERR_TIMEOUT = 2 };
 
 __device__ __forceinline__ unsigned cluster_rank() {
@@ -82,12 +83,17 @@ __device__ __forceinline__ void umma_commit_pair(void* bar) {
         ::"r"(smem_u32(bar)), "h"(mask) : "memory");
 }
 
-template <int BN>
+// ACTS: the epilogue applies `glu` (mode MODE_SWIGLU or MODE_UNARY) and nothing else; a kernel of its own, so that the other
+// epilogues are not touched by it (90 registers; the QKV epilogue takes 162).  It is bound as the plain product is, by the
+// way from L2 to an SM, until a short K makes the activation the longer part.  us, one-SM kernel -> this one: 512 x 6,144 x
+// 2,048 with gelu 24.3 -> 18.4, 1,536 x 2,048 x 1,024 with relu squared 14.3 -> 12.5, 4,096 x 5,632 x 1,024 with the clamped
+// gate 46.6 -> 40.4, 2,048 x 6,144 x 2,048 43.5 -> 42.0.
+template <int BN, bool ACTS>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
 gemm_tcgen05_2sm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                         const __grid_constant__ qkv::Epilogue qkv_e, float* __restrict__ c,
                         bf16* __restrict__ out_act, int m, int n, int k, int ldc, int ld_act, int mode,
-                        int* __restrict__ status, const AddGate add) {
+                        int* __restrict__ status, const AddGate add, const GluArgs glu) {
     constexpr int STAGES = Pair<BN>::STAGES, STAGE_B = Pair<BN>::STAGE_B;
     constexpr unsigned TMEM_COLS = Pair<BN>::TMEM_COLS;
     extern __shared__ unsigned char smem_raw[];
@@ -120,7 +126,7 @@ gemm_tcgen05_2sm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;\n" ::: "memory");
     }
     __shared__ float qkv_norm_w[2 * qkv::HEAD_DIM];
-    if (mode == MODE_QKV) qkv::load_norm_weights(qkv_e, qkv_norm_w, threadIdx.x, THREADS);
+    if (!ACTS && mode == MODE_QKV) qkv::load_norm_weights(qkv_e, qkv_norm_w, threadIdx.x, THREADS);
     pdl_launch();
     tc_fence_before();
     __syncthreads();
@@ -198,7 +204,7 @@ gemm_tcgen05_2sm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
             // requested while the products still run
             bf16 *qkv_dst0 = nullptr, *qkv_dst1 = nullptr;
             qkv::Angles angles;
-            if (mode == MODE_QKV) {
+            if (!ACTS && mode == MODE_QKV) {
                 const int item0 = n0 / qkv::HEAD_DIM, items = qkv_e.num_heads + 2 * qkv_e.num_kv_heads;
                 qkv_dst0 = qkv::destination(qkv_e, row, item0, row < m && item0 < items, status);
                 qkv_dst1 = qkv::destination(qkv_e, row, item0 + 1, row < m && item0 + 1 < items, status);
@@ -207,11 +213,11 @@ gemm_tcgen05_2sm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
             ok = mbar_wait(&acc_full[buf], (local >> 1) & 1);
             if (!ok) break;
             tc_fence_after();
-            if (mode == MODE_QKV)
+            if (!ACTS && mode == MODE_QKV)
                 qkv::two_heads(qkv_e, qkv_norm_w, tmem_base + ((unsigned)(quarter * 32) << 16) + (unsigned)(buf * BN),
                                n0 / qkv::HEAD_DIM, col_half, qkv_dst0, qkv_dst1, angles);
 #pragma unroll 1
-            for (int c0 = col_half * (BN / 2); c0 < (col_half + 1) * (BN / 2) && mode != MODE_QKV; c0 += 32) {
+            for (int c0 = col_half * (BN / 2); c0 < (col_half + 1) * (BN / 2) && (ACTS || mode != MODE_QKV); c0 += 32) {
                 float v[32];
                 tmem_load32(tmem_base + ((unsigned)(quarter * 32) << 16) + (unsigned)(buf * BN + c0), v);
                 const int col = n0 + c0;
@@ -225,10 +231,27 @@ gemm_tcgen05_2sm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
                         for (int i = 0; i < 4; ++i) {
                             const float g0 = v[half * 16 + 2 * i], g1 = v[half * 16 + 2 * i + 1];
                             const float u0 = v[half * 16 + 8 + 2 * i], u1 = v[half * 16 + 9 + 2 * i];
-                            __nv_bfloat162 y = __floats2bfloat162_rn(silu_mul(g0, u0), silu_mul(g1, u1));
+                            __nv_bfloat162 y = !ACTS || glu.kind == GLU_SILU
+                                ? __floats2bfloat162_rn(silu_mul(g0, u0), silu_mul(g1, u1))
+                                : __floats2bfloat162_rn(glu_activation(glu.kind, g0, u0, glu.limit, glu.alpha),
+                                                        glu_activation(glu.kind, g1, u1, glu.limit, glu.alpha));
                             packed[i] = *reinterpret_cast<unsigned*>(&y);
                         }
                         *reinterpret_cast<uint4*>(out_act + (size_t)row * ld_act + (col + half * 16) / 2) =
+                            make_uint4(packed[0], packed[1], packed[2], packed[3]);
+                    }
+                } else if (ACTS) {
+#pragma unroll
+                    for (int i = 0; i < 32; i += 8) {
+                        if (col + i >= n) break;
+                        unsigned packed[4];
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            __nv_bfloat162 y = __floats2bfloat162_rn(unary_activation(glu.kind, v[i + 2 * j]),
+                                                                     unary_activation(glu.kind, v[i + 2 * j + 1]));
+                            packed[j] = *reinterpret_cast<unsigned*>(&y);
+                        }
+                        *reinterpret_cast<uint4*>(out_act + (size_t)row * ld_act + col + i) =
                             make_uint4(packed[0], packed[1], packed[2], packed[3]);
                     }
                 } else {
@@ -274,14 +297,17 @@ gemm_tcgen05_2sm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
 extern "C" int ti_gemm_tcgen05_2sm_supported(int m, int n, int k, int lda, int ldw, int ldc, int mode) {
     if (m < 1 || n < 1 || k < 8 || k % 8 || lda % 8 || ldw % 8) return 0;
     if (mode == MODE_SWIGLU) return n % 16 == 0;
+    if (mode == MODE_UNARY) return n % 8 == 0;
     return n % 4 == 0 && ldc % 4 == 0;
 }
 
 namespace {
 
+template <bool ACTS>
 int launch_pairs(const void* a, const void* w, const qkv::Epilogue& e, float* c, void* out_act, int m, int n,
                  int k, int lda, int ldw, int ldc, int ld_act, int mode, int* status, void* stream,
-                 AddGate add = AddGate{nullptr, 0, nullptr, 1.0f}) {
+                 AddGate add = AddGate{nullptr, 0, nullptr, 1.0f}, GluArgs glu = GluArgs{GLU_SILU, 0.0f, 0.0f}) {
+    auto kernel = gemm_tcgen05_2sm_kernel<256, ACTS>;
     int device = 0, sms = 0;
     cudaGetDevice(&device);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
@@ -290,15 +316,14 @@ int launch_pairs(const void* a, const void* w, const qkv::Epilogue& e, float* c,
     if (int rc = make_map_bf16(&map_w, w, n, k, ldw, 128, "gemm_tcgen05_2sm")) return rc;
     static TiPerDevice configured;
     if (configured.first_use()) {
-        cudaError_t e2 = cudaFuncSetAttribute(gemm_tcgen05_2sm_kernel<256>,
-                                              cudaFuncAttributeMaxDynamicSharedMemorySize, Pair<256>::SMEM);
+        cudaError_t e2 = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Pair<256>::SMEM);
         if (e2 != cudaSuccess) return ti_fail("gemm_tcgen05_2sm: %s", cudaGetErrorString(e2));
         configured.mark();
     }
     const int tiles = ((m + BM - 1) / BM) * ((n + 255) / 256);
     const int pairs = tiles < sms / 2 ? tiles : sms / 2;
-    ti_launch_pdl(gemm_tcgen05_2sm_kernel<256>, 2 * pairs, THREADS, Pair<256>::SMEM, (cudaStream_t)stream,
-                  map_a, map_w, e, c, (bf16*)out_act, m, n, k, ldc, ld_act, mode, status, add);
+    ti_launch_pdl(kernel, 2 * pairs, THREADS, Pair<256>::SMEM, (cudaStream_t)stream, map_a, map_w, e, c,
+                  (bf16*)out_act, m, n, k, ldc, ld_act, mode, status, add, glu);
     return ti_check_launch("gemm_tcgen05_2sm");
 }
 
@@ -317,7 +342,7 @@ extern "C" int ti_gemm_tcgen05_2sm(const void* a, const void* w, float* c, void*
     TI_REQUIRE((uintptr_t)a % 16 == 0 && (uintptr_t)w % 16 == 0, "gemm_tcgen05_2sm: operands must be 16-byte aligned");
     TI_REQUIRE(mode == MODE_SWIGLU ? ((uintptr_t)out_act % 16 == 0 && ld_act % 8 == 0) : (uintptr_t)c % 16 == 0,
                "gemm_tcgen05_2sm: the output must be 16-byte aligned");
-    return launch_pairs(a, w, qkv::Epilogue{}, c, out_act, m, n, k, lda, ldw, ldc, ld_act, mode, status, stream);
+    return launch_pairs<false>(a, w, qkv::Epilogue{}, c, out_act, m, n, k, lda, ldw, ldc, ld_act, mode, status, stream);
 }
 
 // c += scale sigmoid(gate + bias) * (a w^T), or without a gate c += scale * (a w^T): as ti_gemm_tcgen05_gated, K never cut
@@ -331,8 +356,26 @@ extern "C" int ti_gemm_tcgen05_2sm_gated(const void* a, const void* w, float* c,
     TI_REQUIRE((uintptr_t)a % 16 == 0 && (uintptr_t)w % 16 == 0 && (uintptr_t)c % 16 == 0 && (uintptr_t)gate % 16 == 0 &&
                (uintptr_t)bias % 16 == 0 && ld_gate % 4 == 0 && (gate != nullptr) == (bias != nullptr),
                "gemm_tcgen05_2sm_gated: operands, output, the gate's rows and the bias must start on 16 bytes");
-    return launch_pairs(a, w, qkv::Epilogue{}, c, nullptr, m, n, k, lda, ldw, ldc, 0, MODE_ACCUMULATE, status, stream,
+    return launch_pairs<false>(a, w, qkv::Epilogue{}, c, nullptr, m, n, k, lda, ldw, ldc, 0, MODE_ACCUMULATE, status, stream,
                         AddGate{gate, ld_gate, bias, scale});
+}
+
+// As ti_gemm_tcgen05_glu (gemm_tcgen05.cu): out_act[m, n/2] = act(gate, up) of a w^T over groups of 8 gate + 8 up columns, or
+// out_act[m, n] = act(a w^T) with an activation of one value.
+extern "C" int ti_gemm_tcgen05_2sm_glu(const void* a, const void* w, void* out_act, int m, int n, int k, int lda,
+                                       int ldw, int ld_act, int glu_kind, float glu_limit, float glu_alpha, int* status,
+                                       void* stream) {
+    if (m == 0 || n == 0) return 0;
+    TI_REQUIRE((glu_kind >= GLU_SILU && glu_kind <= GLU_GELU_TANH) || glu_kind == ACT_RELU2,
+               "gemm_tcgen05_2sm_glu: activation %d", glu_kind);
+    const int mode = act_is_gated(glu_kind) ? MODE_SWIGLU : MODE_UNARY;
+    TI_REQUIRE(ti_gemm_tcgen05_2sm_supported(m, n, k, lda, ldw, 0, mode),
+               "gemm_tcgen05_2sm_glu: K=%d and the row strides %d, %d must be multiples of 8, N=%d a multiple of 16 (8 "
+               "without a gate)", k, lda, ldw, n);
+    TI_REQUIRE((uintptr_t)a % 16 == 0 && (uintptr_t)w % 16 == 0 && (uintptr_t)out_act % 16 == 0 && ld_act % 8 == 0,
+               "gemm_tcgen05_2sm_glu: operands and output must be 16-byte aligned");
+    return launch_pairs<true>(a, w, qkv::Epilogue{}, nullptr, out_act, m, n, k, lda, ldw, 0, ld_act, mode, status, stream,
+                              AddGate{nullptr, 0, nullptr, 1.0f}, GluArgs{glu_kind, glu_limit, glu_alpha});
 }
 
 // The QKV product of a prompt portion with the epilogue of qkv_epilogue.cuh (head size 128):
@@ -352,7 +395,7 @@ extern "C" int ti_gemm_tcgen05_2sm_qkv(const void* a, const void* w, int m, int 
                (uintptr_t)k_weight % 16 == 0, "gemm_tcgen05_2sm_qkv: operands must be 16-byte aligned, q_out and the pages 32-byte");
     const qkv::Epilogue e{q_weight, k_weight, eps, table, positions, req_of_tok, block_table, bt_stride,
                           (bf16*)pages, num_pages, page_size, write_kv, num_heads, num_kv_heads, (bf16*)q_out};
-    return launch_pairs(a, w, e, nullptr, nullptr, m, n, k, lda, ldw, 0, 0, MODE_QKV, status, stream);
+    return launch_pairs<false>(a, w, e, nullptr, nullptr, m, n, k, lda, ldw, 0, 0, MODE_QKV, status, stream);
 }
 
 TI_TAPED(ti_gemm_tcgen05_2sm)

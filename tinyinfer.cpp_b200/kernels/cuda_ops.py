@@ -299,6 +299,7 @@ class CudaOps(MixerOps, StateOps):
                                                       _vp, _vp]
             b.ti_gemm_skinny_glu.argtypes = [_vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _f, _f, _vp]
             b.ti_gemm_tcgen05_glu.argtypes = [_vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _f, _f, _vp, _vp]
+            b.ti_gemm_tcgen05_2sm_glu.argtypes = b.ti_gemm_tcgen05_glu.argtypes
             b.ti_gemm_tcgen05_2sm.argtypes = [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _vp, _vp]
             qkv_args = [_vp, _vp, _i, _i, _i, _i, _vp, _vp, _f, _vp, _vp, _vp, _vp, _i, _vp, _i, _i, _i,
                         _i, _i, _vp, _vp, _vp]
@@ -433,6 +434,15 @@ class CudaOps(MixerOps, StateOps):
         if self.use_2sm_gemm and tiles >= self.pair_min_tiles:
             return self.bf16.ti_gemm_tcgen05_2sm
         return self.bf16.ti_gemm_tcgen05
+
+    def _tc_glu(self, m: int, n: int, k: int, kind: str):
+        """The same choice among the products whose epilogue applies an activation.  With gelu's tanh the epilogue is the longer
+        half of a tile of short rows, and pairs lose what they gain while they wait for it: us, one SM / pairs, gelu at k 1,024:
+        64 tiles 15.4 / 13.3, 88 tiles 18.4 / 19.4, 352 tiles 38.4 / 39.4; other kinds or k 2,048: equal to a quarter faster."""
+        pairs = self._tc_gemm(m, n) is self.bf16.ti_gemm_tcgen05_2sm
+        if kind == "gelu_tanh" and k <= 1024 and -(-m // 256) * -(-n // 256) > self.num_sms // 2:
+            pairs = False
+        return self.bf16.ti_gemm_tcgen05_2sm_glu if pairs else self.bf16.ti_gemm_tcgen05_glu
 
     def _run_tc_gemm(self, a, w, c, out_act, m, n, k, ldc, ld_act, mode, may_defer=False) -> None:
         """The tcgen05 product of many rows; an output of few tiles has its K cut into runs that a
@@ -787,7 +797,7 @@ class CudaOps(MixerOps, StateOps):
                 return
             if (m > 64 and n % 8 == 0 and out.stride(0) % 8 == 0 and out.data_ptr() % 16 == 0
                     and self.bf16.ti_gemm_tcgen05_supported(m, n, k, h.stride(0), w.stride(0), 0, 0)):
-                self._ok(self.bf16.ti_gemm_tcgen05_glu(
+                self._ok(self._tc_glu(m, n, k, kind)(
                     h.data_ptr(), w.data_ptr(), out.data_ptr(), m, n, k, h.stride(0), w.stride(0), out.stride(0),
                     UNARY_KINDS[kind], 0.0, 0.0, self.status.data_ptr(), self._stream()), self.bf16)
                 return
@@ -848,7 +858,7 @@ class CudaOps(MixerOps, StateOps):
                 and inter % 8 == 0 and h.data_ptr() % 16 == 0 and self.bf16.ti_gemm_tcgen05_supported(
                     m, 2 * inter, k, h.stride(0), w_gate_up.stride(0), 0, 2)):
             # many rows: the activation in the epilogue of the tcgen05 product
-            self._ok(self.bf16.ti_gemm_tcgen05_glu(
+            self._ok(self._tc_glu(m, 2 * inter, k, kind)(
                 h.data_ptr(), w_gate_up.data_ptr(), y.data_ptr(), m, 2 * inter, k, h.stride(0), w_gate_up.stride(0),
                 y.stride(0), GLU_KINDS[kind], float(limit), float(alpha), self.status.data_ptr(), self._stream()),
                 self.bf16)
