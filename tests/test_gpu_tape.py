@@ -76,3 +76,59 @@ def test_layers_that_cannot_be_repeated_run_one_by_one(monkeypatch):
     mixer.w_o = mixer.w_o.float()
     _run(engine, True)
     assert not made, "layers of unlike weights were recorded"
+
+
+def _adapted_parts():
+    """A feed-forward from outside the package: SwiGLU and one more matrix a layer."""
+    from tinyinfer_b200.parts.base import MATRIX, WeightSpec
+    from tinyinfer_b200.parts.mlp import SwiGLU
+
+    class Adapted(SwiGLU):
+        def weight_specs(self):
+            return {**super().weight_specs(), "adapter.weight": WeightSpec((self.hidden_size, self.hidden_size), MATRIX)}
+
+        def load_weights(self, tensors, ops):
+            super().load_weights(tensors, ops)
+            self.adapter = ops.pack_linear(tensors["adapter.weight"])
+
+        def forward(self, ops, h, residual, step):
+            ops.linear(h, self.adapter, residual, accumulate=True)
+            super().forward(ops, h, residual, step)
+
+    class AdaptedAndSaid(Adapted):
+        launches_repeat = True
+    return Adapted, AdaptedAndSaid
+
+
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+@pytest.mark.parametrize("said", [False, True])
+def test_parts_from_outside_the_package_read_their_own_tensors(dtype, said, monkeypatch):
+    from tinyinfer_b200 import Engine
+    from tinyinfer_b200.kernels import tape
+    from tinyinfer_b200.parts import register_part
+    from tinyinfer_b200.parts.mlp import SwiGLU
+    register_part("ffn", "swiglu", _adapted_parts()[said])
+    try:
+        engine = Engine(config=_config(), seed=1, dtype=dtype, device=DEV, num_pages=64, max_requests=3)
+    finally:
+        register_part("ffn", "swiglu", SwiGLU)
+    want = _run(engine, False)
+    made = []
+    real = tape.record
+    monkeypatch.setattr(tape, "record", lambda *a: made.append(real(*a)) or made[-1])
+    for (a, n), (b, m) in zip(want, _run(engine, True)):
+        assert torch.equal(a, b) and n == m
+    assert len(made) == (len(STEPS) if said else 0) and all(r is not None for r in made)
+
+
+def test_a_number_changed_in_one_layer_is_kept(monkeypatch):
+    from tinyinfer_b200 import Engine
+    from tinyinfer_b200.kernels import tape
+    engine = Engine(config=_config(), seed=1, dtype="bfloat16", device=DEV, num_pages=64, max_requests=3)
+    plain = _run(engine, False)
+    engine.model.blocks[3].mixer.scale *= 3.0
+    want = _run(engine, False)
+    assert not torch.equal(plain[0][0], want[0][0])
+    monkeypatch.setattr(tape, "record", lambda *a: pytest.fail("layers of unlike numbers were recorded"))
+    for (a, _), (b, _) in zip(want, _run(engine, True)):
+        assert torch.equal(a, b)

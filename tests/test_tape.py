@@ -1,0 +1,171 @@
+"""What makes a layer's recorded launches valid for the layers like it: parts whose class itself says so, equal in everything but
+their tensors; the addresses of those tensors, and addresses inside them, are the layer's own in every repetition.  A kernel set
+whose entry points note their pointers stands for the device."""
+import ctypes
+import threading
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from tinyinfer_b200.config import PartSpec
+from tinyinfer_b200.kernels import tape
+from tinyinfer_b200.parts.attention import Attention
+from tinyinfer_b200.parts.base import own_state
+from tinyinfer_b200.parts.block import PreNormBlock
+from tinyinfer_b200.parts.mlp import SwiGLU
+from tinyinfer_b200.parts.norm import RMSNorm
+
+
+class NotingLib:
+    """One entry point, ``ti_x(pointer, number)``, and the native repetition of its calls."""
+
+    def __init__(self):
+        self.seen, self.lock = [], threading.Lock()
+        self.ti_x_taped = ctypes.CFUNCTYPE(ctypes.c_int, ctypes.c_void_p)(lambda slots: 0)
+
+        def ti_x(pointer, number):
+            self.seen.append((pointer, number))
+            return 0
+        ti_x.argtypes = [ctypes.c_void_p, ctypes.c_int]
+        self.ti_x = ti_x
+
+    def ti_tape_run(self, calls, first, num_calls, slots, patch_slot, num_patches, values, layers):
+        for layer in range(layers):
+            for p in range(num_patches):
+                slots[patch_slot[p]] = values[layer * num_patches + p]
+            for c in range(num_calls):
+                self.seen.append((slots[first[c]], slots[first[c] + 1]))
+        return 0
+
+
+def _ops():
+    ops = SimpleNamespace(core=NotingLib(), _pending_runs=None, _pending=None, _pending_pair=None, issued=0, launches=0, use_tape=True)
+
+    def x(pointer, number):
+        ops.issued += 1
+        ops.core.ti_x(pointer, number)
+    ops.x = x
+    return ops
+
+
+class Plain(SwiGLU):
+    """Reads its two matrices, one of them from an address inside it."""
+    launches_repeat = True
+
+    def __init__(self):
+        super().__init__(8, 16)
+        self.w_gate_up, self.w_down = torch.zeros(32, 8), torch.zeros(8, 16)
+
+    def forward(self, ops, h, residual, step):
+        ops.x(self.w_gate_up.data_ptr(), 1)
+        ops.x(self.w_gate_up[16:].data_ptr() if step is None else self.w_gate_up.data_ptr() + 16 * 8 * 4, 2)
+        ops.x(self.w_down.data_ptr(), 3)
+
+
+class Adapted(Plain):
+    """One tensor more, as a class outside the package would add it, without a word on its launches."""
+
+    def __init__(self):
+        super().__init__()
+        self.adapter = torch.zeros(4, 8)
+
+    def forward(self, ops, h, residual, step):
+        super().forward(ops, h, residual, step)
+        ops.x(self.adapter.data_ptr(), 4)
+
+
+class AdaptedAndSaid(Adapted):
+    launches_repeat = True
+
+
+def _run(layers):
+    from tinyinfer_b200.kernels.cuda_ops import CudaOps
+    ops = _ops()
+
+    def own(k):
+        tensors, others = [], []
+        return (tensors, others) if own_state(layers[k], tensors, others) else None
+    before = len(ops.core.seen)
+    CudaOps.repeat_layers(ops, len(layers), lambda k: layers[k].forward(ops, None, None, True), own)
+    got = ops.core.seen[before:]
+    python = ops.issued
+    ops.core.seen.clear()
+    for layer in layers:
+        layer.forward(ops, None, None, True)
+    return got, list(ops.core.seen), python
+
+
+@pytest.mark.parametrize("part", [Plain, Adapted, AdaptedAndSaid])
+def test_every_layer_reads_its_own_tensors(part):
+    got, want, python = _run([part() for _ in range(6)])
+    assert got == want
+    per_layer = len(want) // 6
+    assert part is Adapted or python == 6 * per_layer      # launches are counted, repeated ones too
+
+
+def test_classes_speak_for_themselves_alone():
+    assert own_state(Plain(), [], []) and own_state(AdaptedAndSaid(), [], [])
+    assert not own_state(Adapted(), [], [])
+    tensors = []
+    own_state(AdaptedAndSaid(), tensors, [])
+    assert len(tensors) == 3
+    part = Plain()
+    part.forward = lambda *a: None                          # a method replaced on one part
+    assert not own_state(part, [], [])
+    part = Plain()
+    part.table = {"a": torch.zeros(1)}                      # tensors out of sight
+    assert not own_state(part, [], [])
+
+
+def _block(**changed):
+    position = PartSpec("rope_neox", {"head_dim": 16, "theta": 1e4})
+    mixer = Attention(hidden_size=64, num_heads=4, num_kv_heads=2, head_dim=16, qk_norm_eps=1e-6, position=position)
+    block = PreNormBlock(mixer, RMSNorm(64, 1e-6), SwiGLU(64, 96), RMSNorm(64, 1e-6))
+    mixer.w_qkv, mixer.w_o, mixer.q_norm, mixer.k_norm = (torch.zeros(n, 4) for n in (8, 4, 2, 2))
+    block.ffn.w_gate_up, block.ffn.w_down = torch.zeros(8, 4), torch.zeros(4, 4)
+    block.mixer_norm.weight, block.ffn_norm.weight = torch.zeros(4), torch.zeros(4)
+    for path, value in changed.items():
+        *way, name = path.split("__")
+        at = block
+        for w in way:
+            at = getattr(at, w)
+        setattr(at, name, value)
+    return block
+
+
+def _state(block):
+    tensors, others = [], []
+    assert own_state(block, tensors, others)
+    return tensors, others
+
+
+def test_the_parts_of_a_layer_are_seen_through():
+    tensors, _ = _state(_block())
+    assert len(tensors) == 8
+    like = tape.signature(*_state(_block()))
+    assert like == tape.signature(*_state(_block()))
+
+
+@pytest.mark.parametrize("changed", [{"mixer__scale": 0.5}, {"mixer_norm__eps": 1e-3}, {"mixer__position__theta": 3e4},
+                                     {"ffn__w_down": torch.zeros(4, 4, dtype=torch.bfloat16)}, {"mixer__window": 7},
+                                     {"ffn__factor": 2.0}, {"mixer__w_o": None}])
+def test_layers_that_differ_in_anything_but_contents_are_told_apart(changed):
+    assert tape.signature(*_state(_block(**changed))) != tape.signature(*_state(_block()))
+
+
+def test_tensors_that_overlap_are_not_repeated():
+    class Two(Plain):
+        launches_repeat = True
+
+        def __init__(self):
+            super().__init__()
+            self.w_second = self.w_gate_up[8:]
+    made = []
+    real = tape.record
+    try:
+        tape.record = lambda *a: made.append(real(*a)) or made[-1]
+        got, want, _ = _run([Two() for _ in range(5)])
+    finally:
+        tape.record = real
+    assert got == want and made == [None]

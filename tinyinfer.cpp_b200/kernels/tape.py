@@ -9,7 +9,8 @@ replaced.  The first layer is not the one recorded because it has no layer in fr
 
 What makes a recording valid: every launch went through an entry point that has a taped form (else the number of launches and
 of recorded calls differ), no torch operation but allocations and views took place, nothing is held back at the layer's end
-that was not held back at its start, and the layers' own tensors agree in type, shape, strides and alignment.  A recording
+that was not held back at its start, and the layers agree in everything that their launches may depend on (``own_state`` of
+parts/base.py) but the contents of their tensors, whose addresses, and those inside them, are replaced.  A recording
 lives for one pass and holds the tensors allocated under it until the pass has issued its last launch.
 """
 from __future__ import annotations
@@ -71,9 +72,17 @@ def _slot(kind, value) -> int:
     return (0 if value is None else int(value)) & 0xFFFFFFFFFFFFFFFF
 
 
-def signature(tensors) -> tuple:
-    """What two layers' own tensors must agree in for one layer's launches to serve the other."""
-    return tuple((t.dtype, t.shape, t.stride(), t.data_ptr() % 32, getattr(t, "_ti_interleaved", None)) for t in tensors)
+def signature(tensors, others) -> tuple:
+    """What two layers must agree in for one layer's launches to serve the other: all but what their tensors hold."""
+    return [(t.dtype, t.shape, t.stride(), t.data_ptr() % 32, getattr(t, "_ti_interleaved", None)) for t in tensors], others
+
+
+def _inside(spans, value):
+    """(index, offset) of the tensor that the address lies in, behind its start; None: in none of them."""
+    for i, (start, end) in enumerate(spans):
+        if start < value < end:
+            return i, value - start
+    return None
 
 
 def record(ops, run, mine):
@@ -103,9 +112,12 @@ def record(ops, run, mine):
         if start[1:2] != end[1:2] or start[2] is not end[2] or start[3] != end[3]:
             return None
         renamed[start[0].data_ptr()] = end[0].data_ptr()
-    place = {t.data_ptr(): i for i, t in enumerate(mine)}
-    if len(place) != len(mine):
-        return None
+    spans = [(t.data_ptr(), t.data_ptr() + t.element_size() * (1 + sum((n - 1) * s for n, s in zip(t.shape, t.stride()))))
+             for t in mine]
+    in_order = sorted(spans)
+    if any(after[0] < before[1] for before, after in zip(in_order, in_order[1:])):
+        return None                        # an address may stand for either of two tensors
+    place = {first: (i, 0) for i, (first, _) in enumerate(spans)}
     first, slots, patches, sources = [], [], [], []
     for _, _, kinds, args in calls:
         if kinds is None or len(kinds) != len(args):
@@ -113,7 +125,9 @@ def record(ops, run, mine):
         first.append(len(slots))
         for kind, value in zip(kinds, args):
             if kind is ctypes.c_void_p and value:
-                if value in place:
+                if value not in place:
+                    place[value] = _inside(spans, value)
+                if place[value] is not None:
                     patches.append(len(slots))
                     sources.append(place[value])
                 value = renamed.get(value, value)
@@ -123,7 +137,7 @@ def record(ops, run, mine):
               (ctypes.c_ulonglong * max(1, len(slots)))(*slots), (ctypes.c_int * max(1, len(patches)))(*patches), len(patches))
 
     def replay(layers):
-        values = [own[s] for own in ([t.data_ptr() for t in layer] for layer in layers) for s in sources]
+        values = [own[i] + offset for own in ([t.data_ptr() for t in layer] for layer in layers) for i, offset in sources]
         rc = ops.core.ti_tape_run(*packed, (ctypes.c_ulonglong * max(1, len(values)))(*values), len(layers))
         ops.launches += n * len(layers)
         ops.issued += n * len(layers)

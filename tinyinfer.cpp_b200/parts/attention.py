@@ -23,6 +23,7 @@ from .base import (MATRIX, NORM_WEIGHT, PagedKVSpec, Part, WeightSpec, as_float3
 
 class Attention(Part):
     category = "mixer"
+    launches_repeat = True
 
     def __init__(self, hidden_size: int, num_heads: int, num_kv_heads: int, head_dim: int,
                  qk_norm_eps: float, position: PartSpec, window: Optional[int] = None,
@@ -66,9 +67,6 @@ class Attention(Part):
 
     def cache_spec(self):
         return PagedKVSpec(self.num_kv_heads, self.head_dim, self.window)
-
-    def own_tensors(self):
-        return [self.w_qkv, self.w_o, self.q_norm, self.k_norm]
 
     def forward(self, ops, h, residual, step, cache):
         t, dev, act = h.shape[0], h.device, h.dtype

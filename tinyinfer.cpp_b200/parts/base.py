@@ -111,17 +111,17 @@ class Part:
     # a mixer or feed-forward that takes a ``GatedSum`` without a gate (a factor on what it adds) in the
     # place of its residual, besides those that end in a product
     takes_factor = False
+    # every launch of the part goes through the kernel set's entry points and depends on the step, the cache view and the
+    # part's own attributes alone, and those are numbers, texts, tensors and parts of which the same holds: alike layers of
+    # such parts may repeat one another's launches (``own_state``).  A class says so for itself alone: what is derived from
+    # it may read more, so it has to say it again.
+    launches_repeat = False
 
     def weight_specs(self) -> dict[str, WeightSpec]:
         return {}
 
     def load_weights(self, tensors: Mapping[str, torch.Tensor], ops: Any) -> None:
         """Take the tensors named in ``weight_specs`` (already on the device, dtype as stored)."""
-
-    def own_tensors(self):
-        """The device tensors that the part's launches read and that another part of the same specification has in
-        its place, in a fixed order; None: not stated (its layer is then never repeated from a recording)."""
-        return None
 
     def step_lists(self) -> list:
         """Integer lists (``engine.batch.StepList``) that this part wants built on the host for
@@ -131,6 +131,27 @@ class Part:
     def shared_weights(self) -> dict[str, torch.Tensor]:
         """Tensors another part may alias (for instance the embedding table for a tied head)."""
         return {}
+
+
+_PLAIN = frozenset((bool, int, float, str, type(None), torch.dtype))
+
+
+def own_state(part: Part, tensors: list, others: list) -> bool:
+    """Appends the tensors that the part and the parts inside it hold, and all else that tells it from another part (classes,
+    attributes' names, numbers).  Launches of two parts whose lists agree differ by the tensors alone.  False: not known, for
+    a part whose class does not say ``launches_repeat`` or that holds anything else (a function in the place of a method)."""
+    cls, held = type(part), vars(part)
+    if cls.__dict__.get("launches_repeat") is not True:
+        return False
+    others.append((cls, *held))
+    for value in held.values():
+        if type(value) in _PLAIN:
+            others.append(value)
+        elif type(value) is torch.Tensor:
+            tensors.append(value)
+        elif not isinstance(value, Part) or not own_state(value, tensors, others):
+            return False
+    return True
 
 
 def residual_and_factor(target) -> "tuple[torch.Tensor, float]":

@@ -30,16 +30,13 @@ from .norm import LayerNorm
 
 class PreNormBlock(Part):
     category = "block"
+    launches_repeat = True
 
     def __init__(self, mixer, mixer_norm, ffn=None, ffn_norm=None):
         if (ffn is None) != (ffn_norm is None):
             raise ValueError("a feed-forward and its norm come together")
         self.mixer, self.ffn = mixer, ffn
         self.mixer_norm, self.ffn_norm = mixer_norm, ffn_norm
-
-    def own_tensors(self):
-        lists = [p.own_tensors() for p in (self.mixer_norm, self.mixer, self.ffn_norm, self.ffn) if p is not None]
-        return None if any(x is None for x in lists) else [t for x in lists for t in x]
 
     def forward(self, ops, x, step, cache):
         self.mixer.forward(ops, self.mixer_norm.forward(ops, x, step.act_dtype), x, step, cache)
@@ -123,9 +120,6 @@ class ScaledPreNormBlock(PreNormBlock):
     def __init__(self, mixer, mixer_norm, ffn=None, ffn_norm=None, multiplier: float = 1.0):
         super().__init__(mixer, mixer_norm, ffn, ffn_norm)
         self.multiplier = float(multiplier)
-
-    def own_tensors(self):
-        return None
 
     def _add(self, ops, part, run, x):
         if self.multiplier == 1.0:

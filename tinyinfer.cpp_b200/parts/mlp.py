@@ -19,6 +19,7 @@ from .base import MATRIX, Part, WeightSpec, register_part
 
 class SwiGLU(Part):
     category = "ffn"
+    launches_repeat = True
 
     def __init__(self, hidden_size: int, intermediate_size: int):
         self.hidden_size = int(hidden_size)
@@ -39,9 +40,6 @@ class SwiGLU(Part):
             g, u = g.to(torch.float32), u.to(torch.float32)
         self.w_gate_up = ops.pack_gate_up(g, u)
         self.w_down = ops.pack_linear(tensors["down_proj.weight"])
-
-    def own_tensors(self):
-        return [self.w_gate_up, self.w_down]
 
     def forward(self, ops, h, residual, step):
         ops.swiglu_ffn(h, self.w_gate_up, self.w_down, residual, may_defer=True)

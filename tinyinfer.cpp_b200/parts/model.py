@@ -12,7 +12,7 @@ from typing import Callable, Mapping
 import torch
 
 from ..config.plan import ModelPlan
-from .base import FixedStateSpec, PagedKVSpec, Part, WeightSpec, build_part
+from .base import FixedStateSpec, PagedKVSpec, Part, WeightSpec, build_part, own_state
 
 
 class CausalLM:
@@ -145,10 +145,11 @@ class CausalLM:
             parts = [(self.blocks[e.layer], cache_views[(e.cache_slot, e.writes_cache)]) for e in schedule[at:at + count]]
 
             def own(k):
-                mine, view = parts[k][0].own_tensors(), parts[k][1]
+                mine, others, view = [], [], parts[k][1]
                 pages, first = getattr(view, "pages", None), parts[0][1]      # one kind of pages, by one block table
-                same = mine is not None and pages is not None and view.block_table is getattr(first, "block_table", None)
-                return mine + [pages] if same else None
+                if pages is None or view.block_table is not getattr(first, "block_table", None):
+                    return None
+                return (mine + [pages], others) if own_state(parts[k][0], mine, others) else None
 
             def run(k):
                 parts[k][0].forward(ops, x, step, parts[k][1])

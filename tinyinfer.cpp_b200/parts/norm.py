@@ -14,6 +14,7 @@ from .base import NORM_WEIGHT, NORM_ZERO, Part, WeightSpec, as_float32, register
 
 class RMSNorm(Part):
     category = "norm"
+    launches_repeat = True
 
     def __init__(self, size: int, eps: float, tensor: str = "weight", one_plus: bool = False, scalar: bool = False,
                  factor: float = 1.0):
@@ -36,9 +37,6 @@ class RMSNorm(Part):
             self.weight = 1.0 + self.weight          # float32; the kernels multiply by it as it is
         if self.factor != 1.0:
             self.weight = self.factor * self.weight
-
-    def own_tensors(self):
-        return [self.weight]
 
     def forward(self, ops, x: torch.Tensor, out_dtype: torch.dtype) -> torch.Tensor:
         out = torch.empty((x.shape[0], self.size), dtype=out_dtype, device=x.device)

@@ -60,6 +60,7 @@ _TABLES: dict[tuple, torch.Tensor] = {}      # layers with the same constants sh
 
 class RopeNeox(Part):
     category = "position"
+    launches_repeat = True
 
     def __init__(self, head_dim: int, theta: float, rotary_dim: Optional[int] = None):
         rotary_dim = head_dim if rotary_dim is None else int(rotary_dim)
@@ -84,6 +85,7 @@ class RopeNeox(Part):
 
 class RopeInterleaved(RopeNeox):
     """The same frequencies and turn as ``RopeNeox`` on neighbouring pairs ``(2k, 2k + 1)``."""
+    launches_repeat = True
 
     def rotation(self, device) -> Rotation:
         return Rotation("interleaved", self.rotary_dim, super().rotation(device).inv_freq)
@@ -95,6 +97,7 @@ class RopeStretched(RopeNeox):
     ``hi = min(ceil(d(slow)), rotary_dim - 1)`` and ``ramp_k = clamp((k - lo) / max(hi - lo, 0.001),
     0, 1)``, pair ``k`` turns with ``f_k / factor * ramp_k + f_k * (1 - ramp_k)``, and sine and
     cosine are multiplied by ``0.1 ln(factor) + 1``.  ``layout``: ``interleaved`` or ``neox``."""
+    launches_repeat = True
 
     def __init__(self, head_dim: int, theta: float, factor: float, original: float, fast: float, slow: float,
                  rotary_dim: Optional[int] = None, layout: str = "interleaved"):
@@ -131,6 +134,7 @@ class RopeWavelength(RopeNeox):
     """Frequencies scaled by their wavelength ``l = 2 pi / f`` (the scaling of Llama 3.1): ``f`` stays where ``l <
     original / high``, becomes ``f / factor`` where ``l > original / low``, and ``(1 - s) f / factor + s f`` with ``s =
     (original / l - low) / (high - low)`` between the two.  ``layout``: ``neox`` or ``interleaved``."""
+    launches_repeat = True
 
     def __init__(self, head_dim: int, theta: float, factor: float, original: float, low: float, high: float,
                  rotary_dim: Optional[int] = None, layout: str = "neox"):
@@ -167,6 +171,7 @@ class RopeWavelength(RopeNeox):
 class NoPosition(Part):
     """Heads are normed and stored without a rotation."""
     category = "position"
+    launches_repeat = True
 
     def __init__(self, head_dim: int = 0):
         self.head_dim = int(head_dim)
