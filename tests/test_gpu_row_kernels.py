@@ -204,3 +204,26 @@ def test_embedding_rows(ops, hidden):
         out = torch.empty((4, hidden), device=DEV)
         ops.embed(table, tokens, out)
         assert torch.equal(out, table[tokens.long()].float())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("heads,kv,dk", [(16, 4, 128), (31, 1, 64), (32, 1, 64), (60, 4, 64), (61, 4, 64), (60, 4, 128)])
+def test_a_row_of_heads_does_not_depend_on_the_rows_beside_it(ops, heads, kv, dk, dtype):
+    """300 rows and the same rows in runs of 1, 7 and 255, on either side of every number of units and tokens that chooses a
+    launch shape (512 and 1,024 units, 256 tokens)."""
+    t, nq, nk = 300, heads * dk, kv * dk
+    proj, wq, wk, freq = _rand((t, nq + 2 * nk), 1), _rand((nq,), 2), _rand((nk,), 3), _freq(dk)
+    rotation = SimpleNamespace(kind="interleaved", rotary_dim=dk, inv_freq=freq, scale=1.0)
+
+    def rows(first, n):
+        step = _step([n], [first])
+        cache = _cache(step, kv * 2 * dk, dtype)
+        q = torch.empty((n, nq), dtype=dtype, device=DEV)
+        ops.qk_rownorm_rope_store(proj[first:first + n], wq, wk, 1e-6, rotation, step, cache, q, heads, kv, dk, dk)
+        per_page = 2 * dk * kv * PAGE
+        kept = [_stored(cache, step, base * kv * PAGE * dk, h, dk, per_page) for base in (0, 1) for h in range(kv)]
+        return torch.cat([q] + kept, 1)
+    whole = rows(0, t)
+    for run in (1, 7, 255):
+        for first in (0, 20, 45):
+            assert torch.equal(rows(first, run), whole[first:first + run]), (run, first)

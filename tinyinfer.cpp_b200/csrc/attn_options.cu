@@ -170,8 +170,8 @@ template <typename TQ, typename TC, int THREADS, int NU, bool AHEAD>
 __global__ void __launch_bounds__(THREADS, 1024 / THREADS)
 row_heads_units_kernel(const RowHeads p, TC* __restrict__ pages, TQ* __restrict__ q_out, int* __restrict__ status) {
     extern __shared__ __align__(16) float2 turn_table[];
-    constexpr int WARPS_ = THREADS / 32;
-    __shared__ float sums[2][WARPS_];
+    constexpr int SHARES = NU / 2, SUMS = SHARES * THREADS / 32;
+    __shared__ float sums[2][SUMS];
     const int t = blockIdx.x, tid = threadIdx.x, pos = p.positions[t];
     const int hu = p.dk >> 2, qu = p.num_heads * hu, total = qu + (p.write_kv ? p.num_kv_heads * hu : 0);
     const int nq = p.num_heads * p.dk, nk = p.num_kv_heads * p.dk;
@@ -203,7 +203,6 @@ row_heads_units_kernel(const RowHeads p, TC* __restrict__ pages, TQ* __restrict_
     __syncthreads();                                   // the turn tables
     pdl_wait();
     const float* row = p.proj + (size_t)t * p.stride;
-    float2 ss = make_float2(0.0f, 0.0f);               // of the query row, of the key row
 #pragma unroll
     for (int j = 0; j < NU; ++j) {
         const int i = tid + THREADS * j;
@@ -233,17 +232,24 @@ row_heads_units_kernel(const RowHeads p, TC* __restrict__ pages, TQ* __restrict_
     }
     float inv_q = 1.0f, inv_k = 1.0f;
     if (p.norm.on) {
+        // Four units a thread are summed as the two threads of twice as wide a block sum them: a row's bits must not depend
+        // on the number of tokens, which chooses between the two.
 #pragma unroll
-        for (int j = 0; j < NU; ++j) {
-            const float s = fmaf(x[j].w, x[j].w, fmaf(x[j].z, x[j].z, fmaf(x[j].y, x[j].y, x[j].x * x[j].x)));
-            if (tid + THREADS * j < qu) ss.x += s; else ss.y += s;
+        for (int p0 = 0; p0 < SHARES; ++p0) {
+            float2 ss = make_float2(0.0f, 0.0f);       // of the query row, of the key row
+#pragma unroll
+            for (int j = p0; j < NU; j += SHARES) {
+                const float s = fmaf(x[j].w, x[j].w, fmaf(x[j].z, x[j].z, fmaf(x[j].y, x[j].y, x[j].x * x[j].x)));
+                if (tid + THREADS * j < qu) ss.x += s; else ss.y += s;
+            }
+            ss = make_float2(warp_sum(ss.x), warp_sum(ss.y));
+            const int at = p0 * (THREADS / 32) + (tid >> 5);
+            if ((tid & 31) == 0) { sums[0][at] = ss.x; sums[1][at] = ss.y; }
         }
-        ss = make_float2(warp_sum(ss.x), warp_sum(ss.y));
-        if ((tid & 31) == 0) { sums[0][tid >> 5] = ss.x; sums[1][tid >> 5] = ss.y; }
         __syncthreads();
-        ss = make_float2(0.0f, 0.0f);
+        float2 ss = make_float2(0.0f, 0.0f);
 #pragma unroll
-        for (int i = 0; i < WARPS_; ++i) { ss.x += sums[0][i]; ss.y += sums[1][i]; }
+        for (int i = 0; i < SUMS; ++i) { ss.x += sums[0][i]; ss.y += sums[1][i]; }
         inv_q = 1.0f / sqrtf(ss.x / (float)nq + p.norm.eps);
         inv_k = 1.0f / sqrtf(ss.y / (float)nk + p.norm.eps);
     }
