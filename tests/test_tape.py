@@ -11,7 +11,7 @@ import torch
 from tinyinfer_b200.config import PartSpec
 from tinyinfer_b200.kernels import tape
 from tinyinfer_b200.parts.attention import Attention
-from tinyinfer_b200.parts.base import own_state
+from tinyinfer_b200.parts.base import own_layout, own_tensors
 from tinyinfer_b200.parts.block import PreNormBlock
 from tinyinfer_b200.parts.mlp import SwiGLU
 from tinyinfer_b200.parts.norm import RMSNorm
@@ -83,9 +83,11 @@ def _run(layers):
     from tinyinfer_b200.kernels.cuda_ops import CudaOps
     ops = _ops()
 
+    layout = own_layout(layers[0])
+
     def own(k):
-        tensors, others = [], []
-        return (tensors, others) if own_state(layers[k], tensors, others) else None
+        tensors = []
+        return tensors if layout and own_tensors(layers[k], layout, tensors) else None
     before = len(ops.core.seen)
     CudaOps.repeat_layers(ops, len(layers), lambda k: layers[k].forward(ops, None, None, True), own)
     got = ops.core.seen[before:]
@@ -105,17 +107,20 @@ def test_every_layer_reads_its_own_tensors(part):
 
 
 def test_classes_speak_for_themselves_alone():
-    assert own_state(Plain(), [], []) and own_state(AdaptedAndSaid(), [], [])
-    assert not own_state(Adapted(), [], [])
+    assert own_layout(Plain()) and own_layout(AdaptedAndSaid())
+    assert own_layout(Adapted()) is None
     tensors = []
-    own_state(AdaptedAndSaid(), tensors, [])
-    assert len(tensors) == 3
+    assert own_tensors(AdaptedAndSaid(), own_layout(AdaptedAndSaid()), tensors) and len(tensors) == 3
+    assert not own_tensors(Adapted(), own_layout(Plain()), []) and not own_tensors(AdaptedAndSaid(), own_layout(Plain()), [])
     part = Plain()
     part.forward = lambda *a: None                          # a method replaced on one part
-    assert not own_state(part, [], [])
+    assert own_layout(part) is None and not own_tensors(part, own_layout(Plain()), [])
     part = Plain()
     part.table = {"a": torch.zeros(1)}                      # tensors out of sight
-    assert not own_state(part, [], [])
+    assert own_layout(part) is None and not own_tensors(part, own_layout(Plain()), [])
+    part = Plain()
+    del part.w_down
+    assert not own_tensors(part, own_layout(Plain()), [])
 
 
 def _block(**changed):
@@ -134,24 +139,27 @@ def _block(**changed):
     return block
 
 
-def _state(block):
-    tensors, others = [], []
-    assert own_state(block, tensors, others)
-    return tensors, others
+def _alike(other):
+    tensors = [[], []]
+    layout = own_layout(_block())
+    if not all(own_tensors(b, layout, t) for b, t in zip((_block(), other), tensors)):
+        return None
+    assert len(tensors[0]) == 8
+    return tape.alike(tensors)
 
 
 def test_the_parts_of_a_layer_are_seen_through():
-    tensors, _ = _state(_block())
-    assert len(tensors) == 8
-    like = tape.signature(*_state(_block()))
-    assert like == tape.signature(*_state(_block()))
+    other = _block()
+    assert _alike(other)[1] == [t.data_ptr() for t in (
+        other.mixer.w_qkv, other.mixer.w_o, other.mixer.q_norm, other.mixer.k_norm, other.ffn.w_gate_up, other.ffn.w_down,
+        other.mixer_norm.weight, other.ffn_norm.weight)]
 
 
 @pytest.mark.parametrize("changed", [{"mixer__scale": 0.5}, {"mixer_norm__eps": 1e-3}, {"mixer__position__theta": 3e4},
                                      {"ffn__w_down": torch.zeros(4, 4, dtype=torch.bfloat16)}, {"mixer__window": 7},
                                      {"ffn__factor": 2.0}, {"mixer__w_o": None}])
 def test_layers_that_differ_in_anything_but_contents_are_told_apart(changed):
-    assert tape.signature(*_state(_block(**changed))) != tape.signature(*_state(_block()))
+    assert _alike(_block(**changed)) is None
 
 
 def test_tensors_that_overlap_are_not_repeated():

@@ -385,24 +385,24 @@ class CudaOps(MixerOps, StateOps):
             raise KernelError((lib or self.core).ti_last_error().decode("utf-8", "replace"))
 
     def repeat_layers(self, count: int, run, own) -> None:
-        """Runs ``run(0)`` to ``run(count - 1)``: layers of one specification.  ``own(k)`` lists the tensors that layer k reads
-        and whatever else tells it from another layer (``parts.base.own_state``; None: not known).  From the third on, the launches recorded while the second ran are repeated natively where they can be;
-        the result is that of running them one by one.  (0.6B shape, 28 layers, steps of 512 tokens: 3.6 to 4.1 ms
-        of host time a step -> 1.9, of which the repeated launches take 0.65.)"""
-        from .tape import record, signature
+        """Runs ``run(0)`` to ``run(count - 1)``: layers alike in all but the tensors that ``own(k)`` lists (None: layer k is not
+        like layer 0, or not known to be).  From the third on, the launches recorded while the second ran are repeated
+        natively where they can be; the result is that of running them one by one.  (0.6B shape, 28 layers, steps of 512
+        tokens: 3.6 to 4.1 ms of host time a step -> 1.9, of which the repeated launches take 0.65.)"""
+        from .tape import alike, record
         run(0)                                        # the device has something to do while the layers are compared
         layers = [own(k) for k in range(count)] if self.use_tape and count >= 4 else [None]
-        like = None if any(layer is None for layer in layers) else signature(*layers[0])
-        if like is None or any(signature(*layer) != like for layer in layers):
+        addresses = None if any(layer is None for layer in layers) else alike(layers)
+        if addresses is None:
             for k in range(1, count):
                 run(k)
             return
-        replay = record(self, lambda: run(1), layers[1][0])
+        replay = record(self, lambda: run(1), layers[1])
         if replay is None:
             for k in range(2, count):
                 run(k)
             return
-        failed = replay([tensors for tensors, _ in layers[2:]])
+        failed = replay(addresses[2:])
         if failed is not None:
             raise KernelError(failed.ti_last_error().decode("utf-8", "replace"))
 

@@ -9,7 +9,7 @@ replaced.  The first layer is not the one recorded because it has no layer in fr
 
 What makes a recording valid: every launch went through an entry point that has a taped form (else the number of launches and
 of recorded calls differ), no torch operation but allocations and views took place, nothing is held back at the layer's end
-that was not held back at its start, and the layers agree in everything that their launches may depend on (``own_state`` of
+that was not held back at its start, and the layers agree in everything that their launches may depend on (``own_layout`` of
 parts/base.py) but the contents of their tensors, whose addresses, and those inside them, are replaced.  A recording
 lives for one pass and holds the tensors allocated under it until the pass has issued its last launch.
 """
@@ -72,9 +72,23 @@ def _slot(kind, value) -> int:
     return (0 if value is None else int(value)) & 0xFFFFFFFFFFFFFFFF
 
 
-def signature(tensors, others) -> tuple:
-    """What two layers must agree in for one layer's launches to serve the other: all but what their tensors hold."""
-    return [(t.dtype, t.shape, t.stride(), t.data_ptr() % 32, getattr(t, "_ti_interleaved", None)) for t in tensors], others
+def alike(layers):
+    """The addresses of the layers' own tensors, a list a layer; None: the tensors differ in something that launches depend on
+    (or are none)."""
+    try:
+        like = [(t.dtype, t.shape, t.stride(), t.is_contiguous(), t.data_ptr() % 32, getattr(t, "_ti_interleaved", None))
+                for t in layers[0]]
+        addresses = [[t.data_ptr() for t in layer] for layer in layers]
+        for layer, mine in zip(layers[1:], addresses[1:]):
+            if len(mine) != len(like):
+                return None
+            for t, at, (dtype, shape, strides, dense, place, interleaved) in zip(layer, mine, like):
+                if (t.dtype is not dtype or at % 32 != place or t.shape != shape or t.is_contiguous() is not dense
+                        or (not dense and t.stride() != strides) or getattr(t, "_ti_interleaved", None) is not interleaved):
+                    return None
+    except AttributeError:
+        return None
+    return addresses
 
 
 def _inside(spans, value):
@@ -86,8 +100,8 @@ def _inside(spans, value):
 
 
 def record(ops, run, mine):
-    """Runs one layer through ``run()`` and returns its launches as ``replay(layers)``, which takes the own tensors of each
-    layer to repeat them for (in the order of ``mine``, this layer's); None if they cannot be repeated."""
+    """Runs one layer through ``run()`` and returns its launches as ``replay(layers)``, which takes the addresses of the own
+    tensors of each layer to repeat them for (in the order of ``mine``, this layer's); None if they cannot be repeated."""
     calls: list = []
     start = ops._pending_runs
     had_more = ops._pending is not None or ops._pending_pair is not None
@@ -137,7 +151,7 @@ def record(ops, run, mine):
               (ctypes.c_ulonglong * max(1, len(slots)))(*slots), (ctypes.c_int * max(1, len(patches)))(*patches), len(patches))
 
     def replay(layers):
-        values = [own[i] + offset for own in ([t.data_ptr() for t in layer] for layer in layers) for i, offset in sources]
+        values = [own[i] + offset for own in layers for i, offset in sources]
         rc = ops.core.ti_tape_run(*packed, (ctypes.c_ulonglong * max(1, len(values)))(*values), len(layers))
         ops.launches += n * len(layers)
         ops.issued += n * len(layers)

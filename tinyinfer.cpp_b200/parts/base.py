@@ -27,6 +27,7 @@ float32); ``residual``/``x`` is the float32 residual stream ``[T, hidden]``.
 from __future__ import annotations
 
 from dataclasses import dataclass
+from operator import itemgetter
 from typing import Any, Callable, Mapping, Optional
 
 import torch
@@ -113,7 +114,7 @@ class Part:
     takes_factor = False
     # every launch of the part goes through the kernel set's entry points and depends on the step, the cache view and the
     # part's own attributes alone, and those are numbers, texts, tensors and parts of which the same holds: alike layers of
-    # such parts may repeat one another's launches (``own_state``).  A class says so for itself alone: what is derived from
+    # such parts may repeat one another's launches (``own_layout``).  A class says so for itself alone: what is derived from
     # it may read more, so it has to say it again.
     launches_repeat = False
 
@@ -136,21 +137,49 @@ class Part:
 _PLAIN = frozenset((bool, int, float, str, type(None), torch.dtype))
 
 
-def own_state(part: Part, tensors: list, others: list) -> bool:
-    """Appends the tensors that the part and the parts inside it hold, and all else that tells it from another part (classes,
-    attributes' names, numbers).  Launches of two parts whose lists agree differ by the tensors alone.  False: not known, for
-    a part whose class does not say ``launches_repeat`` or that holds anything else (a function in the place of a method)."""
-    cls, held = type(part), vars(part)
-    if cls.__dict__.get("launches_repeat") is not True:
+def _values(names):
+    """Reads the attributes of these names out of a part's dictionary, as a tuple (None: there are none)."""
+    if len(names) == 1:
+        return lambda held, get=itemgetter(*names): (get(held),)
+    return itemgetter(*names) if names else None
+
+
+def own_layout(part: Part):
+    """What another part has to share with this one for its launches to differ by the tensors it holds alone: the class, and
+    every attribute but the contents of tensors, in the parts inside it too.  None: not known, for a part whose class does not
+    say ``launches_repeat`` or that holds anything but numbers, texts, tensors and such parts (a function in the place of a
+    method).  A list with an entry per part: where it is found, its class, and how to read and compare its attributes."""
+    layout, found = [], [(0, None, part)]
+    for at, (parent, name, p) in enumerate(found):
+        held = vars(p)
+        if type(p).__dict__.get("launches_repeat") is not True:
+            return None
+        plain = [n for n, v in held.items() if type(v) in _PLAIN]
+        tensors = [n for n, v in held.items() if type(v) is torch.Tensor]
+        inner = [(at, n, v) for n, v in held.items() if isinstance(v, Part)]
+        if len(plain) + len(tensors) + len(inner) != len(held):
+            return None
+        found += inner
+        read = _values(plain)
+        layout.append((parent, name, type(p), len(held), read, read and read(held), _values(tensors)))
+    return layout
+
+
+def own_tensors(part: Part, layout, into: list) -> bool:
+    """Appends what the part and the parts inside it hold in the places of the layout's tensors; False: the part differs from
+    the layout in anything else."""
+    found = []
+    try:
+        for parent, name, cls, count, read, values, tensors in layout:
+            p = part if name is None else found[parent][name]
+            held = p.__dict__
+            if type(p) is not cls or len(held) != count or (read is not None and read(held) != values):
+                return False
+            found.append(held)
+            if tensors is not None:
+                into += tensors(held)
+    except (KeyError, AttributeError):
         return False
-    others.append((cls, *held))
-    for value in held.values():
-        if type(value) in _PLAIN:
-            others.append(value)
-        elif type(value) is torch.Tensor:
-            tensors.append(value)
-        elif not isinstance(value, Part) or not own_state(value, tensors, others):
-            return False
     return True
 
 

@@ -12,7 +12,7 @@ from typing import Callable, Mapping
 import torch
 
 from ..config.plan import ModelPlan
-from .base import FixedStateSpec, PagedKVSpec, Part, WeightSpec, build_part, own_state
+from .base import FixedStateSpec, PagedKVSpec, Part, WeightSpec, build_part, own_layout, own_tensors
 
 
 class CausalLM:
@@ -144,12 +144,16 @@ class CausalLM:
             count = self._alike[at] if hasattr(ops, "repeat_layers") else 1
             parts = [(self.blocks[e.layer], cache_views[(e.cache_slot, e.writes_cache)]) for e in schedule[at:at + count]]
 
+            layout = []
+
             def own(k):
-                mine, others, view = [], [], parts[k][1]
+                mine, view = [], parts[k][1]
                 pages, first = getattr(view, "pages", None), parts[0][1]      # one kind of pages, by one block table
                 if pages is None or view.block_table is not getattr(first, "block_table", None):
                     return None
-                return (mine + [pages], others) if own_state(parts[k][0], mine, others) else None
+                if not layout:
+                    layout.append(own_layout(parts[0][0]))
+                return mine + [pages] if layout[0] and own_tensors(parts[k][0], layout[0], mine) else None
 
             def run(k):
                 parts[k][0].forward(ops, x, step, parts[k][1])
