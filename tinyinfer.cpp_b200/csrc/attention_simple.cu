@@ -412,168 +412,164 @@ paged_attention_simple_kernel(const TQ* q, const int* __restrict__ rows, const i
     }
 }
 
-// The same for ROWS consecutive tokens a block (no window): a key and its value are read once for all of them, which is what
-// bounds many rows (466 tokens of three prompts, 16 heads of 128: 600 MB from L2, 122 us a layer -> 65).  A row takes the
-// same keys in the same order through the same arithmetic as above, so its bits are those of the kernel above: the sums over
-// the lanes are the same tree, folded for all rows at once (a lane is left with the score of row lane / 4, whose maximum, sum
-// and exponentials it keeps and hands out).
+// The same for up to ROWS consecutive tokens of one request a block (no window): a key and its value are read once for all of
+// them, which is what bounds many rows (466 tokens of three prompts, 16 heads of 128: 600 MB from L2, 122 us a layer -> 65).
+// A row takes the same keys in the same order through the same arithmetic as above, so its bits are those of the kernel above:
+// the sums over the lanes are the same tree, folded for all rows at once (a lane is left with the score of row lane / 4, whose
+// maximum, sum and exponentials it keeps and hands out).  All ROWS scores are made for every key, so rows of different
+// requests gain nothing from one block: 80 single tokens at 1,000 keys walked eight to a block 810 us, by the kernel above 244.
+// tiles[i] = {request row, first flat token, tokens}; blockIdx.z counts a tile's runs of ROWS tokens.
 constexpr int ROWS = 8, ROW_LANES = 32 / ROWS;
 
 template <typename TQ, typename TC, int PER_LANE>
 __global__ void __launch_bounds__(ATT_WARPS * 32, PER_LANE <= 4 ? 2 : 1)
-paged_attention_rows_kernel(const TQ* q, const int* __restrict__ positions, const int* __restrict__ req_of_tok,
+paged_attention_rows_kernel(const TQ* q, const int* __restrict__ tiles, const int* __restrict__ positions,
                             const int* __restrict__ block_table, int bt_stride, const TC* pages, int num_pages, int page_size,
-                            int num_tokens, int num_heads, int num_kv_heads, int head_dim, float scale, TQ* out,
-                            int* __restrict__ status) {
+                            int num_heads, int num_kv_heads, int head_dim, float scale, TQ* out, int* __restrict__ status) {
     __shared__ float so[ATT_WARPS][ROWS / 2][32 * PER_LANE];
     __shared__ float sm[ATT_WARPS][ROWS], sl[ATT_WARPS][ROWS];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int h = blockIdx.y, t0 = blockIdx.x * ROWS, count = min(ROWS, num_tokens - t0);
+    const int* tile = tiles + 3 * blockIdx.x;
+    const int h = blockIdx.y, t0 = tile[1] + ROWS * blockIdx.z, count = min(ROWS, tile[2] - ROWS * (int)blockIdx.z);
+    if (count <= 0) return;
     const int kvh = h / (num_heads / num_kv_heads);
     pdl_launch();
     pdl_wait();
     const size_t to_values = (size_t)num_kv_heads * page_size * head_dim;
     bool bad = false;
-    for (int first = 0; first < count;) {                // the tokens of one request after the other
-        const int r = req_of_tok[t0 + first];
-        int behind = first + 1;
-        while (behind < count && req_of_tok[t0 + behind] == r) ++behind;
-        const int* table = block_table + (size_t)r * bt_stride;
-        const int own = lane / ROW_LANES, n = behind - first;   // this lane's row of the run
-        int pos[ROWS], last = 0, least = 1 << 30;
-        float qv[ROWS][PER_LANE], o[ROWS][PER_LANE];
+    const int* table = block_table + (size_t)tile[0] * bt_stride;
+    const int own = lane / ROW_LANES;                        // this lane's row
+    int pos[ROWS], last = 0, least = 1 << 30;
+    float qv[ROWS][PER_LANE], o[ROWS][PER_LANE];
+#pragma unroll
+    for (int j = 0; j < ROWS; ++j) {
+        const int t = t0 + j;
+        pos[j] = j < count ? positions[t] : -1;
+        last = max(last, pos[j]);
+        least = j < count ? min(least, pos[j]) : least;
+#pragma unroll
+        for (int i = 0; i < PER_LANE; ++i) {
+            const int d = lane + 32 * i;
+            qv[j][i] = j < count && d < head_dim ? to_f32(q[((size_t)t * num_heads + h) * head_dim + d]) : 0.0f;
+            o[j][i] = 0.0f;
+        }
+    }
+    int my_pos = -1;
+#pragma unroll
+    for (int j = 0; j < ROWS; ++j) my_pos = own == j ? pos[j] : my_pos;
+    float m = -INFINITY, l = 0.0f;                   // of row `own`
+    constexpr int DEEP = 2;                          // keys of this warp on their way
+    TC kn[DEEP][PER_LANE], vn[DEEP][PER_LANE];
+    bool there_next[DEEP];
+    // the keys of a warp follow one another: the page is looked up where it changes, and nothing is divided
+    int block = warp / page_size, slot = warp - block * page_size, page = -1;
+    const TC* base = pages;
+    auto turn_page = [&]() {
+        page = block * page_size <= last ? table[block] : -1;
+        base = pages + ((size_t)(page >= 0 && page < num_pages ? page : 0) * 2 * num_kv_heads + kvh) * page_size * head_dim;
+    };
+    turn_page();
+    auto fetch = [&](int p, TC (&kn)[PER_LANE], TC (&vn)[PER_LANE], bool& there) {
+        if (p > last) return;
+        there = page >= 0 && page < num_pages;
+        const TC* kp = base + (size_t)slot * head_dim;
+#pragma unroll
+        for (int i = 0; i < PER_LANE; ++i) {
+            const int d = lane + 32 * i;
+            const bool on = there && d < head_dim;
+            kn[i] = on ? kp[d] : from_f32<TC>(0.0f);
+            vn[i] = on ? kp[to_values + d] : from_f32<TC>(0.0f);
+        }
+        slot += ATT_WARPS;
+        if (slot >= page_size) {
+            do { slot -= page_size; ++block; } while (slot >= page_size);
+            turn_page();
+        }
+    };
+    auto take = [&](int p, TC (&kn)[PER_LANE], TC (&vn)[PER_LANE], bool& there_then) {
+        float kf[PER_LANE], vf[PER_LANE];
+#pragma unroll
+        for (int i = 0; i < PER_LANE; ++i) { kf[i] = to_f32(kn[i]); vf[i] = to_f32(vn[i]); }
+        const bool there = there_then;
+        fetch(p + DEEP * ATT_WARPS, kn, vn, there_then);
+        if (!there) { bad = true; return; }
+        float s[ROWS];
 #pragma unroll
         for (int j = 0; j < ROWS; ++j) {
-            const int t = t0 + first + j;
-            pos[j] = j < n ? positions[t] : -1;
-            last = max(last, pos[j]);
-            least = j < n ? min(least, pos[j]) : least;
+            s[j] = 0.0f;
 #pragma unroll
-            for (int i = 0; i < PER_LANE; ++i) {
-                const int d = lane + 32 * i;
-                qv[j][i] = j < n && d < head_dim ? to_f32(q[((size_t)t * num_heads + h) * head_dim + d]) : 0.0f;
-                o[j][i] = 0.0f;
+            for (int i = 0; i < PER_LANE; ++i) s[j] = fmaf(qv[j][i], kf[i], s[j]);
+        }
+        // sums over the lanes: a lane keeps half of its rows at each exchange until it has one
+#pragma unroll
+        for (int half = ROWS / 2, x = 16; half >= 1; half >>= 1, x >>= 1) {
+            const bool upper = lane & x;
+#pragma unroll
+            for (int j = 0; j < half; ++j) {
+                const float keep = upper ? s[j + half] : s[j], give = upper ? s[j] : s[j + half];
+                s[j] = keep + __shfl_xor_sync(0xffffffffu, give, x);
             }
         }
-        int my_pos = -1;
 #pragma unroll
-        for (int j = 0; j < ROWS; ++j) my_pos = own == j ? pos[j] : my_pos;
-        float m = -INFINITY, l = 0.0f;                   // of row `own`
-        constexpr int DEEP = 2;                          // keys of this warp on their way
-        TC kn[DEEP][PER_LANE], vn[DEEP][PER_LANE];
-        bool there_next[DEEP];
-        // the keys of a warp follow one another: the page is looked up where it changes, and nothing is divided
-        int block = warp / page_size, slot = warp - block * page_size, page = -1;
-        const TC* base = pages;
-        auto turn_page = [&]() {
-            page = block * page_size <= last ? table[block] : -1;
-            base = pages + ((size_t)(page >= 0 && page < num_pages ? page : 0) * 2 * num_kv_heads + kvh) * page_size * head_dim;
-        };
-        turn_page();
-        auto fetch = [&](int p, TC (&kn)[PER_LANE], TC (&vn)[PER_LANE], bool& there) {
-            if (p > last) return;
-            there = page >= 0 && page < num_pages;
-            const TC* kp = base + (size_t)slot * head_dim;
-#pragma unroll
-            for (int i = 0; i < PER_LANE; ++i) {
-                const int d = lane + 32 * i;
-                const bool on = there && d < head_dim;
-                kn[i] = on ? kp[d] : from_f32<TC>(0.0f);
-                vn[i] = on ? kp[to_values + d] : from_f32<TC>(0.0f);
-            }
-            slot += ATT_WARPS;
-            if (slot >= page_size) {
-                do { slot -= page_size; ++block; } while (slot >= page_size);
-                turn_page();
-            }
-        };
-        auto take = [&](int p, TC (&kn)[PER_LANE], TC (&vn)[PER_LANE], bool& there_then) {
-            float kf[PER_LANE], vf[PER_LANE];
-#pragma unroll
-            for (int i = 0; i < PER_LANE; ++i) { kf[i] = to_f32(kn[i]); vf[i] = to_f32(vn[i]); }
-            const bool there = there_then;
-            fetch(p + DEEP * ATT_WARPS, kn, vn, there_then);
-            if (!there) { bad = true; return; }
-            float s[ROWS];
+        for (int x = ROW_LANES / 2; x >= 1; x >>= 1) s[0] += __shfl_xor_sync(0xffffffffu, s[0], x);
+        float alpha = 1.0f, pr = 0.0f;
+        const bool sees = p <= my_pos;
+        if (sees) {
+            const float sc = s[0] * scale, m_new = fmaxf(m, sc);
+            alpha = expf(m - m_new);                 // exp(-inf) = 0 on the first key
+            pr = expf(sc - m_new);
+            l = l * alpha + pr;
+            m = m_new;
+        }
+        if (p <= least && !__any_sync(0xffffffffu, alpha != 1.0f)) {     // every row sees it, no maximum moved
 #pragma unroll
             for (int j = 0; j < ROWS; ++j) {
-                s[j] = 0.0f;
+                const float w = __shfl_sync(0xffffffffu, pr, ROW_LANES * j);
 #pragma unroll
-                for (int i = 0; i < PER_LANE; ++i) s[j] = fmaf(qv[j][i], kf[i], s[j]);
+                for (int i = 0; i < PER_LANE; ++i) o[j][i] = fmaf(w, vf[i], o[j][i]);
             }
-            // sums over the lanes: a lane keeps half of its rows at each exchange until it has one
-#pragma unroll
-            for (int half = ROWS / 2, x = 16; half >= 1; half >>= 1, x >>= 1) {
-                const bool upper = lane & x;
-#pragma unroll
-                for (int j = 0; j < half; ++j) {
-                    const float keep = upper ? s[j + half] : s[j], give = upper ? s[j] : s[j + half];
-                    s[j] = keep + __shfl_xor_sync(0xffffffffu, give, x);
-                }
-            }
-#pragma unroll
-            for (int x = ROW_LANES / 2; x >= 1; x >>= 1) s[0] += __shfl_xor_sync(0xffffffffu, s[0], x);
-            float alpha = 1.0f, pr = 0.0f;
-            const bool sees = p <= my_pos;
-            if (sees) {
-                const float sc = s[0] * scale, m_new = fmaxf(m, sc);
-                alpha = expf(m - m_new);                 // exp(-inf) = 0 on the first key
-                pr = expf(sc - m_new);
-                l = l * alpha + pr;
-                m = m_new;
-            }
-            if (p <= least && !__any_sync(0xffffffffu, alpha != 1.0f)) {     // every row sees it, no maximum moved
-#pragma unroll
-                for (int j = 0; j < ROWS; ++j) {
-                    const float w = __shfl_sync(0xffffffffu, pr, ROW_LANES * j);
-#pragma unroll
-                    for (int i = 0; i < PER_LANE; ++i) o[j][i] = fmaf(w, vf[i], o[j][i]);
-                }
-                return;
-            }
-#pragma unroll
-            for (int j = 0; j < ROWS; ++j) {
-                const float a = __shfl_sync(0xffffffffu, alpha, ROW_LANES * j), w = __shfl_sync(0xffffffffu, pr, ROW_LANES * j);
-                if (p > pos[j]) continue;
-#pragma unroll
-                for (int i = 0; i < PER_LANE; ++i) o[j][i] = fmaf(w, vf[i], o[j][i] * a);
-            }
-        };
-#pragma unroll
-        for (int d = 0; d < DEEP; ++d) fetch(warp + d * ATT_WARPS, kn[d], vn[d], there_next[d]);
-        for (int p = warp; p <= last; p += DEEP * ATT_WARPS) {
-#pragma unroll
-            for (int d = 0; d < DEEP; ++d)
-                if (p + d * ATT_WARPS <= last) take(p + d * ATT_WARPS, kn[d], vn[d], there_next[d]);
+            return;
         }
-        if (lane % ROW_LANES == 0) { sm[warp][own] = m; sl[warp][own] = l; }
 #pragma unroll
-        for (int part = 0; part < 2; ++part) {           // half of the rows at a time meet in shared memory
-            __syncthreads();
+        for (int j = 0; j < ROWS; ++j) {
+            const float a = __shfl_sync(0xffffffffu, alpha, ROW_LANES * j), w = __shfl_sync(0xffffffffu, pr, ROW_LANES * j);
+            if (p > pos[j]) continue;
 #pragma unroll
-            for (int j = 0; j < ROWS / 2; ++j)
-#pragma unroll
-                for (int i = 0; i < PER_LANE; ++i) so[warp][j][lane + 32 * i] = o[part * (ROWS / 2) + j][i];
-            __syncthreads();
-            for (int e = threadIdx.x; e < ROWS / 2 * 32 * PER_LANE; e += ATT_WARPS * 32) {
-                const int j = e / (32 * PER_LANE), d = e % (32 * PER_LANE), row = part * (ROWS / 2) + j;
-                if (row >= n || d >= head_dim) continue;
-                float mm = -INFINITY;
-#pragma unroll
-                for (int w = 0; w < ATT_WARPS; ++w) mm = fmaxf(mm, sm[w][row]);
-                float ltot = 0.0f, acc = 0.0f;
-#pragma unroll
-                for (int w = 0; w < ATT_WARPS; ++w) {
-                    const float wt = sl[w][row] > 0.0f ? expf(sm[w][row] - mm) : 0.0f;
-                    ltot += sl[w][row] * wt;
-                    acc = fmaf(so[w][j][d], wt, acc);
-                }
-                const float inv = 1.0f / ltot;
-                out[((size_t)(t0 + first + row) * num_heads + h) * head_dim + d] = from_f32<TQ>(acc * inv);
-            }
+            for (int i = 0; i < PER_LANE; ++i) o[j][i] = fmaf(w, vf[i], o[j][i] * a);
         }
-        first = behind;
-        if (first < count) __syncthreads();              // the next run's rows take the places of these
+    };
+#pragma unroll
+    for (int d = 0; d < DEEP; ++d) fetch(warp + d * ATT_WARPS, kn[d], vn[d], there_next[d]);
+    for (int p = warp; p <= last; p += DEEP * ATT_WARPS) {
+#pragma unroll
+        for (int d = 0; d < DEEP; ++d)
+            if (p + d * ATT_WARPS <= last) take(p + d * ATT_WARPS, kn[d], vn[d], there_next[d]);
+    }
+    if (lane % ROW_LANES == 0) { sm[warp][own] = m; sl[warp][own] = l; }
+#pragma unroll
+    for (int part = 0; part < 2; ++part) {           // half of the rows at a time meet in shared memory
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < ROWS / 2; ++j)
+#pragma unroll
+            for (int i = 0; i < PER_LANE; ++i) so[warp][j][lane + 32 * i] = o[part * (ROWS / 2) + j][i];
+        __syncthreads();
+        for (int e = threadIdx.x; e < ROWS / 2 * 32 * PER_LANE; e += ATT_WARPS * 32) {
+            const int j = e / (32 * PER_LANE), d = e % (32 * PER_LANE), row = part * (ROWS / 2) + j;
+            if (row >= count || d >= head_dim) continue;
+            float mm = -INFINITY;
+#pragma unroll
+            for (int w = 0; w < ATT_WARPS; ++w) mm = fmaxf(mm, sm[w][row]);
+            float ltot = 0.0f, acc = 0.0f;
+#pragma unroll
+            for (int w = 0; w < ATT_WARPS; ++w) {
+                const float wt = sl[w][row] > 0.0f ? expf(sm[w][row] - mm) : 0.0f;
+                ltot += sl[w][row] * wt;
+                acc = fmaf(so[w][j][d], wt, acc);
+            }
+            const float inv = 1.0f / ltot;
+            out[((size_t)(t0 + row) * num_heads + h) * head_dim + d] = from_f32<TQ>(acc * inv);
+        }
     }
     if (bad && lane == 0) atomicCAS(status, 0, TI_ERR_BAD_PAGE);
 }
@@ -665,21 +661,14 @@ extern "C" int ti_paged_attention_simple(const void* q, int q_dtype, const int* 
     cudaGetDevice(&device);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     const long long blocks = (long long)num_rows * num_heads;
-    // several tokens a block where that leaves every SM one, and no list picks rows out of the step's
-    const bool many = rows == nullptr && window == 0 && blocks >= (long long)ROWS * sms;
     const int per_lane = head_dim <= 32 ? 1 : head_dim <= 64 ? 2 : head_dim <= 128 ? 4 : 8;
 #define LAUNCH(TQ, TC, N, A)                                                                    \
     ti_launch_pdl(paged_attention_simple_kernel<TQ, TC, N, A>, grid, dim3(ATT_WARPS * 32), 0, s, \
         (const TQ*)q, rows, positions, req_of_tok, block_table, bt_stride, (const TC*)pages,     \
         num_pages, page_size, num_heads, num_kv_heads, head_dim, window, scale, (TQ*)out, status)
-#define MANY(TQ, TC, N)                                                                         \
-    ti_launch_pdl(paged_attention_rows_kernel<TQ, TC, N>, dim3((num_rows + ROWS - 1) / ROWS, num_heads), \
-        dim3(ATT_WARPS * 32), 0, s, (const TQ*)q, positions, req_of_tok, block_table, bt_stride,  \
-        (const TC*)pages, num_pages, page_size, num_rows, num_heads, num_kv_heads, head_dim, scale, (TQ*)out, status)
 #define PICK(TQ, TC, N)                                                                         \
     {                                                                                           \
-        if (many) MANY(TQ, TC, N);                                                               \
-        else if (blocks <= sms) LAUNCH(TQ, TC, N, 8);                                            \
+        if (blocks <= sms) LAUNCH(TQ, TC, N, 8);                                                 \
         else if (blocks <= 2 * sms) LAUNCH(TQ, TC, N, 4);                                        \
         else LAUNCH(TQ, TC, N, 1);                                                               \
     }
@@ -691,10 +680,39 @@ extern "C" int ti_paged_attention_simple(const void* q, int q_dtype, const int* 
     TI_DISPATCH_QC(q_dtype, cache_dtype, CALL)
 #undef CALL
 #undef PICK
-#undef MANY
 #undef LAUNCH
     return ti_check_launch("paged_attention_simple");
 }
 
+// The tokens of `tiles` (int32 [num_tiles, 3] = {request row, first flat token, at most tile_rows tokens}, consecutive tokens of
+// one request), without a window: the bits of ti_paged_attention_simple.
+extern "C" int ti_paged_attention_portions(const void* q, int q_dtype, const int* tiles, int num_tiles, int tile_rows,
+                                           const int* positions, const int* block_table, int bt_stride, const void* pages,
+                                           int cache_dtype, int num_pages, int page_size, int num_heads, int num_kv_heads,
+                                           int head_dim, float scale, void* out, int* status, void* stream) {
+    if (num_tiles == 0) return 0;
+    TI_REQUIRE(head_dim >= 1 && head_dim <= MAX_HEAD_DIM, "paged_attention: head_dim %d must be at most %d", head_dim,
+               MAX_HEAD_DIM);
+    TI_REQUIRE(num_heads % num_kv_heads == 0, "paged_attention: %d heads over %d kv heads", num_heads, num_kv_heads);
+    TI_REQUIRE(tile_rows >= 1, "paged_attention: tiles of %d rows", tile_rows);
+    const dim3 grid(num_tiles, num_heads, (tile_rows + ROWS - 1) / ROWS);
+    cudaStream_t s = (cudaStream_t)stream;
+    const int per_lane = head_dim <= 32 ? 1 : head_dim <= 64 ? 2 : head_dim <= 128 ? 4 : 8;
+#define LAUNCH(TQ, TC, N)                                                                       \
+    ti_launch_pdl(paged_attention_rows_kernel<TQ, TC, N>, grid, dim3(ATT_WARPS * 32), 0, s, (const TQ*)q, tiles, positions, \
+        block_table, bt_stride, (const TC*)pages, num_pages, page_size, num_heads, num_kv_heads, head_dim, scale, (TQ*)out, \
+        status)
+#define CALL(TQ, TC)                                                                            \
+    if (per_lane == 1) LAUNCH(TQ, TC, 1);                                                        \
+    else if (per_lane == 2) LAUNCH(TQ, TC, 2);                                                   \
+    else if (per_lane == 4) LAUNCH(TQ, TC, 4);                                                   \
+    else LAUNCH(TQ, TC, 8)
+    TI_DISPATCH_QC(q_dtype, cache_dtype, CALL)
+#undef CALL
+#undef LAUNCH
+    return ti_check_launch("paged_attention_portions");
+}
+
 TI_TAPED(ti_qk_norm_rope_store)
 TI_TAPED(ti_paged_attention_simple)
+TI_TAPED(ti_paged_attention_portions)

@@ -45,6 +45,7 @@ from .mixer_ops import MixerOps
 from .state_ops import StateOps
 
 _CODE = {torch.float32: 0, torch.bfloat16: 1}
+PLAIN_TILE = 64              # tokens of a tile of the 32-bit path's portions, whose blocks take eight of them
 _vp = ctypes.c_void_p
 _i = ctypes.c_int
 _f = ctypes.c_float
@@ -241,6 +242,8 @@ class CudaOps(MixerOps, StateOps):
             _vp, _i, _vp, _vp]
         c.ti_paged_attention_simple.argtypes = [
             _vp, _i, _vp, _vp, _vp, _vp, _i, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _f, _vp, _vp, _vp]
+        c.ti_paged_attention_portions.argtypes = [
+            _vp, _i, _vp, _i, _i, _vp, _vp, _i, _vp, _i, _i, _i, _i, _i, _i, _f, _vp, _vp, _vp]
         c.ti_gemm_split_scratch.argtypes = [_i, _i, _i, ctypes.POINTER(ctypes.c_longlong), ctypes.POINTER(ctypes.c_int)]
         c.ti_gemm_split.argtypes = [_vp, _vp, _vp] + [_i] * 7 + [_vp, _vp, _vp, _vp]
         c.ti_sample.argtypes = [_vp, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp]
@@ -353,10 +356,10 @@ class CudaOps(MixerOps, StateOps):
         """The host-built integer lists (``engine.batch.StepList``) that the attention kernels of
         this kernel set want in every step of an engine with activations of ``act_dtype``: the
         single-token rows, the rows of prompt portions, and the portions cut into tiles of each
-        prompt-attention kernel's own height.  The 32-bit kernels need none."""
-        if act_dtype != torch.bfloat16:
-            return []
+        prompt-attention kernel's own height (for the 32-bit path tiles that its blocks walk in pieces)."""
         from .step_lists import attention_lists, option_tile_lists, row_tile_lists
+        if act_dtype != torch.bfloat16:
+            return attention_lists([PLAIN_TILE])
         self.bf16
         # ... and, where a mixer has announced attention with options, every entry cut into tiles
         # of as many tokens as that kernel's blocks take
@@ -1162,12 +1165,36 @@ class CudaOps(MixerOps, StateOps):
             rows, n_rows = single, n_dec
             if n_rows == 0:
                 return
+        if rows is None and win == 0:
+            rows, n_rows = self._portions_share_keys(q, step, cache, out, num_heads, num_kv_heads, head_dim, scale)
+            if n_rows == 0:
+                return
         self._ok(self.core.ti_paged_attention_simple(
             q.data_ptr(), _code(q, "q"), _ptr(rows), step.positions.data_ptr(),
             step.req_of_tok.data_ptr(), bt.data_ptr(), bt.stride(0), pages.data_ptr(),
             _code(pages, "cache"), pages.shape[0], cache.page_size, n_rows, num_heads,
             num_kv_heads, head_dim, win, float(scale), out.data_ptr(), self.status.data_ptr(),
             self._stream()))
+
+    def _portions_share_keys(self, q, step, cache, out, num_heads, num_kv_heads, head_dim, scale):
+        """The plain attention of a step's portions by the kernel whose blocks read a key once for eight tokens of a request,
+        where it pays; returns the rows that are left (None: all) and their number.  It pays from eight tokens a portion on, if
+        that leaves every SM a block.  us against a block per row, 16 heads of 128: portions of 2 (100 requests) 21.5 / 8.6,
+        4 (64) 15.8 / 11.1, 8 (32) 12.7 / 12.7, 16 (64) 46 / 57, 64 (8) 38 / 63, three of 119 to 197 61 / 140."""
+        lists, pages, bt = step.lists, cache.pages, cache.block_table
+        height = self._tile_rows[0] if q.dtype == torch.bfloat16 else PLAIN_TILE
+        tiles, single = lists.get(f"portion_tiles_{height}"), lists.get("single_rows")
+        t = q.shape[0]
+        if tiles is None or single is None:
+            return None, t
+        left = single.shape[0]
+        if t - left < 8 * (bt.shape[0] - left) or (t - left) * num_heads < 8 * self.num_sms:
+            return None, t
+        self._ok(self.core.ti_paged_attention_portions(
+            q.data_ptr(), _code(q, "q"), tiles.data_ptr(), tiles.shape[0], height, step.positions.data_ptr(), bt.data_ptr(),
+            bt.stride(0), pages.data_ptr(), _code(pages, "cache"), pages.shape[0], cache.page_size, num_heads, num_kv_heads,
+            head_dim, float(scale), out.data_ptr(), self.status.data_ptr(), self._stream()))
+        return single, left
 
     # ---- attention with a distance bias, kept first tokens and an output gate ---------------
     def embed_sinusoid(self, table, token_ids, positions, freq, scale, out):
