@@ -1,6 +1,7 @@
 // Paged flash-decoding for single-token rows (bfloat16 cache, head_dim a multiple of 16 up to 128).
 //
-// A row is one new token of a request; it attends to the keys [lo, pos] of its request's
+// A row is one new token of a request, its only one of the step (its other keys are read before the kernels in
+// front have ended); it attends to the keys [lo, pos] of its request's
 // pages (lo > 0 only with a window).  The keys are cut into tiles of 32; the tiles of a row
 // are dealt to `num_splits` blocks per kv head.  A block is ONE warp: it streams its tiles
 // through a ring of shared-memory stages with cp.async, computes the scores of all query

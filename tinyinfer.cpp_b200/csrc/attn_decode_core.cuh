@@ -256,13 +256,15 @@ __device__ __forceinline__ void decode_item(
         // which follows behind the wait (16 heads, 8 kv heads, us a layer at one request of 20 to 256
         // keys 5.9 to 6.1 with that tile behind the wait -> 4.6 to 4.9, eight of 50 to 250 6.4 to 7.2 ->
         // 5.1 to 6.1; letting one block have the two to six tiles of a short row, so that nothing is
-        // merged, takes 5.4 to 10.2).
+        // merged, takes 5.4 to 10.2).  Not where a row is not split (SINGLE): there are blocks enough to
+        // cover the wait, and the code alone cost more than it gave (64 requests, us a step of 28 layers
+        // with / without: 250 keys 2,021 / 2,014, 1,024 keys 2,916 / 2,889, 4,096 keys 6,426 / 6,268).
         const int new_tile = pos / TILE;
         int early = 0, held_stage = -1;
 #pragma unroll
         for (int s = 0; s < STAGES - 1; ++s) {
-            if (PDL && !LATE_WAIT && my_lo + s < my_hi) {
-                const bool own = my_lo + s == new_tile;
+            if (PDL && !LATE_WAIT && my_lo + s < my_hi && (!SINGLE || my_lo + s < new_tile)) {
+                const bool own = !SINGLE && my_lo + s == new_tile;
                 if (own) {
                     issue(my_lo + s, s, Flag<true>{});
                     held_stage = s;
