@@ -126,3 +126,39 @@ def test_short_portions_in_one_tile_of_keys(ops, monkeypatch, heads, kv, size, m
             taken.clear()
             _check(ops, heads, kv, size, size, False, 64, ctx, [tokens, 1], one_tile=one_tile)
             assert bool(taken) == (not one_tile or tokens > most)
+
+
+@pytest.mark.parametrize("heads,kv,size", [(4, 4, 64), (16, 4, 128)])
+def test_tiles_of_one_token_cut_from_a_portion(ops, heads, kv, size):
+    """Such a token's other keys are written by the kernel in front, so a call that does not say ``alone`` reads nothing of them
+    before that kernel has ended; a call that says it with tiles of several tokens is refused."""
+    from tinyinfer_b200.kernels.step_lists import row_tiles
+    page, ctx, n = 64, 300, 200
+    ti = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    positions, table = ti(list(range(ctx - n, ctx))), torch.arange(5, dtype=torch.int32, device=DEV).view(1, 5)
+    step = SimpleNamespace(positions=positions, req_of_tok=ti([0] * n), cu_q=ti([0, n]), num_requests=1, max_q_len=n, scratch={})
+    proj = torch.randn((n, (heads + 2 * kv) * size), device=DEV)
+    rotation = SimpleNamespace(kind="none", rotary_dim=0, inv_freq=None, scale=1.0)
+    wq, wk = torch.ones(heads * size, device=DEV), torch.ones(kv * size, device=DEV)
+    old = torch.randn((5, kv * page * 2 * size), device=DEV).bfloat16()
+    pages, q = old.clone(), torch.empty((n, heads * size), dtype=torch.bfloat16, device=DEV)
+    cache = SimpleNamespace(pages=pages, block_table=table, page_size=page, writes=True)
+    tiles = ti(row_tiles([n], [ctx - n], 1).tolist())
+    part_o, part_ml = torch.empty((n, heads, 2, size), device=DEV), torch.empty((n, heads, 2, 2), device=DEV)
+    lib, outs = ops.mixers_tc, []
+
+    def attend(out, tiles, alone):
+        return lib.ti_attn_options_tc(
+            q.data_ptr(), tiles.data_ptr(), tiles.shape[0], n, positions.data_ptr(), table.data_ptr(), 5, pages.data_ptr(), 5, page,
+            heads, kv, size, size, 0, 0, 0, size ** -0.5, 0.0, None, None, None, 0, 0, 2, part_o.data_ptr(), part_ml.data_ptr(), 1,
+            alone, out.data_ptr(), ops.status.data_ptr(), torch.cuda.current_stream().cuda_stream)
+    for wait in [True] + [False] * 20:
+        pages.copy_(old)
+        ops.qk_rownorm_rope_store(proj, wq, wk, 1e-6, rotation, step, cache, q, heads, kv, size, size)
+        if wait:
+            torch.cuda.synchronize()
+        outs.append(torch.empty_like(q))
+        assert attend(outs[-1], tiles, 0) == 0
+    ops.check_status()
+    assert all(torch.equal(o, outs[0]) for o in outs[1:])
+    assert attend(outs[0], tiles[:n // 2], 1) != 0

@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(WARPS * 32)
 attn_options_tc_kernel(const bf16* q, const int* __restrict__ tiles, const int* __restrict__ positions,
                        const int* __restrict__ block_table, int bt_stride, const bf16* pages, int num_pages,
                        int page_size, int num_heads, int num_kv_heads, int dk, int dv, int gp, int head_blocks,
-                       int nsplit, TcOptions opt, bf16* __restrict__ out, float* __restrict__ part_o,
+                       int nsplit, int alone, TcOptions opt, bf16* __restrict__ out, float* __restrict__ part_o,
                        float* __restrict__ part_ml, int* __restrict__ status) {
     constexpr int NT_O = DVS / 8;
     constexpr bool KS = MODE == 1;
@@ -228,9 +228,9 @@ attn_options_tc_kernel(const bf16* q, const int* __restrict__ tiles, const int* 
     };
 
     if (MODE != 0 && kt_lo < kt_hi) lookup(kt_lo);
-    if (MODE != 0 && ntok == 1) {
-        // a single token: all keys but its own are older than this step, so the first tile is on its way while the
-        // kernels before still run; the own key's row follows behind the wait
+    if (MODE != 0 && alone) {
+        // its request's only token: all keys but its own are older than this step, so the first tile is on its way while
+        // the kernels before still run; the own key's row follows behind the wait
         const bool last = kt_lo < kt_hi && kt_lo == pos_last / BN;
         if (kt_lo < kt_hi) issue(kt_lo, 0, pos_last);
         pdl_wait();
@@ -631,14 +631,16 @@ extern "C" int ti_attn_options_tc_group_rows(int num_heads, int num_kv_heads) {
 // [tokens, heads, nsplit, dv] and [tokens, heads, nsplit, 2] when nsplit > 1.  key_split: every tile has at
 // most 16 rows (tokens x group_rows), and the warps of a block share them and split a tile's keys (1) or,
 // with shared rows, the slices of the value columns (2; every tile is then a single token, and a group of more
-// than 16 heads is spread over blocks of 16).
+// than 16 heads is spread over blocks of 16).  alone, with key_split: every tile is its request's only token of the step, whose
+// other keys no kernel of the step writes; they are then asked for before the wait for the kernels in front.  (A tile of one
+// token may also be cut from a portion, whose keys the kernel in front has just written.)
 extern "C" int ti_attn_options_tc(const void* q, const int* tiles, int num_tiles, int num_tokens,
                                   const int* positions, const int* block_table, int bt_stride, const void* pages,
                                   int num_pages, int page_size, int num_heads, int num_kv_heads, int dk, int dv,
                                   int shared_rows, int window, int chunk, float scale, float softcap,
                                   const float* head_scale, const float* sink, const float* gate, int gate_stride,
                                   int gate_per_head, int nsplit, float* part_o, float* part_ml, int key_split,
-                                  void* out, int* status, void* stream) {
+                                  int alone, void* out, int* status, void* stream) {
     if (num_tiles == 0) return 0;
     TI_REQUIRE(num_heads % num_kv_heads == 0, "attn_options_tc: %d heads over %d kv heads", num_heads, num_kv_heads);
     TI_REQUIRE(ti_attn_options_tc_supported(dk, dv, page_size, shared_rows),
@@ -646,6 +648,7 @@ extern "C" int ti_attn_options_tc(const void* q, const int* tiles, int num_tiles
                "(a multiple of 16) are not supported", dk, dv, page_size);
     TI_REQUIRE(nsplit >= 1 && nsplit <= 64 && (nsplit == 1 || (part_o && part_ml)), "attn_options_tc: runs and scratch");
     TI_REQUIRE(num_tiles <= 65535, "attn_options_tc: %d tiles exceed the grid limit", num_tiles);
+    TI_REQUIRE(!alone || num_tiles == num_tokens, "attn_options_tc: %d tiles for %d tokens that are alone", num_tiles, num_tokens);
     TI_REQUIRE(key_split != 1 || ti_attn_options_tc_group_rows(num_heads, num_kv_heads) <= 16,
                "attn_options_tc: warps split the keys only when a tile has at most 16 rows");
     int gp = ti_attn_options_tc_group_rows(num_heads, num_kv_heads);
@@ -679,7 +682,7 @@ extern "C" int ti_attn_options_tc(const void* q, const int* tiles, int num_tiles
         }                                                                                                 \
         ti_launch_pdl((attn_options_tc_kernel<DVS, MODE>), grid, dim3(WARPS * 32), smem, s,                       \
             (const bf16*)q, tiles, positions, block_table, bt_stride, (const bf16*)pages, num_pages,       \
-            page_size, num_heads, num_kv_heads, dk, dv, gp, head_blocks, nsplit, opt, (bf16*)out, part_o,   \
+            page_size, num_heads, num_kv_heads, dk, dv, gp, head_blocks, nsplit, alone, opt, (bf16*)out, part_o,   \
             part_ml, status);                                                                             \
     }
     switch (dvs) {

@@ -91,7 +91,7 @@ class MixerOps:
             b.ti_head_project_tc_supported.argtypes = [_i, _i, _i, _i]
             b.ti_head_project_tc.argtypes = [_vp, _i, _i, _vp, _i, _i, _vp, _i, _i, _i, _i, _vp]
             b.ti_attn_options_tc.argtypes = [_vp, _vp, _i, _i, _vp, _vp, _i, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _i,
-                                             _f, _f, _vp, _vp, _vp, _i, _i, _i, _vp, _vp, _i, _vp, _vp, _vp]
+                                             _f, _f, _vp, _vp, _vp, _i, _i, _i, _vp, _vp, _i, _i, _vp, _vp, _vp]
             b.ti_attn_options_umma_tokens.argtypes = [_i] * 6
             b.ti_attn_options_umma.argtypes = [_vp, _vp, _i, _i, _vp, _vp, _i, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _i,
                                                _f, _f, _vp, _vp, _vp, _i, _i, _vp, _vp, _vp]
@@ -410,6 +410,7 @@ class MixerOps:
             # count depends on the step's shape and the model's bounds alone
             nsplit, part_o, part_ml = 1, None, None
             slices = dv // (128 if dv % 128 == 0 else 64 if dv % 64 == 0 else 32 if dv % 32 == 0 else 16)
+            # every token its request's only one of the step: its other keys are older, and the kernel may read them early
             single = getattr(step, "max_q_len", 0) == 1
             # single tokens of few heads: the warps of a block share the rows and split the keys (1) or,
             # over shared rows, the slices of the value columns (2)
@@ -437,7 +438,7 @@ class MixerOps:
                 int(bool(shared_rows)), int(window or 0), int(chunk or 0), float(scale), float(softcap or 0.0),
                 _ptr(head_scale), _ptr(sink), _ptr(gate), gate.stride(0) if gate is not None else 0,
                 int(bool(gate_per_head)), nsplit, _ptr(part_o), _ptr(part_ml),
-                mode, out.data_ptr(),
+                mode, int(single), out.data_ptr(),
                 self.status.data_ptr(), self._stream()), self.mixers_tc)
             return
         self._mx(self.mixers.ti_attention_options(
