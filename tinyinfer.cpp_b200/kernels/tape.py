@@ -17,9 +17,12 @@ from __future__ import annotations
 
 import ctypes
 import struct
+from bisect import bisect
 
 import torch
 from torch.overrides import TorchFunctionMode
+
+_LAST = 1 << 64
 
 # what a layer may ask of a tensor, and views of it: nothing of these runs on the device
 _QUESTIONS = {"data_ptr", "stride", "is_contiguous", "numel", "size", "dim", "element_size", "__get__", "__len__", "__hash__",
@@ -91,12 +94,11 @@ def alike(layers):
     return addresses
 
 
-def _inside(spans, value):
-    """(index, offset) of the tensor that the address lies in, behind its start; None: in none of them."""
-    for i, (start, end) in enumerate(spans):
-        if start < value < end:
-            return i, value - start
-    return None
+def _inside(in_order, value):
+    """(index, offset) of the tensor that the address lies in; None: in none of them."""
+    at = bisect(in_order, (value, _LAST, 0)) - 1
+    start, end, i = in_order[at]
+    return (i, value - start) if at >= 0 and value < end else None
 
 
 def record(ops, run, mine):
@@ -126,12 +128,14 @@ def record(ops, run, mine):
         if start[1:2] != end[1:2] or start[2] is not end[2] or start[3] != end[3]:
             return None
         renamed[start[0].data_ptr()] = end[0].data_ptr()
-    spans = [(t.data_ptr(), t.data_ptr() + t.element_size() * (1 + sum((n - 1) * s for n, s in zip(t.shape, t.stride()))))
-             for t in mine]
-    in_order = sorted(spans)
+    in_order = []
+    for i, t in enumerate(mine):
+        n = t.numel() if t.is_contiguous() else 1 + sum((n - 1) * s for n, s in zip(t.shape, t.stride()))
+        in_order.append((t.data_ptr(), t.data_ptr() + t.element_size() * n, i))
+    in_order.sort()
     if any(after[0] < before[1] for before, after in zip(in_order, in_order[1:])):
         return None                        # an address may stand for either of two tensors
-    place = {first: (i, 0) for i, (first, _) in enumerate(spans)}
+    place = {}
     first, slots, patches, sources = [], [], [], []
     for _, _, kinds, args in calls:
         if kinds is None or len(kinds) != len(args):
@@ -140,7 +144,7 @@ def record(ops, run, mine):
         for kind, value in zip(kinds, args):
             if kind is ctypes.c_void_p and value:
                 if value not in place:
-                    place[value] = _inside(spans, value)
+                    place[value] = _inside(in_order, value)
                 if place[value] is not None:
                     patches.append(len(slots))
                     sources.append(place[value])
