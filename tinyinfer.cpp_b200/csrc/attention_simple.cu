@@ -418,19 +418,23 @@ paged_attention_simple_kernel(const TQ* q, const int* __restrict__ rows, const i
 // the sums over the lanes are the same tree, folded for all rows at once (a lane is left with the score of row lane / 4, whose
 // maximum, sum and exponentials it keeps and hands out).  All ROWS scores are made for every key, so rows of different
 // requests gain nothing from one block: 80 single tokens at 1,000 keys walked eight to a block 810 us, by the kernel above 244.
-// tiles[i] = {request row, first flat token, tokens}; blockIdx.z counts a tile's runs of ROWS tokens.
+// tiles[i] = {request row, first flat token, tokens}, of at most runs * ROWS tokens.  The grid has the heads of a run beside one
+// another and a tile's last tokens first, so that the blocks with the most keys come first (466 tokens of three prompts 52 to
+// 61 us; a tile of 64 tokens with its runs last in the grid 73).
 constexpr int ROWS = 8, ROW_LANES = 32 / ROWS;
 
 template <typename TQ, typename TC, int PER_LANE>
 __global__ void __launch_bounds__(ATT_WARPS * 32, PER_LANE <= 4 ? 2 : 1)
-paged_attention_rows_kernel(const TQ* q, const int* __restrict__ tiles, const int* __restrict__ positions,
+paged_attention_rows_kernel(const TQ* q, const int* __restrict__ tiles, int runs, const int* __restrict__ positions,
                             const int* __restrict__ block_table, int bt_stride, const TC* pages, int num_pages, int page_size,
                             int num_heads, int num_kv_heads, int head_dim, float scale, TQ* out, int* __restrict__ status) {
     __shared__ float so[ATT_WARPS][ROWS / 2][32 * PER_LANE];
     __shared__ float sm[ATT_WARPS][ROWS], sl[ATT_WARPS][ROWS];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int* tile = tiles + 3 * blockIdx.x;
-    const int h = blockIdx.y, t0 = tile[1] + ROWS * blockIdx.z, count = min(ROWS, tile[2] - ROWS * (int)blockIdx.z);
+    const int run = blockIdx.x / num_heads, h = blockIdx.x - run * num_heads;
+    const int* tile = tiles + 3 * (run / runs);
+    const int first = ROWS * (runs - 1 - run % runs), t0 = tile[1] + first;
+    const int count = min(ROWS, tile[2] - first);
     if (count <= 0) return;
     const int kvh = h / (num_heads / num_kv_heads);
     pdl_launch();
@@ -695,11 +699,12 @@ extern "C" int ti_paged_attention_portions(const void* q, int q_dtype, const int
                MAX_HEAD_DIM);
     TI_REQUIRE(num_heads % num_kv_heads == 0, "paged_attention: %d heads over %d kv heads", num_heads, num_kv_heads);
     TI_REQUIRE(tile_rows >= 1, "paged_attention: tiles of %d rows", tile_rows);
-    const dim3 grid(num_tiles, num_heads, (tile_rows + ROWS - 1) / ROWS);
+    const int runs = (tile_rows + ROWS - 1) / ROWS;
+    const dim3 grid((unsigned)num_heads * num_tiles * runs);
     cudaStream_t s = (cudaStream_t)stream;
     const int per_lane = head_dim <= 32 ? 1 : head_dim <= 64 ? 2 : head_dim <= 128 ? 4 : 8;
 #define LAUNCH(TQ, TC, N)                                                                       \
-    ti_launch_pdl(paged_attention_rows_kernel<TQ, TC, N>, grid, dim3(ATT_WARPS * 32), 0, s, (const TQ*)q, tiles, positions, \
+    ti_launch_pdl(paged_attention_rows_kernel<TQ, TC, N>, grid, dim3(ATT_WARPS * 32), 0, s, (const TQ*)q, tiles, runs, positions, \
         block_table, bt_stride, (const TC*)pages, num_pages, page_size, num_heads, num_kv_heads, head_dim, scale, (TQ*)out, \
         status)
 #define CALL(TQ, TC)                                                                            \

@@ -45,7 +45,7 @@ from .mixer_ops import MixerOps
 from .state_ops import StateOps
 
 _CODE = {torch.float32: 0, torch.bfloat16: 1}
-PLAIN_TILE = 64              # tokens of a tile of the 32-bit path's portions, whose blocks take eight of them
+PLAIN_RUN = 8                # tokens of a portion that a block of the 32-bit path's attention takes
 _vp = ctypes.c_void_p
 _i = ctypes.c_int
 _f = ctypes.c_float
@@ -356,10 +356,10 @@ class CudaOps(MixerOps, StateOps):
         """The host-built integer lists (``engine.batch.StepList``) that the attention kernels of
         this kernel set want in every step of an engine with activations of ``act_dtype``: the
         single-token rows, the rows of prompt portions, and the portions cut into tiles of each
-        prompt-attention kernel's own height (for the 32-bit path tiles that its blocks walk in pieces)."""
-        from .step_lists import attention_lists, option_tile_lists, row_tile_lists
+        prompt-attention kernel's own height (the 32-bit path: the single-token rows and the portions' runs)."""
+        from .step_lists import attention_lists, option_tile_lists, plain_attention_lists, row_tile_lists
         if act_dtype != torch.bfloat16:
-            return attention_lists([PLAIN_TILE])
+            return plain_attention_lists(PLAIN_RUN)
         self.bf16
         # ... and, where a mixer has announced attention with options, every entry cut into tiles
         # of as many tokens as that kernel's blocks take
@@ -1180,15 +1180,17 @@ class CudaOps(MixerOps, StateOps):
         """The plain attention of a step's portions by the kernel whose blocks read a key once for eight tokens of a request,
         where it pays; returns the rows that are left (None: all) and their number.  It pays from eight tokens a portion on, if
         that leaves every SM a block.  us against a block per row, 16 heads of 128: portions of 2 (100 requests) 21.5 / 8.6,
-        4 (64) 15.8 / 11.1, 8 (32) 12.7 / 12.7, 16 (64) 46 / 57, 64 (8) 38 / 63, three of 119 to 197 61 / 140."""
+        4 (64) 15.8 / 11.1, 8 (32) 11.5 / 12.7, 16 (64) 42 / 56, 64 (8) 33 / 61, three of 119 to 197 52 to 61 / 124, 200 tokens
+        beside 60 single ones 73 / 98.  (bfloat16 heads that the tensor-core kernels refuse come in those kernels' tiles,
+        whose blocks without a token cost something: 16 tokens of 64 52 to 55.)"""
         lists, pages, bt = step.lists, cache.pages, cache.block_table
-        height = self._tile_rows[0] if q.dtype == torch.bfloat16 else PLAIN_TILE
-        tiles, single = lists.get(f"portion_tiles_{height}"), lists.get("single_rows")
+        name, height = (("portion_tiles", self._tile_rows[0]) if q.dtype == torch.bfloat16 else ("portion_runs", PLAIN_RUN))
+        tiles, single = lists.get(f"{name}_{height}"), lists.get("single_rows")
         t = q.shape[0]
         if tiles is None or single is None:
             return None, t
-        left = single.shape[0]
-        if t - left < 8 * (bt.shape[0] - left) or (t - left) * num_heads < 8 * self.num_sms:
+        left, least = single.shape[0], max(8, height // 4)
+        if t - left < least * (bt.shape[0] - left) or (t - left) * num_heads < 8 * self.num_sms:
             return None, t
         self._ok(self.core.ti_paged_attention_portions(
             q.data_ptr(), _code(q, "q"), tiles.data_ptr(), tiles.shape[0], height, step.positions.data_ptr(), bt.data_ptr(),

@@ -51,6 +51,15 @@ def row_tiles(q_lens: Sequence[int], starts: Sequence[int], tokens: int) -> np.n
     return np.stack([req, cu[req] + lo, np.minimum(tokens, q[req] - lo)], axis=1).astype(np.int64).reshape(-1, 3)
 
 
+def portion_runs(q_lens: Sequence[int], starts: Sequence[int], tokens: int) -> np.ndarray:
+    """The tiles of ``row_tiles`` without the single tokens, those with the longest contexts first (they take longest)."""
+    tiles = row_tiles(q_lens, starts, tokens)
+    q = np.asarray(q_lens, dtype=np.int64)
+    tiles = tiles[q[tiles[:, 0]] > 1]
+    ends = (np.asarray(starts, dtype=np.int64) - np.cumsum(q) + q)[tiles[:, 0]] + tiles[:, 1] + tiles[:, 2]
+    return tiles[np.argsort(-ends, kind="stable")]
+
+
 def option_tiles(q_lens: Sequence[int], starts: Sequence[int], tokens: int) -> np.ndarray:
     """The tiles of ``row_tiles`` with the longest contexts first (they take longest); none for a step of single
     tokens, which another kernel takes."""
@@ -71,6 +80,12 @@ def option_tile_lists(token_counts: Sequence[int]):
     from ..engine.batch import StepList
     return [StepList(f"option_tiles_{n}", partial(option_tiles, tokens=n), uses_starts=True)
             for n in sorted(set(token_counts))]
+
+
+def plain_attention_lists(tokens: int):
+    from ..engine.batch import StepList
+    return [StepList("single_rows", single_rows),
+            StepList(f"portion_runs_{tokens}", partial(portion_runs, tokens=tokens), uses_starts=True)]
 
 
 def attention_lists(tile_heights: Sequence[int]):
