@@ -162,3 +162,9 @@ def test_tiles_of_one_token_cut_from_a_portion(ops, heads, kv, size):
     ops.check_status()
     assert all(torch.equal(o, outs[0]) for o in outs[1:])
     assert attend(outs[0], tiles[:n // 2], 1) != 0
+
+
+@pytest.mark.parametrize("dk,dv,shared,blocks", [(16, 16, 0, 4), (64, 64, 0, 4), (128, 128, 0, 2), (192, 128, 0, 2), (288, 256, 1, 2),
+                                                 (576, 512, 1, 1)])
+def test_runs_are_counted_by_the_blocks_that_fit(ops, dk, dv, shared, blocks):
+    assert ops.mixers_tc.ti_attn_options_tc_run_blocks(dk, dv, shared) == blocks

@@ -589,6 +589,16 @@ extern "C" int ti_attn_options_tc_supported(int dk, int dv, int page_size, int s
            (!shared_rows || dv <= dk) && smem_bytes(dk, dv, shared_rows, BM) <= 227 * 1024;
 }
 
+// Blocks an SM that a step of single tokens counts on when it cuts the keys of a row into runs: as many as lie in its shared
+// memory beside one another, at most four, counted with the 64 rows of queries that a portion's block stages.  (Single tokens
+// stage 16, by which three blocks of heads of 128 would fit: us a decode step of 8 requests at 3,000 keys and 32 at 300 396
+// and 669 with two, 424 and 685 with three.  Shared rows of 576 fit once: 359 and 628, with two counted on 388 and 640; of
+// 288 twice: 244 and 322, with one 256 and 337.)
+extern "C" int ti_attn_options_tc_run_blocks(int dk, int dv, int shared_rows) {
+    const int fit = (int)(227 * 1024 / smem_bytes(dk, dv, shared_rows, BM));
+    return fit > 4 ? 4 : fit < 1 ? 1 : fit;
+}
+
 extern "C" int ti_head_project_tc_supported(int n_in, int n_out, int x_stride_t, int x_stride_h) {
     return n_in >= 16 && n_in % 16 == 0 && n_out % 8 == 0 && x_stride_t % 8 == 0 && x_stride_h % 8 == 0 &&
            (size_t)BM * (n_in * 2 + 16) + (size_t)STAGES * HPK * HP_WROW <= 227 * 1024;
@@ -663,10 +673,25 @@ extern "C" int ti_attn_options_tc(const void* q, const int* tiles, int num_tiles
                "and at most %d slices", WARPS);
     dim3 grid(num_kv_heads * head_blocks * (key_split == 2 ? 1 : dv / dvs), num_tiles, nsplit);
     cudaStream_t s = (cudaStream_t)stream;
-    // Single tokens: 164 KB of shared memory an SM are room for the blocks that the caller counts on, and the products
-    // behind this kernel, which start under it and keep the split it leaves, read their rows from the L1 that remains
-    // (three rows of 2,048, the two feed-forward products behind it: 16 + 15 us with three blocks' worth set aside, 12 + 10
-    // with this).
+    // Single tokens: shared memory is set aside for the blocks that the caller counts on (ti_attn_options_tc_run_blocks) and
+    // no more, by a hint of this launch: the products behind this kernel, which start under it and keep the split it leaves,
+    // read their rows from the L1 that remains.  us a decode step, 72 % (196 KB) for every size / this: 8 requests of 500 and
+    // 3,000 keys, heads of 128 (147 KB) 363 / 355 and 405 / 396, shared rows of 576 319 / 317 and 392 / 388; all of it 405 and
+    // 447, 350 and 421; 50 % (room for fewer blocks) 370 and 446, 331 and 413.
+    const size_t aside = ti_attn_options_tc_run_blocks(dk, dv, shared_rows) * (smem + 1024);
+    const int percent = aside < 228 * 1024 ? (int)((aside * 100 + 228 * 1024 - 1) / (228 * 1024)) : 100;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(WARPS * 32);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    attr[1].val.sharedMemCarveout = percent;
+    cfg.attrs = attr;
+    cfg.numAttrs = key_split ? 2 : 1;
 #define LAUNCH(DVS, MODE)                                                                                       \
     {                                                                                                     \
         static TiPerDevice configured;                                                                    \
@@ -675,13 +700,10 @@ extern "C" int ti_attn_options_tc(const void* q, const int* tiles, int num_tiles
             cudaError_t e = cudaFuncSetAttribute(attn_options_tc_kernel<DVS, MODE>,                             \
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024); \
             if (e != cudaSuccess) return ti_fail("attn_options_tc: %s", cudaGetErrorString(e));           \
-            if (MODE != 0)                                                                                \
-                cudaFuncSetAttribute(attn_options_tc_kernel<DVS, MODE>, cudaFuncAttributePreferredSharedMemoryCarveout, 72); \
             configured.mark();                                                                            \
             allowed = 227 * 1024;                                                                         \
         }                                                                                                 \
-        ti_launch_pdl((attn_options_tc_kernel<DVS, MODE>), grid, dim3(WARPS * 32), smem, s,                       \
-            (const bf16*)q, tiles, positions, block_table, bt_stride, (const bf16*)pages, num_pages,       \
+        cudaLaunchKernelEx(&cfg, attn_options_tc_kernel<DVS, MODE>, (const bf16*)q, tiles, positions, block_table, bt_stride, (const bf16*)pages, num_pages,       \
             page_size, num_heads, num_kv_heads, dk, dv, gp, head_blocks, nsplit, alone, opt, (bf16*)out, part_o,   \
             part_ml, status);                                                                             \
     }

@@ -71,22 +71,13 @@ class MixerOps:
             gp *= 2
         return gp
 
-    @staticmethod
-    def _key_run_blocks_per_sm(dk: int, dv: int, shared_rows: bool) -> int:
-        """Single tokens: how many blocks of ``attention_options`` an SM should get when the keys of a row are cut into
-        runs: as many as lie in its shared memory beside one another (64 query rows, two stages of 64 keys and
-        values), two to four.  A third block that has to wait for a place costs more than it brings (measured with
-        heads of 128: a decode step 0.76 -> 0.83 ms); four of heads of 64 fit (0.41 -> 0.38 ms)."""
-        row = 2 * dk + 16
-        block = 64 * row + 2 * 64 * (row + (0 if shared_rows else 2 * dv + 16))
-        return max(2, min(4, 227 * 1024 // block))
-
     @property
     def mixers_tc(self):
         if self._mixers_tc is None:
             b = load_library("bf16_mixers")
             b.ti_last_error.restype = ctypes.c_char_p
             b.ti_attn_options_tc_supported.argtypes = [_i, _i, _i, _i]
+            b.ti_attn_options_tc_run_blocks.argtypes = [_i, _i, _i]
             b.ti_attn_options_tc_group_rows.argtypes = [_i, _i]
             b.ti_head_project_tc_supported.argtypes = [_i, _i, _i, _i]
             b.ti_head_project_tc.argtypes = [_vp, _i, _i, _vp, _i, _i, _vp, _i, _i, _i, _i, _vp]
@@ -421,8 +412,8 @@ class MixerOps:
                 slices = dv // 256
             head_blocks = -(-(num_heads // num_kv_heads) // (min(gp, 16) if mode == 2 else gp))
             blocks = tiles.shape[0] * num_kv_heads * head_blocks * (1 if mode == 2 else slices)
-            per_sm = self._key_run_blocks_per_sm(dk, dv // slices, shared_rows)
-            if single and blocks < per_sm * self.num_sms:
+            per_sm = self.mixers_tc.ti_attn_options_tc_run_blocks(dk, dv, int(bool(shared_rows))) if single else 0
+            if blocks < per_sm * self.num_sms:
                 most = step.max_position or step.max_ctx_len
                 for bound in (window, chunk):
                     if bound:
