@@ -1184,7 +1184,8 @@ class CudaOps(MixerOps, StateOps):
         beside 60 single ones 73 / 98.  (bfloat16 heads that the tensor-core kernels refuse come in those kernels' tiles,
         whose blocks without a token cost something: 16 tokens of 64 52 to 55.)"""
         lists, pages, bt = step.lists, cache.pages, cache.block_table
-        name, height = (("portion_tiles", self._tile_rows[0]) if q.dtype == torch.bfloat16 else ("portion_runs", PLAIN_RUN))
+        half = q.dtype == pages.dtype == torch.bfloat16
+        name, height = ("portion_tiles", self._tile_rows[0]) if half else ("portion_runs", PLAIN_RUN)
         tiles, single = lists.get(f"{name}_{height}"), lists.get("single_rows")
         t = q.shape[0]
         if tiles is None or single is None:
