@@ -66,3 +66,61 @@ def test_numbers_at_the_ends_of_their_range(ops):
     assert torch.equal(out[3][w[:, 50] != 0], -w[:, 50].float().sign()[w[:, 50] != 0] * float("inf"))
     assert torch.equal(out[4], torch.full((130,), 0.5 * 3.4028234e38, device="cuda"))
     ops.check_status()
+
+
+@pytest.mark.parametrize("m", [1, 4, 6, 40, 130])
+@pytest.mark.parametrize("n,k", [(130, 200), (256, 1024), (1024, 520), (40, 4104)])
+def test_infinite_weights(ops, m, n, k):
+    """An infinite weight gives what a product in float32 gives, also where a row's element has a part that is zero."""
+    g = torch.Generator(device="cuda").manual_seed(m)
+    a = torch.randn((m, k), generator=g, device="cuda")
+    a[:, 3] = 1.0                                             # two parts are zero
+    a[:, 5] = 0.0
+    a[0, 7] = -float("inf")
+    w = torch.randn((n, k), generator=g, device="cuda").bfloat16()
+    w[1, 3], w[2, 3], w[5, 9], w[6, 5] = float("inf"), -float("inf"), float("inf"), float("inf")
+    w[7, 3], w[7, 9], w[8, 2] = float("inf"), -float("inf"), float("nan")
+    want = a.double() @ w.double().T
+    out = torch.empty((m, n), device="cuda")
+    for before in (None, 2.5):
+        if before is not None:
+            out.fill_(before)
+        ops.linear(a, w, out, accumulate=before is not None)
+        finite = torch.isfinite(want)
+        assert torch.equal(torch.isnan(out), torch.isnan(want))
+        assert torch.equal(out[~finite & ~torch.isnan(want)].double(), want[~finite & ~torch.isnan(want)])
+        assert bool(((out.double() - want - (before or 0.0)).abs()[finite] <= 1e-4 * k ** 0.5).all())
+    assert bool(torch.isinf(want[1:, 1]).all()) and bool(torch.isnan(want[:, 6]).all())
+    ops.check_status()
+
+
+@pytest.mark.parametrize("m", [3, 6, 40])
+@pytest.mark.parametrize("exponent", [-90, -105, -110, -115, -120, -126, -133, -140])
+def test_small_elements(ops, m, exponent):
+    """Elements whose last bits lie below what bfloat16 holds are cut short by less than 2^-133 each, and by nothing from 2^-109
+    on; the weights lift the sums out of the range where float32 itself runs short."""
+    n, k = 130, 600
+    g = torch.Generator(device="cuda").manual_seed(-exponent)
+    a = (1.0 + torch.rand((m, k), generator=g, device="cuda")) * 2.0 ** -60 * 2.0 ** (exponent + 60)
+    w = (torch.randn((n, k), generator=g, device="cuda") * 2.0 ** 60).bfloat16()
+    want = a.double() @ w.double().T
+    out = torch.empty((m, n), device="cuda")
+    ops.linear(a, w, out)
+    cut = 0.0 if exponent >= -109 else 2.0 ** -133 * w.double().abs().sum(1)
+    assert bool(((out.double() - want).abs() <= _bound(a, w, k) + cut).all())
+    ops.check_status()
+
+
+@pytest.mark.parametrize("n,k", [(512, 1024), (300, 2048), (130, 4096)])
+def test_terms_of_one_sign(ops, n, k):
+    """A tensor core cuts its sums off, so terms of one sign leave an error of one sign.  A run's four sums of sixteen terms in
+    three parts lose less than four units of 2^-23 of the run, the sums in registers half a unit each and to either side."""
+    g = torch.Generator(device="cuda").manual_seed(k)
+    a, w = torch.rand((64, k), generator=g, device="cuda") + 0.05, (torch.rand((n, k), generator=g, device="cuda") + 0.05).bfloat16()
+    want = a.double() @ w.double().T
+    for m in (2, 16, 64):
+        out = torch.empty((m, n), device="cuda")
+        ops.linear(a[:m], w, out)
+        off = (out.double() - want[:m]) / want[:m]
+        assert abs(float(off.mean())) < 4 * 2.0 ** -23 and float(off.norm() / off.numel() ** 0.5) < 5 * 2.0 ** -23
+    ops.check_status()

@@ -1,8 +1,9 @@
 // Product of float32 rows with bfloat16 weights on the 5th-generation tensor cores, without rounding the rows:
 // C[M,N] (+)= A[M,K] * W[N,K]^T.
 //
-// A float32 number is the sum of three bfloat16 numbers (its 24 significant bits in runs of eight), and a product of two
-// bfloat16 numbers is exact in float32, so W times the three parts of A is W times A.  What a tensor core does not do is
+// A float32 number is the sum of three bfloat16 numbers (its 24 significant bits in runs of eight; bfloat16 ends at 2^-133, so
+// an element below 2^-109 may be cut short, by less than 2^-133), and a product of two bfloat16 numbers is exact in float32,
+// so W times the three parts of A is W times A.  What a tensor core does not do is
 // round its sums to nearest (they are cut off, which over a thousand terms adds up to 1e-6 of the result), so sums are made
 // there over 64 terms only and then added, rounded to nearest, in registers.  Against 64 bits an element is off by 0.9e-7 of
 // the norm (K = 1,024, normal terms; one fused multiply-add per term in runs of 256: 2.9e-7).
@@ -16,7 +17,8 @@
 // the M side and the three parts of NT tokens beside one another as the N side (a product of 16 columns takes the tensor
 // core as long as one of 48: it reads W), warps 4 to 7 read a stage's sums out of tensor memory while the next ones multiply,
 // warps 8 to 15 read A, cut it into its parts and write them to shared memory in the swizzle that the products read.  An
-// infinite or NaN element of A stays itself; an infinite weight gives NaN where a part is zero.
+// infinite or NaN element of A stays itself; an infinite weight gives NaN where a part is zero, so an element that is NaN is
+// made again by multiply-adds.
 //
 // What bounds it: few rows by the stream of W and, for small W, by the launch, a run's chain (450 to 900 cycles) and the adding
 // of the sums that blocks have left; many by a stage's products (four of 192 columns) and the cutting of A.  us against the
@@ -78,6 +80,19 @@ __device__ __forceinline__ void three_parts(const float (&x)[8], uint4 (&parts)[
 #pragma unroll
     for (int r = 0; r < 3; ++r) parts[r] = make_uint4(q[r][0], q[r][1], q[r][2], q[r][3]);
 }
+// Elements of one row of W by multiply-adds: of the tokens t, t + step, ... whose bits are set
+__device__ __noinline__ void plain_sums(unsigned tokens, int t, int step, const float* a, int lda, const bf16* w, int k, float* c, int ldc,
+                                        int accumulate) {
+    for (; tokens; t += step, tokens >>= 1) {
+        if (!(tokens & 1)) continue;
+        const float* row = a + (size_t)t * lda;
+        float sum = 0.0f;
+        for (int i = 0; i < k && sum == sum; ++i) sum = fmaf(row[i], __bfloat162float(w[i]), sum);
+        float* p = c + (size_t)t * ldc;
+        *p = accumulate ? *p + sum : sum;
+    }
+}
+
 // 16 columns of each of the three parts of a stage's sums (`apart` columns from one another), all on their way at once
 __device__ __forceinline__ void load_sums(unsigned taddr, unsigned apart, float (&v)[3][16]) {
     unsigned r[3][16];
@@ -135,8 +150,9 @@ __device__ __forceinline__ void add_parts(const float* part, int nt, int parts, 
 
 template <int NT>
 __global__ void __launch_bounds__(THREADS, Split<NT>::BLOCKS)
-gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const float* a, float* c, float* ws, int* __restrict__ tickets,
-                  int m, int n, int k, int lda, int ldc, int accumulate, int vec, int fine, int* __restrict__ status) {
+gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const float* a, const bf16* __restrict__ w, float* c, float* ws,
+                  int* __restrict__ tickets, int m, int n, int k, int lda, int ldw, int ldc, int accumulate, int vec, int fine,
+                  int* __restrict__ status) {
     using T = Split<NT>;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -306,9 +322,12 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const float* a, flo
     if (*ticket_slot && !*failed_slot) {                 // four threads a row of W
         pdl_wait();                                      // C belongs to the chain
         const int row = threadIdx.x & (BW - 1), t0 = threadIdx.x / BW, n_row = n0 + row;
+        unsigned again = 0;                              // tokens t0, t0 + 4, ... whose sum is NaN
         auto out = [&](int t, float v) {
             float* p = c + (size_t)(m0 + t) * ldc + n_row;
-            *p = accumulate ? *p + v : v;
+            if (v != v) again |= 1u << (t >> 2);
+            if (!accumulate) *p = v;
+            else if (v == v) *p += v;
         };
         const float* part = ws + (size_t)tile * parts * NT * BW + row;
         if (n_row >= n) {
@@ -321,6 +340,9 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const float* a, flo
         } else {
             add_parts<4, 4, false>(part, NT, parts, tokens, t0, out);
         }
+        if (again)
+            plain_sums(again, t0, 4, a + (size_t)m0 * lda, lda, w + (size_t)n_row * ldw, k, c + (size_t)m0 * ldc + n_row, ldc,
+                       accumulate);
     }
     if (!ok) atomicCAS(status, 0, TI_ERR_TIMEOUT);
     tc_fence_before();
@@ -355,8 +377,8 @@ Cut choose_cut(int m, int n, int k) {
 }
 
 template <int NT>
-int launch(const CUtensorMap& map_w, const float* a, float* c, float* ws, int* tickets, int m, int n, int k, int lda, int ldc,
-           int accumulate, const Cut& cut, int* status, cudaStream_t s) {
+int launch(const CUtensorMap& map_w, const float* a, const bf16* w, float* c, float* ws, int* tickets, int m, int n, int k, int lda,
+           int ldw, int ldc, int accumulate, const Cut& cut, int* status, cudaStream_t s) {
     static TiPerDevice configured;
     if (configured.first_use()) {
         cudaError_t e = cudaFuncSetAttribute(gemm_split_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, Split<NT>::SMEM);
@@ -366,8 +388,8 @@ int launch(const CUtensorMap& map_w, const float* a, float* c, float* ws, int* t
     const int vec = (uintptr_t)a % 16 == 0 && lda % 4 == 0;
     const dim3 grid((m + NT - 1) / NT, (n + BW - 1) / BW, cut.splits);
     TI_REQUIRE(grid.y <= 65535, "gemm_split: %d rows of weights exceed the grid limit", n);
-    ti_launch_pdl(gemm_split_kernel<NT>, grid, dim3(THREADS), Split<NT>::SMEM, s, map_w, a, c, ws, tickets, m, n, k, lda, ldc,
-                  accumulate, vec, cut.fine, status);
+    ti_launch_pdl(gemm_split_kernel<NT>, grid, dim3(THREADS), Split<NT>::SMEM, s, map_w, a, w, c, ws, tickets, m, n, k, lda,
+                  ldw, ldc, accumulate, vec, cut.fine, status);
     return ti_check_launch("gemm_split");
 }
 
@@ -393,8 +415,8 @@ extern "C" int ti_gemm_split(const float* a, const void* w, float* c, int m, int
     CUtensorMap map_w;
     if (int rc = make_map_bf16(&map_w, w, n, k, ldw, BW, "gemm_split")) return rc;
     cudaStream_t s = (cudaStream_t)stream;
-    if (token_tile(m) == 16) return launch<16>(map_w, a, c, ws, tickets, m, n, k, lda, ldc, accumulate, cut, status, s);
-    return launch<64>(map_w, a, c, ws, tickets, m, n, k, lda, ldc, accumulate, cut, status, s);
+    auto run = token_tile(m) == 16 ? launch<16> : launch<64>;
+    return run(map_w, a, (const bf16*)w, c, ws, tickets, m, n, k, lda, ldw, ldc, accumulate, cut, status, s);
 }
 
 TI_TAPED(ti_gemm_split)
