@@ -10,8 +10,8 @@
 //
 // One order of summation for every number of rows: a run of 64 terms gives first part + (second + third part); chunk sum =
 // its eight runs, ascending, from zero; total = chunk sums, ascending, from zero; C = total or C + total.  A block may have
-// all of a tile (the total lies in shared memory), some of its chunks or some of its runs (every chunk's or run's sum goes to
-// scratch and the tile's last block adds them in that order).
+// all of a tile, some of its chunks or, for few rows, some of its runs (every chunk's or run's sum goes to scratch and the
+// tile's last block adds them in that order).
 //
 // Roles of a block of 512 threads: warp 0 brings W by TMA (128 rows x 64 columns a stage), warp 1 issues the products, W as
 // the M side and the three parts of NT tokens beside one another as the N side (a product of 16 columns takes the tensor
@@ -21,11 +21,12 @@
 // made again by multiply-adds.
 //
 // What bounds it: few rows by the stream of W and, for small W, by the launch, a run's chain (450 to 900 cycles) and the adding
-// of the sums that blocks have left; many by a stage's products (four of 192 columns) and the cutting of A.  us against the
-// multiply-adds of gemm_simple.cu: 466 x 6,144 x 1,024 182 -> 51, 466 x 1,024 x 3,072 93 -> 34, 64 x 4,096 x 4,096 120 -> 31,
-// three rows of 151,936 x 1,024 125 -> 65, of 4,096 x 12,288 99 -> 25, of 1,024 x 3,072 9.7 -> 9.3; a single row of a small
-// matrix pays for the longer chain (6,144 x 1,024 5.1 -> 8.0, 4,096 x 4,096 10.8 -> 11.1).  With three products of NT columns in
-// place of one of 3 NT 466 x 6,144 x 1,024 took 63, three rows of 151,936 x 1,024 85.
+// of the sums that blocks have left (gemm_split_few_kernel); many by a stage's products (four of 192 columns) and the cutting of
+// A.  us against the multiply-adds of gemm_simple.cu: 466 x 6,144 x 1,024 182 -> 51, 466 x 1,024 x 3,072 93 -> 34, 64 x 4,096 x
+// 4,096 120 -> 31, six rows of 6,144 x 1,024 12.2 -> 10.9, three rows of 151,936 x 1,024 125 -> 51, of 4,096 x 4,096 34 -> 11.5, of
+// 1,024 x 3,072 9.0 -> 8.6; one and two rows of a small matrix still pay for the longer chain (4,096 x 1,024 4.4 and 4.8 -> 6.3
+// and 6.5, 1,024 x 2,048 4.4 and 5.4 -> 5.6 and 5.7, 6,144 x 1,024 5.0 and 5.4 -> 6.7 and 6.9, 1,024 x 3,072 4.7 and 5.8 -> 6.4 and
+// 7.2).  With three products of NT columns in place of one of 3 NT 466 x 6,144 x 1,024 took 63.
 #include "sm100.cuh"
 #include "tape.cuh"
 
@@ -94,6 +95,21 @@ __device__ __noinline__ void plain_sums(unsigned tokens, int t, int step, const 
 }
 
 // 16 columns of each of the three parts of a stage's sums (`apart` columns from one another), all on their way at once
+__device__ __forceinline__ void tmem_load16(unsigned taddr, float (&v)[16]) {
+    unsigned r[16];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+          "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+        asm volatile("" : "+r"(r[j]));                   // not used before the wait
+        v[j] = __uint_as_float(r[j]);
+    }
+}
 __device__ __forceinline__ void load_sums(unsigned taddr, unsigned apart, float (&v)[3][16]) {
     unsigned r[3][16];
 #pragma unroll
@@ -115,12 +131,12 @@ __device__ __forceinline__ void load_sums(unsigned taddr, unsigned apart, float 
         }
 }
 
-// C of one row of W from the sums that a tile's blocks have left: every fourth token from t0 on, TS of them and PS sums asked
+// C of one row of W from the sums that a tile's blocks have left: every STEP-th token from t0 on, TS of them and PS sums asked
 // for at a time; chunks in ascending order or, RUNS, the runs of a chunk first.
-template <int TS, int PS, bool RUNS, typename Out>
+template <int TS, int PS, bool RUNS, int STEP, typename Out>
 __device__ __forceinline__ void add_parts(const float* part, int nt, int parts, int tokens, int t0, Out out) {
     static_assert(!RUNS || PS % CHUNK == 0, "whole chunks of runs");
-    for (; t0 < tokens; t0 += 4 * TS) {
+    for (; t0 < tokens; t0 += STEP * TS) {
         float all[TS];
 #pragma unroll
         for (int i = 0; i < TS; ++i) all[i] = 0.0f;
@@ -130,7 +146,7 @@ __device__ __forceinline__ void add_parts(const float* part, int nt, int parts, 
             for (int p = 0; p < PS; ++p)
 #pragma unroll
                 for (int i = 0; i < TS; ++i)
-                    got[p][i] = p0 + p < parts && t0 + 4 * i < tokens ? __ldcg(part + ((size_t)(p0 + p) * nt + t0 + 4 * i) * BW) : 0.0f;
+                    got[p][i] = p0 + p < parts && t0 + STEP * i < tokens ? __ldcg(part + ((size_t)(p0 + p) * nt + t0 + STEP * i) * BW) : 0.0f;
 #pragma unroll
             for (int p = 0; p < PS; ++p) {
                 if (p0 + p >= parts) continue;
@@ -144,14 +160,14 @@ __device__ __forceinline__ void add_parts(const float* part, int nt, int parts, 
         }
 #pragma unroll
         for (int i = 0; i < TS; ++i)
-            if (t0 + 4 * i < tokens) out(t0 + 4 * i, all[i]);
+            if (t0 + STEP * i < tokens) out(t0 + STEP * i, all[i]);
     }
 }
 
 template <int NT>
 __global__ void __launch_bounds__(THREADS, Split<NT>::BLOCKS)
 gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const float* a, const bf16* __restrict__ w, float* c, float* ws,
-                  int* __restrict__ tickets, int m, int n, int k, int lda, int ldw, int ldc, int accumulate, int vec, int fine,
+                  int* __restrict__ tickets, int m, int n, int k, int lda, int ldw, int ldc, int accumulate, int vec,
                   int* __restrict__ status) {
     using T = Split<NT>;
     extern __shared__ unsigned char smem_raw[];
@@ -168,11 +184,11 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const float* a, con
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int m0 = blockIdx.x * NT, n0 = blockIdx.y * BW;
-    // the block's stages: whole chunks of them or, `fine`, any
-    const int stages_all = (k + BK - 1) / BK, splits = gridDim.z, per = fine ? 1 : CHUNK;
-    const int parts = (stages_all + per - 1) / per;      // sums that a tile's blocks leave, if there are several
-    const int kb_lo = (int)((long long)parts * blockIdx.z / splits) * per;
-    const int kb_hi = min(stages_all, (int)((long long)parts * (blockIdx.z + 1) / splits) * per);
+    // the block's stages: whole chunks of them
+    const int stages_all = (k + BK - 1) / BK, splits = gridDim.z;
+    const int parts = (stages_all + CHUNK - 1) / CHUNK;  // sums that a tile's blocks leave, if there are several
+    const int kb_lo = (int)((long long)parts * blockIdx.z / splits) * CHUNK;
+    const int kb_hi = min(stages_all, (int)((long long)parts * (blockIdx.z + 1) / splits) * CHUNK);
     auto stage_w = [&](int s) { return smem + s * T::STAGE; };
     auto stage_a = [&](int s, int part) { return smem + s * T::STAGE + T::STAGE_W + part * T::STAGE_A; };
 
@@ -279,7 +295,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const float* a, con
         float acc[NT];
         for (int kb = kb_lo, it = 0; kb < kb_hi; ++kb, ++it) {
             const int buf = it % T::SUMS;
-            const bool first = kb % CHUNK == 0 || fine, last = kb % CHUNK == CHUNK - 1 || kb + 1 == stages_all || fine;
+            const bool first = kb % CHUNK == 0, last = kb % CHUNK == CHUNK - 1 || kb + 1 == stages_all;
             ok = __all_sync(0xffffffffu, mbar_wait(&sum_full[buf], (it / T::SUMS) & 1));
             if (!ok) break;
             tc_fence_after();
@@ -295,7 +311,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const float* a, con
             if (lane == 0) mbar_arrive(&sum_empty[buf]);
             if (!last) continue;
             if (splits > 1) {
-                float* part = ws + ((size_t)tile * parts + kb / per) * NT * BW + row;
+                float* part = ws + ((size_t)tile * parts + kb / CHUNK) * NT * BW + row;
 #pragma unroll
                 for (int t = 0; t < NT; ++t)
                     if (t < tokens) part[t * BW] = acc[t];
@@ -333,12 +349,10 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const float* a, con
         if (n_row >= n) {
         } else if (splits == 1) {
             for (int t = t0; t < tokens; t += 4) out(t, total[t * BW + row]);
-        } else if (fine) {
-            add_parts<1, 16, true>(part, NT, parts, tokens, t0, out);
         } else if (tokens <= 4) {
-            add_parts<1, 16, false>(part, NT, parts, tokens, t0, out);
+            add_parts<1, 16, false, 4>(part, NT, parts, tokens, t0, out);
         } else {
-            add_parts<4, 4, false>(part, NT, parts, tokens, t0, out);
+            add_parts<4, 4, false, 4>(part, NT, parts, tokens, t0, out);
         }
         if (again)
             plain_sums(again, t0, 4, a + (size_t)m0 * lda, lda, w + (size_t)n_row * ldw, k, c + (size_t)m0 * ldc + n_row, ldc,
@@ -353,24 +367,225 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const float* a, con
     }
 }
 
+// Up to four rows.  The three parts of four tokens lie beside one another in the 16 columns of one product, a warp cuts a
+// stage's rows, and a block of 256 threads is small enough that the next launch's blocks find a place beside it and have their
+// weights on the way while this one ends.  us at 1 and 4 rows, the kernel above / this: 4,096 x 1,024 7.1 / 6.3 and 7.8 / 6.7,
+// 1,024 x 2,048 8.8 / 5.6 and 9.3 / 6.9, 6,144 x 1,024 7.8 / 6.7 and 8.6 / 7.3, 1,024 x 3,072 9.2 / 6.4 and 9.6 / 8.7,
+// 151,936 x 1,024 64.1 / 50.6 and 64.5 / 51.6.  A cluster's blocks that exchange their sums through shared memory start later:
+// 4,096 x 1,024 7.8, 1,024 x 2,048 6.8 at one row.
+constexpr int FEW = 4, FEW_THREADS = 256;
+struct Few {
+    static constexpr int STAGE = BW * BK * 2 + 16 * BK * 2, STAGES = 4, SUMS = 4, CUTTERS = 2, AHEAD = 4;
+    static constexpr int BARS = STAGES * STAGE, SMEM = BARS + 256 + 1024;
+    static constexpr unsigned TMEM_COLS = SUMS * 16;
+};
+
+__global__ void __launch_bounds__(FEW_THREADS, 3)
+gemm_split_few_kernel(const __grid_constant__ CUtensorMap map_w, const float* a, const bf16* __restrict__ w, float* c, float* ws,
+                      int* __restrict__ tickets, int m, int n, int k, int lda, int ldw, int ldc, int accumulate, int vec, int fine,
+                      int* __restrict__ status) {
+    using T = Few;
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    unsigned long long* bars = (unsigned long long*)(smem + T::BARS);
+    unsigned long long *full = bars, *empty = bars + T::STAGES, *sum_full = bars + 2 * T::STAGES, *sum_empty = sum_full + T::SUMS;
+    unsigned* tmem_slot = (unsigned*)(sum_empty + T::SUMS);
+    int* ticket_slot = (int*)(tmem_slot + 1);
+    int* failed_slot = ticket_slot + 1;
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n0 = blockIdx.x * BW;
+    const int stages_all = (k + BK - 1) / BK, splits = gridDim.y, per = fine ? 1 : CHUNK;
+    const int parts = (stages_all + per - 1) / per;
+    const int kb_lo = (int)((long long)parts * blockIdx.y / splits) * per;
+    const int kb_hi = min(stages_all, (int)((long long)parts * (blockIdx.y + 1) / splits) * per);
+    auto stage_w = [&](int s) { return smem + s * T::STAGE; };
+    auto stage_a = [&](int s) { return smem + s * T::STAGE + BW * BK * 2; };
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < T::STAGES; ++s) { mbar_init(&full[s], 2); mbar_init(&empty[s], 1); }
+        for (int b = 0; b < T::SUMS; ++b) { mbar_init(&sum_full[b], 1); mbar_init(&sum_empty[b], 4); }
+        *failed_slot = 0;
+        mbar_fence_init();
+    }
+    if (warp == 1) tmem_alloc(tmem_slot, T::TMEM_COLS);
+    for (int i = threadIdx.x; i < T::STAGES * 128; i += FEW_THREADS)         // rows without a token stay zeros
+        *reinterpret_cast<uint4*>(stage_a(i >> 7) + (i & 127) * 16) = make_uint4(0u, 0u, 0u, 0u);
+    fence_async_smem();
+    pdl_launch();
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const unsigned tmem_base = *tmem_slot;
+    const int stages = kb_hi - kb_lo;
+
+    bool ok = true;
+    float all[FEW] = {};                                 // one block a tile: the total
+    if (warp == 0) {
+        if (lane == 0) {                                 // the weights do not depend on the kernel before this one
+            for (int it = 0; it < stages && ok; ++it) {
+                const int s = it % T::STAGES;
+                ok = mbar_wait(&empty[s], ((it / T::STAGES) & 1) ^ 1);
+                if (!ok) break;
+                mbar_expect_tx(&full[s], BW * BK * 2);
+                tma_load_2d(stage_w(s), &map_w, &full[s], (kb_lo + it) * BK, n0);
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            const unsigned idesc = umma_idesc(BW, 16);
+            const unsigned long long dw0 = umma_desc(stage_w(0)), da0 = umma_desc(stage_a(0));
+            for (int it = 0; it < stages && ok; ++it) {
+                const int s = it % T::STAGES, buf = it % T::SUMS;
+                ok = mbar_wait(&sum_empty[buf], ((it / T::SUMS) & 1) ^ 1);
+                if (ok) ok = mbar_wait(&full[s], (it / T::STAGES) & 1);
+                if (!ok) break;
+                tc_fence_after();
+                const unsigned long long step = (unsigned long long)(s * (T::STAGE >> 4));
+#pragma unroll
+                for (int kk = 0; kk < BK / 16; ++kk)
+                    umma_bf16(tmem_base + buf * 16, dw0 + step + (unsigned long long)(kk * 2), da0 + step + (unsigned long long)(kk * 2),
+                              idesc, kk != 0);
+                umma_commit(&empty[s]);
+                umma_commit(&sum_full[buf]);
+            }
+        }
+    } else if (warp < 4) {
+        // a lane has eight neighbouring columns of a token; the two warps take the stages in turn
+        const int t = lane >> 3, piece = lane & 7, team = warp - 2;
+        const float* row = a + (size_t)t * lda;
+        float v[T::AHEAD][8];
+        auto fetch = [&](int it, float (&v)[8]) {
+            if (it >= stages || t >= m) return;
+            const int col = (kb_lo + it) * BK + piece * 8;
+            if (vec && col + 8 <= k) {
+                const float4 x = *reinterpret_cast<const float4*>(row + col), y = *reinterpret_cast<const float4*>(row + col + 4);
+                v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w; v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
+            } else {
+#pragma unroll
+                for (int e = 0; e < 8; ++e) v[e] = col + e < k ? row[col + e] : 0.0f;
+            }
+        };
+        pdl_wait();
+#pragma unroll
+        for (int d = 0; d < T::AHEAD; ++d) fetch(team + d * T::CUTTERS, v[d]);
+        for (int first = team; first < stages && ok; first += T::AHEAD * T::CUTTERS) {
+#pragma unroll
+            for (int d = 0; d < T::AHEAD; ++d) {
+                const int it = first + d * T::CUTTERS, s = it % T::STAGES;
+                if (it >= stages || !ok) break;
+                ok = __all_sync(0xffffffffu, mbar_wait(&empty[s], ((it / T::STAGES) & 1) ^ 1));
+                if (!ok) break;
+                if (t < m) {
+                    uint4 part[3];
+                    three_parts(v[d], part);
+#pragma unroll
+                    for (int q = 0; q < 3; ++q) {
+                        const int at = q * FEW + t;
+                        *reinterpret_cast<uint4*>(stage_a(s) + at * 128 + (piece ^ (at & 7)) * 16) = part[q];
+                    }
+                }
+                fence_async_smem();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&full[s]);
+                fetch(it + T::AHEAD * T::CUTTERS, v[d]);
+            }
+        }
+    } else {
+        const int row = (warp & 3) * 32 + lane;
+        const unsigned lane_addr = (unsigned)((warp & 3) * 32) << 16;
+        pdl_wait();                                       // the scratch and the tickets belong to the chain
+        float acc[FEW];
+        for (int kb = kb_lo, it = 0; kb < kb_hi; ++kb, ++it) {
+            const int buf = it % T::SUMS;
+            const bool first = kb % CHUNK == 0 || fine, last = kb % CHUNK == CHUNK - 1 || kb + 1 == stages_all || fine;
+            ok = __all_sync(0xffffffffu, mbar_wait(&sum_full[buf], (it / T::SUMS) & 1));
+            if (!ok) break;
+            tc_fence_after();
+            float v[16];
+            tmem_load16(tmem_base + lane_addr + buf * 16, v);
+#pragma unroll
+            for (int t = 0; t < FEW; ++t)
+                acc[t] = (first ? 0.0f : acc[t]) + (v[t] + (v[FEW + t] + v[2 * FEW + t]));
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sum_empty[buf]);
+            if (!last) continue;
+            float* part = ws + ((size_t)blockIdx.x * parts + kb / per) * FEW * BW + row;
+#pragma unroll
+            for (int t = 0; t < FEW; ++t) {
+                if (splits > 1) { if (t < m) part[t * BW] = acc[t]; }
+                else all[t] += acc[t];
+            }
+        }
+        if (splits > 1) {
+            // the tile is complete when all its blocks have stored their sums; the last one adds them
+            drain_sync();
+            if (threadIdx.x == 128) {
+                __threadfence();
+                const bool finish = atomicAdd(&tickets[blockIdx.x], 1) == splits - 1;
+                if (finish) tickets[blockIdx.x] = 0;
+                *ticket_slot = finish;
+                __threadfence();
+            }
+        }
+    }
+    if (!ok) *failed_slot = 1;
+    __syncthreads();
+    if (!*failed_slot && (splits == 1 ? warp >= 4 : *ticket_slot)) {
+        pdl_wait();                                       // C belongs to the chain
+        const int row = threadIdx.x & (BW - 1), t0 = splits == 1 ? 0 : threadIdx.x / BW;
+        unsigned again = 0;                               // tokens whose sum is NaN
+        auto store = [&](int t, float v) {
+            float* p = c + (size_t)t * ldc + n0 + row;
+            *p = accumulate ? *p + v : v;
+        };
+        auto out = [&](int t, float v) {
+            if (v != v) again |= 1u << t;
+            else store(t, v);
+        };
+        const float* part = ws + (size_t)blockIdx.x * parts * FEW * BW + row;
+        if (n0 + row >= n) {
+        } else if (splits == 1) {
+#pragma unroll
+            for (int t = 0; t < FEW; ++t)
+                if (t < m) out(t, all[t]);
+        } else if (fine && m <= 2) {
+            add_parts<1, 32, true, 2>(part, FEW, parts, m, t0, out);
+        } else if (fine) {
+            add_parts<2, 16, true, 2>(part, FEW, parts, m, t0, out);
+        } else {
+            add_parts<2, 8, false, 2>(part, FEW, parts, m, t0, out);
+        }
+        if (again) plain_sums(again, 0, 1, a, lda, w + (size_t)(n0 + row) * ldw, k, c + n0 + row, ldc, accumulate);
+    }
+    if (!ok) atomicCAS(status, 0, TI_ERR_TIMEOUT);
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_dealloc(tmem_base, T::TMEM_COLS);
+    }
+}
+
 int token_tile(int m) { return m <= 16 ? 16 : 64; }
 
-// Blocks that share a tile: as many as fill the SMs once (twice where two blocks fit on one), a chunk or more each or,
-// where that leaves SMs idle and there are few sums to add (up to 4 rows, K of 320 to 1,024), a run or more: us at 3 and 16 rows of
-// 1,024 x 1,024 with chunks 8.7 / 10.8, with runs 6.6 / 11.5, of 1,024 x 3,072 9.6 / 13.0 and 10.4 / 22.3.
+// How a tile's K is shared.  Up to four rows: some two blocks an SM, a run or more each or, where a tile gets fewer blocks than
+// twice its chunks, whole chunks, whose sums are fewer to add (us at 1 and 4 rows, runs / chunks: 1,024 x 3,072 6.4 / 7.9 and
+// 8.7 / 8.7, 4,096 x 4,096 10.8 / 11.1 and 13.6 / 11.5); four runs are not shared (256 x 256 4.4 / 3.5).  More rows: as many
+// blocks as fill the SMs once (twice where two fit on one), a chunk or more each.
 struct Cut { int splits, fine; long long floats; int tickets; };
 Cut choose_cut(int m, int n, int k) {
     int device = 0, sms = 148;
     cudaGetDevice(&device);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    const int nt = token_tile(m), stages = (k + BK - 1) / BK, chunks = (stages + CHUNK - 1) / CHUNK;
-    const long long tiles = (long long)((m + nt - 1) / nt) * ((n + BW - 1) / BW), room = (long long)sms * (nt == 16 ? 2 : 1);
+    const bool few = m <= FEW;
+    const int nt = few ? FEW : token_tile(m), stages = (k + BK - 1) / BK, chunks = (stages + CHUNK - 1) / CHUNK;
+    const long long tiles = (long long)((m + nt - 1) / nt) * ((n + BW - 1) / BW), room = (long long)sms * (nt <= 16 ? 2 : 1);
     const long long s = room / tiles;
     Cut cut;
-    cut.fine = s > chunks && stages > chunks && m <= 4 && stages > 4 && stages <= 16;
+    cut.fine = few && s >= 2 * chunks && stages > 4;
     const int most = cut.fine ? stages : chunks;
     cut.splits = s < 1 ? 1 : s > most ? most : (int)s;
-    if (cut.splits == 1) cut.fine = 0;
     cut.floats = cut.splits > 1 ? tiles * most * nt * BW : 0;
     cut.tickets = cut.splits > 1 ? (int)tiles : 0;
     return cut;
@@ -389,7 +604,21 @@ int launch(const CUtensorMap& map_w, const float* a, const bf16* w, float* c, fl
     const dim3 grid((m + NT - 1) / NT, (n + BW - 1) / BW, cut.splits);
     TI_REQUIRE(grid.y <= 65535, "gemm_split: %d rows of weights exceed the grid limit", n);
     ti_launch_pdl(gemm_split_kernel<NT>, grid, dim3(THREADS), Split<NT>::SMEM, s, map_w, a, w, c, ws, tickets, m, n, k, lda,
-                  ldw, ldc, accumulate, vec, cut.fine, status);
+                  ldw, ldc, accumulate, vec, status);
+    return ti_check_launch("gemm_split");
+}
+
+int launch_few(const CUtensorMap& map_w, const float* a, const bf16* w, float* c, float* ws, int* tickets, int m, int n, int k,
+               int lda, int ldw, int ldc, int accumulate, const Cut& cut, int* status, cudaStream_t s) {
+    static TiPerDevice configured;
+    if (configured.first_use()) {
+        cudaError_t e = cudaFuncSetAttribute(gemm_split_few_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Few::SMEM);
+        if (e != cudaSuccess) return ti_fail("gemm_split: %s", cudaGetErrorString(e));
+        configured.mark();
+    }
+    const int vec = (uintptr_t)a % 16 == 0 && lda % 4 == 0;
+    ti_launch_pdl(gemm_split_few_kernel, dim3((n + BW - 1) / BW, cut.splits), dim3(FEW_THREADS), Few::SMEM, s, map_w, a, w, c, ws,
+                  tickets, m, n, k, lda, ldw, ldc, accumulate, vec, cut.fine, status);
     return ti_check_launch("gemm_split");
 }
 
@@ -415,7 +644,7 @@ extern "C" int ti_gemm_split(const float* a, const void* w, float* c, int m, int
     CUtensorMap map_w;
     if (int rc = make_map_bf16(&map_w, w, n, k, ldw, BW, "gemm_split")) return rc;
     cudaStream_t s = (cudaStream_t)stream;
-    auto run = token_tile(m) == 16 ? launch<16> : launch<64>;
+    auto run = m <= FEW ? launch_few : token_tile(m) == 16 ? launch<16> : launch<64>;
     return run(map_w, a, (const bf16*)w, c, ws, tickets, m, n, k, lda, ldw, ldc, accumulate, cut, status, s);
 }
 

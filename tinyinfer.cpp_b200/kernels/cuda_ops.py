@@ -178,8 +178,8 @@ class CudaOps(MixerOps, StateOps):
         self.few_tc_min_bytes = 1 << 25
         self._few_tickets = None
         # float32 rows times bfloat16 weights on the tensor cores, from this many weights on (smaller ones: a launch of
-        # the multiply-add kernel is shorter, 128 x 128 at one row 2.6 against 4.0 us; at 256 x 256 one row pays 4.9 for
-        # 3.4, three save 4.9 for 7.0, 64 7.2 for 14.7)
+        # the multiply-add kernel is shorter, 128 x 128 at one row 2.4 us; 256 x 256, multiply-adds / this, one row
+        # 3.0 / 3.5, three 6.6 / 3.7, 40 15.8 / 6.6)
         self.split_products = True
         self.split_from = 1 << 16
         # prompt attention with two heads per block (csrc/attn_prefill_tc2.cu) from this many
