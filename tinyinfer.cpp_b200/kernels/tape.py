@@ -16,7 +16,6 @@ lives for one pass and holds the tensors allocated under it until the pass has i
 from __future__ import annotations
 
 import ctypes
-import struct
 from bisect import bisect
 
 import torch
@@ -71,7 +70,7 @@ class _Tap:
 
 def _slot(kind, value) -> int:
     if kind is ctypes.c_float:
-        return struct.unpack("<I", struct.pack("<f", value))[0]
+        return int.from_bytes(bytes(ctypes.c_float(value)), "little")        # rounds as a direct call does, to infinity too
     return (0 if value is None else int(value)) & 0xFFFFFFFFFFFFFFFF
 
 
