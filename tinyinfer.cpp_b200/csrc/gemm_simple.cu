@@ -1,9 +1,9 @@
 // Matrix product on the CUDA cores: C[M,N] (+)= A[M,K] * W[N,K]^T.
 //
-// This is the true 32-bit path (float32 multiply-add, no tensor cores, no reduced-precision
-// mode) and the fallback for operand types or sizes that the tensor-core kernels refuse.
-// Operands may be float32 or bfloat16 in any combination (widening bfloat16 is exact).
-// Float32 rows with bfloat16 weights of some size take gemm_split.cu instead.
+// Float32 multiply-adds, no tensor cores, no reduced-precision mode: the part of the 32-bit path that gemm_split.cu does not
+// take (float32 weights, and bfloat16 weights of less than 65,536 elements or off a 16-byte boundary), and the fallback for
+// operand types or sizes that the tensor-core kernels refuse.  Operands may be float32 or bfloat16 in any combination
+// (widening bfloat16 is exact).
 //
 // One order of summation for every element, whatever kernel computes it: K is cut into segments
 // of SEG terms, a segment is accumulated in float32 with one fused multiply-add per term, k

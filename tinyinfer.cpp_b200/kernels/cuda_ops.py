@@ -441,7 +441,9 @@ class CudaOps(MixerOps, StateOps):
     def _tc_glu(self, m: int, n: int, k: int, kind: str):
         """The same choice among the products whose epilogue applies an activation.  With gelu's tanh the epilogue is the longer
         half of a tile of short rows, and pairs lose what they gain while they wait for it: us, one SM / pairs, gelu at k 1,024:
-        64 tiles 15.4 / 13.3, 88 tiles 18.4 / 19.4, 352 tiles 38.4 / 39.4; other kinds or k 2,048: equal to a quarter faster."""
+        64 tiles 15.4 / 13.3, 88 tiles 18.4 / 19.4, 352 tiles 38.4 / 39.4; other kinds or k 2,048: equal to a quarter faster.
+        Longer rows with their weights in L2 lie within 2 % of one another from 88 tiles on (k 1,152 18.1 / 18.2, 1,536 21.5 /
+        21.9, 2,048 26.1 / 26.6; 352 tiles 42.4 / 42.0, 53.1 / 52.9, 68.0 / 69.2) and gain with 64 (1,536 18.2 / 14.2)."""
         pairs = self._tc_gemm(m, n) is self.bf16.ti_gemm_tcgen05_2sm
         if kind == "gelu_tanh" and k <= 1024 and -(-m // 256) * -(-n // 256) > self.num_sms // 2:
             pairs = False
