@@ -183,4 +183,4 @@ def test_numbers_are_handed_on_as_a_direct_call_hands_them_on():
     for value in (0.1, -3, 1e39, -1e39, 1e-46, float("inf")):
         bits = tape._slot(ctypes.c_float, value)
         assert ctypes.c_float.from_buffer_copy(bits.to_bytes(4, "little")).value == ctypes.c_float(value).value
-    assert tape._slot(ctypes.c_int, -2) == 2 ** 64 - 2 and tape._slot(ctypes.c_void_p, None) == 0
+    assert tape._slot(ctypes.c_int, -2) == 2 ** 64 - 2 and tape._slot(ctypes.c_int, True) == 1

@@ -71,7 +71,7 @@ class _Tap:
 def _slot(kind, value) -> int:
     if kind is ctypes.c_float:
         return int.from_bytes(bytes(ctypes.c_float(value)), "little")        # rounds as a direct call does, to infinity too
-    return (0 if value is None else int(value)) & 0xFFFFFFFFFFFFFFFF
+    return value & 0xFFFFFFFFFFFFFFFF
 
 
 def alike(layers):
@@ -134,21 +134,25 @@ def record(ops, run, mine):
     in_order.sort()
     if any(after[0] < before[1] for before, after in zip(in_order, in_order[1:])):
         return None                        # an address may stand for either of two tensors
-    place = {}
+    place = {}                             # pointer -> where it lies in the layer's own tensors (None: elsewhere)
     first, slots, patches, sources = [], [], [], []
+    pointer = ctypes.c_void_p
     for _, _, kinds, args in calls:
         if kinds is None or len(kinds) != len(args):
             return None
         first.append(len(slots))
         for kind, value in zip(kinds, args):
-            if kind is ctypes.c_void_p and value:
+            if kind is not pointer:
+                slots.append(_slot(kind, value))
+            elif not value:
+                slots.append(0)
+            else:
                 if value not in place:
                     place[value] = _inside(in_order, value)
                 if place[value] is not None:
                     patches.append(len(slots))
                     sources.append(place[value])
-                value = renamed.get(value, value)
-            slots.append(_slot(kind, value))
+                slots.append(renamed.get(value, value))
     n = len(calls)
     packed = ((ctypes.c_void_p * n)(*[c[0] for c in calls]), (ctypes.c_int * n)(*first), n,
               (ctypes.c_ulonglong * max(1, len(slots)))(*slots), (ctypes.c_int * max(1, len(patches)))(*patches), len(patches))
