@@ -127,8 +127,8 @@ def test_terms_of_one_sign(ops, n, k):
 
 
 @pytest.mark.parametrize("n,k", [(128, 256), (128, 320), (2560, 700), (40, 8192), (1024, 16392), (129, 1030)])
-def test_up_to_four_rows(ops, n, k):
-    """They have a kernel of their own, whose blocks share a tile's K by runs, by chunks or not at all: the bits of a product of
+def test_few_rows(ops, n, k):
+    """Up to eight rows have a kernel of their own, whose blocks share a tile's K by runs, by chunks or not at all: the bits of a product of
     more rows, next to one another and with rows off a 16-byte boundary, stored and added."""
     g = torch.Generator(device="cuda").manual_seed(n)
     a = torch.randn((70, k), generator=g, device="cuda")
@@ -137,7 +137,7 @@ def test_up_to_four_rows(ops, n, k):
     whole = torch.empty((70, n), device="cuda")
     ops.linear(a, w, whole)
     assert bool(((whole.double() - a.double() @ w.double().T).abs() <= _bound(a, w, k)).all())
-    for m in (1, 2, 3, 4):
+    for m in (1, 2, 3, 4, 5, 7, 8):
         for first in (0, 9):
             rows = torch.empty(m * (k + 3) + 1, device="cuda")[1:].view(m, k + 3)[:, :k] if first else torch.empty((m, k), device="cuda")
             rows.copy_(a[first:first + m])

@@ -3,10 +3,10 @@
 //
 // A float32 number is the sum of three bfloat16 numbers (its 24 significant bits in runs of eight; bfloat16 ends at 2^-133, so
 // an element below 2^-109 may be cut short, by less than 2^-133), and a product of two bfloat16 numbers is exact in float32,
-// so W times the three parts of A is W times A.  What a tensor core does not do is
-// round its sums to nearest (they are cut off, which over a thousand terms adds up to 1e-6 of the result), so sums are made
-// there over 64 terms only and then added, rounded to nearest, in registers.  Against 64 bits an element is off by 0.9e-7 of
-// the norm (K = 1,024, normal terms; one fused multiply-add per term in runs of 256: 2.9e-7).
+// so W times the three parts of A is W times A.  What a tensor core does not do is round its sums to nearest (they are cut
+// off, which over a thousand terms adds up to 1e-6 of the result), so sums are made there over 64 terms only and then added,
+// rounded to nearest, in registers.  Against 64 bits an element is off by 0.9e-7 of the norm (K = 1,024, normal terms; one
+// fused multiply-add per term in runs of 256: 2.9e-7).
 //
 // One order of summation for every number of rows: a run of 64 terms gives first part + (second + third part); chunk sum =
 // its eight runs, ascending, from zero; total = chunk sums, ascending, from zero; C = total or C + total.  A block may have
@@ -21,10 +21,10 @@
 // made again by multiply-adds.
 //
 // What bounds it: few rows by the stream of W and, for small W, by the launch, a run's chain (450 to 900 cycles) and the adding
-// of the sums that blocks have left (gemm_split_few_kernel); many by a stage's products (four of 192 columns) and the cutting of
-// A.  us against the multiply-adds of gemm_simple.cu: 466 x 6,144 x 1,024 182 -> 51, 466 x 1,024 x 3,072 93 -> 34, 64 x 4,096 x
-// 4,096 120 -> 31, six rows of 6,144 x 1,024 12.2 -> 10.9, three rows of 151,936 x 1,024 125 -> 51, of 4,096 x 4,096 34 -> 11.5, of
-// 1,024 x 3,072 9.0 -> 8.6; one and two rows of a small matrix still pay for the longer chain (4,096 x 1,024 4.4 and 4.8 -> 6.3
+// of the sums that blocks have left (gemm_split_few_kernel); many by the cutting of A and the handing on of stages (466 x 6,144 x
+// 1,024: the tensor pipe is busy 16 % of the time, issue slots 40 %, memory 3 %).  us against the multiply-adds of gemm_simple.cu: 466 x 6,144 x 1,024 182 -> 51, 466 x 1,024 x 3,072 93 -> 34, 64 x 4,096 x
+// 4,096 120 -> 31, six rows of 6,144 x 1,024 12.3 -> 8.8, three rows of 151,936 x 1,024 125 -> 51, of 4,096 x 4,096 34 -> 11.4, of
+// 1,024 x 3,072 9.0 -> 8.9; one and two rows of a small matrix still pay for the longer chain (4,096 x 1,024 4.4 and 4.8 -> 6.3
 // and 6.5, 1,024 x 2,048 4.4 and 5.4 -> 5.6 and 5.7, 6,144 x 1,024 5.0 and 5.4 -> 6.7 and 6.9, 1,024 x 3,072 4.7 and 5.8 -> 6.4 and
 // 7.2).  With three products of NT columns in place of one of 3 NT 466 x 6,144 x 1,024 took 63.
 #include "sm100.cuh"
@@ -110,6 +110,8 @@ __device__ __forceinline__ void tmem_load16(unsigned taddr, float (&v)[16]) {
         v[j] = __uint_as_float(r[j]);
     }
 }
+__device__ __forceinline__ void tmem_load_cols(unsigned taddr, float (&v)[16]) { tmem_load16(taddr, v); }
+__device__ __forceinline__ void tmem_load_cols(unsigned taddr, float (&v)[32]) { tmem_load32(taddr, v); }
 __device__ __forceinline__ void load_sums(unsigned taddr, unsigned apart, float (&v)[3][16]) {
     unsigned r[3][16];
 #pragma unroll
@@ -367,24 +369,28 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const float* a, con
     }
 }
 
-// Up to four rows.  The three parts of four tokens lie beside one another in the 16 columns of one product, a warp cuts a
+// Up to eight rows.  The three parts of four or eight tokens lie beside one another in the columns of one product, a warp cuts a
 // stage's rows, and a block of 256 threads is small enough that the next launch's blocks find a place beside it and have their
-// weights on the way while this one ends.  us at 1 and 4 rows, the kernel above / this: 4,096 x 1,024 7.1 / 6.3 and 7.8 / 6.7,
-// 1,024 x 2,048 8.8 / 5.6 and 9.3 / 6.9, 6,144 x 1,024 7.8 / 6.7 and 8.6 / 7.3, 1,024 x 3,072 9.2 / 6.4 and 9.6 / 8.7,
-// 151,936 x 1,024 64.1 / 50.6 and 64.5 / 51.6.  A cluster's blocks that exchange their sums through shared memory start later:
-// 4,096 x 1,024 7.8, 1,024 x 2,048 6.8 at one row.
-constexpr int FEW = 4, FEW_THREADS = 256;
-struct Few {
-    static constexpr int STAGE = BW * BK * 2 + 16 * BK * 2, STAGES = 4, SUMS = 4, CUTTERS = 2, AHEAD = 4;
+// weights on the way while this one ends.  us at 1, 4 and 8 rows, the kernel above / this: 4,096 x 1,024 7.1 / 6.2, 7.8 / 6.7 and
+// 10.9 / 8.0, 1,024 x 2,048 8.8 / 5.5, 9.2 / 7.1 and 10.3 / 8.8, 6,144 x 1,024 7.8 / 6.8, 8.6 / 7.3 and 10.8 / 8.9, 1,024 x 3,072
+// 9.2 / 6.3, 9.7 / 9.0 and 11.8 / 11.3, 151,936 x 1,024 at 1, 4 and 6 rows 63.6 / 50.2, 64.5 / 51.1 and 65.7 / 55.8.  A cluster's
+// blocks that exchange their sums through shared memory start later: 4,096 x 1,024 7.8, 1,024 x 2,048 6.8 at one row.
+constexpr int FEW = 8, FEW_THREADS = 256;
+template <int NT> struct Few {                           // NT: tokens, 4 or 8
+    static constexpr int COLS = NT == 4 ? 16 : 32;       // their parts, and columns without a token
+    static constexpr int STAGE = BW * BK * 2 + COLS * BK * 2, STAGES = NT == 4 ? 4 : 3, SUMS = 4, CUTTERS = 2;
+    static constexpr int PIECES = NT / 4, AHEAD = 4 / PIECES;
     static constexpr int BARS = STAGES * STAGE, SMEM = BARS + 256 + 1024;
-    static constexpr unsigned TMEM_COLS = SUMS * 16;
+    static constexpr unsigned TMEM_COLS = SUMS * COLS;
 };
+static_assert(3 * (Few<4>::SMEM + 1024) <= 228 * 1024 && 3 * (Few<8>::SMEM + 1024) <= 228 * 1024, "shared memory");
 
+template <int NT>
 __global__ void __launch_bounds__(FEW_THREADS, 3)
 gemm_split_few_kernel(const __grid_constant__ CUtensorMap map_w, const float* a, const bf16* __restrict__ w, float* c, float* ws,
                       int* __restrict__ tickets, int m, int n, int k, int lda, int ldw, int ldc, int accumulate, int vec, int fine,
                       int* __restrict__ status) {
-    using T = Few;
+    using T = Few<NT>;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     unsigned long long* bars = (unsigned long long*)(smem + T::BARS);
@@ -408,8 +414,8 @@ gemm_split_few_kernel(const __grid_constant__ CUtensorMap map_w, const float* a,
         mbar_fence_init();
     }
     if (warp == 1) tmem_alloc(tmem_slot, T::TMEM_COLS);
-    for (int i = threadIdx.x; i < T::STAGES * 128; i += FEW_THREADS)         // rows without a token stay zeros
-        *reinterpret_cast<uint4*>(stage_a(i >> 7) + (i & 127) * 16) = make_uint4(0u, 0u, 0u, 0u);
+    for (int i = threadIdx.x; i < T::STAGES * T::COLS * 8; i += FEW_THREADS)         // rows without a token stay zeros
+        *reinterpret_cast<uint4*>(stage_a(i / (T::COLS * 8)) + i % (T::COLS * 8) * 16) = make_uint4(0u, 0u, 0u, 0u);
     fence_async_smem();
     pdl_launch();
     tc_fence_before();
@@ -419,7 +425,7 @@ gemm_split_few_kernel(const __grid_constant__ CUtensorMap map_w, const float* a,
     const int stages = kb_hi - kb_lo;
 
     bool ok = true;
-    float all[FEW] = {};                                 // one block a tile: the total
+    float all[NT] = {};                                 // one block a tile: the total
     if (warp == 0) {
         if (lane == 0) {                                 // the weights do not depend on the kernel before this one
             for (int it = 0; it < stages && ok; ++it) {
@@ -432,7 +438,7 @@ gemm_split_few_kernel(const __grid_constant__ CUtensorMap map_w, const float* a,
         }
     } else if (warp == 1) {
         if (lane == 0) {
-            const unsigned idesc = umma_idesc(BW, 16);
+            const unsigned idesc = umma_idesc(BW, T::COLS);
             const unsigned long long dw0 = umma_desc(stage_w(0)), da0 = umma_desc(stage_a(0));
             for (int it = 0; it < stages && ok; ++it) {
                 const int s = it % T::STAGES, buf = it % T::SUMS;
@@ -443,26 +449,31 @@ gemm_split_few_kernel(const __grid_constant__ CUtensorMap map_w, const float* a,
                 const unsigned long long step = (unsigned long long)(s * (T::STAGE >> 4));
 #pragma unroll
                 for (int kk = 0; kk < BK / 16; ++kk)
-                    umma_bf16(tmem_base + buf * 16, dw0 + step + (unsigned long long)(kk * 2), da0 + step + (unsigned long long)(kk * 2),
+                    umma_bf16(tmem_base + buf * T::COLS, dw0 + step + (unsigned long long)(kk * 2), da0 + step + (unsigned long long)(kk * 2),
                               idesc, kk != 0);
                 umma_commit(&empty[s]);
                 umma_commit(&sum_full[buf]);
             }
         }
     } else if (warp < 4) {
-        // a lane has eight neighbouring columns of a token; the two warps take the stages in turn
-        const int t = lane >> 3, piece = lane & 7, team = warp - 2;
-        const float* row = a + (size_t)t * lda;
-        float v[T::AHEAD][8];
-        auto fetch = [&](int it, float (&v)[8]) {
-            if (it >= stages || t >= m) return;
+        // a lane has eight neighbouring columns of a token, or of two; the two warps take the stages in turn
+        const int piece = lane & 7, team = warp - 2;
+        float v[T::AHEAD][T::PIECES][8];
+        auto fetch = [&](int it, float (&v)[T::PIECES][8]) {
             const int col = (kb_lo + it) * BK + piece * 8;
-            if (vec && col + 8 <= k) {
-                const float4 x = *reinterpret_cast<const float4*>(row + col), y = *reinterpret_cast<const float4*>(row + col + 4);
-                v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w; v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
-            } else {
 #pragma unroll
-                for (int e = 0; e < 8; ++e) v[e] = col + e < k ? row[col + e] : 0.0f;
+            for (int i = 0; i < T::PIECES; ++i) {
+                const int t = (lane >> 3) + 4 * i;
+                if (it >= stages || t >= m) continue;
+                const float* row = a + (size_t)t * lda;
+                if (vec && col + 8 <= k) {
+                    const float4 x = *reinterpret_cast<const float4*>(row + col), y = *reinterpret_cast<const float4*>(row + col + 4);
+                    v[i][0] = x.x; v[i][1] = x.y; v[i][2] = x.z; v[i][3] = x.w;
+                    v[i][4] = y.x; v[i][5] = y.y; v[i][6] = y.z; v[i][7] = y.w;
+                } else {
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) v[i][e] = col + e < k ? row[col + e] : 0.0f;
+                }
             }
         };
         pdl_wait();
@@ -475,12 +486,15 @@ gemm_split_few_kernel(const __grid_constant__ CUtensorMap map_w, const float* a,
                 if (it >= stages || !ok) break;
                 ok = __all_sync(0xffffffffu, mbar_wait(&empty[s], ((it / T::STAGES) & 1) ^ 1));
                 if (!ok) break;
-                if (t < m) {
+#pragma unroll
+                for (int i = 0; i < T::PIECES; ++i) {
+                    const int t = (lane >> 3) + 4 * i;
+                    if (t >= m) continue;
                     uint4 part[3];
-                    three_parts(v[d], part);
+                    three_parts(v[d][i], part);
 #pragma unroll
                     for (int q = 0; q < 3; ++q) {
-                        const int at = q * FEW + t;
+                        const int at = q * NT + t;
                         *reinterpret_cast<uint4*>(stage_a(s) + at * 128 + (piece ^ (at & 7)) * 16) = part[q];
                     }
                 }
@@ -494,25 +508,25 @@ gemm_split_few_kernel(const __grid_constant__ CUtensorMap map_w, const float* a,
         const int row = (warp & 3) * 32 + lane;
         const unsigned lane_addr = (unsigned)((warp & 3) * 32) << 16;
         pdl_wait();                                       // the scratch and the tickets belong to the chain
-        float acc[FEW];
+        float acc[NT];
         for (int kb = kb_lo, it = 0; kb < kb_hi; ++kb, ++it) {
             const int buf = it % T::SUMS;
             const bool first = kb % CHUNK == 0 || fine, last = kb % CHUNK == CHUNK - 1 || kb + 1 == stages_all || fine;
             ok = __all_sync(0xffffffffu, mbar_wait(&sum_full[buf], (it / T::SUMS) & 1));
             if (!ok) break;
             tc_fence_after();
-            float v[16];
-            tmem_load16(tmem_base + lane_addr + buf * 16, v);
+            float v[T::COLS];
+            tmem_load_cols(tmem_base + lane_addr + buf * T::COLS, v);
 #pragma unroll
-            for (int t = 0; t < FEW; ++t)
-                acc[t] = (first ? 0.0f : acc[t]) + (v[t] + (v[FEW + t] + v[2 * FEW + t]));
+            for (int t = 0; t < NT; ++t)
+                acc[t] = (first ? 0.0f : acc[t]) + (v[t] + (v[NT + t] + v[2 * NT + t]));
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&sum_empty[buf]);
             if (!last) continue;
-            float* part = ws + ((size_t)blockIdx.x * parts + kb / per) * FEW * BW + row;
+            float* part = ws + ((size_t)blockIdx.x * parts + kb / per) * NT * BW + row;
 #pragma unroll
-            for (int t = 0; t < FEW; ++t) {
+            for (int t = 0; t < NT; ++t) {
                 if (splits > 1) { if (t < m) part[t * BW] = acc[t]; }
                 else all[t] += acc[t];
             }
@@ -543,18 +557,18 @@ gemm_split_few_kernel(const __grid_constant__ CUtensorMap map_w, const float* a,
             if (v != v) again |= 1u << t;
             else store(t, v);
         };
-        const float* part = ws + (size_t)blockIdx.x * parts * FEW * BW + row;
+        const float* part = ws + (size_t)blockIdx.x * parts * NT * BW + row;
         if (n0 + row >= n) {
         } else if (splits == 1) {
 #pragma unroll
-            for (int t = 0; t < FEW; ++t)
+            for (int t = 0; t < NT; ++t)
                 if (t < m) out(t, all[t]);
         } else if (fine && m <= 2) {
-            add_parts<1, 32, true, 2>(part, FEW, parts, m, t0, out);
+            add_parts<1, 32, true, 2>(part, NT, parts, m, t0, out);
         } else if (fine) {
-            add_parts<2, 16, true, 2>(part, FEW, parts, m, t0, out);
+            add_parts<NT / 2, 64 / NT, true, 2>(part, NT, parts, m, t0, out);
         } else {
-            add_parts<2, 8, false, 2>(part, FEW, parts, m, t0, out);
+            add_parts<NT / 2, 32 / NT, false, 2>(part, NT, parts, m, t0, out);
         }
         if (again) plain_sums(again, 0, 1, a, lda, w + (size_t)(n0 + row) * ldw, k, c + n0 + row, ldc, accumulate);
     }
@@ -567,9 +581,10 @@ gemm_split_few_kernel(const __grid_constant__ CUtensorMap map_w, const float* a,
     }
 }
 
+int few_tile(int m) { return m <= 4 ? 4 : 8; }
 int token_tile(int m) { return m <= 16 ? 16 : 64; }
 
-// How a tile's K is shared.  Up to four rows: some two blocks an SM, a run or more each or, where a tile gets fewer blocks than
+// How a tile's K is shared.  Up to eight rows: some two blocks an SM, a run or more each or, where a tile gets fewer blocks than
 // twice its chunks, whole chunks, whose sums are fewer to add (us at 1 and 4 rows, runs / chunks: 1,024 x 3,072 6.4 / 7.9 and
 // 8.7 / 8.7, 4,096 x 4,096 10.8 / 11.1 and 13.6 / 11.5); four runs are not shared (256 x 256 4.4 / 3.5).  More rows: as many
 // blocks as fill the SMs once (twice where two fit on one), a chunk or more each.
@@ -579,7 +594,7 @@ Cut choose_cut(int m, int n, int k) {
     cudaGetDevice(&device);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     const bool few = m <= FEW;
-    const int nt = few ? FEW : token_tile(m), stages = (k + BK - 1) / BK, chunks = (stages + CHUNK - 1) / CHUNK;
+    const int nt = few ? few_tile(m) : token_tile(m), stages = (k + BK - 1) / BK, chunks = (stages + CHUNK - 1) / CHUNK;
     const long long tiles = (long long)((m + nt - 1) / nt) * ((n + BW - 1) / BW), room = (long long)sms * (nt <= 16 ? 2 : 1);
     const long long s = room / tiles;
     Cut cut;
@@ -608,17 +623,18 @@ int launch(const CUtensorMap& map_w, const float* a, const bf16* w, float* c, fl
     return ti_check_launch("gemm_split");
 }
 
+template <int NT>
 int launch_few(const CUtensorMap& map_w, const float* a, const bf16* w, float* c, float* ws, int* tickets, int m, int n, int k,
                int lda, int ldw, int ldc, int accumulate, const Cut& cut, int* status, cudaStream_t s) {
     static TiPerDevice configured;
     if (configured.first_use()) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_split_few_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Few::SMEM);
+        cudaError_t e = cudaFuncSetAttribute(gemm_split_few_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, Few<NT>::SMEM);
         if (e != cudaSuccess) return ti_fail("gemm_split: %s", cudaGetErrorString(e));
         configured.mark();
     }
     const int vec = (uintptr_t)a % 16 == 0 && lda % 4 == 0;
-    ti_launch_pdl(gemm_split_few_kernel, dim3((n + BW - 1) / BW, cut.splits), dim3(FEW_THREADS), Few::SMEM, s, map_w, a, w, c, ws,
-                  tickets, m, n, k, lda, ldw, ldc, accumulate, vec, cut.fine, status);
+    ti_launch_pdl(gemm_split_few_kernel<NT>, dim3((n + BW - 1) / BW, cut.splits), dim3(FEW_THREADS), Few<NT>::SMEM, s, map_w, a, w, c,
+                  ws, tickets, m, n, k, lda, ldw, ldc, accumulate, vec, cut.fine, status);
     return ti_check_launch("gemm_split");
 }
 
@@ -644,7 +660,7 @@ extern "C" int ti_gemm_split(const float* a, const void* w, float* c, int m, int
     CUtensorMap map_w;
     if (int rc = make_map_bf16(&map_w, w, n, k, ldw, BW, "gemm_split")) return rc;
     cudaStream_t s = (cudaStream_t)stream;
-    auto run = m <= FEW ? launch_few : token_tile(m) == 16 ? launch<16> : launch<64>;
+    auto run = m <= 4 ? launch_few<4> : m <= FEW ? launch_few<8> : token_tile(m) == 16 ? launch<16> : launch<64>;
     return run(map_w, a, (const bf16*)w, c, ws, tickets, m, n, k, lda, ldw, ldc, accumulate, cut, status, s);
 }
 
