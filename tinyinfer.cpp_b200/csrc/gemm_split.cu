@@ -22,11 +22,12 @@
 //
 // What bounds it: few rows by the stream of W and, for small W, by the launch, a run's chain (450 to 900 cycles) and the adding
 // of the sums that blocks have left (gemm_split_few_kernel); many by the cutting of A and the handing on of stages (466 x 6,144 x
-// 1,024: the tensor pipe is busy 16 % of the time, issue slots 40 %, memory 3 %).  us against the multiply-adds of gemm_simple.cu: 466 x 6,144 x 1,024 182 -> 51, 466 x 1,024 x 3,072 93 -> 34, 64 x 4,096 x
-// 4,096 120 -> 31, six rows of 6,144 x 1,024 12.3 -> 8.8, three rows of 151,936 x 1,024 125 -> 51, of 4,096 x 4,096 34 -> 11.4, of
-// 1,024 x 3,072 9.0 -> 8.9; one and two rows of a small matrix still pay for the longer chain (4,096 x 1,024 4.4 and 4.8 -> 6.3
-// and 6.5, 1,024 x 2,048 4.4 and 5.4 -> 5.6 and 5.7, 6,144 x 1,024 5.0 and 5.4 -> 6.7 and 6.9, 1,024 x 3,072 4.7 and 5.8 -> 6.4 and
-// 7.2).  With three products of NT columns in place of one of 3 NT 466 x 6,144 x 1,024 took 63.
+// 1,024: the tensor pipe is busy 16 % of the time, issue slots 40 %, memory 3 %).  us against the multiply-adds of
+// gemm_simple.cu: 466 x 6,144 x 1,024 182 -> 50, 466 x 1,024 x 3,072 93 -> 34, 64 x 4,096 x 4,096 120 -> 31, six rows of 6,144 x
+// 1,024 12.3 -> 8.8, three rows of 151,936 x 1,024 125 -> 51, of 4,096 x 4,096 34 -> 11.4, of 1,024 x 3,072 9.0 -> 8.9; one and two
+// rows of a small matrix still pay for the longer chain (4,096 x 1,024 4.4 and 4.8 -> 6.2 and 6.4, 1,024 x 2,048 4.4 and 5.4 -> 5.5
+// and 5.7, 6,144 x 1,024 5.0 and 5.4 -> 6.7 and 6.9, 1,024 x 3,072 4.7 and 5.8 -> 6.4 and 7.0).  With three products of NT columns
+// in place of one of 3 NT 466 x 6,144 x 1,024 took 63.
 #include "sm100.cuh"
 #include "tape.cuh"
 
@@ -82,8 +83,8 @@ __device__ __forceinline__ void three_parts(const float (&x)[8], uint4 (&parts)[
     for (int r = 0; r < 3; ++r) parts[r] = make_uint4(q[r][0], q[r][1], q[r][2], q[r][3]);
 }
 // Elements of one row of W by multiply-adds: of the tokens t, t + step, ... whose bits are set
-__device__ __noinline__ void plain_sums(unsigned tokens, int t, int step, const float* a, int lda, const bf16* w, int k, float* c, int ldc,
-                                        int accumulate) {
+__device__ __noinline__ void plain_sums(unsigned tokens, int t, int step, const float* a, int lda, const bf16* w, int k, float* c,
+                                        int ldc, int accumulate) {
     for (; tokens; t += step, tokens >>= 1) {
         if (!(tokens & 1)) continue;
         const float* row = a + (size_t)t * lda;
